@@ -856,11 +856,12 @@ __global__ void five_to_nine(i64 n, const double *__restrict__ c4, const double 
         a9[4 * n + f] = 1.0;
         return;
     }
+    // place (dI + 1) 3 + (dJ + 1), as every 9-point reader has it
     a9[4 * n + f] = diag[f];
-    a9[1 * n + f] = -c4[2 * n + f];  // (0, -1)
-    a9[7 * n + f] = -c4[3 * n + f];  // (0, +1)
-    a9[3 * n + f] = -c4[f];          // (-1, 0)
-    a9[5 * n + f] = -c4[n + f];      // (+1, 0)
+    a9[1 * n + f] = -c4[f];          // (-1, 0)
+    a9[7 * n + f] = -c4[n + f];      // (+1, 0)
+    a9[3 * n + f] = -c4[2 * n + f];  // (0, -1)
+    a9[5 * n + f] = -c4[3 * n + f];  // (0, +1)
 }
 
 // -- the small levels in one launch, in shared memory ---------------------------------------
