@@ -664,80 +664,153 @@ constexpr int kInvertThreads = 1024;
 // The coarsest operator is a 9-point stencil: ordered along its shorter side first its
 // matrix is banded with half-bandwidth b = min(nx, ny) + 1 (at most 17 for 256 nodes), and
 // its LU factors without pivoting fit shared memory (n rows of 2b + 1).  One block
-// factorises it (b^2 updates a step between two barriers), then one thread a column
-// solves L U x = e_c into the dense inverse the V-cycle applies.  A pivot smaller than
-// 1e-12 of its row (a matrix that needs pivoting, or a singular one) sets *fallback and the
-// pivoting Gauss-Jordan below computes the inverse instead.
-constexpr int kBandThreads = 512;
+// factorises it, a warp a row and a lane a column of the moving b x b window, one barrier a
+// step: the multipliers stay unscaled until the end (every thread scales its own by the
+// step's reciprocal pivot), so no step waits for a scaled column.  A second kernel then
+// solves L U x = e_c with a thread a column, the b unknowns a row still touches in registers
+// (right-looking: b independent multiply-adds a row, the factors' columns read from shared
+// memory by all lanes at once), into the dense inverse the V-cycle applies.  The work is one
+// serial chain of 3 n rows, so the time is rows times latency: with the substitutions
+// reading global memory row by row and a serial scan of every pivot row, 208 nodes
+// (b = 9, an 801 x 201 mesh) took 374 us and 153 nodes (b = 10, 1025 x 513) 284 us; now
+// 37 + 37 us and 28 + 31 us.  A pivot smaller than 1e-12 of its row (a matrix that needs pivoting, or a singular
+// one) sets *fallback and the pivoting Gauss-Jordan below computes the inverse instead.
 constexpr int kBandMax = 17;
+constexpr int kBandPad = kBandMax + 1;  // a factor column's stride, in doubles (even: 16-byte loads)
+constexpr int kSolveThreads = 32;       // columns a block of coarsest_band_solve: a warp
 
 __host__ __device__ __forceinline__ int band_half(i64 nx, i64 ny) {
     return (int)(nx < ny ? nx : ny) + 1;
 }
 
 __host__ __device__ __forceinline__ size_t band_smem(i64 nx, i64 ny) {
-    return sizeof(double) * (size_t)(nx * ny) * (size_t)(2 * band_half(nx, ny) + 1);
+    return sizeof(double) * (size_t)(nx * ny) * (size_t)(2 * band_half(nx, ny) + 2);
 }
 
-__global__ void __launch_bounds__(kBandThreads) coarsest_band_invert(
-    i64 nx, i64 ny, const double *__restrict__ a9, double *__restrict__ M,
+// The node at place o of the band's order and the other way round.
+__device__ __forceinline__ int band_order(int node, int nx, int ny) {
+    return nx < ny ? (node % ny) * nx + node / ny : node;
+}
+__device__ __forceinline__ int band_node(int o, int nx, int ny) {
+    return nx < ny ? (o % nx) * ny + o / nx : o;
+}
+
+// factors: column k of L below the diagonal at [k kBandPad + j - 1] (row k + j), column k of
+// U above it at [(n + k) kBandPad + j - 1] (row k - j), the reciprocal pivots after both.
+__global__ void __launch_bounds__(32 * kBandMax) coarsest_band_factor(
+    int nx, int ny, const double *__restrict__ a9, double *__restrict__ factors,
     int *__restrict__ fallback) {
     extern __shared__ double band[];  // row r: band[r * W + (c - r + b)], |c - r| <= b
-    const int n = (int)(nx * ny);
-    const bool across = nx < ny;  // order x fastest when x is the shorter side
+    const int n = nx * ny;
     const int b = band_half(nx, ny), W = 2 * b + 1;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    auto order_of = [&](int node) {
-        return across ? (node % (int)ny) * (int)nx + node / (int)ny : node;
-    };
-    auto node_of = [&](int o) { return across ? (o % (int)nx) * (int)ny + o / (int)nx : o; };
+    double *inv = band + n * W;  // the reciprocal pivots
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     for (int e = tid; e < n * W; e += nt) band[e] = 0.0;
     __syncthreads();
     for (int node = tid; node < n; node += nt) {
-        const int i = node / (int)ny, j = node % (int)ny, r = order_of(node);
+        const int i = node / ny, j = node % ny, r = band_order(node, nx, ny);
         for (int di = -1; di <= 1; ++di)
             for (int dj = -1; dj <= 1; ++dj) {
                 const int i2 = i + di, j2 = j + dj;
                 if (i2 < 0 || i2 >= nx || j2 < 0 || j2 >= ny) continue;
-                const int c = order_of(i2 * (int)ny + j2);
+                const int c = band_order(i2 * ny + j2, nx, ny);
                 band[r * W + (c - r + b)] = a9[(i64)((di + 1) * 3 + (dj + 1)) * n + node];
             }
     }
     __syncthreads();
+    // row k + 1 + warp, column k + 1 + lane of step k's window
+    double *mine = band + (warp + 1) * W + b + lane - warp;
+    const double *left = band + (warp + 1) * W + b - 1 - warp, *up = band + b + 1 + lane;
+    const double *diag = band + b;
     for (int k = 0; k < n; ++k) {
-        const double piv = band[k * W + b];
-        if (tid == 0) {
-            double row = 0.0;
-            for (int q = 0; q < W; ++q) row = fmax(row, fabs(band[k * W + q]));
-            if (!(fabs(piv) > 1e-12 * row)) *fallback = 1;
-        }
-        const int last = min(n - 1, k + b);
-        for (int r = k + 1 + tid; r <= last; r += nt) band[r * W + (k - r + b)] /= piv;
+        const double r = 1.0 / *diag;
+        if (tid == 0) inv[k] = r;
+        if (lane < b && k + 1 + lane < n && k + 1 + warp < n)
+            *mine = fma(-(*left * r), *up, *mine);
         __syncthreads();
-        const int m = last - k;  // rows and columns k + 1 .. last
-        for (int e = tid; e < m * m; e += nt) {
-            const int r = k + 1 + e / m, c = k + 1 + e % m;
-            band[r * W + (c - r + b)] -= band[r * W + (k - r + b)] * band[k * W + (c - k + b)];
-        }
-        __syncthreads();
+        mine += W;
+        left += W;
+        up += W;
+        diag += W;
     }
-    if (*fallback) return;
-    for (int col = tid; col < n; col += nt) {
-        const int oc = order_of(col);
-        // L y = e (unit lower, band b), y in M's column col: y_r = 0 for r < oc
-        for (int o = 0; o < oc; ++o) M[(i64)node_of(o) * n + col] = 0.0;
-        for (int o = oc; o < n; ++o) {
-            double y = o == oc ? 1.0 : 0.0;
-            for (int q = max(oc, o - b); q < o; ++q)
-                y -= band[o * W + (q - o + b)] * M[(i64)node_of(q) * n + col];
-            M[(i64)node_of(o) * n + col] = y;
+    for (int k = tid; k < n; k += nt) {
+        const double r = inv[k];
+        double row = 0.0;
+        double *L = factors + k * kBandPad, *U = factors + (n + k) * kBandPad;
+        for (int j = 1; j <= kBandPad; ++j) {
+            const bool below = j <= b && k + j < n, above = j <= b && k - j >= 0;
+            L[j - 1] = below ? band[(k + j) * W + b - j] * r : 0.0;
+            U[j - 1] = above ? band[(k - j) * W + b + j] : 0.0;
+            // row k's own entries: its multipliers and its part of U
+            if (above) row = fmax(row, fabs(band[k * W + b - j] * inv[k - j]));
+            if (below) row = fmax(row, fabs(band[k * W + b + j]));
         }
-        // U x = y, in place
-        for (int o = n - 1; o >= 0; --o) {
-            double x = M[(i64)node_of(o) * n + col];
-            for (int q = o + 1; q <= min(n - 1, o + b); ++q)
-                x -= band[o * W + (q - o + b)] * M[(i64)node_of(q) * n + col];
-            M[(i64)node_of(o) * n + col] = x / band[o * W + b];
+        const double piv = band[k * W + b];
+        row = fmax(row, fabs(piv));
+        if (!(fabs(piv) > 1e-12 * row)) *fallback = 1;
+        factors[2 * n * kBandPad + k] = r;
+    }
+}
+
+// M[., col] = (L U)^-1 e_col, a thread a column: KB at least b, even.  The window w[j] holds
+// row o + j's (forward) or o - j's (backward) remaining right-hand side.  The forward
+// results go through M; the backward pass reads its own column's values kAhead rows early.
+template <int KB>
+__global__ void __launch_bounds__(kSolveThreads) coarsest_band_solve(
+    int nx, int ny, const double *__restrict__ factors, double *__restrict__ M,
+    const int *__restrict__ fallback) {
+    extern __shared__ __align__(16) double f[];
+    if (*fallback) return;
+    const int n = nx * ny;
+    // the first KB of every factor column, then the reciprocal pivots
+    for (int e = threadIdx.x; e < 2 * n * KB; e += kSolveThreads) {
+        const int k = e / KB;
+        f[e] = factors[k * kBandPad + (e - k * KB)];
+    }
+    double *inv = f + 2 * n * KB;
+    for (int e = threadIdx.x; e < n; e += kSolveThreads) inv[e] = factors[2 * n * kBandPad + e];
+    __syncthreads();
+    const int col = blockIdx.x * kSolveThreads + threadIdx.x;
+    const int oc = col < n ? band_order(col, nx, ny) : -1;
+    double w[KB + 1];
+#pragma unroll
+    for (int j = 0; j <= KB; ++j) w[j] = 0.0;
+    for (int o = 0; o < n; ++o) {
+        const double y = o == oc ? w[0] + 1.0 : w[0];
+        const double2 *L = reinterpret_cast<const double2 *>(f + o * KB);
+#pragma unroll
+        for (int j = 0; j < KB / 2; ++j) {
+            const double2 l = L[j];
+            w[2 * j] = fma(-l.x, y, w[2 * j + 1]);
+            w[2 * j + 1] = fma(-l.y, y, w[2 * j + 2]);
+        }
+        w[KB] = 0.0;
+        if (col < n) M[(i64)band_node(o, nx, ny) * n + col] = y;
+    }
+    constexpr int kAhead = 8;
+    double ahead[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+        ahead[q] = col < n && n - 1 - q >= 0 ? M[(i64)band_node(n - 1 - q, nx, ny) * n + col] : 0.0;
+#pragma unroll
+    for (int j = 0; j <= KB; ++j) w[j] = 0.0;
+    for (int top = n - 1; top >= 0; top -= kAhead) {
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int o = top - q;
+            if (o < 0) break;
+            const double x = (w[0] + ahead[q]) * inv[o];
+            const int next = o - kAhead;
+            ahead[q] = col < n && next >= 0 ? M[(i64)band_node(next, nx, ny) * n + col] : 0.0;
+            const double2 *U = reinterpret_cast<const double2 *>(f + (n + o) * KB);
+#pragma unroll
+            for (int j = 0; j < KB / 2; ++j) {
+                const double2 u = U[j];
+                w[2 * j] = fma(-u.x, x, w[2 * j + 1]);
+                w[2 * j + 1] = fma(-u.y, x, w[2 * j + 2]);
+            }
+            w[KB] = 0.0;
+            if (col < n) M[(i64)band_node(o, nx, ny) * n + col] = x;
         }
     }
 }
@@ -1473,7 +1546,7 @@ struct bt_poisson {
     double region_value = 0.0;
     bool has_region = false;
     std::vector<bt::Level> levels;
-    bt::Buffer inv, status;
+    bt::Buffer inv, status, band;  // the coarsest inverse; the band's factors
     bool built = false;        // hierarchy matches the current diagonal
     bool transposed = false;   // the fine operator is A's transpose (bt_poisson_set_transposed)
     bt::Buffer c4_plain;       // A's own coefficients while the operator is transposed
@@ -1588,8 +1661,24 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     double *inv = p->inv.as<double>(Lc.n * Lc.n);
     const double *a9c = Lc.a9.as<double>(9 * Lc.n);
     if (band_half(Lc.nx, Lc.ny) <= kBandMax) {
-        BT_LAUNCH(p->ctx, coarsest_band_invert, 1, kBandThreads, band_smem(Lc.nx, Lc.ny), st,
-                  Lc.nx, Lc.ny, a9c, inv, status + 1);
+        const int nx = (int)Lc.nx, ny = (int)Lc.ny, n = nx * ny, b = band_half(nx, ny);
+        double *factors = p->band.as<double>((size_t)n * (2 * kBandPad + 1));
+        BT_LAUNCH(p->ctx, coarsest_band_factor, 1, 32 * b, band_smem(nx, ny), st, nx, ny, a9c,
+                  factors, status + 1);
+        const unsigned grid = blocks_for(n, kSolveThreads);
+        const auto smem = [&](int kb) { return sizeof(double) * (size_t)n * (2 * kb + 1); };
+        if (b <= 6)
+            BT_LAUNCH(p->ctx, coarsest_band_solve<6>, grid, kSolveThreads, smem(6), st, nx, ny,
+                      factors, inv, status + 1);
+        else if (b <= 10)
+            BT_LAUNCH(p->ctx, coarsest_band_solve<10>, grid, kSolveThreads, smem(10), st, nx, ny,
+                      factors, inv, status + 1);
+        else if (b <= 14)
+            BT_LAUNCH(p->ctx, coarsest_band_solve<14>, grid, kSolveThreads, smem(14), st, nx, ny,
+                      factors, inv, status + 1);
+        else
+            BT_LAUNCH(p->ctx, coarsest_band_solve<18>, grid, kSolveThreads, smem(18), st, nx, ny,
+                      factors, inv, status + 1);
         BT_LAUNCH(p->ctx, coarsest_invert, 1, kInvertThreads, 0, st, Lc.nx, Lc.ny, a9c, inv,
                   status, status + 1);
     } else {
@@ -1621,8 +1710,13 @@ void setup_tail(bt_poisson *p) {
     BT_CUDA(cudaFuncSetAttribute(smooth_staged<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big9));
     // the largest band any solver's coarsest level needs (the attribute is the kernel's,
     // shared by every solver of the process: never set it to one mesh's own size)
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_invert, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * kCoarsest * (2 * kBandMax + 1))));
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * kCoarsest * (2 * kBandMax + 2))));
+    const int solve = (int)(sizeof(double) * kCoarsest * (2 * kBandPad + 1));
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<14>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<18>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
     if (p->tail_start <= 0) return;
     const TailLayout T = tail_layout(p->levels, p->tail_start);
     p->tail_smem = T.total();
