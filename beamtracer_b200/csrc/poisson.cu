@@ -1425,18 +1425,53 @@ __device__ __forceinline__ double max_nan(double m, double v) {
     return (v > m || v != v) ? v : m;
 }
 
-// max |v| over the array (one block, deterministic; NaN if any entry is NaN)
-__global__ void max_abs(const double *__restrict__ v, i64 n, double *__restrict__ out) {
-    __shared__ double part[256];
-    double s = 0.0;
-    for (i64 f = threadIdx.x; f < n; f += blockDim.x) s = max_nan(s, fabs(v[f]));
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = blockDim.x / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) part[threadIdx.x] = max_nan(part[threadIdx.x], part[threadIdx.x + off]);
+// x += d and *out = max |d| (NaN if any entry is NaN): Newton's update and its size in one
+// pass over the vectors.  Every block leaves its maximum, the block that finishes last (a
+// ticket counter, reset by it) takes theirs; a maximum does not depend on the order.  One
+// block alone took 307 us for 525,825 nodes; the grid's 296 blocks 9 us with the
+// addition.
+__global__ void __launch_bounds__(kDotThreads) add_max(const double *__restrict__ d, i64 n,
+                                                       double *__restrict__ x,
+                                                       double *__restrict__ partial,
+                                                       unsigned *__restrict__ ticket,
+                                                       double *__restrict__ out) {
+    __shared__ double part[kDotThreads / 32];
+    __shared__ bool is_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto block_max = [&](double m) {
+        for (int off = 16; off > 0; off >>= 1)
+            m = max_nan(m, __shfl_down_sync(0xffffffffu, m, off));
+        if (lane == 0) part[warp] = m;
         __syncthreads();
+        m = part[0];
+        for (int w = 1; w < kDotThreads / 32; ++w) m = max_nan(m, part[w]);
+        __syncthreads();
+        return m;
+    };
+    double m = 0.0;
+    for (i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x; f < n;
+         f += (i64)gridDim.x * blockDim.x) {
+        const double v = d[f];
+        x[f] += v;
+        m = max_nan(m, fabs(v));
     }
-    if (threadIdx.x == 0) *out = part[0];
+    m = block_max(m);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = m;
+        __threadfence();
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    m = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+        m = max_nan(m, __ldcg(partial + b));
+    m = block_max(m);
+    if (threadIdx.x == 0) {
+        *out = m;
+        *ticket = 0u;
+    }
 }
 
 // the right-hand side: rho / eps0 + c on free nodes, 0 on fixed ones; phi's fixed values set
@@ -1956,16 +1991,22 @@ double read_scalar(bt_poisson *p, const double *dev) {
     return host[0];
 }
 
+// The finishing-block counter of the passes over vectors (zero between them).
+unsigned *dot_ticket(bt_poisson *p) {
+    unsigned *ticket = p->dot_ticket.as<unsigned>(1);
+    if (!p->ticket_ready) {
+        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), p->ctx->stream));
+        p->ticket_ready = true;
+    }
+    return ticket;
+}
+
 // One dot pass (dot_pass) over the n-vectors w and V's rows q < m; out gets its sums.
 template <int MODE>
 void dot_launch(bt_poisson *p, const double *V, const double *h, double *w, int m, double *out) {
     double *partial = p->dot_partial.as<double>((size_t)kDotBlocks * kDotMax);
-    unsigned *ticket = p->dot_ticket.as<unsigned>(1);
+    unsigned *ticket = dot_ticket(p);
     cudaStream_t st = p->ctx->stream;
-    if (!p->ticket_ready) {
-        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
-        p->ticket_ready = true;
-    }
     BT_REQUIRE(m >= 1 && m <= kDotMax, "poisson: a dot pass takes 1 to 32 vectors");
 #define BT_DOT(MQ)                                                                              \
     BT_LAUNCH(p->ctx, (dot_pass<MQ, MODE>), kDotBlocks, kDotThreads, 0, st, V, h, w, p->n, m,  \
@@ -2240,8 +2281,9 @@ extern "C" int bt_poisson_solve(bt_poisson *p, double *phi, const double *rho, d
                 double left = 0.0;
                 total_cycles += bt::gmres(p, r0, d, tol * (fnorm > 0.0 ? fnorm : 1.0),
                                           max_cycles, &left);
-                BT_LAUNCH(p->ctx, bt::add_into, bt::blocks_for(n, 256), 256, 0, st, d, n, phi);
-                BT_LAUNCH(p->ctx, bt::max_abs, 1, 256, 0, st, d, n, scal + 8);
+                BT_LAUNCH(p->ctx, bt::add_max, bt::kDotBlocks, bt::kDotThreads, 0, st, d, n, phi,
+                          p->dot_partial.as<double>((size_t)bt::kDotBlocks * bt::kDotMax),
+                          bt::dot_ticket(p), scal + 8);
                 BT_CHECK_LAUNCH();
                 const double change = bt::read_scalar(p, scal + 8);
                 if (!std::isfinite(change))
