@@ -29,7 +29,7 @@ constexpr double kEps0 = 8.8541878188e-12;  // scipy.constants.epsilon_0 (CODATA
 struct Axis {
     i64 n = 0, nc = 0;
     bool coarsened = false;
-    Buffer lo, w, cidx;  // per fine node: coarse index and its weight; per coarse: fine index
+    Buffer lo, w;        // per fine node: coarse index and its weight
     Buffer r0, rw;       // per coarse node: its first fine node and kRestrict weights from there
 };
 
@@ -48,13 +48,6 @@ struct Level {
     double *cur = nullptr;  // which of x, x2 holds the level's x while a V-cycle is recorded
     Axis ax, ay;            // the map to the next coarser level
 };
-
-__device__ __forceinline__ double pw(const int32_t *lo, const double *w, i64 k, i64 I) {
-    const i64 l = lo[k];
-    if (l == I) return w[k];
-    if (l + 1 == I) return 1.0 - w[k];
-    return 0.0;
-}
 
 // -- the fine operator (mirrors oracle/poisson.py:coefficients) ---------------------------
 
@@ -214,74 +207,104 @@ struct Fine {
     const uint8_t *active;
     const int32_t *lox, *loy;
     const double *wx, *wy;
-    const int32_t *cix, *ciy;  // fine index of each coarse node
     const int32_t *rx0, *ry0;  // restriction: first fine node of each coarse node
     const double *rxw, *ryw;   //   and kRestrict weights from it (zero: not a neighbour)
     i64 ncx, ncy;
 };
 
-__device__ __forceinline__ double fine_coef(const Fine &F, i64 f, int di, int dj) {
-    if (F.a9) return F.a9[(i64)((di + 1) * 3 + (dj + 1)) * (F.nx * F.ny) + f];
-    const i64 n = F.nx * F.ny;
-    if (di == 0 && dj == 0) return F.diag[f];
-    if (di == -1 && dj == 0) return -F.c4[f];
-    if (di == 1 && dj == 0) return -F.c4[n + f];
-    if (di == 0 && dj == -1) return -F.c4[2 * n + f];
-    if (di == 0 && dj == 1) return -F.c4[3 * n + f];
-    return 0.0;
+// The weights of the coarse nodes I - 1, I, I + 1 at the kRestrict + 2 fine nodes from
+// first - 1 on (zero off the axis).
+__device__ __forceinline__ void axis_weights(const int32_t *__restrict__ lo,
+                                             const double *__restrict__ w, i64 n, int first, int I,
+                                             double (&p)[kRestrict + 2][3]) {
+#pragma unroll
+    for (int a = 0; a < kRestrict + 2; ++a) {
+        const int k = first - 1 + a;
+        const bool in = k >= 0 && k < (int)n;
+        const int l = in ? lo[k] : -4;
+        const double v = in ? w[k] : 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            p[a][d] = l == I + d - 1 ? v : (l + 1 == I + d - 1 ? 1.0 - v : 0.0);
+    }
 }
 
-__global__ void galerkin(Fine F, double *__restrict__ a9c, uint8_t *__restrict__ active_c) {
-    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    const i64 nc = F.ncx * F.ncy;
+// A thread a coarse node.  Its row is a product over the axes: with the weights of both
+// axes in registers, each fine row's three neighbour rows are contracted along y, then
+// along x -- some 54 multiply-adds a fine node and no branch but the fine node's own, and
+// the loads of a fine row of nodes are all in flight together.  Testing every pair of fine
+// neighbour and coarse node instead (a branch and an index a term) took 60 us a level of a
+// 1025 x 513 mesh, its levels of a few thousand nodes as long as the finest; so the finest
+// takes 22 us and the others 14.
+constexpr int kGalerkinThreads = 64;
+
+template <bool NINE>
+__global__ void __launch_bounds__(kGalerkinThreads)
+    galerkin(Fine F, double *__restrict__ a9c, uint8_t *__restrict__ active_c) {
+    const i64 nc = F.ncx * F.ncy, n = F.nx * F.ny;
+    const int t = blockIdx.x * kGalerkinThreads + threadIdx.x;
     if (t >= nc) return;
-    const i64 I = t / F.ncy, J = t - I * F.ncy;
-    double acc[9];
+    const int ny = (int)F.ny, ncy = (int)F.ncy;
+    const int I = t / ncy, J = t - I * ncy;
+    const int k0 = F.rx0[I], l0 = F.ry0[J];
+    double px[kRestrict + 2][3], py[kRestrict + 2][3], acc[3][3];
+    axis_weights(F.lox, F.wx, F.nx, k0, I, px);
+    axis_weights(F.loy, F.wy, F.ny, l0, J, py);
 #pragma unroll
-    for (int q = 0; q < 9; ++q) acc[q] = 0.0;
-    const i64 k0 = I > 0 ? F.cix[I - 1] : 0, k1 = I < F.ncx - 1 ? F.cix[I + 1] : F.nx - 1;
-    const i64 l0 = J > 0 ? F.ciy[J - 1] : 0, l1 = J < F.ncy - 1 ? F.ciy[J + 1] : F.ny - 1;
-    const int span = F.a9 ? 1 : 0;  // the 9-point fine stencil reaches diagonals
-    for (i64 k = k0; k <= k1; ++k) {
-        const double pk = pw(F.lox, F.wx, k, I);
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) acc[d][e] = 0.0;
+    // 1 where a fine node is in the mesh and free
+    auto free_at = [&](int k, int l) {
+        return k >= 0 && k < (int)F.nx && l >= 0 && l < ny && F.active[(i64)k * ny + l] ? 1.0 : 0.0;
+    };
+#pragma unroll
+    for (int a = 0; a < kRestrict; ++a) {
+        const double pk = px[a + 1][1];
         if (pk == 0.0) continue;
-        for (i64 l = l0; l <= l1; ++l) {
-            const double pl = pw(F.loy, F.wy, l, J);
-            if (pl == 0.0) continue;
-            const i64 f = k * F.ny + l;
-            if (!F.active[f]) continue;
+        const int k = k0 + a;
+#pragma unroll
+        for (int c = 0; c < kRestrict; ++c) {
+            const double pl = py[c + 1][1];
+            const int l = l0 + c;
+            if (pl == 0.0 || free_at(k, l) == 0.0) continue;
+            const i64 f = (i64)k * ny + l;
             const double wgt = pk * pl * (F.weight ? F.weight[f] : 1.0);
-            for (int di = -1; di <= 1; ++di) {
-                const i64 k2 = k + di;
-                if (k2 < 0 || k2 >= F.nx) continue;
-                for (int dj = -1; dj <= 1; ++dj) {
-                    if (!span && di != 0 && dj != 0) continue;
-                    const i64 l2 = l + dj;
-                    if (l2 < 0 || l2 >= F.ny) continue;
-                    const i64 f2 = k2 * F.ny + l2;
-                    if (!F.active[f2]) continue;
-                    const double a = fine_coef(F, f, di, dj);
-                    if (a == 0.0) continue;
-                    const i64 ix = F.lox[k2], iy = F.loy[l2];
-                    const double wx = F.wx[k2], wy = F.wy[l2];
-                    for (int sx = 0; sx < 2; ++sx) {
-                        const double px = sx ? 1.0 - wx : wx;
-                        const i64 I2 = ix + sx;
-                        if (px == 0.0 || I2 - I < -1 || I2 - I > 1) continue;
-                        for (int sy = 0; sy < 2; ++sy) {
-                            const double py = sy ? 1.0 - wy : wy;
-                            const i64 J2 = iy + sy;
-                            if (py == 0.0 || J2 - J < -1 || J2 - J > 1) continue;
-                            acc[(I2 - I + 1) * 3 + (J2 - J + 1)] += wgt * a * px * py;
-                        }
-                    }
-                }
+            double m[3][3];  // the fine row, held neighbours left out
+            if (NINE) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int e = 0; e < 3; ++e)
+                        m[d][e] = F.a9[(i64)(3 * d + e) * n + f] * free_at(k + d - 1, l + e - 1);
+            } else {
+                m[0][0] = m[0][2] = m[2][0] = m[2][2] = 0.0;
+                m[1][1] = F.diag[f];
+                m[0][1] = -F.c4[f] * free_at(k - 1, l);
+                m[2][1] = -F.c4[n + f] * free_at(k + 1, l);
+                m[1][0] = -F.c4[2 * n + f] * free_at(k, l - 1);
+                m[1][2] = -F.c4[3 * n + f] * free_at(k, l + 1);
+            }
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                double row[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    row[d] = fma(m[d][0], py[c][e], fma(m[d][1], py[c + 1][e], m[d][2] * py[c + 2][e]));
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    acc[d][e] = fma(wgt, fma(px[a][d], row[0],
+                                             fma(px[a + 1][d], row[1], px[a + 2][d] * row[2])),
+                                    acc[d][e]);
             }
         }
     }
-    const bool on = acc[4] != 0.0;
+    const bool on = acc[1][1] != 0.0;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) a9c[(i64)q * nc + t] = on ? acc[q] : (q == 4 ? 1.0 : 0.0);
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int e = 0; e < 3; ++e)
+            a9c[(i64)(3 * d + e) * nc + t] = on ? acc[d][e] : (d == 1 && e == 1 ? 1.0 : 0.0);
     active_c[t] = on ? 1 : 0;
 }
 
@@ -1562,8 +1585,6 @@ void build_axis(Axis &A, i64 n) {
                cudaMemcpyHostToDevice);
     cudaMemcpy(A.lo.as<int32_t>(n), lo.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice);
     cudaMemcpy(A.w.as<double>(n), w.data(), n * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(A.cidx.as<int32_t>(A.nc), cidx.data(), A.nc * sizeof(int32_t),
-               cudaMemcpyHostToDevice);
 }
 
 }  // namespace
@@ -1619,7 +1640,7 @@ struct bt_poisson {
 namespace bt {
 namespace {
 
-void refresh_tail_image(bt_poisson *p);
+void refresh_tail_image(bt_poisson *p, bool tables = false);
 
 Fine fine_of(Level &L, Level &C, bool first) {
     Fine F{};
@@ -1641,8 +1662,6 @@ Fine fine_of(Level &L, Level &C, bool first) {
     F.loy = L.ay.lo.as<int32_t>(L.ny);
     F.wx = L.ax.w.as<double>(L.nx);
     F.wy = L.ay.w.as<double>(L.ny);
-    F.cix = L.ax.cidx.as<int32_t>(L.ax.nc);
-    F.ciy = L.ay.cidx.as<int32_t>(L.ay.nc);
     F.rx0 = L.ax.r0.as<int32_t>(L.ax.nc);
     F.ry0 = L.ay.r0.as<int32_t>(L.ay.nc);
     F.rxw = L.ax.rw.as<double>(kRestrict * L.ax.nc);
@@ -1683,8 +1702,13 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     for (size_t l = 0; l + 1 < p->levels.size(); ++l) {
         Level &L = p->levels[l], &C = p->levels[l + 1];
         Fine F = fine_of(L, C, l == 0);
-        BT_LAUNCH(p->ctx, galerkin, blocks_for(C.n, 128), 128, 0, st, F, C.a9.as<double>(9 * C.n),
-                                                        C.active.as<uint8_t>(C.n));
+        const unsigned grid = blocks_for(C.n, kGalerkinThreads);
+        if (F.a9)
+            BT_LAUNCH(p->ctx, galerkin<true>, grid, kGalerkinThreads, 0, st, F,
+                      C.a9.as<double>(9 * C.n), C.active.as<uint8_t>(C.n));
+        else
+            BT_LAUNCH(p->ctx, galerkin<false>, grid, kGalerkinThreads, 0, st, F,
+                      C.a9.as<double>(9 * C.n), C.active.as<uint8_t>(C.n));
     }
     Level &Lc = p->levels.back();
     if (p->levels.size() == 1)
@@ -1780,12 +1804,12 @@ void setup_tail(bt_poisson *p) {
     BT_CUDA(cudaMemcpy(p->tail_plans.as<TailPlan>(T.plan.size()), T.plan.data(),
                        sizeof(TailPlan) * T.plan.size(), cudaMemcpyHostToDevice));
     p->tail_image.get(T.image());
-    refresh_tail_image(p);
+    refresh_tail_image(p, true);
 }
 
-// Copy the tail levels' coefficients, transfer tables and active flags into the tail's
-// static image (after the hierarchy's coefficients change).
-void refresh_tail_image(bt_poisson *p) {
+// Copy the tail levels' coefficients and active flags into the tail's static image (after
+// the hierarchy's coefficients change), with the transfer tables when it is laid out.
+void refresh_tail_image(bt_poisson *p, bool tables) {
     if (p->tail_start <= 0) return;
     cudaStream_t st = p->ctx->stream;
     const TailLayout T = tail_layout(p->levels, p->tail_start);
@@ -1804,6 +1828,7 @@ void refresh_tail_image(bt_poisson *p) {
         if (l + 1 == levels) continue;
         const Fine F = fine_of(L, p->levels[l + 1], false);
         copy(d + P.a9, L.a9.as<double>(9 * L.n), sizeof(double) * 9 * L.n);
+        if (!tables) continue;
         copy(d + P.wx, F.wx, sizeof(double) * P.nx);
         copy(d + P.wy, F.wy, sizeof(double) * P.ny);
         copy(d + P.rxw, F.rxw, sizeof(double) * kRestrict * P.ncx);
