@@ -219,6 +219,102 @@ __device__ __forceinline__ double div_known(double a, double b, double rb) {
     return fma(r, rb, q);
 }
 
+// -- square roots and quotients without a branch -----------------------------------------------
+//
+// The compiler's IEEE division and square root each end in a branch to a rarely taken
+// routine, so no two of them, nor the loads and sums between, are scheduled into one another:
+// a chain of a dozen per trajectory step ran behind one another with one warp a scheduler.
+// Num<true> gives the same bits as straight-line code, and `odd()` afterwards is true where it
+// might not (an operand outside 2^-400 .. 2^400 other than zero, a divisor whose significand
+// is all ones); the caller then computes everything again with Num<false>, the IEEE
+// operations.  The operands' exponents are gathered in two integer extremes, tested once.
+//
+// The methods are Markstein's (IBM J. Res. Develop. 34(1), 1990): a Newton step from the
+// hardware's approximations (20 bits) of third order, then corrections by exact remainders.
+// - root: y = 1 / sqrt(s) to within 2^-53 relative, g = s y within 2 ulps, and
+//   g + (s - g^2) y / 2 is sqrt(s) to within 2^-50 ulps before its rounding.  A root closer
+//   than that to a rounding boundary M + 1/2 (scaled to 53 bits) has s = M^2 + M + c with
+//   |c| < 64: two significands for each even c, all of them tested.
+// - inverse: within an ulp of 1 / b, one more step by its remainder rounds to 1 / b unless
+//   b's significand is all ones (Markstein's theorem 8).
+// - over: with rb the rounded 1 / b, a quotient within an ulp of a / b plus its remainder
+//   times rb rounds to a / b (theorem 7); a rb is within 1.5 ulps, so two corrections.
+// A zero dividend gives +0, and root(0) is +0.
+template <bool FAST>
+struct Num {
+    static constexpr bool fast = FAST;
+    static constexpr unsigned kLow = (1023u - 400u) << 20, kHigh = (1023u + 400u) << 20;
+    bool flag = false;
+    unsigned low = 0xffffffffu, high = 0u;  // the operands' smallest and largest high words
+
+    __device__ __forceinline__ bool odd() const { return flag || low < kLow - 1u || high > kHigh; }
+    // an operand that may be zero (high word 0 wraps past every exponent) but not tiny
+    __device__ __forceinline__ void not_tiny(double v) {
+        if (FAST) low = min(low, (unsigned)(__double2hiint(v) & 0x7fffffff) - 1u);
+    }
+    // nor huge, infinite or not a number
+    __device__ __forceinline__ void in_range(double v) {
+        if (!FAST) return;
+        const unsigned t = (unsigned)(__double2hiint(v) & 0x7fffffff);
+        low = min(low, t - 1u);
+        high = max(high, t);
+    }
+
+    // sqrt(s), s >= 0 or NaN, and an approximation y of its reciprocal for `inverse` (no
+    // number for s = 0)
+    __device__ __forceinline__ double root(double s, double &y) {
+        if (!FAST) {
+            y = 0.0;
+            return sqrt(s);
+        }
+        in_range(s);
+        double y0;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(s));
+        // e = 1 - s y0^2 to second order: y0 (1 + e / 2 + 3 e^2 / 8)
+        const double e = fma(-(s * y0), y0, 1.0);
+        y = fma(fma(0.375, e, 0.5), e * y0, y0);
+        const double g = s * y;
+        const double r = fma(fma(-g, g, s), 0.5 * y, g);
+        return __double2hiint(s) == 0 ? 0.0 : r;
+    }
+    __device__ __forceinline__ double root(double s) {
+        double y;
+        return root(s, y);
+    }
+    // the rounded 1 / b from an approximation y within 2 ulps, b a root or in range (0 with
+    // IEEE operations, where `over` divides)
+    __device__ __forceinline__ double inverse(double b, double y) {
+        if (!FAST) return 0.0;
+        flag |= __double2loint(b) == -1;
+        y = fma(fma(-b, y, 1.0), y, y);
+        return fma(fma(-b, y, 1.0), y, y);
+    }
+    __device__ __forceinline__ double inverse(double b) {
+        if (!FAST) return 0.0;
+        in_range(b);
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+        // e = 1 - b y to third order: y (1 + e + e^2)
+        const double e = fma(-b, y, 1.0);
+        return inverse(b, fma(fma(e, e, e), y, y));
+    }
+    // a / b, rb the inverse of b.  A huge or infinite a or one that is no number gives such a
+    // quotient: the caller has its results' range tested (in_range).
+    __device__ __forceinline__ double over(double a, double b, double rb) {
+        if (!FAST) return a / b;
+        not_tiny(a);
+        double q = a * rb;
+        q = fma(fma(-q, b, a), rb, q);
+        return fma(fma(-q, b, a), rb, q);
+    }
+    __device__ __forceinline__ double div(double a, double b) { return over(a, b, inverse(b)); }
+    // a / b for a divisor known in advance (div_known; FAST: rb is not 0)
+    __device__ __forceinline__ double known(double a, double b, double rb) {
+        if (!FAST) return div_known(a, b, rb);
+        return over(a, b, rb);
+    }
+};
+
 // The Lorentz factor sqrt(1 + |u|^2 / c^2) of a proper velocity u (1 for inv_c2 = 0).
 __device__ __forceinline__ double lorentz(double u0, double u1, double u2, double inv_c2) {
     return sqrt(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2);

@@ -37,26 +37,18 @@ struct Trace {
     Shapes shapes;
 };
 
-__device__ __forceinline__ i64 node_cell(double x, const double *__restrict__ nodes, i64 n) {
-    i64 lo = 0, hi = n - 1;
-    if (x >= nodes[n - 1]) {
-        lo = n - 2;
-    } else if (x > nodes[0]) {
-        while (hi - lo > 1) {
-            const i64 mid = (lo + hi) / 2;
-            if (nodes[mid] <= x)
-                lo = mid;
-            else
-                hi = mid;
-        }
-    }
-    return lo;
-}
-
-__device__ __forceinline__ double uniform_x(double x, const double *__restrict__ nodes, i64 n,
-                                            double x0, double h) {
-    const i64 c = node_cell(x, nodes, n);
-    return x0 + h * ((double)c + (x - nodes[c]) / (nodes[c + 1] - nodes[c]));
+// The cell of x on a graded axis: the last node at or before x, within the axis (0 left of
+// it or for a NaN).  `hint` is where the search starts: a trajectory's points lie in its last
+// cell or beside it, so the walk reads two or three nodes where a bisection read eleven
+// of 1025, each waiting for the one before.
+__device__ __forceinline__ int node_cell(double x, const double *__restrict__ nodes, int n,
+                                         int hint) {
+    if (!(x > nodes[0])) return 0;
+    if (x >= nodes[n - 1]) return n - 2;
+    int c = hint;
+    while (x < nodes[c]) --c;
+    while (x >= nodes[c + 1]) ++c;
+    return c;
 }
 
 __device__ __forceinline__ i64 finest_patch(const bt_trace_args &a, i64 P, double px, double py) {
@@ -89,51 +81,67 @@ __device__ __forceinline__ PatchGeom patch_geom(const bt_trace_args &a, i64 pp) 
 // follow them give what the 64-bit conversions give.
 __device__ __forceinline__ int clamp_index(int i, int lo, int hi) { return min(max(i, lo), hi); }
 
-// E at the point (sx, sy) in cells of patch g from its origin (the finest patch holding the
-// point; trace_trajectories_2d_pyccel.py:212-269).
-__device__ __forceinline__ void edge_field_cells(const bt_trace_args &a, const PatchGeom &g,
-                                                 double sx, double sy, double &ex, double &ey) {
-    const int pnx = (int)g.pnx, pny = (int)g.pny;
-    double s = sx + 0.5;
-    int i = clamp_index(__double2int_rd(s), 0, pnx - 1);
-    int j = clamp_index(__double2int_rd(sy), 0, pny - 2);
-    double u = s - (double)i;
-    double w = sy - (double)j;
-    const double *fx = a.fxs + g.ofx + (i64)i * pny + j;
-    double f00 = __ldg(fx), f01 = __ldg(fx + 1), f10 = __ldg(fx + pny), f11 = __ldg(fx + pny + 1);
-    double low = f00 + w * (f01 - f00);
-    double high = f10 + w * (f11 - f10);
-    ex = low + u * (high - low);
-    s = sy + 0.5;
-    i = clamp_index(__double2int_rd(sx), 0, pnx - 2);
-    j = clamp_index(__double2int_rd(s), 0, pny - 1);
-    u = sx - (double)i;
-    w = s - (double)j;
-    const double *fy = a.fys + g.ofy + (i64)i * (pny + 1) + j;
-    f00 = __ldg(fy);
-    f01 = __ldg(fy + 1);
-    f10 = __ldg(fy + pny + 1);
-    f11 = __ldg(fy + pny + 2);
-    low = f00 + w * (f01 - f00);
-    high = f10 + w * (f11 - f10);
-    ey = low + u * (high - low);
+// The cell i of s among cells 0 .. last and the weight w in it.
+__device__ __forceinline__ int cell_weight(double s, int last, double &w) {
+    const int i = clamp_index(__double2int_rd(s), 0, last);
+    w = s - (double)i;
+    return i;
 }
 
-// E at (lq, qy), the uniform x and the mesh y, on patch g.
-__device__ __forceinline__ void edge_field(const bt_trace_args &a, const PatchGeom &g, double lq,
-                                           double qy, double &ex, double &ey) {
-    edge_field_cells(a, g, div_known(lq - g.pox, g.phh, g.rphh),
-                     div_known(qy - g.poy, g.phh, g.rphh), ex, ey);
+__device__ __forceinline__ double bilinear(const double *__restrict__ f, int stride, double u,
+                                           double w) {
+    const double f00 = __ldg(f), f01 = __ldg(f + 1);
+    const double f10 = __ldg(f + stride), f11 = __ldg(f + stride + 1);
+    const double low = f00 + w * (f01 - f00);
+    const double high = f10 + w * (f11 - f10);
+    return low + u * (high - low);
+}
+
+// E at the point (sx, sy) in cells of patch g from its origin (the finest patch holding the
+// point; trace_trajectories_2d_pyccel.py:212-269).  The straight-line form takes the cell of
+// s + 1/2 from the cell c of s -- it is c, or c + 1 where s + 1/2, as rounded, has reached
+// it -- without a second pair of conversions, and calls a point whose cell is clamped odd.
+template <class N>
+__device__ __forceinline__ void edge_field_cells(N &num, const bt_trace_args &a,
+                                                 const PatchGeom &g, double sx, double sy,
+                                                 double &ex, double &ey) {
+    const int pnx = (int)g.pnx, pny = (int)g.pny;
+    const double hx = sx + 0.5, hy = sy + 0.5;
+    int ix, jx, iy, jy;
+    double ux, wx, uy, wy;
+    if (N::fast) {
+        const int i = __double2int_rd(sx), j = __double2int_rd(sy);
+        const double fi = (double)i, fj = (double)j;
+        const bool up_i = hx >= fi + 1.0, up_j = hy >= fj + 1.0;
+        ix = clamp_index(i + (up_i ? 1 : 0), 0, pnx - 1);
+        jx = clamp_index(j, 0, pny - 2);
+        iy = clamp_index(i, 0, pnx - 2);
+        jy = clamp_index(j + (up_j ? 1 : 0), 0, pny - 1);
+        num.flag |= iy != i || jx != j;
+        uy = sx - fi;
+        wx = sy - fj;
+        ux = hx - (up_i ? fi + 1.0 : fi);
+        wy = hy - (up_j ? fj + 1.0 : fj);
+    } else {
+        ix = cell_weight(hx, pnx - 1, ux);
+        jx = cell_weight(sy, pny - 2, wx);
+        iy = cell_weight(sx, pnx - 2, uy);
+        jy = cell_weight(hy, pny - 1, wy);
+    }
+    ex = bilinear(a.fxs + g.ofx + (i64)ix * pny + jx, pny, ux, wx);
+    ey = bilinear(a.fys + g.ofy + (i64)iy * (pny + 1) + jy, pny + 1, uy, wy);
 }
 
 // (B_z, B_r) of an on-axis profile at axial position z and radius r (fields.py:250-279,
-// term by term: the derivatives interpolated between samples, then the series in r).
-__device__ __forceinline__ void axial_field(const bt_magnetic &m, double z, double r,
-                                            double &bz_out, double &br_out) {
+// term by term: the derivatives interpolated between samples, then the series in r); rhz
+// the reciprocal of the samples' spacing.
+template <class N>
+__device__ __forceinline__ void axial_field(N &num, const bt_magnetic &m, double rhz, double z,
+                                            double r, double &bz_out, double &br_out) {
     const i64 n = m.n;
     const int K = m.order + 1;
-    const double s = (z - m.z0) / m.hz;
-    i64 i = (i64)floor(s);
+    const double s = num.known(z - m.z0, m.hz, rhz);
+    i64 i = (i64)__double2int_rd(s);
     if (i < 3)
         i = 3;
     else if (i > n - 5)
@@ -170,17 +178,18 @@ __device__ __forceinline__ void axial_field(const bt_magnetic &m, double z, doub
 
 // The Cartesian B at (q0, q1, q2): mode 1 on a cylindrical mesh ((cy, cz) the radial unit
 // vector, r the radius), mode 2 a planar mesh with the solenoid axis on y = axis_y.
-__device__ __forceinline__ void magnetic_at(const bt_magnetic &m, double q0, double q1, double r,
-                                            double cy, double cz, double *b) {
+template <class N>
+__device__ __forceinline__ void magnetic_at(N &num, const bt_magnetic &m, double rhz, double q0,
+                                            double q1, double r, double cy, double cz, double *b) {
     double bz, br;
     if (m.mode == 1) {
-        axial_field(m, q0, r, bz, br);
+        axial_field(num, m, rhz, q0, r, bz, br);
         b[0] = bz;
         b[1] = br * cy;
         b[2] = br * cz;
     } else {
         const double yr = q1 - m.axis_y;
-        axial_field(m, q0, fabs(yr), bz, br);
+        axial_field(num, m, rhz, q0, fabs(yr), bz, br);
         b[0] = bz;
         b[1] = yr < 0.0 ? -br : br;
         b[2] = 0.0;
@@ -190,12 +199,13 @@ __device__ __forceinline__ void magnetic_at(const bt_magnetic &m, double q0, dou
 // v <- Boris's kick over tau in the fields e, b (non-relativistic; tracer.py:605-621):
 // v- = v + (tau/2) q/m E, t = (tau/2) q/m B, v+ = v- + (v- + v- x t) x 2t / (1 + t^2),
 // then + (tau/2) q/m E; the operations in the oracle's order.
-__device__ __forceinline__ void kick(double *v, const double *e, const double *b, double tau,
-                                     double qm) {
+template <class N>
+__device__ __forceinline__ void kick(N &num, double *v, const double *e, const double *b,
+                                     double tau, double qm) {
     const double f = 0.5 * tau * qm;
     const double m0 = v[0] + f * e[0], m1 = v[1] + f * e[1], m2 = v[2] + f * e[2];
     const double t0 = f * b[0], t1 = f * b[1], t2 = f * b[2];
-    const double d = 2.0 / (1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
+    const double d = num.div(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
     const double s0 = d * t0, s1 = d * t1, s2 = d * t2;
     const double p0 = m0 + (m1 * t2 - m2 * t1);
     const double p1 = m1 + (m2 * t0 - m0 * t2);
@@ -210,9 +220,372 @@ __device__ __forceinline__ void kick(double *v, const double *e, const double *b
 
 // 1 / gamma of a proper velocity: exactly 1 without relativity (inv_c2 = 0), which the
 // non-general kernels fold away.
-template <bool GENERAL>
-__device__ __forceinline__ double inv_gamma(double u0, double u1, double u2, double inv_c2) {
-    return GENERAL ? 1.0 / lorentz(u0, u1, u2, inv_c2) : 1.0;
+template <bool GENERAL, class N>
+__device__ __forceinline__ double inv_gamma(N &num, double u0, double u1, double u2,
+                                            double inv_c2) {
+    return GENERAL ? num.div(1.0, num.root(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2)) : 1.0;
+}
+
+// What a trajectory's steps share: its mesh (its candidate's in a batch), its base patch,
+// the spacings' reciprocals, its charge over mass and its current.
+struct Geo {
+    double ox, oy, h, rh, rhz;
+    PatchGeom base;
+    double qm, dq, fraction, inv_c2;
+    int P, n_x_nodes;
+    bool graded;
+    bool same;  // one patch, which is the mesh: cell coordinates serve both
+    bool fast;  // the straight-line arithmetic may be tried (every reciprocal is one)
+};
+
+// A point on the mesh: its radius or distance from the axis (the mesh's second coordinate)
+// with the root's reciprocal, its uniform x, its cell on a graded axis, its cell coordinates.
+struct Place {
+    double r, y, lx, sx, sy;
+    int cell;
+};
+
+// The state of a trajectory between steps: position, velocity, place, and the pace it sets --
+// the local spacing, the speed's square and the spacing over the speed (-1 at rest) -- with
+// Boris the fields at the last step's end (q/m E, or E and B).
+struct State {
+    double x[3], v[3];
+    Place at;
+    double gv, hloc, speed2, dt0;
+    double e[3], b[3];
+    bool have;
+};
+
+// A step's deposit: the shares of the four nodes of its midpoint's cell.
+struct Share {
+    uint32_t key;
+    double c00, c01, c10, c11;
+};
+
+// x on the uniform axis (its own value on a mesh that is not graded), its graded cell found
+// from `hint` on.
+template <bool GENERAL, class N>
+__device__ __forceinline__ double uniform_x(N &num, const bt_trace_args &a, const Geo &G, double x,
+                                            int hint, int &cell) {
+    cell = hint;
+    if (!GENERAL || !G.graded) return x;
+    const double *nodes = a.x_nodes;
+    const int c = cell = node_cell(x, nodes, G.n_x_nodes, hint);
+    return G.ox + G.h * ((double)c + num.div(x - nodes[c], nodes[c + 1] - nodes[c]));
+}
+
+template <int CYL, bool GENERAL, class N>
+__device__ __forceinline__ void locate(N &num, const bt_trace_args &a, const Geo &G,
+                                       const double *q, int hint, Place &W) {
+    W.y = 0.0;
+    W.r = q[1];
+    if (CYL == 1)
+        W.r = num.root(q[1] * q[1] + q[2] * q[2], W.y);
+    else if (CYL == 2)
+        W.r = G.oy + fabs(q[1] - G.oy);
+    W.lx = uniform_x<GENERAL>(num, a, G, q[0], hint, W.cell);
+    W.sx = num.known(W.lx - G.ox, G.h, G.rh);
+    W.sy = num.known(W.r - G.oy, G.h, G.rh);
+}
+
+// The pace of a state at its place.
+template <bool GENERAL, bool MAG, class N>
+__device__ __forceinline__ void set_pace(N &num, const bt_trace_args &a, const Geo &G, State &S) {
+    double hloc = G.h;
+    if (GENERAL) {
+        for (int qq = 0; qq < G.P - 1; ++qq) {
+            const double *pr = a.patch_real + qq * 7;
+            if (S.at.lx >= __ldg(pr + 3) && S.at.lx <= __ldg(pr + 5) && S.at.r >= __ldg(pr + 4) &&
+                S.at.r <= __ldg(pr + 6)) {
+                hloc = __ldg(pr + 2);
+                break;
+            }
+        }
+        if (G.graded) {
+            const double dxc = a.x_nodes[S.at.cell + 1] - a.x_nodes[S.at.cell];
+            if (MAG) {
+                // the NumPy tracer's spacing: the smaller of the cell's edge and h
+                if (dxc < hloc) hloc = dxc;
+            } else {
+                const double d2 = num.known(dxc, G.h, G.rh);
+                if (d2 < 1.0) hloc = hloc * d2;
+            }
+        }
+    }
+    S.hloc = hloc;
+    const double s = S.v[0] * S.v[0] + S.v[1] * S.v[1] + S.v[2] * S.v[2];
+    double y;
+    const double root = num.root(s, y);
+    const double speed = GENERAL ? S.gv * root : root;
+    S.speed2 = speed * speed;
+    // (at rest the quotient is not used; Num<true> then calls the step odd)
+    const double time = GENERAL ? num.div(hloc, speed) : num.over(hloc, speed, num.inverse(speed, y));
+    S.dt0 = speed > 0.0 ? time : -1.0;
+}
+
+// E and, with MAG, B at the point q located at W.
+template <int CYL, bool GENERAL, bool MAG, class N>
+__device__ __forceinline__ void fields_at(N &num, const bt_trace_args &a, const bt_magnetic &mag,
+                                          const Geo &G, const double *q, const Place &W, double *E,
+                                          double *B) {
+    double cy = 0.0, cz = 0.0;
+    if (CYL == 1) {
+        // (selected, not branched around: with Num<true> the quotients cost no branch)
+        const bool off_axis = W.r > 0.0;
+        const double ir = num.inverse(W.r, W.y);
+        const double uy = num.over(q[1], W.r, ir), uz = num.over(q[2], W.r, ir);
+        cy = off_axis ? uy : 0.0;
+        cz = off_axis ? uz : 0.0;
+    } else if (CYL == 2) {
+        cy = 1.0;
+        if (q[1] < G.oy) cy = -1.0;
+    }
+    double ex, ey;
+    if ((N::fast && !GENERAL) || G.same) {  // (the straight-line form is for G.same only)
+        edge_field_cells(num, a, G.base, W.sx, W.sy, ex, ey);
+    } else {
+        const PatchGeom g = GENERAL ? patch_geom(a, finest_patch(a, G.P, W.lx, W.r)) : G.base;
+        edge_field_cells(num, a, g, num.div(W.lx - g.pox, g.phh), num.div(W.r - g.poy, g.phh), ex,
+                         ey);
+    }
+    E[0] = ex;
+    if (CYL != 0) {
+        E[1] = ey * cy;
+        E[2] = ey * cz;
+    } else {
+        E[1] = ey;
+        E[2] = 0.0;
+    }
+    if (MAG) magnetic_at(num, mag, G.rhz, q[0], q[1], W.r, cy, cz, B);
+}
+
+// g = q/m (E + u x B) (tracer.py:519-529), or q/m E.
+template <bool MAG>
+__device__ __forceinline__ void pull(double qm, const double *E, const double *B, const double *u,
+                                     double *g) {
+    if (MAG) {
+        g[0] = qm * (E[0] + (u[1] * B[2] - u[2] * B[1]));
+        g[1] = qm * (E[1] + (u[2] * B[0] - u[0] * B[2]));
+        g[2] = qm * (E[2] + (u[0] * B[1] - u[1] * B[0]));
+    } else {
+        g[0] = qm * E[0];
+        g[1] = qm * E[1];
+        g[2] = qm * E[2];
+    }
+}
+
+// One step from S to T, its deposit in D and its step time in dt_out; the rounding of every
+// operation is the reference's.  FAST: straight-line arithmetic (Num<true>), false where it
+// may not hold -- the caller steps again with FAST false.
+//
+// FAST also takes the step as limited by the speed, whose time the step before has left in
+// S.dt0, and only checks that the acceleration would not shorten it, with a margin of 1e-9
+// against rounding: |a| < 2 v^2 / h, all squared, no root or quotient.  So the time does not
+// wait for the first field: the points of the second stage (x + dt/2 v) and of the first are
+// looked up together, as are those of the third (which needs the first stage's field) and
+// the fourth (the second's), the chain of a Runge-Kutta step two lookups long instead of
+// four with the step time's two roots and quotient between.  A step limited by the
+// acceleration (a beam starting nearly at rest) is taken twice.
+//
+// Bound by latency still: one warp a scheduler on 20,000 rings, 1,013 instructions of 500 in
+// FP64 a step (8 cycles each behind another, 2 of issue).  A window of 64 Runge-Kutta steps of
+// 20,000 rings at 801 x 201 takes 132 us (216 with IEEE roots and quotients and a step time
+// that waits for the field); 64 Boris steps of 100,000 ions on a graded 1025 x 513 mesh in
+// a solenoid 965 us before, some 550 now.
+template <int CYL, int INTEG, bool GENERAL, bool MAG, bool FAST>
+__device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magnetic &mag,
+                                        const Geo &G, const State &S, State &T, Share &D,
+                                        double &dt_out) {
+    Num<FAST> num;
+    const double qm = G.qm, inv_c2 = G.inv_c2;
+    const double gv = GENERAL ? S.gv : 1.0;
+    double E[3], B[3] = {0.0, 0.0, 0.0}, a1[3];
+    if (INTEG != 0 && S.have) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            E[c] = S.e[c];
+            if (MAG) B[c] = S.b[c];
+        }
+    } else {
+        fields_at<CYL, GENERAL, MAG>(num, a, mag, G, S.x, S.at, E, B);
+    }
+    if (INTEG != 0 && !MAG && S.have) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a1[c] = E[c];  // the end of the last step's q/m E
+    } else {
+        pull<MAG>(qm, E, B, S.v, a1);
+    }
+    const double acc2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
+    double dt = S.dt0;
+    if (FAST) {
+        num.flag |= !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2));
+        num.flag |= !(dt > 0.0);
+    } else {
+        const double accel = num.root(acc2);
+        if (accel > 0.0) {
+            const double d2 = sqrt(2.0 * S.hloc / accel);
+            if (dt < 0.0 || d2 < dt) dt = d2;
+        }
+        if (dt < 0.0) dt = S.hloc;
+    }
+    dt = G.fraction * dt;
+    const double hdt = 0.5 * dt;
+    double *y = T.x, *w = T.v;
+    Place Wq;
+    if (INTEG != 0) {
+        // half a kick, the drift, the field there and the other half
+        double k[3];
+        if (MAG) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) k[c] = S.v[c];
+            kick(num, k, E, B, hdt, qm);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) y[c] = S.x[c] + dt * k[c];
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) k[c] = S.v[c] + hdt * a1[c];
+            const double gk = inv_gamma<GENERAL>(num, k[0], k[1], k[2], inv_c2);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) y[c] = S.x[c] + dt * gk * k[c];
+        }
+        locate<CYL, GENERAL>(num, a, G, y, S.at.cell, T.at);
+        fields_at<CYL, GENERAL, MAG>(num, a, mag, G, y, T.at, E, B);
+        if (MAG) {
+            kick(num, k, E, B, hdt, qm);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                w[c] = k[c];
+                T.e[c] = E[c];
+                T.b[c] = B[c];
+            }
+        } else {
+            double g[3];
+            pull<false>(qm, E, B, k, g);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                w[c] = k[c] + hdt * g[c];
+                T.e[c] = g[c];
+            }
+        }
+        T.have = true;
+    } else {
+        double q[3], k2[3], k3[3], k4[3], g[3], sx[3], sv[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sx[c] = gv * S.v[c];
+            sv[c] = a1[c];
+            q[c] = S.x[c] + hdt * gv * S.v[c];
+            k2[c] = S.v[c] + hdt * a1[c];
+        }
+        const double g2 = inv_gamma<GENERAL>(num, k2[0], k2[1], k2[2], inv_c2);
+        locate<CYL, GENERAL>(num, a, G, q, S.at.cell, Wq);
+        fields_at<CYL, GENERAL, MAG>(num, a, mag, G, q, Wq, E, B);
+        pull<MAG>(qm, E, B, k2, g);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sx[c] = sx[c] + 2.0 * g2 * k2[c];
+            sv[c] = sv[c] + 2.0 * g[c];
+            q[c] = S.x[c] + hdt * g2 * k2[c];
+            k3[c] = S.v[c] + hdt * g[c];
+        }
+        const double g3 = inv_gamma<GENERAL>(num, k3[0], k3[1], k3[2], inv_c2);
+        locate<CYL, GENERAL>(num, a, G, q, S.at.cell, Wq);
+        fields_at<CYL, GENERAL, MAG>(num, a, mag, G, q, Wq, E, B);
+        pull<MAG>(qm, E, B, k3, g);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sx[c] = sx[c] + 2.0 * g3 * k3[c];
+            sv[c] = sv[c] + 2.0 * g[c];
+            q[c] = S.x[c] + dt * g3 * k3[c];
+            k4[c] = S.v[c] + dt * g[c];
+        }
+        const double g4 = inv_gamma<GENERAL>(num, k4[0], k4[1], k4[2], inv_c2);
+        locate<CYL, GENERAL>(num, a, G, q, S.at.cell, Wq);
+        fields_at<CYL, GENERAL, MAG>(num, a, mag, G, q, Wq, E, B);
+        pull<MAG>(qm, E, B, k4, g);
+        const double dt6 = num.known(dt, 6.0, 1.0 / 6.0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            y[c] = S.x[c] + dt6 * (sx[c] + g4 * k4[c]);
+            w[c] = S.v[c] + dt6 * (sv[c] + g[c]);
+        }
+        T.have = false;
+        locate<CYL, GENERAL>(num, a, G, y, S.at.cell, T.at);
+    }
+    const double gw = T.gv = inv_gamma<GENERAL>(num, w[0], w[1], w[2], inv_c2);
+    set_pace<GENERAL, MAG>(num, a, G, T);
+
+    // the deposit of the step's Hermite midpoint (:372-423); a / 8 is a * 0.125 exactly
+    double m0 = 0.5 * (S.x[0] + y[0]) + dt * (gv * S.v[0] - gw * w[0]) * 0.125;
+    double m1 = 0.5 * (S.x[1] + y[1]) + dt * (gv * S.v[1] - gw * w[1]) * 0.125;
+    const double m2 = 0.5 * (S.x[2] + y[2]) + dt * (gv * S.v[2] - gw * w[2]) * 0.125;
+    if (CYL == 1)
+        m1 = num.root(m1 * m1 + m2 * m2);
+    else if (CYL == 2)
+        m1 = G.oy + fabs(m1 - G.oy);
+    int cell;
+    m0 = uniform_x<GENERAL>(num, a, G, m0, S.at.cell, cell);
+    const bool one = !GENERAL || G.P == 1;
+    const PatchGeom g = one ? G.base : patch_geom(a, finest_patch(a, G.P, m0, m1));
+    const double rphh = one ? g.rphh : 0.0;
+    // quotients by the patch's spacing
+    auto cells_of = [&](double v) { return one ? num.known(v, g.phh, rphh) : num.div(v, g.phh); };
+    const int pnx = (int)g.pnx, pny = (int)g.pny;
+    int i = __double2int_rd(cells_of(m0 - g.pox));
+    int j = __double2int_rd(cells_of(m1 - g.poy));
+    double u = cells_of(m0 - (g.pox + g.phh * (double)i));
+    double wr;
+    if (CYL == 1) {
+        const double low = g.poy + g.phh * (double)j;
+        const double high = low + g.phh;
+        wr = num.div(m1 * m1 - low * low, high * high - low * low);
+    } else {
+        wr = cells_of(m1 - (g.poy + g.phh * (double)j));
+    }
+    if (i < 0) {
+        u = 0.0;
+        i = 0;
+    } else if (i >= pnx - 1) {
+        u = 1.0;
+        i = pnx - 2;
+    }
+    if (j < 0) {
+        wr = 0.0;
+        j = 0;
+    } else if (j >= pny - 1) {
+        wr = 1.0;
+        j = pny - 2;
+    }
+    D.key = (uint32_t)(g.ofn + (i64)i * pny + j);
+    const double ch = G.dq * dt;
+    D.c00 = (1.0 - u) * (1.0 - wr) * ch;
+    D.c01 = (1.0 - u) * wr * ch;
+    D.c10 = u * (1.0 - wr) * ch;
+    D.c11 = u * wr * ch;
+    dt_out = dt;
+    // (an intermediate value out of range leaves the end state, or its root, out of range)
+    num.in_range(y[0]);
+    if (CYL != 1) num.in_range(y[1]);
+    return !num.odd();
+}
+
+// The same with IEEE operations, out of line: for the steps the straight-line form refuses.
+template <int CYL, int INTEG, bool GENERAL, bool MAG>
+__device__ __noinline__ void advance_plain(const bt_trace_args &a, const bt_magnetic &mag,
+                                           const Geo &G, const State &S, State &T, Share &D) {
+    double dt;
+    advance<CYL, INTEG, GENERAL, MAG, false>(a, mag, G, S, T, D, dt);
+}
+
+// The place and pace of a state whose position and velocity are set.
+template <int CYL, bool GENERAL, bool MAG>
+__device__ __noinline__ void begin_plain(const bt_trace_args &a, const Geo &G, State &S) {
+    Num<false> num;
+    S.gv = inv_gamma<GENERAL>(num, S.v[0], S.v[1], S.v[2], G.inv_c2);
+    locate<CYL, GENERAL>(num, a, G, S.x, S.at.cell, S.at);
+    // (the root's reciprocal, for the straight-line quotients by the radius)
+    S.at.y = S.at.r > 0.0 ? 1.0 / S.at.r : 0.0;
+    set_pace<GENERAL, MAG>(num, a, G, S);
 }
 
 // The kernel is specialised on the geometry (0 planar, 1 cylindrical, 2 symmetry plane),
@@ -229,10 +602,6 @@ __device__ __forceinline__ double inv_gamma(double u0, double u1, double u2, dou
 // window with live trajectories sets *records_end to `end`, the end of its slots, so the
 // deposit sorts no window that had none.
 //
-// At most 168 registers, so that an SM holds three blocks: measured as fast as the
-// registers the compiler wants on a window of one block per SM (the einzel lens) and
-// faster on larger windows and on concurrent solves, whose warps hide each other's latency.
-//
 // One thread's window (m < stride): whether its trajectory is still live afterwards.
 template <int CYL, int INTEG, bool GENERAL, bool MAG, bool BATCH>
 __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restrict__ act,
@@ -245,406 +614,163 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
     }
     const bt_trace_args &a = tr.a;
     const i64 k = act[m];
-    const i64 P = GENERAL ? a.n_patches : 1;
     // the one patch of a non-general mesh (of the trajectory's candidate in a batch)
     const i64 cand = BATCH ? (i64)__ldg(tr.cand + k) : 0;
-    PatchGeom base = patch_geom(a, cand);
-    base.rphh = known_reciprocal(base.phh);
-    const double rh = BATCH ? base.rphh : known_reciprocal(a.h);
-    const i64 nx = BATCH ? base.pnx : tr.nx, ny = BATCH ? base.pny : tr.ny;
-    const double origin_x = BATCH ? base.pox : a.origin_x;
-    const double origin_y = BATCH ? base.poy : a.origin_y;
-    const double h = BATCH ? base.phh : a.h;
+    Geo G;
+    G.P = GENERAL ? (int)a.n_patches : 1;
+    G.base = patch_geom(a, cand);
+    G.base.rphh = known_reciprocal(G.base.phh);
+    const i64 nx = BATCH ? G.base.pnx : tr.nx, ny = BATCH ? G.base.pny : tr.ny;
+    G.ox = BATCH ? G.base.pox : a.origin_x;
+    G.oy = BATCH ? G.base.poy : a.origin_y;
+    G.h = BATCH ? G.base.phh : a.h;
+    G.rh = BATCH ? G.base.rphh : known_reciprocal(a.h);
+    G.rhz = MAG ? known_reciprocal(tr.mag.hz) : 1.0;
+    G.qm = a.qm[k];
+    G.dq = a.dq[k];
+    G.fraction = a.step_fraction;
+    G.inv_c2 = a.inv_c2;
+    G.graded = GENERAL && a.graded != 0;
+    G.n_x_nodes = (int)a.n_x_nodes;
+    G.same = G.P == 1 && G.base.pox == G.ox && G.base.poy == G.oy && G.base.phh == G.h;
+    G.fast = G.rh != 0.0 && G.base.rphh != 0.0 && G.rhz != 0.0 && (GENERAL || G.same);
     const double upper_x = BATCH ? __ldg(a.patch_real + cand * 7 + 5) : a.upper_x;
     const double upper_y = BATCH ? __ldg(a.patch_real + cand * 7 + 6) : a.upper_y;
     const i64 *__restrict__ cells = BATCH ? a.cells + __ldg(tr.cell_off + cand) : a.cells;
-    constexpr int cyl = CYL;
-    const double inv_c2 = a.inv_c2;
     const i64 n = a.n;
-    const bool graded = GENERAL && a.graded != 0;
-    double x0 = a.x[k], x1 = a.x[n + k], x2 = a.x[2 * n + k];
-    double v0 = a.v[k], v1 = a.v[n + k], v2 = a.v[2 * n + k];
-    const double qmk = a.qm[k];
-    const double dqk = a.dq[k];
+    State now;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        now.x[c] = a.x[c * n + k];
+        now.v[c] = a.v[c * n + k];
+        now.e[c] = now.b[c] = 0.0;
+    }
+    now.have = false;
+    now.at.cell = 0;
+    {
+        State first = now;
+        const Geo g = G;
+        begin_plain<CYL, GENERAL, MAG>(a, g, first);
+        now = first;
+    }
     const i64 slot = a.path_slot[k];
     i64 ns = a.steps[k];
     i64 st = -1;
-    constexpr int nstage = INTEG == 0 ? 4 : 2;
-    int have = 0;
-    double ca0 = 0.0, ca1 = 0.0, ca2 = 0.0;
-    double cE[3] = {0, 0, 0}, cB[3] = {0, 0, 0};  // with B: the fields at the step's end
-    // A one-patch mesh whose patch is the mesh: the first gather of a step is at the point
-    // where the exit test of the step before found the radius and the cell coordinates;
-    // they are kept (the same expressions on the same values).
-    const bool reuse = !GENERAL && !MAG && base.pox == origin_x && base.poy == origin_y &&
-                       base.phh == h;
-    double start_r = 0.0, start_sx = 0.0, start_sy = 0.0;
-    if (reuse) {
-        start_r = x1;
-        if (cyl == 1)
-            start_r = radius(x1, x2);
-        else if (cyl == 2)
-            start_r = origin_y + fabs(x1 - origin_y);
-        start_sx = div_known(x0 - origin_x, h, rh);
-        start_sy = div_known(start_r - origin_y, h, rh);
-    }
+    // the first planes in registers: a step's crossing test is two comparisons a plane
+    constexpr int kHeldPlanes = 2;
+    double held[kHeldPlanes];
+#pragma unroll
+    for (int p = 0; p < kHeldPlanes; ++p)
+        held[p] = p < a.n_planes ? a.planes[p] : __longlong_as_double(0x7ff8000000000000LL);
     // The records of consecutive steps in one cell are summed into one (the run's): it goes
     // to the slot of the run's last step, the slots of its other steps hold the sentinel.
     i64 run_slot = -1;
     uint32_t run_key = sentinel;
     double r00 = 0.0, r01 = 0.0, r10 = 0.0, r11 = 0.0;
+    // a point below the mesh (only a malformed geometry puts one there) takes its first cell,
+    // where the reference indexes outside the table
+    auto last_cell = [](double u, i64 nodes) {
+        return max(min(__double2int_rz(u), (int)nodes - 2), 0);
+    };
+    auto cell_at = [&](const Place &W) {
+        return __ldg(cells + (i64)last_cell(W.sx, nx) * (ny - 1) + last_cell(W.sy, ny));
+    };
     int s = 0;
     for (; s < S; ++s) {
         if (ns >= a.max_steps) break;
-        double rr = x1;
-        if (cyl == 1)
-            rr = radius(x1, x2);
-        else if (cyl == 2)
-            rr = origin_y + fabs(x1 - origin_y);
-        double lx = x0;
-        if (graded) lx = uniform_x(x0, a.x_nodes, a.n_x_nodes, origin_x, h);
-        double hloc = h;
-        for (i64 qq = 0; qq < P - 1; ++qq) {
-            const double *pr = a.patch_real + qq * 7;
-            if (lx >= __ldg(pr + 3) && lx <= __ldg(pr + 5) && rr >= __ldg(pr + 4) &&
-                rr <= __ldg(pr + 6)) {
-                hloc = __ldg(pr + 2);
-                break;
-            }
+        State next;
+        Share D;
+        double dt;
+        const bool ok = advance<CYL, INTEG, GENERAL, MAG, true>(a, tr.mag, G, now, next, D, dt);
+        // the end's cell in the electrode table: asked for here, where the lookup runs beside
+        // the rest of the step's arithmetic
+        i64 cell = cell_at(next.at);
+        if (!(ok && G.fast)) {
+            // copies, so that only this branch keeps anything in memory
+            const State from = now;
+            const Geo g = G;
+            State to;
+            Share d;
+            advance_plain<CYL, INTEG, GENERAL, MAG>(a, tr.mag, g, from, to, d);
+            to.at.y = to.at.r > 0.0 ? 1.0 / to.at.r : 0.0;
+            next = to;
+            D = d;
+            cell = cell_at(next.at);
         }
-        if (graded) {
-            const i64 cg = node_cell(x0, a.x_nodes, a.n_x_nodes);
-            if (MAG) {
-                // the NumPy tracer's spacing: the smaller of the cell's edge and h
-                const double dxc = a.x_nodes[cg + 1] - a.x_nodes[cg];
-                if (dxc < hloc) hloc = dxc;
-            } else {
-                const double d2 = (a.x_nodes[cg + 1] - a.x_nodes[cg]) / h;
-                if (d2 < 1.0) hloc = hloc * d2;
-            }
-        }
-        const double gv = inv_gamma<GENERAL>(v0, v1, v2, inv_c2);
-        double q0 = x0, q1 = x1, q2 = x2;
-        double kx0 = v0, kx1 = v1, kx2 = v2;
-        double sx0 = 0, sx1 = 0, sx2 = 0, sv0 = 0, sv1 = 0, sv2 = 0;
-        double w0 = 0, w1 = 0, w2 = 0, y0, y1, y2;
-        double dt = 0.0, hdt = 0.0, dt6 = 0.0;
-        for (int stage = 0; stage < nstage; ++stage) {
-            double gk = inv_gamma<GENERAL>(kx0, kx1, kx2, inv_c2);
-            double g0, g1, g2;
-            double E[3], B[3];
-            if (MAG && stage == 0 && have != 0) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    E[c] = cE[c];
-                    B[c] = cB[c];
-                }
-            }
-            if (MAG && !(stage == 0 && have != 0)) {
-                double qy = q1, cy = 0.0, cz = 0.0;
-                if (cyl == 1) {
-                    const double r = radius(q1, q2);
-                    if (r > 0.0) {
-                        cy = q1 / r;
-                        cz = q2 / r;
-                    }
-                    qy = r;
-                }
-                double lq = q0;
-                if (graded) lq = uniform_x(q0, a.x_nodes, a.n_x_nodes, origin_x, h);
-                double ex, ey;
-                const PatchGeom g = GENERAL ? patch_geom(a, finest_patch(a, P, lq, qy)) : base;
-                edge_field(a, g, lq, qy, ex, ey);
-                if (cyl != 0) {
-                    E[0] = ex;
-                    E[1] = ey * cy;
-                    E[2] = ey * cz;
-                } else {
-                    E[0] = ex;
-                    E[1] = ey;
-                    E[2] = 0.0;
-                }
-                magnetic_at(tr.mag, q0, q1, qy, cy, cz, B);
-            }
-            if (MAG) {
-                // q/m (E + v x B) at the stage velocity (tracer.py:519-529)
-                const double c0 = kx1 * B[2] - kx2 * B[1];
-                const double c1 = kx2 * B[0] - kx0 * B[2];
-                const double c2 = kx0 * B[1] - kx1 * B[0];
-                g0 = qmk * (E[0] + c0);
-                g1 = qmk * (E[1] + c1);
-                g2 = qmk * (E[2] + c2);
-            } else if (stage == 0 && have != 0) {
-                g0 = ca0;
-                g1 = ca1;
-                g2 = ca2;
-            } else {
-                const bool kept = reuse && stage == 0;
-                double qy = q1, cy = 0.0, cz = 0.0;
-                if (cyl == 1) {
-                    const double r = kept ? start_r : radius(q1, q2);
-                    if (r > 0.0) {
-                        cy = q1 / r;
-                        cz = q2 / r;
-                    }
-                    qy = r;
-                } else if (cyl == 2) {
-                    cy = 1.0;
-                    if (q1 < origin_y) cy = -1.0;
-                    qy = origin_y + fabs(q1 - origin_y);
-                }
-                double lq = q0;
-                if (graded) lq = uniform_x(q0, a.x_nodes, a.n_x_nodes, origin_x, h);
-                double ex, ey;
-                const PatchGeom g = GENERAL ? patch_geom(a, finest_patch(a, P, lq, qy)) : base;
-                if (kept)
-                    edge_field_cells(a, g, start_sx, start_sy, ex, ey);
-                else
-                    edge_field(a, g, lq, qy, ex, ey);
-                if (cyl != 0) {
-                    g0 = qmk * ex;
-                    g1 = qmk * (ey * cy);
-                    g2 = qmk * (ey * cz);
-                } else {
-                    g0 = qmk * ex;
-                    g1 = qmk * ey;
-                    g2 = qmk * 0.0;
-                }
-            }
-            if (stage == 0) {
-                const double a0 = g0, a1 = g1, a2 = g2;
-                const double speed = gv * sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-                const double accel = sqrt(a0 * a0 + a1 * a1 + a2 * a2);
-                dt = -1.0;
-                if (speed > 0.0) dt = hloc / speed;
-                if (accel > 0.0) {
-                    const double d2 = sqrt(2.0 * hloc / accel);
-                    if (dt < 0.0 || d2 < dt) dt = d2;
-                }
-                if (dt < 0.0) dt = hloc;
-                dt = a.step_fraction * dt;
-                hdt = 0.5 * dt;
-                dt6 = div_known(dt, 6.0, 1.0 / 6.0);
-                if (INTEG != 0 && MAG) {
-                    // Boris with B: the kick over half the step, then the drift
-                    double u[3] = {v0, v1, v2};
-                    kick(u, E, B, hdt, qmk);
-                    kx0 = u[0];
-                    kx1 = u[1];
-                    kx2 = u[2];
-                    q0 = x0 + dt * kx0;
-                    q1 = x1 + dt * kx1;
-                    q2 = x2 + dt * kx2;
-                    continue;
-                }
-                if (INTEG != 0) {
-                    kx0 = v0 + hdt * a0;
-                    kx1 = v1 + hdt * a1;
-                    kx2 = v2 + hdt * a2;
-                    gk = inv_gamma<GENERAL>(kx0, kx1, kx2, inv_c2);
-                    q0 = x0 + dt * gk * kx0;
-                    q1 = x1 + dt * gk * kx1;
-                    q2 = x2 + dt * gk * kx2;
-                    continue;
-                }
-                sx0 = gv * v0;
-                sx1 = gv * v1;
-                sx2 = gv * v2;
-                sv0 = a0;
-                sv1 = a1;
-                sv2 = a2;
-                q0 = x0 + hdt * gv * v0;
-                q1 = x1 + hdt * gv * v1;
-                q2 = x2 + hdt * gv * v2;
-                kx0 = v0 + hdt * a0;
-                kx1 = v1 + hdt * a1;
-                kx2 = v2 + hdt * a2;
-            } else if (INTEG != 0 && MAG) {
-                // Boris with B: the second kick in the fields at the end of the step
-                double u[3] = {kx0, kx1, kx2};
-                kick(u, E, B, hdt, qmk);
-                w0 = u[0];
-                w1 = u[1];
-                w2 = u[2];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    cE[c] = E[c];
-                    cB[c] = B[c];
-                }
-                have = 1;
-            } else if (INTEG != 0) {
-                w0 = kx0 + hdt * g0;
-                w1 = kx1 + hdt * g1;
-                w2 = kx2 + hdt * g2;
-                ca0 = g0;
-                ca1 = g1;
-                ca2 = g2;
-                have = 1;
-            } else if (stage == 1 || stage == 2) {
-                sx0 = sx0 + 2.0 * gk * kx0;
-                sx1 = sx1 + 2.0 * gk * kx1;
-                sx2 = sx2 + 2.0 * gk * kx2;
-                sv0 = sv0 + 2.0 * g0;
-                sv1 = sv1 + 2.0 * g1;
-                sv2 = sv2 + 2.0 * g2;
-                const double f = stage == 1 ? hdt : dt;
-                q0 = x0 + f * gk * kx0;
-                q1 = x1 + f * gk * kx1;
-                q2 = x2 + f * gk * kx2;
-                kx0 = v0 + f * g0;
-                kx1 = v1 + f * g1;
-                kx2 = v2 + f * g2;
-            } else {
-                sx0 = sx0 + gk * kx0;
-                sx1 = sx1 + gk * kx1;
-                sx2 = sx2 + gk * kx2;
-                sv0 = sv0 + g0;
-                sv1 = sv1 + g1;
-                sv2 = sv2 + g2;
-            }
-        }
-        if (INTEG == 0) {
-            y0 = x0 + dt6 * sx0;
-            y1 = x1 + dt6 * sx1;
-            y2 = x2 + dt6 * sx2;
-            w0 = v0 + dt6 * sv0;
-            w1 = v1 + dt6 * sv1;
-            w2 = v2 + dt6 * sv2;
+        if (run_slot >= 0 && D.key == run_key) {
+            // the step stays in the run's cell: its charge joins the run's record
+            keys[run_slot] = sentinel;
+            r00 = r00 + D.c00;
+            r01 = r01 + D.c01;
+            r10 = r10 + D.c10;
+            r11 = r11 + D.c11;
         } else {
-            y0 = q0;
-            y1 = q1;
-            y2 = q2;
+            if (run_slot >= 0) {
+                keys[run_slot] = run_key;
+                rec[run_slot] = DepositRec{r00, r01, r10, r11};
+            }
+            run_key = D.key;
+            r00 = D.c00;
+            r01 = D.c01;
+            r10 = D.c10;
+            r11 = D.c11;
         }
-
-        // the deposit record of the step's Hermite midpoint (:372-423)
-        const double gw = inv_gamma<GENERAL>(w0, w1, w2, inv_c2);
-        // (a / 8 is a * 0.125 exactly)
-        double m0 = 0.5 * (x0 + y0) + dt * (gv * v0 - gw * w0) * 0.125;
-        double m1 = 0.5 * (x1 + y1) + dt * (gv * v1 - gw * w1) * 0.125;
-        const double m2 = 0.5 * (x2 + y2) + dt * (gv * v2 - gw * w2) * 0.125;
-        if (cyl == 1)
-            m1 = radius(m1, m2);
-        else if (cyl == 2)
-            m1 = origin_y + fabs(m1 - origin_y);
-        if (graded) m0 = uniform_x(m0, a.x_nodes, a.n_x_nodes, origin_x, h);
-        {
-            const PatchGeom g = GENERAL ? patch_geom(a, finest_patch(a, P, m0, m1)) : base;
-            const int pnx = (int)g.pnx, pny = (int)g.pny;
-            const double pox = g.pox, poy = g.poy, phh = g.phh, rphh = g.rphh;
-            int i = __double2int_rd(div_known(m0 - pox, phh, rphh));
-            int j = __double2int_rd(div_known(m1 - poy, phh, rphh));
-            double u = div_known(m0 - (pox + phh * (double)i), phh, rphh);
-            double w;
-            if (cyl == 1) {
-                const double low = poy + phh * (double)j;
-                const double high = low + phh;
-                w = (m1 * m1 - low * low) / (high * high - low * low);
-            } else {
-                w = div_known(m1 - (poy + phh * (double)j), phh, rphh);
-            }
-            if (i < 0) {
-                u = 0.0;
-                i = 0;
-            } else if (i >= pnx - 1) {
-                u = 1.0;
-                i = pnx - 2;
-            }
-            if (j < 0) {
-                w = 0.0;
-                j = 0;
-            } else if (j >= pny - 1) {
-                w = 1.0;
-                j = pny - 2;
-            }
-            const uint32_t key = (uint32_t)(g.ofn + (i64)i * pny + j);
-            const double q = dqk * dt;
-            const double c00 = (1.0 - u) * (1.0 - w) * q, c01 = (1.0 - u) * w * q;
-            const double c10 = u * (1.0 - w) * q, c11 = u * w * q;
-            if (run_slot >= 0 && key == run_key) {
-                // the step stays in the run's cell: its charge joins the run's record
-                keys[run_slot] = sentinel;
-                r00 = r00 + c00;
-                r01 = r01 + c01;
-                r10 = r10 + c10;
-                r11 = r11 + c11;
-            } else {
-                if (run_slot >= 0) {
-                    keys[run_slot] = run_key;
-                    rec[run_slot] = DepositRec{r00, r01, r10, r11};
-                }
-                run_key = key;
-                r00 = c00;
-                r01 = c01;
-                r10 = c10;
-                r11 = c11;
-            }
-            run_slot = (i64)s * stride + m;
-        }
+        run_slot = (i64)s * stride + m;
         ns = ns + 1;
 
-        for (i64 p = 0; p < a.n_planes; ++p) {
-            const double xp = a.planes[p];
-            const double before = x0 - xp;
-            const double after = y0 - xp;
-            if ((before < 0.0) != (after < 0.0)) {
-                const double sc = before / (before - after);
-                i64 *cnt = a.counts + k * a.n_planes + p;
-                const i64 c = *cnt;
-                if (c < a.capacity) {
-                    double *hit = a.hits + ((k * a.n_planes + p) * a.capacity + c) * 8;
-                    hit[0] = xp;
-                    hit[1] = x1 + sc * (y1 - x1);
-                    hit[2] = x2 + sc * (y2 - x2);
-                    hit[3] = gv * v0 + sc * (gw * w0 - gv * v0);
-                    hit[4] = gv * v1 + sc * (gw * w1 - gv * v1);
-                    hit[5] = gv * v2 + sc * (gw * w2 - gv * v2);
-                    hit[6] = after >= 0.0 ? 1.0 : -1.0;
-                    hit[7] = 1.0 * (double)ns;
+        bool crossing = a.n_planes > kHeldPlanes;
+#pragma unroll
+        for (int p = 0; p < kHeldPlanes; ++p)
+            crossing |= (now.x[0] < held[p]) != (next.x[0] < held[p]);
+        if (crossing) {
+            for (i64 p = 0; p < a.n_planes; ++p) {
+                const double xp = a.planes[p];
+                const double before = now.x[0] - xp;
+                const double after = next.x[0] - xp;
+                if ((before < 0.0) != (after < 0.0)) {
+                    const double sc = before / (before - after);
+                    i64 *cnt = a.counts + k * a.n_planes + p;
+                    const i64 c = *cnt;
+                    if (c < a.capacity) {
+                        double *hit = a.hits + ((k * a.n_planes + p) * a.capacity + c) * 8;
+                        const double gv = GENERAL ? now.gv : 1.0;
+                        const double gw = GENERAL ? next.gv : 1.0;
+                        hit[0] = xp;
+                        hit[1] = now.x[1] + sc * (next.x[1] - now.x[1]);
+                        hit[2] = now.x[2] + sc * (next.x[2] - now.x[2]);
+                        hit[3] = gv * now.v[0] + sc * (gw * next.v[0] - gv * now.v[0]);
+                        hit[4] = gv * now.v[1] + sc * (gw * next.v[1] - gv * now.v[1]);
+                        hit[5] = gv * now.v[2] + sc * (gw * next.v[2] - gv * now.v[2]);
+                        hit[6] = after >= 0.0 ? 1.0 : -1.0;
+                        hit[7] = 1.0 * (double)ns;
+                    }
+                    *cnt = c + 1;
                 }
-                *cnt = c + 1;
             }
         }
-        x0 = y0;
-        x1 = y1;
-        x2 = y2;
-        v0 = w0;
-        v1 = w1;
-        v2 = w2;
+        now = next;
 
-        double px = x0, py = x1;
-        if (cyl == 1)
-            py = radius(x1, x2);
-        else if (cyl == 2)
-            py = origin_y + fabs(x1 - origin_y);
+        const double px = now.at.lx, py = now.at.r;
         if (slot >= 0) {
             const i64 c = a.path_count[slot];
             if (c < a.path_capacity) {
-                a.paths[(slot * a.path_capacity + c) * 2 + 0] = px;
+                a.paths[(slot * a.path_capacity + c) * 2 + 0] = now.x[0];
                 a.paths[(slot * a.path_capacity + c) * 2 + 1] = py;
             }
             a.path_count[slot] = c + 1;
         }
-        if (graded) px = uniform_x(px, a.x_nodes, a.n_x_nodes, origin_x, h);
         if (px >= upper_x) {
             st = 0;
-        } else if (px < origin_x) {
+        } else if (px < G.ox) {
             st = 1;
-        } else if (py > upper_y || (cyl == 0 && py < origin_y)) {
+        } else if (py > upper_y || (CYL == 0 && py < G.oy)) {
             st = 2;
         } else {
-            const double ux = div_known(px - origin_x, h, rh);
-            const double uy = div_known(py - origin_y, h, rh);
-            start_r = py;
-            start_sx = ux;
-            start_sy = uy;
-            // a point below the mesh (only a malformed geometry puts one there) takes
-            // its first cell, where the reference indexes outside the table
-            const int i = max(min(__double2int_rz(ux), (int)nx - 2), 0);
-            const int j = max(min(__double2int_rz(uy), (int)ny - 2), 0);
-            const i64 cell = __ldg(cells + (i64)i * (ny - 1) + j);
+            const double ux = now.at.sx, uy = now.at.sy;
             if (MAG && cell >= 0) {
                 st = -2;  // the caller tests the electrodes' shapes
             } else if (cell >= 0) {
+                const int i = last_cell(ux, nx), j = last_cell(uy, ny);
                 const i64 R = a.refine;
                 i64 si = (i64)((ux - (double)i) * (double)R);
                 if (si < 0)
@@ -664,9 +790,9 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
                     // the candidate's own electrodes, tested here at the point's mesh
                     // coordinates: the caller's test of a paused trajectory
                     const i64 s0 = __ldg(tr.shape_first + cand);
-                    const Shapes S{__ldg(tr.shape_first + cand + 1) - s0, tr.shapes.kind + s0,
-                                   tr.shapes.offset + s0, tr.shapes.params};
-                    const i64 hit = inside_solid(S, px, py);
+                    const Shapes sh{__ldg(tr.shape_first + cand + 1) - s0, tr.shapes.kind + s0,
+                                    tr.shapes.offset + s0, tr.shapes.params};
+                    const i64 hit = inside_solid(sh, px, py);
                     if (hit >= 0) {
                         st = 3;
                         a.electrode[k] = hit;
@@ -688,12 +814,11 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
     // the slots of the steps not taken hold no record
     for (; s < S; ++s) keys[(i64)s * stride + m] = sentinel;
     if (st == -1 && ns >= a.max_steps) st = 4;
-    a.x[k] = x0;
-    a.x[n + k] = x1;
-    a.x[2 * n + k] = x2;
-    a.v[k] = v0;
-    a.v[n + k] = v1;
-    a.v[2 * n + k] = v2;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        a.x[c * n + k] = now.x[c];
+        a.v[c * n + k] = now.v[c];
+    }
     a.steps[k] = ns;
     a.status[k] = st;
     return st == -1;
@@ -701,10 +826,11 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
 
 // The window: every thread's trajectory, then each block's count of live trajectories and
 // every thread's flag, for compact_live.  BATCH: the trajectories of many candidate meshes
-// in one launch (Trace::cand).
-template <int CYL, int INTEG, bool GENERAL, bool MAG, bool BATCH>
-__global__ void __launch_bounds__(128, 3)
-    trace_window(Trace tr, const i64 *__restrict__ act, const i64 *__restrict__ live, i64 stride,
+// in one launch (Trace::cand).  BLOCKS: the blocks an SM is to hold, which bounds a thread's
+// registers (255 for two, 168 for three; see trace_all for which is launched).
+template <int CYL, int INTEG, bool GENERAL, bool MAG, bool BATCH, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS)
+    trace_window(const __grid_constant__ Trace tr, const i64 *__restrict__ act, const i64 *__restrict__ live, i64 stride,
                  int S, uint32_t *__restrict__ keys, DepositRec *__restrict__ rec,
                  uint32_t sentinel, i64 *__restrict__ records_end, i64 end,
                  uint32_t *__restrict__ block_live, uint8_t *__restrict__ alive) {
@@ -984,13 +1110,23 @@ void trace_all(bt_ctx *ctx, const bt_trace_args *args, const bt_magnetic *mag, i
                     bt::Timed timed(ctx, "trace_window");
                     grid = (unsigned)bt::blocks_for(bound, 128);
                     const int64_t launched = ctx->launch_count;
-#define BT_TRACE_CASE_B(C, I, G, M, B)                                                          \
+                    // A window whose blocks fit two a multiprocessor has warps to spare for
+                    // none: 255 registers let the lookups' chains run side by side (20,000
+                    // rings, 157 blocks: 132 us a window against 159 with 168 registers).
+                    // A larger one hides latency with a third block (40,000 rings: 7.3 ms a
+                    // trace against 8.3), as do the magnetic trace's (52 ms against 64) and a
+                    // batch's thousands of blocks.
+                    const bool wide = !mag && !batch && grid <= (unsigned)(2 * ctx->num_sms);
+#define BT_TRACE_CASE_N(C, I, G, M, B, N)                                                       \
     if (a.cylindrical == C && (a.integrator != 0) == (I != 0) && general == G &&                 \
-        (mag != nullptr) == M && (batch != nullptr) == B)                                        \
-        BT_LAUNCH(ctx, (bt::trace_window<C, I, G, M, B>), grid, 128, 0, st, tr, act_a,            \
+        (mag != nullptr) == M && (batch != nullptr) == B && wide == (N == 2))                    \
+        BT_LAUNCH(ctx, (bt::trace_window<C, I, G, M, B, N>), grid, 128, 0, st, tr, act_a,         \
                   live + lv, bound, S, keys[cur] + used, rec[cur] + used, sentinel,               \
                   records_end + cur, used + need, block_live, alive);
-#define BT_TRACE_CASE(C, I, G, M) BT_TRACE_CASE_B(C, I, G, M, false)
+#define BT_TRACE_CASE_B(C, I, G, M, B) BT_TRACE_CASE_N(C, I, G, M, B, 3)
+#define BT_TRACE_CASE(C, I, G, M)                                                               \
+    BT_TRACE_CASE_N(C, I, G, M, false, 3)                                                         \
+    if (!M) { BT_TRACE_CASE_N(C, I, G, false, false, 2) }
                     BT_TRACE_CASE(0, 0, false, false) BT_TRACE_CASE(0, 0, true, false)
                     BT_TRACE_CASE(0, 1, false, false) BT_TRACE_CASE(0, 1, true, false)
                     BT_TRACE_CASE(1, 0, false, false) BT_TRACE_CASE(1, 0, true, false)
@@ -1006,6 +1142,7 @@ void trace_all(bt_ctx *ctx, const bt_trace_args *args, const bt_magnetic *mag, i
                     BT_TRACE_CASE_B(2, 0, false, false, true) BT_TRACE_CASE_B(2, 1, false, false, true)
 #undef BT_TRACE_CASE
 #undef BT_TRACE_CASE_B
+#undef BT_TRACE_CASE_N
                     BT_REQUIRE(ctx->launch_count > launched,
                                "trace: no kernel for these settings");
                 }
