@@ -37,73 +37,111 @@ __device__ __forceinline__ int finest3(const bt_trace3d_args &a, double p0, doub
 }
 
 // The reference's nested trilinear form at corner index ci (:231-236).
-__device__ __forceinline__ double trilinear(const double *__restrict__ f, i64 ci, i64 dj, i64 di,
+__device__ __forceinline__ double trilinear(const double *__restrict__ f, i64 ci, int dj, i64 di,
                                             double a, double b, double c) {
-    return (1.0 - a) * ((1.0 - b) * ((1.0 - c) * __ldg(f + ci) + c * __ldg(f + ci + 1)) +
-                        b * ((1.0 - c) * __ldg(f + ci + dj) + c * __ldg(f + ci + dj + 1))) +
-           a * ((1.0 - b) * ((1.0 - c) * __ldg(f + ci + di) + c * __ldg(f + ci + di + 1)) +
-                b * ((1.0 - c) * __ldg(f + ci + di + dj) + c * __ldg(f + ci + di + dj + 1)));
+    f += ci;
+    return (1.0 - a) * ((1.0 - b) * ((1.0 - c) * __ldg(f) + c * __ldg(f + 1)) +
+                        b * ((1.0 - c) * __ldg(f + dj) + c * __ldg(f + dj + 1))) +
+           a * ((1.0 - b) * ((1.0 - c) * __ldg(f + di) + c * __ldg(f + di + 1)) +
+                b * ((1.0 - c) * __ldg(f + di + dj) + c * __ldg(f + di + dj + 1)));
 }
 
-// E and B at a point: mirrored below a symmetry plane, E from the finest patch holding it
-// (:173-335).
-__device__ __forceinline__ Fields3 fields3(const bt_trace3d_args &a, i64 nx, i64 ny, i64 nz,
-                                           double p0, double p1, double p2) {
-    double s1 = 1.0, s2 = 1.0;
-    if (a.mirror_y != 0 && p1 < a.origin_y) {
-        p1 = 2.0 * a.origin_y - p1;
-        s1 = -1.0;
-    }
-    if (a.mirror_z != 0 && p2 < a.origin_z) {
-        p2 = 2.0 * a.origin_z - p2;
-        s2 = -1.0;
-    }
-    const int pp = finest3(a, p0, p1, p2);
-    const i64 *pi = a.patch_int + pp * 8;
-    const double *pr = a.patch_real + pp * 10;
-    const int pnx = (int)__ldg(pi), pny = (int)__ldg(pi + 1), pnz = (int)__ldg(pi + 2);
-    const i64 ofx = __ldg(pi + 3), ofy = __ldg(pi + 4), ofz = __ldg(pi + 5);
-    const double phh = __ldg(pr + 3);
-    const double sx = (p0 - __ldg(pr)) / phh, sy = (p1 - __ldg(pr + 1)) / phh;
-    const double sz = (p2 - __ldg(pr + 2)) / phh;
-    Fields3 F;
+// A field box's shape and its edge arrays' offsets.
+struct Box3 {
+    int nx, ny, nz;
+    i64 ofx, ofy, ofz;
+};
+
+// E at the point (sx, sy, sz) in cells of a box; s1, s2 the signs a mirror gives.
+__device__ __forceinline__ void edges3(const bt_trace3d_args &a, const Box3 &g, double sx, double sy,
+                                       double sz, double s1, double s2, double *e) {
+    const int pnx = g.nx, pny = g.ny, pnz = g.nz;
     // E_x on (pnx + 1, pny, pnz) at (sx + 1/2, sy, sz)
     double s = sx + 0.5;
     int i = clamp3(__double2int_rd(s), 0, pnx - 1);
     int j = clamp3(__double2int_rd(sy), 0, pny - 2);
     int k = clamp3(__double2int_rd(sz), 0, pnz - 2);
-    const double c = sz - (double)k;
-    F.e[0] = trilinear(a.fxs, ofx + (i64)i * pny * pnz + (i64)j * pnz + k, pnz, (i64)pny * pnz,
-                       s - (double)i, sy - (double)j, c);
+    const int jb = j;
+    const double c = sz - (double)k, b = sy - (double)j;
+    e[0] = trilinear(a.fxs, g.ofx + ((i64)i * pny + j) * pnz + k, pnz, (i64)pny * pnz, s - (double)i,
+                     b, c);
     // E_y on (pnx, pny + 1, pnz) at (sx, sy + 1/2, sz)
     i = clamp3(__double2int_rd(sx), 0, pnx - 2);
     s = sy + 0.5;
     j = clamp3(__double2int_rd(s), 0, pny - 1);
     const double ax = sx - (double)i;
-    i64 di = (i64)(pny + 1) * pnz;
-    F.e[1] = s1 * trilinear(a.fys, ofy + i * di + (i64)j * pnz + k, pnz, di, ax, s - (double)j, c);
+    e[1] = s1 * trilinear(a.fys, g.ofy + ((i64)i * (pny + 1) + j) * pnz + k, pnz,
+                          (i64)(pny + 1) * pnz, ax,
+                          s - (double)j, c);
     // E_z on (pnx, pny, pnz + 1) at (sx, sy, sz + 1/2)
-    j = clamp3(__double2int_rd(sy), 0, pny - 2);
     s = sz + 0.5;
     k = clamp3(__double2int_rd(s), 0, pnz - 1);
-    di = (i64)pny * (pnz + 1);
-    F.e[2] = s2 * trilinear(a.fzs, ofz + i * di + (i64)j * (pnz + 1) + k, pnz + 1, di, ax,
-                            sy - (double)j, s - (double)k);
+    e[2] = s2 * trilinear(a.fzs, g.ofz + ((i64)i * pny + jb) * (pnz + 1) + k, pnz + 1,
+                          (i64)pny * (pnz + 1), ax, b, s - (double)k);
+}
+
+// What a trajectory's steps share: the base mesh, its patch, the spacings' reciprocals.
+struct Geo3 {
+    int nx, ny, nz;   // the base mesh's nodes
+    Box3 base;        // the base patch
+    i64 first;        // its first charge node
+    double h, rh, qm, dq;
+};
+
+// A point on the mesh: mirrored below a symmetry plane (with the signs that gives E), in
+// cells of the base mesh from its origin.
+struct Place3 {
+    double p[3], s[3], s1, s2;
+};
+
+template <class N>
+__device__ __forceinline__ void locate3(N &num, const bt_trace3d_args &a, const Geo3 &G,
+                                        const double *q, Place3 &W) {
+    W.s1 = W.s2 = 1.0;
+    W.p[0] = q[0];
+    W.p[1] = q[1];
+    W.p[2] = q[2];
+    const bool my = a.mirror_y != 0 && q[1] < a.origin_y, mz = a.mirror_z != 0 && q[2] < a.origin_z;
+    W.p[1] = my ? 2.0 * a.origin_y - q[1] : q[1];
+    W.p[2] = mz ? 2.0 * a.origin_z - q[2] : q[2];
+    W.s1 = my ? -1.0 : 1.0;
+    W.s2 = mz ? -1.0 : 1.0;
+    W.s[0] = num.known(W.p[0] - a.origin_x, G.h, G.rh);
+    W.s[1] = num.known(W.p[1] - a.origin_y, G.h, G.rh);
+    W.s[2] = num.known(W.p[2] - a.origin_z, G.h, G.rh);
+}
+
+// E (from the finest patch holding the point) and B at a place (:173-335).
+template <bool HASB, class N>
+__device__ __forceinline__ Fields3 fields3(N &num, const bt_trace3d_args &a, const Geo3 &G,
+                                           const Place3 &W) {
+    Fields3 F;
+    if (N::fast) {
+        edges3(a, G.base, W.s[0], W.s[1], W.s[2], W.s1, W.s2, F.e);
+    } else {
+        const int pp = finest3(a, W.p[0], W.p[1], W.p[2]);
+        const i64 *pi = a.patch_int + pp * 8;
+        const double *pr = a.patch_real + pp * 10;
+        const double phh = __ldg(pr + 3);
+        const Box3 g{(int)__ldg(pi), (int)__ldg(pi + 1), (int)__ldg(pi + 2),
+                     __ldg(pi + 3), __ldg(pi + 4), __ldg(pi + 5)};
+        edges3(a, g, (W.p[0] - __ldg(pr)) / phh, (W.p[1] - __ldg(pr + 1)) / phh,
+               (W.p[2] - __ldg(pr + 2)) / phh, W.s1, W.s2, F.e);
+    }
     F.b[0] = F.b[1] = F.b[2] = 0.0;
-    if (a.has_b != 0) {
+    if (HASB) {
         // B on the base mesh's nodes (3, nx, ny, nz), the weights summed in corner order
-        const double tx = (p0 - a.origin_x) / a.h, ty = (p1 - a.origin_y) / a.h;
-        const double tz = (p2 - a.origin_z) / a.h;
-        const int bi = clamp3(__double2int_rd(tx), 0, (int)nx - 2);
-        const int bj = clamp3(__double2int_rd(ty), 0, (int)ny - 2);
-        const int bk = clamp3(__double2int_rd(tz), 0, (int)nz - 2);
-        const double u = tx - (double)bi, w = ty - (double)bj, z = tz - (double)bk;
+        const int bi = clamp3(__double2int_rd(W.s[0]), 0, G.nx - 2);
+        const int bj = clamp3(__double2int_rd(W.s[1]), 0, G.ny - 2);
+        const int bk = clamp3(__double2int_rd(W.s[2]), 0, G.nz - 2);
+        const double u = W.s[0] - (double)bi, w = W.s[1] - (double)bj, z = W.s[2] - (double)bk;
         const double wt[8] = {(1.0 - u) * (1.0 - w) * (1.0 - z), (1.0 - u) * (1.0 - w) * z,
                               (1.0 - u) * w * (1.0 - z),         (1.0 - u) * w * z,
                               u * (1.0 - w) * (1.0 - z),         u * (1.0 - w) * z,
                               u * w * (1.0 - z),                 u * w * z};
-        const i64 nb = nx * ny * nz, dj = nz, dI = ny * nz;
-        const i64 base = (i64)bi * dI + (i64)bj * dj + bk;
+        const i64 nb = (i64)G.nx * G.ny * G.nz;
+        const i64 dj = G.nz, dI = (i64)G.ny * G.nz;
+        const i64 base = ((i64)bi * G.ny + bj) * G.nz + bk;
         const i64 off[8] = {0, 1, dj, dj + 1, dI, dI + 1, dI + dj, dI + dj + 1};
         double comp[3];
 #pragma unroll
@@ -114,22 +152,30 @@ __device__ __forceinline__ Fields3 fields3(const bt_trace3d_args &a, i64 nx, i64
             for (int q = 1; q < 8; ++q) f = f + wt[q] * __ldg(bn + off[q]);
             comp[n0] = f;
         }
-        F.b[0] = s1 * s2 * comp[0];
-        F.b[1] = s2 * comp[1];
-        F.b[2] = s1 * comp[2];
+        F.b[0] = W.s1 * W.s2 * comp[0];
+        F.b[1] = W.s2 * comp[1];
+        F.b[2] = W.s1 * comp[2];
     }
     return F;
+}
+
+// 1 / gamma of a proper velocity: 1 with Num<true>, whose steps are not relativistic.
+template <class N>
+__device__ __forceinline__ double inv_gamma3(N &, double u0, double u1, double u2, double inv_c2) {
+    return N::fast ? 1.0 : 1.0 / sqrt(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2);
 }
 
 // The relativistic Boris push (J. P. Boris, 1970) of u by the scaled fields e (the kicks)
 // and b (the rotation by t = b / gamma, s = 2 t / (1 + t^2)): what the reference's kernel
 // calls mpiparticles' relativistic_boris_update for.
-__device__ __forceinline__ void boris_push(double *u, const double *e, const double *b,
+template <class N>
+__device__ __forceinline__ void boris_push(N &num, double *u, const double *e, const double *b,
                                            double inv_c2) {
     const double m0 = u[0] + e[0], m1 = u[1] + e[1], m2 = u[2] + e[2];
-    const double g = sqrt(1.0 + (m0 * m0 + m1 * m1 + m2 * m2) * inv_c2);
-    const double t0 = b[0] / g, t1 = b[1] / g, t2 = b[2] / g;
-    const double f = 2.0 / (1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
+    const double g = N::fast ? 1.0 : sqrt(1.0 + (m0 * m0 + m1 * m1 + m2 * m2) * inv_c2);
+    const double t0 = N::fast ? b[0] : b[0] / g, t1 = N::fast ? b[1] : b[1] / g,
+                 t2 = N::fast ? b[2] : b[2] / g;
+    const double f = num.div(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
     const double s0 = f * t0, s1 = f * t1, s2 = f * t2;
     const double p0 = m0 + (m1 * t2 - m2 * t1);
     const double p1 = m1 + (m2 * t0 - m0 * t2);
@@ -137,10 +183,6 @@ __device__ __forceinline__ void boris_push(double *u, const double *e, const dou
     u[0] = m0 + (p1 * s2 - p2 * s1) + e[0];
     u[1] = m1 + (p2 * s0 - p0 * s2) + e[1];
     u[2] = m2 + (p0 * s1 - p1 * s0) + e[2];
-}
-
-__device__ __forceinline__ double inv_gamma3(double u0, double u1, double u2, double inv_c2) {
-    return 1.0 / sqrt(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2);
 }
 
 // A deposit point's corner node (among `nodes` of a box of (bnx, bny, bnz) from `first`) and
@@ -220,13 +262,196 @@ struct Trace3 {
     uint32_t jsentinel;   // a slot with no current record
 };
 
+// The state of a trajectory between steps, as the 2D trace's: its place and the pace it sets
+// (the local spacing, the speed's square, the spacing over the speed or -1 at rest), with
+// Boris the fields at the last step's end.
+struct State3 {
+    double x[3], v[3];
+    Place3 at;
+    double gv, hloc, speed2, dt0;
+    Fields3 end;
+    bool have;
+};
+
+// A step's deposit: its time, its midpoint's box on the charge's patch and on the base mesh.
+struct Deposit3 {
+    double dt;
+    Box charge, mesh;
+};
+
+template <class N>
+__device__ __forceinline__ void set_pace3(N &num, const bt_trace3d_args &a, const Geo3 &G,
+                                          State3 &S) {
+    S.gv = inv_gamma3(num, S.v[0], S.v[1], S.v[2], a.inv_c2);
+    S.hloc = G.h;
+    if (!N::fast) {
+        // the spacing of the finest patch at the step's start (:148-163)
+        const int q = finest3(a, S.at.p[0], S.at.p[1], S.at.p[2]);
+        if (q < (int)a.n_patches - 1) S.hloc = __ldg(a.patch_real + q * 10 + 3);
+    }
+    double y;
+    const double root = num.root(S.v[0] * S.v[0] + S.v[1] * S.v[1] + S.v[2] * S.v[2], y);
+    const double speed = N::fast ? root : S.gv * root;
+    S.speed2 = speed * speed;
+    const double time = num.over(S.hloc, speed, num.inverse(speed, y));
+    S.dt0 = speed > 0.0 ? time : -1.0;
+}
+
+// q/m (E + v x B) at the velocity u.
+template <bool HASB, class N>
+__device__ __forceinline__ void pull3(N &, double qm, const Fields3 &F, const double *u, double gk,
+                                      double *g) {
+    if (N::fast && !HASB) {
+        g[0] = qm * F.e[0];
+        g[1] = qm * F.e[1];
+        g[2] = qm * F.e[2];
+    } else if (N::fast) {
+        g[0] = qm * (F.e[0] + u[1] * F.b[2] - u[2] * F.b[1]);
+        g[1] = qm * (F.e[1] + u[2] * F.b[0] - u[0] * F.b[2]);
+        g[2] = qm * (F.e[2] + u[0] * F.b[1] - u[1] * F.b[0]);
+    } else {
+        g[0] = qm * (F.e[0] + gk * u[1] * F.b[2] - gk * u[2] * F.b[1]);
+        g[1] = qm * (F.e[1] + gk * u[2] * F.b[0] - gk * u[0] * F.b[2]);
+        g[2] = qm * (F.e[2] + gk * u[0] * F.b[1] - gk * u[1] * F.b[0]);
+    }
+}
+
+// One step from S to T and its deposit: the 2D trace's `advance` in three dimensions (the
+// same straight-line roots and quotients, the same step time known in advance, false where
+// either may not hold).  With IEEE operations a step was 2,429 instructions, its quotients by
+// the spacing and its roots behind one another: 509 us a window of 32 Runge-Kutta steps of
+// 100,000 trajectories; 1,620 instructions and 346 us now, the L1 data path busy 62 % of them
+// with the 96 corner loads a step.  Three blocks a multiprocessor (168 registers) hide more
+// of the loads than two with 255 (384 us).
+template <int INTEG, bool HASB, bool FAST>
+__device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G, const State3 &S,
+                                         State3 &T, Deposit3 &D) {
+    Num<FAST> num;
+    const double qm = G.qm, inv_c2 = a.inv_c2, gv = FAST ? 1.0 : S.gv;
+    Fields3 F;
+    if (INTEG != 0 && S.have)
+        F = S.end;
+    else
+        F = fields3<HASB>(num, a, G, S.at);
+    double a1[3];
+    pull3<HASB>(num, qm, F, S.v, gv, a1);
+    const double acc2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
+    double dt = S.dt0;
+    if (FAST) {
+        num.flag |= !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2));
+        num.flag |= !(dt > 0.0);
+    } else {
+        const double accel = sqrt(acc2);
+        if (accel > 0.0) {
+            const double d2 = sqrt(2.0 * S.hloc / accel);
+            if (dt < 0.0 || d2 < dt) dt = d2;
+        }
+        if (dt < 0.0) dt = S.hloc;
+    }
+    dt = a.step_fraction * dt;
+    const double hdt = 0.5 * dt;
+    double *y = T.x, *w = T.v;
+    if (INTEG != 0) {
+        // Boris: a half step's kick--rotate--kick, the drift, the second at the end
+        const double tau = 0.5 * hdt * qm;
+        double u[3] = {S.v[0], S.v[1], S.v[2]};
+        double e[3] = {tau * F.e[0], tau * F.e[1], tau * F.e[2]};
+        double b[3] = {tau * F.b[0], tau * F.b[1], tau * F.b[2]};
+        boris_push(num, u, e, b, inv_c2);
+        const double gk = inv_gamma3(num, u[0], u[1], u[2], inv_c2);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) y[c] = S.x[c] + dt * gk * u[c];
+        locate3(num, a, G, y, T.at);
+        F = fields3<HASB>(num, a, G, T.at);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            e[c] = tau * F.e[c];
+            b[c] = tau * F.b[c];
+        }
+        boris_push(num, u, e, b, inv_c2);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) w[c] = u[c];
+        T.end = F;
+        T.have = true;
+    } else {
+        const double dt6 = num.known(dt, 6.0, 1.0 / 6.0);
+        double sx[3], sv[3], q[3], k[3], g[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            sx[c] = gv * S.v[c];
+            sv[c] = a1[c];
+            q[c] = S.x[c] + hdt * gv * S.v[c];
+            k[c] = S.v[c] + hdt * a1[c];
+        }
+#pragma unroll
+        for (int stage = 1; stage < 4; ++stage) {
+            Place3 W;
+            locate3(num, a, G, q, W);
+            F = fields3<HASB>(num, a, G, W);
+            const double gk = inv_gamma3(num, k[0], k[1], k[2], inv_c2);
+            pull3<HASB>(num, qm, F, k, gk, g);
+            const double f = stage == 1 ? hdt : dt;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (stage < 3) {
+                    sx[c] = sx[c] + 2.0 * gk * k[c];
+                    sv[c] = sv[c] + 2.0 * g[c];
+                    q[c] = S.x[c] + f * gk * k[c];
+                    k[c] = S.v[c] + f * g[c];
+                } else {
+                    y[c] = S.x[c] + dt6 * (sx[c] + gk * k[c]);
+                    w[c] = S.v[c] + dt6 * (sv[c] + g[c]);
+                }
+            }
+        }
+        T.have = false;
+        locate3(num, a, G, y, T.at);
+    }
+    set_pace3(num, a, G, T);
+    const double gw = FAST ? 1.0 : T.gv;
+    // the space charge dq dt at the step's Hermite midpoint (:451-519); a / 8 is a * 0.125
+    double m[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        m[c] = 0.5 * (S.x[c] + y[c]) + dt * (gv * S.v[c] - gw * w[c]) * 0.125;
+    Place3 M;
+    locate3(num, a, G, m, M);
+    D.mesh = box3(0, G.nx, G.ny, G.nz, M.s[0], M.s[1], M.s[2]);
+    if (FAST) {
+        D.charge = D.mesh;
+        D.charge.cc += G.first;
+    } else {
+        const int pp = finest3(a, M.p[0], M.p[1], M.p[2]);
+        const i64 *pi = a.patch_int + pp * 8;
+        const double *pr = a.patch_real + pp * 10;
+        const double phh = __ldg(pr + 3);
+        D.charge = box3(__ldg(pi + 7), (int)__ldg(pi), (int)__ldg(pi + 1), (int)__ldg(pi + 2),
+                        (M.p[0] - __ldg(pr)) / phh, (M.p[1] - __ldg(pr + 1)) / phh,
+                        (M.p[2] - __ldg(pr + 2)) / phh);
+    }
+    D.dt = dt;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) num.in_range(y[c] - 1.0);
+    return !num.odd();
+}
+
+template <int INTEG, bool HASB>
+__device__ __noinline__ void advance3_plain(const bt_trace3d_args &a, const Geo3 &G,
+                                            const State3 &S, State3 &T, Deposit3 &D) {
+    advance3<INTEG, HASB, false>(a, G, S, T, D);
+}
+
 // One window of trajectory m (of the active list): at most S steps from its state.  The
 // charge of a run of consecutive steps in one cell is summed into one cell record (key: the
 // cell's lower corner node), written to the slot (s n_active + m) of the run's last step s;
 // with has_j, each step's current shares go to the slots ((s n_active + m) 24 + 8 component
 // + corner).  The slots with no record hold the sentinels.  alive[m]: the trajectory has not ended (cleared here when
 // it does, with its status written); *live counts the ones still going after the window.
-__global__ void __launch_bounds__(128) trace3d_window(Trace3 T, uint8_t *__restrict__ alive,
+// TRY: the straight-line step is tried first, on one patch that is the mesh, without
+// relativity; the others take the IEEE operations in line.
+template <int INTEG, bool HASB, bool TRY>
+__global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__ Trace3 T,
+                                                      uint8_t *__restrict__ alive,
                                                       uint32_t *__restrict__ keys,
                                                       CellRec *__restrict__ recs,
                                                       uint32_t *__restrict__ jkeys,
@@ -242,131 +467,58 @@ __global__ void __launch_bounds__(128) trace3d_window(Trace3 T, uint8_t *__restr
     if (alive[m]) {
         const i64 k = a.active[m];
         const i64 n = a.n;
-        const i64 nx = T.nx, ny = T.ny, nz = T.nz;
-        double x0 = a.x[k], x1 = a.x[n + k], x2 = a.x[2 * n + k];
-        double v0 = a.v[k], v1 = a.v[n + k], v2 = a.v[2 * n + k];
-        const double qmk = a.qm[k], dqk = a.dq[k], inv_c2 = a.inv_c2;
+        Geo3 G;
+        G.nx = (int)T.nx;
+        G.ny = (int)T.ny;
+        G.nz = (int)T.nz;
+        const i64 *pi = a.patch_int + (a.n_patches - 1) * 8;
+        G.base = Box3{G.nx, G.ny, G.nz, __ldg(pi + 3), __ldg(pi + 4), __ldg(pi + 5)};
+        G.first = __ldg(pi + 7);
+        G.h = a.h;
+        G.rh = known_reciprocal(a.h);
+        G.qm = a.qm[k];
+        G.dq = a.dq[k];
+        const double dqk = G.dq;
+        State3 now;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            now.x[c] = a.x[c * n + k];
+            now.v[c] = a.v[c * n + k];
+            now.end.e[c] = now.end.b[c] = 0.0;
+        }
+        now.have = false;
+        {
+            Num<false> num;
+            locate3(num, a, G, now.x, now.at);
+            set_pace3(num, a, G, now);
+        }
         const i64 slot = a.path_slot[k];
         i64 ns = a.steps[k];
         i64 st = -1;
-        bool have = false;
-        Fields3 cache{};
         // the current run of steps in one cell: its slot, key and summed shares
         i64 run_slot = -1;
         uint32_t run_key = T.sentinel;
         double run[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (; s < S && ns < a.max_steps; ++s) {
-            // the spacing of the finest patch at the step's start (:148-163)
-            double p1 = x1, p2 = x2;
-            if (a.mirror_y != 0 && p1 < a.origin_y) p1 = 2.0 * a.origin_y - p1;
-            if (a.mirror_z != 0 && p2 < a.origin_z) p2 = 2.0 * a.origin_z - p2;
-            double hloc = a.h;
+            State3 next;
+            Deposit3 D;
+            bool ok = false;
+            if (TRY) ok = advance3<INTEG, HASB, true>(a, G, now, next, D);
+            if (!TRY) advance3<INTEG, HASB, false>(a, G, now, next, D);
+            if (TRY && !ok) {
+                // copies, so that only this branch keeps anything in memory
+                const State3 from = now;
+                const Geo3 g = G;
+                State3 to;
+                Deposit3 d;
+                advance3_plain<INTEG, HASB>(a, g, from, to, d);
+                next = to;
+                D = d;
+            }
             {
-                const int q = finest3(a, x0, p1, p2);
-                if (q < (int)a.n_patches - 1) hloc = __ldg(a.patch_real + q * 10 + 3);
-            }
-            const double gv = inv_gamma3(v0, v1, v2, inv_c2);
-            Fields3 F = (a.integrator != 0 && have) ? cache : fields3(a, nx, ny, nz, x0, x1, x2);
-            double gk = inv_gamma3(v0, v1, v2, inv_c2);
-            double g0 = qmk * (F.e[0] + gk * v1 * F.b[2] - gk * v2 * F.b[1]);
-            double g1 = qmk * (F.e[1] + gk * v2 * F.b[0] - gk * v0 * F.b[2]);
-            double g2 = qmk * (F.e[2] + gk * v0 * F.b[1] - gk * v1 * F.b[0]);
-            const double speed = gv * sqrt(v0 * v0 + v1 * v1 + v2 * v2);
-            const double accel = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
-            double dt = -1.0;
-            if (speed > 0.0) dt = hloc / speed;
-            if (accel > 0.0) {
-                const double d2 = sqrt(2.0 * hloc / accel);
-                if (dt < 0.0 || d2 < dt) dt = d2;
-            }
-            if (dt < 0.0) dt = hloc;
-            dt = a.step_fraction * dt;
-            const double hdt = 0.5 * dt;
-            double y0, y1, y2, w0, w1, w2;
-            if (a.integrator != 0) {
-                // Boris: a half step's kick--rotate--kick, the drift, the second at the end
-                const double tau = 0.5 * hdt * qmk;
-                double u[3] = {v0, v1, v2};
-                double e[3] = {tau * F.e[0], tau * F.e[1], tau * F.e[2]};
-                double b[3] = {tau * F.b[0], tau * F.b[1], tau * F.b[2]};
-                boris_push(u, e, b, inv_c2);
-                gk = inv_gamma3(u[0], u[1], u[2], inv_c2);
-                y0 = x0 + dt * gk * u[0];
-                y1 = x1 + dt * gk * u[1];
-                y2 = x2 + dt * gk * u[2];
-                F = fields3(a, nx, ny, nz, y0, y1, y2);
-                e[0] = tau * F.e[0];
-                e[1] = tau * F.e[1];
-                e[2] = tau * F.e[2];
-                b[0] = tau * F.b[0];
-                b[1] = tau * F.b[1];
-                b[2] = tau * F.b[2];
-                boris_push(u, e, b, inv_c2);
-                w0 = u[0];
-                w1 = u[1];
-                w2 = u[2];
-                cache = F;
-                have = true;
-            } else {
-                const double dt6 = dt / 6.0;
-                double sx0 = gv * v0, sx1 = gv * v1, sx2 = gv * v2;
-                double sv0 = g0, sv1 = g1, sv2 = g2;
-                double q0 = x0 + hdt * gv * v0, q1 = x1 + hdt * gv * v1, q2 = x2 + hdt * gv * v2;
-                double k0 = v0 + hdt * g0, k1 = v1 + hdt * g1, k2 = v2 + hdt * g2;
-                for (int stage = 1; stage < 4; ++stage) {
-                    F = fields3(a, nx, ny, nz, q0, q1, q2);
-                    gk = inv_gamma3(k0, k1, k2, inv_c2);
-                    g0 = qmk * (F.e[0] + gk * k1 * F.b[2] - gk * k2 * F.b[1]);
-                    g1 = qmk * (F.e[1] + gk * k2 * F.b[0] - gk * k0 * F.b[2]);
-                    g2 = qmk * (F.e[2] + gk * k0 * F.b[1] - gk * k1 * F.b[0]);
-                    if (stage < 3) {
-                        sx0 = sx0 + 2.0 * gk * k0;
-                        sx1 = sx1 + 2.0 * gk * k1;
-                        sx2 = sx2 + 2.0 * gk * k2;
-                        sv0 = sv0 + 2.0 * g0;
-                        sv1 = sv1 + 2.0 * g1;
-                        sv2 = sv2 + 2.0 * g2;
-                        const double f = stage == 1 ? hdt : dt;
-                        q0 = x0 + f * gk * k0;
-                        q1 = x1 + f * gk * k1;
-                        q2 = x2 + f * gk * k2;
-                        k0 = v0 + f * g0;
-                        k1 = v1 + f * g1;
-                        k2 = v2 + f * g2;
-                    } else {
-                        sx0 = sx0 + gk * k0;
-                        sx1 = sx1 + gk * k1;
-                        sx2 = sx2 + gk * k2;
-                        sv0 = sv0 + g0;
-                        sv1 = sv1 + g1;
-                        sv2 = sv2 + g2;
-                    }
-                }
-                y0 = x0 + dt6 * sx0;
-                y1 = x1 + dt6 * sx1;
-                y2 = x2 + dt6 * sx2;
-                w0 = v0 + dt6 * sv0;
-                w1 = v1 + dt6 * sv1;
-                w2 = v2 + dt6 * sv2;
-            }
-            // the space charge dq dt at the step's Hermite midpoint (:451-519)
-            const double gw = inv_gamma3(w0, w1, w2, inv_c2);
-            const double m0 = 0.5 * (x0 + y0) + dt * (gv * v0 - gw * w0) / 8.0;
-            double m1 = 0.5 * (x1 + y1) + dt * (gv * v1 - gw * w1) / 8.0;
-            double m2 = 0.5 * (x2 + y2) + dt * (gv * v2 - gw * w2) / 8.0;
-            if (a.mirror_y != 0 && m1 < a.origin_y) m1 = 2.0 * a.origin_y - m1;
-            if (a.mirror_z != 0 && m2 < a.origin_z) m2 = 2.0 * a.origin_z - m2;
-            {
-                const int pp = finest3(a, m0, m1, m2);
-                const i64 *pi = a.patch_int + pp * 8;
-                const double *pr = a.patch_real + pp * 10;
-                const double phh = __ldg(pr + 3);
-                const Box B = box3(__ldg(pi + 7), (int)__ldg(pi), (int)__ldg(pi + 1),
-                                   (int)__ldg(pi + 2), (m0 - __ldg(pr)) / phh,
-                                   (m1 - __ldg(pr + 1)) / phh, (m2 - __ldg(pr + 2)) / phh);
                 double w[8];
-                shares8(B, dqk * dt, w);
-                const uint32_t key = (uint32_t)B.cc;
+                shares8(D.charge, dqk * D.dt, w);
+                const uint32_t key = (uint32_t)D.charge.cc;
                 const i64 at = (i64)s * na + m;
                 if (run_slot >= 0 && key == run_key) {
                     keys[run_slot] = T.sentinel;  // the run moves on to this step's slot
@@ -389,53 +541,45 @@ __global__ void __launch_bounds__(128) trace3d_window(Trace3 T, uint8_t *__restr
             }
             if (j_on) {
                 // the current element dq (x' - x) on the base mesh (:520-565)
-                double jd[3] = {dqk * (y0 - x0), dqk * (y1 - x1), dqk * (y2 - x2)};
-                if (a.mirror_y != 0 && 0.5 * (x1 + y1) < a.origin_y) jd[1] = -jd[1];
-                if (a.mirror_z != 0 && 0.5 * (x2 + y2) < a.origin_z) jd[2] = -jd[2];
-                const Box B = box3(0, (int)nx, (int)ny, (int)nz, (m0 - a.origin_x) / a.h,
-                                   (m1 - a.origin_y) / a.h, (m2 - a.origin_z) / a.h);
+                double jd[3] = {dqk * (next.x[0] - now.x[0]), dqk * (next.x[1] - now.x[1]),
+                                dqk * (next.x[2] - now.x[2])};
+                if (a.mirror_y != 0 && 0.5 * (now.x[1] + next.x[1]) < a.origin_y) jd[1] = -jd[1];
+                if (a.mirror_z != 0 && 0.5 * (now.x[2] + next.x[2]) < a.origin_z) jd[2] = -jd[2];
                 const i64 at = ((i64)s * na + m) * 24;
-                const i64 nb = nx * ny * nz;
+                const i64 nb = T.nx * T.ny * T.nz;
 #pragma unroll
                 for (int jc = 0; jc < 3; ++jc) {
-                    Box C = B;
-                    C.cc = B.cc + jc * nb;
+                    Box C = D.mesh;
+                    C.cc += jc * nb;
                     records8(C, jd[jc], jkeys + at + 8 * jc, jvals + at + 8 * jc);
                 }
             }
             ns = ns + 1;
             for (i64 p = 0; p < a.n_planes; ++p) {
                 const double xp = a.planes[p];
-                const double before = x0 - xp, after = y0 - xp;
+                const double before = now.x[0] - xp, after = next.x[0] - xp;
                 if ((before < 0.0) != (after < 0.0)) {
                     const double sc = before / (before - after);
                     i64 *cnt = a.counts + k * a.n_planes + p;
                     const i64 c = *cnt;
                     if (c < a.capacity) {
                         double *hit = a.hits + ((k * a.n_planes + p) * a.capacity + c) * 8;
+                        const double gv = now.gv, gw = next.gv;
                         hit[0] = xp;
-                        hit[1] = x1 + sc * (y1 - x1);
-                        hit[2] = x2 + sc * (y2 - x2);
-                        hit[3] = gv * v0 + sc * (gw * w0 - gv * v0);
-                        hit[4] = gv * v1 + sc * (gw * w1 - gv * v1);
-                        hit[5] = gv * v2 + sc * (gw * w2 - gv * v2);
+                        hit[1] = now.x[1] + sc * (next.x[1] - now.x[1]);
+                        hit[2] = now.x[2] + sc * (next.x[2] - now.x[2]);
+                        hit[3] = gv * now.v[0] + sc * (gw * next.v[0] - gv * now.v[0]);
+                        hit[4] = gv * now.v[1] + sc * (gw * next.v[1] - gv * now.v[1]);
+                        hit[5] = gv * now.v[2] + sc * (gw * next.v[2] - gv * now.v[2]);
                         hit[6] = after >= 0.0 ? 1.0 : -1.0;
                         hit[7] = 1.0 * (double)ns;
                     }
                     *cnt = c + 1;
                 }
             }
-            x0 = y0;
-            x1 = y1;
-            x2 = y2;
-            v0 = w0;
-            v1 = w1;
-            v2 = w2;
+            now = next;
             // the end of the step: off the mesh or in an electrode (:587-641)
-            const double px = x0;
-            double py = x1, pz = x2;
-            if (a.mirror_y != 0 && py < a.origin_y) py = 2.0 * a.origin_y - py;
-            if (a.mirror_z != 0 && pz < a.origin_z) pz = 2.0 * a.origin_z - pz;
+            const double px = now.at.p[0], py = now.at.p[1], pz = now.at.p[2];
             if (slot >= 0) {
                 const i64 c = a.path_count[slot];
                 if (c < a.path_capacity) {
@@ -453,12 +597,11 @@ __global__ void __launch_bounds__(128) trace3d_window(Trace3 T, uint8_t *__restr
             } else if (py > a.upper_y || py < a.origin_y || pz > a.upper_z || pz < a.origin_z) {
                 st = 2;
             } else {
-                const double ux = (px - a.origin_x) / a.h, uy = (py - a.origin_y) / a.h;
-                const double uz = (pz - a.origin_z) / a.h;
-                const int i = min(__double2int_rz(ux), (int)nx - 2);
-                const int j = min(__double2int_rz(uy), (int)ny - 2);
-                const int kz = min(__double2int_rz(uz), (int)nz - 2);
-                const i64 cell = __ldg(a.cells + ((i64)i * (ny - 1) + j) * (nz - 1) + kz);
+                const double ux = now.at.s[0], uy = now.at.s[1], uz = now.at.s[2];
+                const int i = min(__double2int_rz(ux), G.nx - 2);
+                const int j = min(__double2int_rz(uy), G.ny - 2);
+                const int kz = min(__double2int_rz(uz), G.nz - 2);
+                const i64 cell = __ldg(a.cells + ((i64)i * (G.ny - 1) + j) * (G.nz - 1) + kz);
                 if (cell >= 0) {
                     const int R = (int)a.refine;
                     const int si = clamp3(__double2int_rz((ux - (double)i) * (double)R), 0, R - 1);
@@ -486,12 +629,11 @@ __global__ void __launch_bounds__(128) trace3d_window(Trace3 T, uint8_t *__restr
             recs[run_slot] = r;
         }
         if (st == -1 && ns >= a.max_steps) st = 4;
-        a.x[k] = x0;
-        a.x[n + k] = x1;
-        a.x[2 * n + k] = x2;
-        a.v[k] = v0;
-        a.v[n + k] = v1;
-        a.v[2 * n + k] = v2;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            a.x[c * n + k] = now.x[c];
+            a.v[c * n + k] = now.v[c];
+        }
         a.steps[k] = ns;
         if (st != -1) {
             a.status[k] = st;
@@ -699,6 +841,14 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
     BT_REQUIRE(T.nx >= 2 && T.ny >= 2 && T.nz >= 2, "trace3d: the mesh needs 2 x 2 x 2 nodes");
     const i64 nb = T.nx * T.ny * T.nz;
     BT_REQUIRE(!a.has_j || 3 * nb < (int64_t)0xffffffffLL, "trace3d: too many current nodes");
+    // one patch that is the mesh, whose spacing has a reciprocal, and no relativity
+    bool fast = a.n_patches == 1 && a.inv_c2 == 0.0 && known_reciprocal(a.h) != 0.0;
+    if (fast) {
+        double row[10];
+        BT_CUDA(cudaMemcpyAsync(row, a.patch_real, sizeof(row), cudaMemcpyDeviceToHost, ctx->stream));
+        BT_CUDA(cudaStreamSynchronize(ctx->stream));
+        fast = row[0] == a.origin_x && row[1] == a.origin_y && row[2] == a.origin_z && row[3] == a.h;
+    }
     T.S = window > 0 ? (int)window : 32;
     T.sentinel = (uint32_t)a.n_nodes;
     T.jsentinel = (uint32_t)(3 * nb);
@@ -725,8 +875,15 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
         BT_CUDA(cudaMemsetAsync(live, 0, sizeof(unsigned long long), st));
         {
             Timed timed(ctx, "trace3d_window");
-            BT_LAUNCH(ctx, trace3d_window, blocks_for(na, 128), 128, 0, st, T, alive, keys, recs,
-                      jkeys, jvals, live);
+#define BT_TRACE3D_CASE(I, B, F)                                                                \
+    if ((a.integrator != 0) == (I != 0) && (a.has_b != 0) == B && fast == F)                     \
+        BT_LAUNCH(ctx, (trace3d_window<I, B, F>), blocks_for(na, 128), 128, 0, st, T, alive, keys, \
+                  recs, jkeys, jvals, live);
+            BT_TRACE3D_CASE(0, false, true) BT_TRACE3D_CASE(0, false, false)
+            BT_TRACE3D_CASE(0, true, true) BT_TRACE3D_CASE(0, true, false)
+            BT_TRACE3D_CASE(1, false, true) BT_TRACE3D_CASE(1, false, false)
+            BT_TRACE3D_CASE(1, true, true) BT_TRACE3D_CASE(1, true, false)
+#undef BT_TRACE3D_CASE
         }
         BT_CHECK_LAUNCH();
         {
