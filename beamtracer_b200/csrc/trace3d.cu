@@ -6,11 +6,12 @@
 // magnetic field on the base mesh's nodes, symmetry planes at the lower y and z faces, the
 // plane crossings, kept paths, exit and electrode sub-cell tests: the reference's step term
 // by term in FP64 with no contracted multiply-add, so a trajectory ends bit for bit where the
-// reference's kernel ends it.  Instead of adding to the charge with atomics, every step writes
-// its eight node shares as (node, value) records to slots fixed by (window step, trajectory,
-// corner); after each window the records are sorted by node (stable) and summed per node in
-// record order, so the node charges are the same on every run.  The current elements (has_j)
-// take the same way on the base mesh's 3 nx ny nz components.
+// reference's kernel ends it.  Instead of adding to the charge with atomics, the steps write
+// their cells' corner shares as records to slots fixed by (window step, trajectory); after
+// each window the records are sorted by cell (stable), summed per cell in record order and
+// gathered by the nodes, so the node charges are the same on every run.  The current elements
+// (has_j) take the same way, one record of three components' eight shares a step (a record a
+// share, 24 keys to sort a step, took 119 ms a trace of 100,000 trajectories; 11 ms so).
 #include <algorithm>
 #include <vector>
 
@@ -214,11 +215,15 @@ __device__ __forceinline__ Box box3(i64 first, int bnx, int bny, int bnz, double
     return {first + (i64)i * bny * bnz + (i64)j * bnz + k, bnz, (i64)bny * bnz, a, b, c};
 }
 
-// A cell's charge record: the shares of its eight corners, in the corner order (k, then j,
-// then i offsets: q = 4 di + 2 dj + dk), two 32-byte sectors.
-struct __align__(64) CellRec {
-    double c[8];
+// A cell's record: the shares of its eight corners, in the corner order (k, then j, then i
+// offsets: q = 4 di + 2 dj + dk) -- of the charge (two 32-byte sectors), or of the current
+// element's three components one after the other (six).
+template <int N>
+struct __align__(64) Rec {
+    double c[N];
 };
+using CellRec = Rec<8>;
+using CurrentRec = Rec<24>;
 
 // The eight shares of q, in the reference's corner order (:512-519).
 __device__ __forceinline__ void shares8(const Box &B, double q, double *w) {
@@ -231,21 +236,6 @@ __device__ __forceinline__ void shares8(const Box &B, double q, double *w) {
     w[5] = a * (1.0 - b) * c * q;
     w[6] = a * b * (1.0 - c) * q;
     w[7] = a * b * c * q;
-}
-
-// The eight shares of q as records, in the reference's corner order (:512-519).
-__device__ __forceinline__ void records8(const Box &B, double q, uint32_t *key, double *val) {
-    const double a = B.a, b = B.b, c = B.c;
-    const i64 o[8] = {0, 1, B.dj, B.dj + 1, B.di, B.di + 1, B.di + B.dj, B.di + B.dj + 1};
-    const double w[8] = {(1.0 - a) * (1.0 - b) * (1.0 - c) * q, (1.0 - a) * (1.0 - b) * c * q,
-                         (1.0 - a) * b * (1.0 - c) * q,         (1.0 - a) * b * c * q,
-                         a * (1.0 - b) * (1.0 - c) * q,         a * (1.0 - b) * c * q,
-                         a * b * (1.0 - c) * q,                 a * b * c * q};
-#pragma unroll
-    for (int q8 = 0; q8 < 8; ++q8) {
-        key[q8] = (uint32_t)(B.cc + o[q8]);
-        val[q8] = w[q8];
-    }
 }
 
 }  // namespace
@@ -444,9 +434,10 @@ __device__ __noinline__ void advance3_plain(const bt_trace3d_args &a, const Geo3
 // One window of trajectory m (of the active list): at most S steps from its state.  The
 // charge of a run of consecutive steps in one cell is summed into one cell record (key: the
 // cell's lower corner node), written to the slot (s n_active + m) of the run's last step s;
-// with has_j, each step's current shares go to the slots ((s n_active + m) 24 + 8 component
-// + corner).  The slots with no record hold the sentinels.  alive[m]: the trajectory has not ended (cleared here when
-// it does, with its status written); *live counts the ones still going after the window.
+// with has_j, each step's current shares go to the slot (s n_active + m) of the current's
+// records.  The slots with no record hold the sentinels.  alive[m]: the trajectory has not
+// ended (cleared here when it does, with its status written); *live counts the ones still
+// going after the window.
 // TRY: the straight-line step is tried first, on one patch that is the mesh, without
 // relativity; the others take the IEEE operations in line.
 template <int INTEG, bool HASB, bool TRY>
@@ -455,7 +446,7 @@ __global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__
                                                       uint32_t *__restrict__ keys,
                                                       CellRec *__restrict__ recs,
                                                       uint32_t *__restrict__ jkeys,
-                                                      double *__restrict__ jvals,
+                                                      CurrentRec *__restrict__ jrecs,
                                                       unsigned long long *__restrict__ live) {
     const bt_trace3d_args &a = T.a;
     const i64 m = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -545,13 +536,14 @@ __global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__
                                 dqk * (next.x[2] - now.x[2])};
                 if (a.mirror_y != 0 && 0.5 * (now.x[1] + next.x[1]) < a.origin_y) jd[1] = -jd[1];
                 if (a.mirror_z != 0 && 0.5 * (now.x[2] + next.x[2]) < a.origin_z) jd[2] = -jd[2];
-                const i64 at = ((i64)s * na + m) * 24;
-                const i64 nb = T.nx * T.ny * T.nz;
+                const i64 at = (i64)s * na + m;
+                jkeys[at] = (uint32_t)D.mesh.cc;
 #pragma unroll
                 for (int jc = 0; jc < 3; ++jc) {
-                    Box C = D.mesh;
-                    C.cc += jc * nb;
-                    records8(C, jd[jc], jkeys + at + 8 * jc, jvals + at + 8 * jc);
+                    double w[8];
+                    shares8(D.mesh, jd[jc], w);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) jrecs[at].c[8 * jc + q] = w[q];
                 }
             }
             ns = ns + 1;
@@ -645,26 +637,8 @@ __global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__
     // the slots of the steps not taken hold no record
     for (; s < S; ++s) {
         keys[(i64)s * na + m] = T.sentinel;
-        if (j_on) {
-            const i64 jt = ((i64)s * na + m) * 24;
-            for (int q = 0; q < 24; ++q) jkeys[jt + q] = T.jsentinel;
-        }
+        if (j_on) jkeys[(i64)s * na + m] = T.jsentinel;
     }
-}
-
-// target[key] += the values of each run of equal sorted keys, in record order (one thread
-// a run, from its head).
-__global__ void run_sums(const uint32_t *__restrict__ K, const uint32_t *__restrict__ I,
-                         const double *__restrict__ vals, const i64 *__restrict__ count,
-                         i64 n_host, double *__restrict__ target) {
-    const i64 r = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    const i64 n = count ? *count : n_host;
-    if (r >= n) return;
-    const uint32_t key = K[r];
-    if (r > 0 && K[r - 1] == key) return;
-    double s = target[key];
-    for (i64 q = r; q < n && K[q] == key; ++q) s += vals[I[q]];
-    target[key] = s;
 }
 
 // The cells' sums: the records of a cell lie together after the sort, in runs of hundreds
@@ -675,13 +649,14 @@ __global__ void run_sums(const uint32_t *__restrict__ K, const uint32_t *__restr
 // order by cell_chains.  The sums depend on the records alone.  (One thread a run, waiting
 // for each record behind the one before, took 343 us for 1.6 M records in cells of some 500;
 // the two kernels take 50 us.)  The cells of no record hold zeros.
+template <int N>
 __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K,
                                                   const uint32_t *__restrict__ I,
-                                                  const CellRec *__restrict__ recs,
+                                                  const Rec<N> *__restrict__ recs,
                                                   const i64 *__restrict__ count,
-                                                  CellRec *__restrict__ cells,
-                                                  CellRec *__restrict__ first,
-                                                  CellRec *__restrict__ last,
+                                                  Rec<N> *__restrict__ cells,
+                                                  Rec<N> *__restrict__ first,
+                                                  Rec<N> *__restrict__ last,
                                                   uint8_t *__restrict__ ends,
                                                   uint8_t *__restrict__ owns) {
     const i64 n = *count;
@@ -691,12 +666,12 @@ __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K
     const i64 r = w * 32 + lane;
     const bool valid = r < n;
     const uint32_t key = valid ? K[r] : 0xffffffffu;
-    CellRec sum;
+    Rec<N> sum;
     if (valid) {
         sum = recs[I[r]];
     } else {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) sum.c[c] = 0.0;
+        for (int c = 0; c < N; ++c) sum.c[c] = 0.0;
     }
     bool head = valid && (r == 0 || K[r - 1] != key);
     const bool tail = valid && (r + 1 >= n || K[r + 1] != key);
@@ -704,7 +679,7 @@ __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K
         const bool before = __shfl_up_sync(0xffffffffu, head, off);
         const bool add = lane >= off && !head;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < N; ++c) {
             const double v = __shfl_up_sync(0xffffffffu, sum.c[c], off);
             if (add) sum.c[c] = v + sum.c[c];
         }
@@ -730,18 +705,19 @@ __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K
     }
 }
 
+template <int N>
 __global__ void __launch_bounds__(256) cell_chains(const uint32_t *__restrict__ K,
                                                    const i64 *__restrict__ count,
-                                                   CellRec *__restrict__ cells,
-                                                   const CellRec *__restrict__ first,
-                                                   const CellRec *__restrict__ last,
+                                                   Rec<N> *__restrict__ cells,
+                                                   const Rec<N> *__restrict__ first,
+                                                   const Rec<N> *__restrict__ last,
                                                    const uint8_t *__restrict__ ends,
                                                    const uint8_t *__restrict__ owns) {
     const i64 n_warps = (*count + 31) / 32;
-    // eight threads a warp's piece: one a corner
+    // N threads a warp's piece: one a value
     const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    const i64 w0 = t >> 3;
-    const int c = (int)(t & 7);
+    const i64 w0 = t / N;
+    const int c = (int)(t - w0 * N);
     if (w0 >= n_warps || !owns[w0]) return;
     double s = last[w0].c[c];
     for (i64 w = w0 + 1; w < n_warps; ++w) {
@@ -752,7 +728,23 @@ __global__ void __launch_bounds__(256) cell_chains(const uint32_t *__restrict__ 
 }
 
 // charge[node] += its shares of the eight cells it is a corner of, in a fixed order (the
-// corner q = 4 di + 2 dj + dk of the cell at node - (di, dj, dk)), within its patch.
+// corner q = 4 di + 2 dj + dk of the cell at node - (di, dj, dk)), within a box of
+// (pnx, pny, pnz) nodes, the node's place in it `local`; `shift` selects a record's component.
+template <int N>
+__device__ __forceinline__ double corner_sum(const Rec<N> *__restrict__ cells, i64 node, i64 local,
+                                             i64 pnx, i64 pny, i64 pnz, int shift) {
+    const i64 i = local / (pny * pnz), j = (local / pnz) % pny, k = local % pnz;
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
+        const i64 ci = i - di, cj = j - dj, ck = k - dk;
+        if (ci < 0 || cj < 0 || ck < 0 || ci > pnx - 2 || cj > pny - 2 || ck > pnz - 2) continue;
+        s = s + cells[node - di * pny * pnz - dj * pnz - dk].c[shift + q];
+    }
+    return s;
+}
+
 __global__ void node_gather3(const CellRec *__restrict__ cells, const i64 *__restrict__ patch_int,
                              int n_patches, i64 n_nodes, double *__restrict__ charge) {
     const i64 node = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -764,16 +756,16 @@ __global__ void node_gather3(const CellRec *__restrict__ cells, const i64 *__res
     const i64 *pi = patch_int + p * 8;
     const i64 pnx = pi[0], pny = pi[1], pnz = pi[2], local = node - pi[7];
     if (local < 0 || local >= pnx * pny * pnz) return;
-    const i64 i = local / (pny * pnz), j = (local / pnz) % pny, k = local % pnz;
-    double s = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
-        const i64 ci = i - di, cj = j - dj, ck = k - dk;
-        if (ci < 0 || cj < 0 || ck < 0 || ci > pnx - 2 || cj > pny - 2 || ck > pnz - 2) continue;
-        s = s + cells[node - di * pny * pnz - dj * pnz - dk].c[q];
-    }
-    charge[node] += s;
+    charge[node] += corner_sum(cells, node, local, pnx, pny, pnz, 0);
+}
+
+// The current's three components on the base mesh's nodes (blockIdx.y the component).
+__global__ void node_gather_current(const CurrentRec *__restrict__ cells, i64 nx, i64 ny, i64 nz,
+                                    double *__restrict__ current) {
+    const i64 node = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    const i64 n = nx * ny * nz;
+    if (node >= n) return;
+    current[blockIdx.y * n + node] += corner_sum(cells, node, node, nx, ny, nz, 8 * (int)blockIdx.y);
 }
 
 __global__ void fill_flags(uint8_t *__restrict__ flags, i64 n, uint8_t value) {
@@ -793,14 +785,23 @@ int key_bits(uint64_t max_key) {
     return b;
 }
 
-// Sort a window's records by node and add each node's run, in record order, to target.
-void deposit_runs(bt_ctx *ctx, const uint32_t *keys, const double *vals, i64 n, uint32_t sentinel,
-                  double *target) {
+// A window's records (`slots` keys, those with the sentinel left out) sorted by cell and
+// summed per cell in record order into `cells` (n_cells, zeroed first).
+template <int N>
+void sum_cells(bt_ctx *ctx, const uint32_t *keys, const Rec<N> *recs, i64 slots, uint32_t sentinel,
+               Rec<N> *cells, i64 n_cells) {
+    cudaStream_t st = ctx->stream;
+    const i64 pieces = (slots + 31) / 32;
+    Rec<N> *first = ctx->t3_pieces.as<Rec<N>>(2 * pieces), *last = first + pieces;
+    uint8_t *flags = ctx->t3_flags.as<uint8_t>(2 * pieces);
     uint32_t *sk = nullptr, *sv = nullptr;
     const i64 *count = nullptr;
-    radix_sort_pairs(ctx, keys, n, nullptr, key_bits(sentinel), sentinel, &sk, &sv, &count);
-    BT_LAUNCH(ctx, run_sums, blocks_for(n, 256), 256, 0, ctx->stream, sk, sv, vals, count, n,
-              target);
+    radix_sort_pairs(ctx, keys, slots, nullptr, key_bits(sentinel), sentinel, &sk, &sv, &count);
+    BT_CUDA(cudaMemsetAsync(cells, 0, sizeof(Rec<N>) * n_cells, st));
+    BT_LAUNCH(ctx, cell_warps<N>, blocks_for(pieces * 32, 256), 256, 0, st, sk, sv, recs, count,
+              cells, first, last, flags, flags + pieces);
+    BT_LAUNCH(ctx, cell_chains<N>, blocks_for(pieces * N, 256), 256, 0, st, sk, count, cells, first,
+              last, flags, flags + pieces);
     BT_CHECK_LAUNCH();
 }
 
@@ -851,19 +852,17 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
     }
     T.S = window > 0 ? (int)window : 32;
     T.sentinel = (uint32_t)a.n_nodes;
-    T.jsentinel = (uint32_t)(3 * nb);
+    T.jsentinel = (uint32_t)nb;
     const i64 na = a.n_active;
-    const i64 slots = (i64)T.S * na, jslots = a.has_j ? (i64)T.S * na * 24 : 0;
-    BT_REQUIRE(slots < (i64)0xffffffffLL && jslots < (i64)0xffffffffLL,
+    const i64 slots = (i64)T.S * na;
+    BT_REQUIRE(slots < (i64)0xffffffffLL && (!a.has_j || 24 * slots < (i64)0xffffffffLL),
                "trace3d: too many records a window (use a shorter window)");
     uint32_t *keys = ctx->t3_keys.as<uint32_t>(slots);
     CellRec *recs = ctx->t3_vals.as<CellRec>(slots);
     CellRec *cells = ctx->t3_cells.as<CellRec>(a.n_nodes);
-    const i64 pieces = (slots + 31) / 32;
-    CellRec *first = ctx->t3_pieces.as<CellRec>(2 * pieces), *last = first + pieces;
-    uint8_t *flags = ctx->t3_flags.as<uint8_t>(2 * pieces);
-    uint32_t *jkeys = a.has_j ? ctx->t3_jkeys.as<uint32_t>(jslots) : nullptr;
-    double *jvals = a.has_j ? ctx->t3_jvals.as<double>(jslots) : nullptr;
+    uint32_t *jkeys = a.has_j ? ctx->t3_jkeys.as<uint32_t>(slots) : nullptr;
+    CurrentRec *jrecs = a.has_j ? ctx->t3_jvals.as<CurrentRec>(slots) : nullptr;
+    CurrentRec *jcells = a.has_j ? ctx->t3_jcells.as<CurrentRec>(nb) : nullptr;
     uint8_t *alive = ctx->t3_alive.as<uint8_t>(na);
     auto *live = ctx->t3_live.as<unsigned long long>(1);
     unsigned long long *host = static_cast<unsigned long long *>(ctx->host.get(64));
@@ -878,7 +877,7 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
 #define BT_TRACE3D_CASE(I, B, F)                                                                \
     if ((a.integrator != 0) == (I != 0) && (a.has_b != 0) == B && fast == F)                     \
         BT_LAUNCH(ctx, (trace3d_window<I, B, F>), blocks_for(na, 128), 128, 0, st, T, alive, keys, \
-                  recs, jkeys, jvals, live);
+                  recs, jkeys, jrecs, live);
             BT_TRACE3D_CASE(0, false, true) BT_TRACE3D_CASE(0, false, false)
             BT_TRACE3D_CASE(0, true, true) BT_TRACE3D_CASE(0, true, false)
             BT_TRACE3D_CASE(1, false, true) BT_TRACE3D_CASE(1, false, false)
@@ -886,22 +885,16 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
 #undef BT_TRACE3D_CASE
         }
         BT_CHECK_LAUNCH();
-        {
-            // the window's cell records: sorted by cell, summed per cell, gathered per node
-            uint32_t *sk = nullptr, *sv = nullptr;
-            const i64 *count = nullptr;
-            radix_sort_pairs(ctx, keys, slots, nullptr, key_bits(T.sentinel), T.sentinel, &sk, &sv,
-                             &count);
-            BT_CUDA(cudaMemsetAsync(cells, 0, sizeof(CellRec) * a.n_nodes, st));
-            BT_LAUNCH(ctx, cell_warps, blocks_for(pieces * 32, 256), 256, 0, st, sk, sv, recs, count,
-                      cells, first, last, flags, flags + pieces);
-            BT_LAUNCH(ctx, cell_chains, blocks_for(pieces * 8, 256), 256, 0, st, sk, count, cells,
-                      first, last, flags, flags + pieces);
-            BT_LAUNCH(ctx, node_gather3, blocks_for(a.n_nodes, 256), 256, 0, st, cells, a.patch_int,
-                      (int)a.n_patches, a.n_nodes, a.charge);
-            BT_CHECK_LAUNCH();
+        // the window's records: sorted by cell, summed per cell, gathered per node
+        sum_cells<8>(ctx, keys, recs, slots, T.sentinel, cells, a.n_nodes);
+        BT_LAUNCH(ctx, node_gather3, blocks_for(a.n_nodes, 256), 256, 0, st, cells, a.patch_int,
+                  (int)a.n_patches, a.n_nodes, a.charge);
+        if (a.has_j) {
+            sum_cells<24>(ctx, jkeys, jrecs, slots, T.jsentinel, jcells, nb);
+            BT_LAUNCH(ctx, node_gather_current, dim3(blocks_for(nb, 256), 3), 256, 0, st, jcells,
+                      T.nx, T.ny, T.nz, a.current);
         }
-        if (a.has_j) deposit_runs(ctx, jkeys, jvals, jslots, T.jsentinel, a.current);
+        BT_CHECK_LAUNCH();
         BT_CUDA(cudaMemcpyAsync(host, live, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
         BT_CUDA(cudaStreamSynchronize(st));
         if (*host == 0) return;
