@@ -40,6 +40,7 @@ struct Level {
     Buffer c4;      // level 0: cw, ce, cs, cn (4 n)
     Buffer diag;    // level 0: the diagonal (with the reaction)
     Buffer base;    // level 0: the diagonal without the reaction
+    Buffer rdiag;   // the reciprocal of the diagonal (a smoothing update multiplies by it)
     Buffer weight;  // level 0: the control volumes W
     Buffer a9;      // coarse levels: 9 coefficients per node, (dI + 1) * 3 + (dJ + 1)
     Buffer active;  // uint8: free (level 0) or a nonzero row (coarse)
@@ -193,10 +194,13 @@ __global__ void fixed_adjoint(i64 nx, i64 ny, const double *__restrict__ c4,
 }
 
 __global__ void add_diag(i64 n, const double *__restrict__ base, const double *__restrict__ reaction,
-                         const uint8_t *__restrict__ active, double *__restrict__ diag) {
+                         const uint8_t *__restrict__ active, double *__restrict__ diag,
+                         double *__restrict__ rdiag) {
     const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    diag[t] = base[t] + ((reaction && active[t]) ? reaction[t] : 0.0);
+    const double d = base[t] + ((reaction && active[t]) ? reaction[t] : 0.0);
+    diag[t] = d;
+    rdiag[t] = 1.0 / d;
 }
 
 // -- Galerkin coarse operator -----------------------------------------------------------
@@ -240,7 +244,8 @@ constexpr int kGalerkinThreads = 64;
 
 template <bool NINE>
 __global__ void __launch_bounds__(kGalerkinThreads)
-    galerkin(Fine F, double *__restrict__ a9c, uint8_t *__restrict__ active_c) {
+    galerkin(Fine F, double *__restrict__ a9c, double *__restrict__ rdiag_c,
+             uint8_t *__restrict__ active_c) {
     const i64 nc = F.ncx * F.ncy, n = F.nx * F.ny;
     const int t = blockIdx.x * kGalerkinThreads + threadIdx.x;
     if (t >= nc) return;
@@ -305,13 +310,31 @@ __global__ void __launch_bounds__(kGalerkinThreads)
 #pragma unroll
         for (int e = 0; e < 3; ++e)
             a9c[(i64)(3 * d + e) * nc + t] = on ? acc[d][e] : (d == 1 && e == 1 ? 1.0 : 0.0);
+    rdiag_c[t] = on ? 1.0 / acc[1][1] : 1.0;
     active_c[t] = on ? 1 : 0;
 }
 
 // -- smoothing, residual, transfer ---------------------------------------------------------
 
+// A Gauss-Seidel update of a node from its neighbours, on a 5-point row (coefficients west,
+// east, south, north) or a 9-point row (the eight neighbours' in row order).  Two chains of
+// fused multiply-adds and the diagonal's reciprocal: a colour phase is one such update a
+// thread between barriers, so its time is the update's latency -- 17 dependent roundings
+// and an IEEE quotient, some 240 cycles, before; some 56 so.  Every form of the smoothing
+// (a launch a colour, staged tiles, the coarse levels in one launch) takes these updates.
+__device__ __forceinline__ double update5(double b, double cw, double ce, double cs, double cn,
+                                          double xw, double xe, double xs, double xn, double rd) {
+    return (fma(ce, xe, fma(cw, xw, b)) + fma(cn, xn, cs * xs)) * rd;
+}
+__device__ __forceinline__ double update9(double b, const double (&a)[8], const double (&x)[8],
+                                          double rd) {
+    const double p = fma(-a[3], x[3], fma(-a[2], x[2], fma(-a[1], x[1], fma(-a[0], x[0], b))));
+    const double q = fma(a[7], x[7], fma(a[6], x[6], fma(a[5], x[5], a[4] * x[4])));
+    return (p - q) * rd;
+}
+
 __global__ void smooth5(i64 nx, i64 ny, const double *__restrict__ c4,
-                        const double *__restrict__ diag, const uint8_t *__restrict__ active,
+                        const double *__restrict__ rdiag, const uint8_t *__restrict__ active,
                         const double *__restrict__ b, double *__restrict__ x, int colour) {
     const i64 n = nx * ny;
     const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -323,12 +346,9 @@ __global__ void smooth5(i64 nx, i64 ny, const double *__restrict__ c4,
     if (j >= ny) return;
     const i64 f = i * ny + j;
     if (!active[f]) return;
-    double s = b[f];
-    if (i > 0) s += c4[f] * x[f - ny];
-    if (i < nx - 1) s += c4[n + f] * x[f + ny];
-    if (j > 0) s += c4[2 * n + f] * x[f - 1];
-    if (j < ny - 1) s += c4[3 * n + f] * x[f + 1];
-    x[f] = s / diag[f];
+    x[f] = update5(b[f], c4[f], c4[n + f], c4[2 * n + f], c4[3 * n + f], i > 0 ? x[f - ny] : 0.0,
+                   i < nx - 1 ? x[f + ny] : 0.0, j > 0 ? x[f - 1] : 0.0,
+                   j < ny - 1 ? x[f + 1] : 0.0, rdiag[f]);
 }
 
 // How the item functions load the vectors they read (plain loads; a kernel whose blocks
@@ -343,37 +363,26 @@ __host__ __device__ __forceinline__ i64 colour_count(i64 nx, i64 ny, int colour)
     return ((nx - ci + 1) / 2) * ((ny - cj + 1) / 2);
 }
 
-template <class Load>
-__device__ __forceinline__ void smooth9_item(i64 t, i64 nx, i64 ny, const double *__restrict__ a9,
-                                             const uint8_t *__restrict__ active,
-                                             const double *__restrict__ b, double *x, int colour,
-                                             Load load) {
+__global__ void smooth9(i64 nx, i64 ny, const double *__restrict__ a9,
+                        const double *__restrict__ rdiag, const uint8_t *__restrict__ active,
+                        const double *__restrict__ b, double *__restrict__ x, int colour) {
+    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= colour_count(nx, ny, colour)) return;
     const i64 n = nx * ny;
     const int ci = colour >> 1, cj = colour & 1;
     const i64 hy = (ny - cj + 1) / 2;
     const i64 i = 2 * (t / hy) + ci, j = 2 * (t % hy) + cj;
     const i64 f = i * ny + j;
     if (!active[f]) return;
-    double s = load(b + f);
+    double a[8], v[8];
 #pragma unroll
-    for (int di = -1; di <= 1; ++di) {
-#pragma unroll
-        for (int dj = -1; dj <= 1; ++dj) {
-            if (di == 0 && dj == 0) continue;
-            const i64 i2 = i + di, j2 = j + dj;
-            if (i2 < 0 || i2 >= nx || j2 < 0 || j2 >= ny) continue;
-            s -= a9[(i64)((di + 1) * 3 + (dj + 1)) * n + f] * load(x + i2 * ny + j2);
-        }
+    for (int q = 0, k = 0; q < 9; ++q) {
+        if (q == 4) continue;
+        const i64 i2 = i + q / 3 - 1, j2 = j + q % 3 - 1;
+        a[k] = a9[(i64)q * n + f];
+        v[k++] = i2 >= 0 && i2 < nx && j2 >= 0 && j2 < ny ? x[i2 * ny + j2] : 0.0;
     }
-    x[f] = s / a9[4 * n + f];
-}
-
-__global__ void smooth9(i64 nx, i64 ny, const double *__restrict__ a9,
-                        const uint8_t *__restrict__ active, const double *__restrict__ b,
-                        double *__restrict__ x, int colour) {
-    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= colour_count(nx, ny, colour)) return;
-    smooth9_item(t, nx, ny, a9, active, b, x, colour, PlainLoad{});
+    x[f] = update9(b[f], a, v, rdiag[f]);
 }
 
 // -- smoothing staged through shared memory -------------------------------------------------
@@ -429,7 +438,7 @@ __host__ __device__ inline size_t stage_smem(bool nine, int tx, int ty, int halo
 // form).
 template <bool NINE, int R>
 __device__ __forceinline__ void smooth_staged_tile(
-    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ diag,
+    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ rdiag,
     const double *__restrict__ a9, const uint8_t *__restrict__ active,
     const double *__restrict__ b, const double *__restrict__ xin, double *__restrict__ xout,
     int tx, int ty, const Phases &ph, const Fine &F, const double *__restrict__ xc, i64 bx,
@@ -438,7 +447,8 @@ __device__ __forceinline__ void smooth_staged_tile(
     // xc, when not NULL: the coarse correction, prolonged onto x as it is read (the values
     // prolong_add would leave in xin)
     extern __shared__ double sm[];
-    constexpr int Q = NINE ? 9 : 5;  // coefficients per node (5-point: w, e, s, n, diagonal)
+    // coefficients per node, the reciprocal diagonal in the diagonal's place (5-point: last)
+    constexpr int Q = NINE ? 9 : 5;
     constexpr int K = NINE ? 4 : 2;  // colours
     const int halo = stage_halo(ph.count);
     const int wx = tx + 2 * halo, wy = ty + 2 * halo, m = wx * wy, per = m / K, hy = wy / 2;
@@ -472,14 +482,14 @@ __device__ __forceinline__ void smooth_staged_tile(
             if (NINE) {
                 double q9[9];
 #pragma unroll
-                for (int q = 0; q < 9; ++q) q9[q] = a9[(i64)q * n + f];
+                for (int q = 0; q < 9; ++q) q9[q] = q == 4 ? rdiag[f] : a9[(i64)q * n + f];
 #pragma unroll
                 for (int q = 0; q < 9; ++q) coef[q * m + pos] = q9[q];
             } else {
                 double q5[5];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) q5[q] = c4[(i64)q * n + f];
-                q5[4] = diag[f];
+                q5[4] = rdiag[f];
 #pragma unroll
                 for (int q = 0; q < 5; ++q) coef[q * m + pos] = q5[q];
             }
@@ -527,23 +537,18 @@ __device__ __forceinline__ void smooth_staged_tile(
             for (int r = 0; r < R; ++r) {
                 if (ring[k][r] <= kk) continue;  // phase kk is exact from ring kk + 1 inward
                 const int pos = k * per + tid + r * nt, q = xi[k][r];
-                double s = bs[pos];
                 if (NINE) {
-                    s -= coef[pos] * xs[q - wy - 1];
-                    s -= coef[m + pos] * xs[q - wy];
-                    s -= coef[2 * m + pos] * xs[q - wy + 1];
-                    s -= coef[3 * m + pos] * xs[q - 1];
-                    s -= coef[5 * m + pos] * xs[q + 1];
-                    s -= coef[6 * m + pos] * xs[q + wy - 1];
-                    s -= coef[7 * m + pos] * xs[q + wy];
-                    s -= coef[8 * m + pos] * xs[q + wy + 1];
+                    const double c[8] = {coef[pos],         coef[m + pos],     coef[2 * m + pos],
+                                         coef[3 * m + pos], coef[5 * m + pos], coef[6 * m + pos],
+                                         coef[7 * m + pos], coef[8 * m + pos]};
+                    const double v[8] = {xs[q - wy - 1], xs[q - wy],     xs[q - wy + 1], xs[q - 1],
+                                         xs[q + 1],      xs[q + wy - 1], xs[q + wy],     xs[q + wy + 1]};
+                    xs[q] = update9(bs[pos], c, v, coef[4 * m + pos]);
                 } else {
-                    s += coef[pos] * xs[q - wy];
-                    s += coef[m + pos] * xs[q + wy];
-                    s += coef[2 * m + pos] * xs[q - 1];
-                    s += coef[3 * m + pos] * xs[q + 1];
+                    xs[q] = update5(bs[pos], coef[pos], coef[m + pos], coef[2 * m + pos],
+                                    coef[3 * m + pos], xs[q - wy], xs[q + wy], xs[q - 1], xs[q + 1],
+                                    coef[4 * m + pos]);
                 }
-                xs[q] = s / coef[4 * m + pos];
             }
         }
         __syncthreads();
@@ -558,11 +563,11 @@ __device__ __forceinline__ void smooth_staged_tile(
 
 template <bool NINE, int R>
 __global__ void __launch_bounds__(kStageThreads) smooth_staged(
-    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ diag,
+    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ rdiag,
     const double *__restrict__ a9, const uint8_t *__restrict__ active,
     const double *__restrict__ b, const double *__restrict__ xin, double *__restrict__ xout,
     int tx, int ty, Phases ph, Fine F, const double *__restrict__ xc) {
-    smooth_staged_tile<NINE, R>(nx, ny, c4, diag, a9, active, b, xin, xout, tx, ty, ph, F, xc,
+    smooth_staged_tile<NINE, R>(nx, ny, c4, rdiag, a9, active, b, xin, xout, tx, ty, ph, F, xc,
                                 blockIdx.x, blockIdx.y);
 }
 
@@ -982,7 +987,8 @@ struct TailLevel {
 // bytes from the byte block; x, b, r doubles from the dynamic block.
 struct TailPlan {
     int nx, ny, n, ncx, ncy;
-    int x, b, r, a9;         // x: (nx + 2) (ny + 2) with a ring of zeros; b, r: n; a9: 9 n
+    int x, b, r, a9, rd;     // x: (nx + 2) (ny + 2) with a ring of zeros; b, r: n; a9: 9 n; the
+                             // reciprocal diagonal: n
     int wx, wy, rxw, ryw;    // transfer weights to the next level
     int lox, loy, rx0, ry0;  // transfer indices (ints)
     int act;                 // active flags (bytes)
@@ -1006,23 +1012,18 @@ __device__ __forceinline__ void tail_smooth(const TailPlan &P, const double *sm,
     const int ci = colour >> 1, cj = colour & 1;
     const int hx = (nx - ci + 1) >> 1, hy = (ny - cj + 1) >> 1;
     double *x = smd + P.x;
-    const double *b = smd + P.b, *a9 = sm + P.a9;
+    const double *b = smd + P.b, *a9 = sm + P.a9, *rd = sm + P.rd;
     for (int t = tid; t < hx * hy; t += nt) {
         const int ti = t / hy;
         const int i = 2 * ti + ci, j = 2 * (t - ti * hy) + cj;
         const int f = i * ny + j;
         if (!act[f]) continue;
         const int q = (i + 1) * W + j + 1;
-        double s = b[f];
-        s -= a9[f] * x[q - W - 1];
-        s -= a9[n + f] * x[q - W];
-        s -= a9[2 * n + f] * x[q - W + 1];
-        s -= a9[3 * n + f] * x[q - 1];
-        s -= a9[5 * n + f] * x[q + 1];
-        s -= a9[6 * n + f] * x[q + W - 1];
-        s -= a9[7 * n + f] * x[q + W];
-        s -= a9[8 * n + f] * x[q + W + 1];
-        x[q] = s / a9[4 * n + f];
+        const double c[8] = {a9[f],         a9[n + f],     a9[2 * n + f], a9[3 * n + f],
+                             a9[5 * n + f], a9[6 * n + f], a9[7 * n + f], a9[8 * n + f]};
+        const double v[8] = {x[q - W - 1], x[q - W],     x[q - W + 1], x[q - 1],
+                             x[q + 1],     x[q + W - 1], x[q + W],     x[q + W + 1]};
+        x[q] = update9(b[f], c, v, rd[f]);
     }
 }
 
@@ -1213,6 +1214,8 @@ TailLayout tail_layout(const std::vector<Level> &levels, int first) {
             P.ncy = (int)levels[l + 1].ny;
             P.a9 = T.doubles;
             T.doubles += 9 * P.n;
+            P.rd = T.doubles;
+            T.doubles += P.n;
             P.wx = T.doubles;
             T.doubles += P.nx;
             P.wy = T.doubles;
@@ -1698,17 +1701,17 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     Level &L0 = p->levels[0];
     BT_LAUNCH(p->ctx, add_diag, blocks_for(p->n, 256), 256, 0, st, p->n, L0.base.as<double>(p->n), reaction,
                                                     L0.active.as<uint8_t>(p->n),
-                                                    L0.diag.as<double>(p->n));
+                                                    L0.diag.as<double>(p->n), L0.rdiag.as<double>(p->n));
     for (size_t l = 0; l + 1 < p->levels.size(); ++l) {
         Level &L = p->levels[l], &C = p->levels[l + 1];
         Fine F = fine_of(L, C, l == 0);
         const unsigned grid = blocks_for(C.n, kGalerkinThreads);
         if (F.a9)
             BT_LAUNCH(p->ctx, galerkin<true>, grid, kGalerkinThreads, 0, st, F,
-                      C.a9.as<double>(9 * C.n), C.active.as<uint8_t>(C.n));
+                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
         else
             BT_LAUNCH(p->ctx, galerkin<false>, grid, kGalerkinThreads, 0, st, F,
-                      C.a9.as<double>(9 * C.n), C.active.as<uint8_t>(C.n));
+                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
     }
     Level &Lc = p->levels.back();
     if (p->levels.size() == 1)
@@ -1828,6 +1831,7 @@ void refresh_tail_image(bt_poisson *p, bool tables) {
         if (l + 1 == levels) continue;
         const Fine F = fine_of(L, p->levels[l + 1], false);
         copy(d + P.a9, L.a9.as<double>(9 * L.n), sizeof(double) * 9 * L.n);
+        copy(d + P.rd, L.rdiag.as<double>(L.n), sizeof(double) * L.n);
         if (!tables) continue;
         copy(d + P.wx, F.wx, sizeof(double) * P.nx);
         copy(d + P.wy, F.wy, sizeof(double) * P.ny);
@@ -1884,15 +1888,15 @@ void smooth(bt_poisson *p, size_t l, bool pre, const Fine *pf = nullptr,
             const double *add = start == 0 ? xc : nullptr;
             if (five && own <= 2)
                 BT_LAUNCH(p->ctx, (smooth_staged<false, 2>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, L.c4.as<double>(4 * L.n), L.diag.as<double>(L.n),
+                          L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
                           (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add);
             else if (five && own == 3)
                 BT_LAUNCH(p->ctx, (smooth_staged<false, 3>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, L.c4.as<double>(4 * L.n), L.diag.as<double>(L.n),
+                          L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
                           (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add);
             else if (!five && own == 1)
                 BT_LAUNCH(p->ctx, (smooth_staged<true, 1>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, (const double *)nullptr, (const double *)nullptr,
+                          L.ny, (const double *)nullptr, L.rdiag.as<double>(L.n),
                           L.a9.as<double>(9 * L.n), act, b, in, out, tx, ty, ph, F, add);
             else
                 BT_REQUIRE(false, "poisson: staged smoothing tile too large for its block");
@@ -1906,11 +1910,11 @@ void smooth(bt_poisson *p, size_t l, bool pre, const Fine *pf = nullptr,
         if (five) {
             const i64 per = L.nx * ((L.ny + 1) / 2);
             BT_LAUNCH(p->ctx, smooth5, blocks_for(per, T), T, 0, st, L.nx, L.ny,
-                      L.c4.as<double>(4 * L.n), L.diag.as<double>(L.n), act, b, x, c);
+                      L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n), act, b, x, c);
         } else {
             const i64 per = colour_count(L.nx, L.ny, c);
             BT_LAUNCH(p->ctx, smooth9, blocks_for(per, T), T, 0, st, L.nx, L.ny,
-                      L.a9.as<double>(9 * L.n), act, b, x, c);
+                      L.a9.as<double>(9 * L.n), L.rdiag.as<double>(L.n), act, b, x, c);
         }
     }
 }
@@ -2185,6 +2189,7 @@ extern "C" int bt_poisson_create(bt_ctx *ctx, const bt_mesh_desc *m, bt_poisson 
                 L.b.as<double>(L.n);
                 L.r.as<double>(L.n);
                 L.active.as<uint8_t>(L.n);
+                L.rdiag.as<double>(L.n);
                 if (p->levels.size() == 1) {
                     L.c4.as<double>(4 * L.n);
                     L.diag.as<double>(L.n);
@@ -2483,6 +2488,7 @@ struct BatchLevel {
     int cand;
     i64 nx, ny, n;
     const double *c4, *diag, *a9;  // level 0: c4, diag; coarse levels: a9
+    const double *rdiag;
     const uint8_t *active;
     double *x, *x2, *b, *r;
     Fine F;           // to the next level
@@ -2543,7 +2549,7 @@ __global__ void __launch_bounds__(kStageThreads)
     const double *in = from ? L.x2 : L.x;
     double *out = from ? L.x : L.x2;
     const Fine none{};
-    smooth_staged_tile<NINE, R>(L.nx, L.ny, L.c4, L.diag, L.a9, L.active, L.b, in, out, tx, ty,
+    smooth_staged_tile<NINE, R>(L.nx, L.ny, L.c4, L.rdiag, L.a9, L.active, L.b, in, out, tx, ty,
                                 ph, prolong ? L.F : none, prolong ? L.xc : nullptr, bx, by,
                                 zero_in != 0);
 }
@@ -3075,6 +3081,7 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                     } else {
                         e.a9 = L.a9.as<double>(9 * L.n);
                     }
+                    e.rdiag = L.rdiag.as<double>(L.n);
                     e.active = L.active.as<uint8_t>(L.n);
                     e.x = L.x.as<double>(L.n);
                     e.x2 = L.x2.as<double>(L.n);
