@@ -236,11 +236,14 @@ class Context:
         handle = P()
         check(lib().bt_ctx_create(self.device, ctypes.byref(handle)))
         self.handle = handle
+        #: the stream of the last `use_stream` (None: the context's own)
+        self.stream: int | None = None
 
     def use_stream(self, stream: int) -> None:
         """Queue work on ``stream`` (a ``cudaStream_t`` as an int; 0: CUDA's default stream,
         which is torch's default stream)."""
         check(lib().bt_ctx_set_stream(self.handle, P(stream) if stream else None))
+        self.stream = stream
 
     def set_timing(self, on: bool) -> None:
         """Record the launch times of the library's kernels (CUDA events on its stream)."""
@@ -299,17 +302,19 @@ def context(device: int | None = None) -> Context:
     """
     import torch
 
-    if not torch.cuda.is_available():
-        raise RuntimeError("beamtracer_b200 needs a CUDA device")
-    if device is None:
-        device = torch.cuda.current_device()
     contexts = getattr(_local, "contexts", None)
     if contexts is None:
+        if not torch.cuda.is_available():
+            raise RuntimeError("beamtracer_b200 needs a CUDA device")
         contexts = _local.contexts = {}
+    if device is None:
+        device = torch.cuda.current_device()
     ctx = contexts.get(device)
     if ctx is None:
         ctx = contexts[device] = Context(device)
-    ctx.use_stream(torch.cuda.current_stream(device).cuda_stream)
+    stream = torch.cuda.current_stream(device).cuda_stream
+    if stream != ctx.stream:
+        ctx.use_stream(stream)
     return ctx
 
 
@@ -318,15 +323,35 @@ def exported_symbols() -> list[str]:
     return list(SIGNATURES)
 
 
+@functools.cache
+def _tensor_types() -> tuple:
+    """torch's tensor class, its dense layout and the element types of the library's arrays."""
+    import torch
+
+    return (torch.Tensor, torch.strided,
+            frozenset((torch.float64, torch.int64, torch.int32, torch.uint8)))  # fmt: skip
+
+
+def is_tensor(array) -> bool:
+    """A torch CUDA tensor whose address, type and shape may be read from it directly: one
+    that exports ``__cuda_array_interface__`` (which takes some 5 us to build where these
+    take 0.2; a call of the kernel catalogue reads a dozen)."""
+    tensor, strided, dtypes = _tensor_types()
+    return (type(array) is tensor and array.is_cuda and array.dtype in dtypes
+            and array.layout is strided and not array.requires_grad)  # fmt: skip
+
+
 def dptr(array) -> int:
     """The device address of a CUDA array (``__cuda_array_interface__``), 0 for None."""
     if array is None:
         return 0
+    if is_tensor(array):
+        return array.data_ptr() if array.numel() else 0
     return int(array.__cuda_array_interface__["data"][0])
 
 
 def is_device_array(array) -> bool:
-    return hasattr(array, "__cuda_array_interface__")
+    return is_tensor(array) or hasattr(array, "__cuda_array_interface__")
 
 
 def np_ptr(array: np.ndarray | None) -> int:

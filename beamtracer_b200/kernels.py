@@ -38,6 +38,13 @@ _I8 = "<i8"
 
 
 def _check_device(array, typestr: str, name: str) -> None:
+    if _lib.is_tensor(array):
+        kind = "float64" if typestr == _F8 else "int64"
+        if str(array.dtype) != "torch." + kind:
+            raise TypeError(f"{name} must be {kind}, got {array.dtype}")
+        if not array.is_contiguous():
+            raise TypeError(f"{name} must be C-contiguous")
+        return
     iface = array.__cuda_array_interface__
     if iface["typestr"] != typestr:
         kind = "float64" if typestr == _F8 else "int64"
@@ -85,12 +92,16 @@ class _Staging:
 
 
 def _size(array) -> int:
+    if _lib.is_tensor(array):
+        return array.numel()
     if _lib.is_device_array(array):
         return int(np.prod(array.__cuda_array_interface__["shape"]))
     return int(np.asarray(array).size)
 
 
 def _shape(array) -> tuple:
+    if _lib.is_tensor(array):
+        return tuple(array.shape)
     if _lib.is_device_array(array):
         return tuple(array.__cuda_array_interface__["shape"])
     return tuple(np.shape(array))
