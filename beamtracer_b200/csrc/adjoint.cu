@@ -37,78 +37,86 @@ struct Grid {
     const double *fx, *fy;
     int nx, ny;
     double ox, oy, h, rh;
+    double ih;  // 1 / h
 };
 
 __device__ __forceinline__ int clamp_cell(int i, int lo, int hi) { return min(max(i, lo), hi); }
 
-// The field lookup of trace.cu (edge_field_cells, the same expressions) at cell coordinates
-// (sx, sy), with its cells, weights and the derivatives along them.
-struct Lookup {
+// A field evaluation at a stage point, with what its reverse needs: the lookups' cells and
+// weights (of E_x and E_y, trace.cu's edge_field_cells, the same expressions), E_y, the
+// derivatives of the two along the weights, the radius' reciprocal and unit vector.
+struct Stage {
     int ix, jx, iy, jy;
     double ux, wx, uy, wy;
-    double ex, ey;
+    double ey;
     double dex_du, dex_dw, dey_du, dey_dw;
+    double cy, cz, ir;
 };
 
-__device__ __forceinline__ void lookup(const Grid &G, double sx, double sy, Lookup &g) {
-    double s = sx + 0.5;
-    int i = clamp_cell(__double2int_rd(s), 0, G.nx - 1);
-    int j = clamp_cell(__double2int_rd(sy), 0, G.ny - 2);
-    double u = s - (double)i;
-    double w = sy - (double)j;
-    const double *f = G.fx + (i64)i * G.ny + j;
+// q/m E at a point, as trace.cu forms it (the radius and its unit vector in cylindrical
+// geometry).  Num<true>: straight-line roots and quotients (common.cuh), and the cells of
+// s + 1/2 from those of s, a clamped point called odd -- as the trace's own step.
+template <int CYL, class N>
+__device__ __forceinline__ void accel(N &num, const Grid &G, double qm, const double *q, double *a,
+                                      Stage &g) {
+    double qy = q[1];
+    g.cy = g.cz = g.ir = 0.0;
+    if (CYL == 1) {
+        double y;
+        qy = num.root(q[1] * q[1] + q[2] * q[2], y);
+        const bool off_axis = qy > 0.0;
+        const double ir = N::fast ? num.inverse(qy, y) : 1.0 / qy;
+        const double uy = num.over(q[1], qy, ir), uz = num.over(q[2], qy, ir);
+        g.cy = off_axis ? uy : 0.0;
+        g.cz = off_axis ? uz : 0.0;
+        g.ir = off_axis ? ir : 0.0;
+    }
+    const double sx = num.known(q[0] - G.ox, G.h, G.rh), sy = num.known(qy - G.oy, G.h, G.rh);
+    const double hx = sx + 0.5, hy = sy + 0.5;
+    if (N::fast) {
+        const int i = __double2int_rd(sx), j = __double2int_rd(sy);
+        const double fi = (double)i, fj = (double)j;
+        const bool up_i = hx >= fi + 1.0, up_j = hy >= fj + 1.0;
+        g.ix = clamp_cell(i + (up_i ? 1 : 0), 0, G.nx - 1);
+        g.jx = clamp_cell(j, 0, G.ny - 2);
+        g.iy = clamp_cell(i, 0, G.nx - 2);
+        g.jy = clamp_cell(j + (up_j ? 1 : 0), 0, G.ny - 1);
+        num.flag |= g.iy != i || g.jx != j;
+        g.uy = sx - fi;
+        g.wx = sy - fj;
+        g.ux = hx - (up_i ? fi + 1.0 : fi);
+        g.wy = hy - (up_j ? fj + 1.0 : fj);
+    } else {
+        g.ix = clamp_cell(__double2int_rd(hx), 0, G.nx - 1);
+        g.jx = clamp_cell(__double2int_rd(sy), 0, G.ny - 2);
+        g.iy = clamp_cell(__double2int_rd(sx), 0, G.nx - 2);
+        g.jy = clamp_cell(__double2int_rd(hy), 0, G.ny - 1);
+        g.ux = hx - (double)g.ix;
+        g.wx = sy - (double)g.jx;
+        g.uy = sx - (double)g.iy;
+        g.wy = hy - (double)g.jy;
+    }
+    const double *f = G.fx + (i64)g.ix * G.ny + g.jx;
     double f00 = __ldg(f), f01 = __ldg(f + 1), f10 = __ldg(f + G.ny), f11 = __ldg(f + G.ny + 1);
-    double low = f00 + w * (f01 - f00);
-    double high = f10 + w * (f11 - f10);
-    g.ex = low + u * (high - low);
-    g.ix = i;
-    g.jx = j;
-    g.ux = u;
-    g.wx = w;
+    double low = f00 + g.wx * (f01 - f00), high = f10 + g.wx * (f11 - f10);
+    const double ex = low + g.ux * (high - low);
     g.dex_du = high - low;
-    g.dex_dw = (1.0 - u) * (f01 - f00) + u * (f11 - f10);
-    s = sy + 0.5;
-    i = clamp_cell(__double2int_rd(sx), 0, G.nx - 2);
-    j = clamp_cell(__double2int_rd(s), 0, G.ny - 1);
-    u = sx - (double)i;
-    w = s - (double)j;
-    f = G.fy + (i64)i * (G.ny + 1) + j;
+    g.dex_dw = (1.0 - g.ux) * (f01 - f00) + g.ux * (f11 - f10);
+    f = G.fy + (i64)g.iy * (G.ny + 1) + g.jy;
     f00 = __ldg(f);
     f01 = __ldg(f + 1);
     f10 = __ldg(f + G.ny + 1);
     f11 = __ldg(f + G.ny + 2);
-    low = f00 + w * (f01 - f00);
-    high = f10 + w * (f11 - f10);
-    g.ey = low + u * (high - low);
-    g.iy = i;
-    g.jy = j;
-    g.uy = u;
-    g.wy = w;
+    low = f00 + g.wy * (f01 - f00);
+    high = f10 + g.wy * (f11 - f10);
+    g.ey = low + g.uy * (high - low);
     g.dey_du = high - low;
-    g.dey_dw = (1.0 - u) * (f01 - f00) + u * (f11 - f10);
-}
-
-// q/m E at a point, as trace.cu forms it (the radius and its unit vector in cylindrical
-// geometry).
-template <int CYL>
-__device__ __forceinline__ void accel(const Grid &G, double qm, const double *q, double *a) {
-    double qy = q[1], cy = 0.0, cz = 0.0;
+    g.dey_dw = (1.0 - g.uy) * (f01 - f00) + g.uy * (f11 - f10);
+    a[0] = qm * ex;
     if (CYL == 1) {
-        const double r = radius(q[1], q[2]);
-        if (r > 0.0) {
-            cy = q[1] / r;
-            cz = q[2] / r;
-        }
-        qy = r;
-    }
-    Lookup g;
-    lookup(G, div_known(q[0] - G.ox, G.h, G.rh), div_known(qy - G.oy, G.h, G.rh), g);
-    if (CYL == 1) {
-        a[0] = qm * g.ex;
-        a[1] = qm * (g.ey * cy);
-        a[2] = qm * (g.ey * cz);
+        a[1] = qm * (g.ey * g.cy);
+        a[2] = qm * (g.ey * g.cz);
     } else {
-        a[0] = qm * g.ex;
         a[1] = qm * g.ey;
         a[2] = qm * 0.0;
     }
@@ -120,37 +128,53 @@ struct StepTape {
     double a[4][3];        // the stage accelerations
     double q[3][3];        // the stage points of stages 2-4
     double u[3][3];        // the stage velocities of stages 2-4
-    double dt, speed, accn;
+    Stage s[4];            // the stages' field evaluations
+    double dt;
+    double rate;           // the step size's sensitivity: dt_bar rate (v or a1) joins v's or a1's
     int branch;            // the step size from 0: h, 1: h / |v|, 2: sqrt(2 h / |a|)
 };
 
-template <int CYL>
-__device__ __forceinline__ void step_forward(const Grid &G, double qm, double f, const double *x,
+// Num<true> takes the step size the speed sets and checks that the acceleration's is not
+// shorter (trace.cu's `advance`); true where the straight-line step holds.
+template <int CYL, bool FAST>
+__device__ __forceinline__ bool step_forward(const Grid &G, double qm, double f, const double *x,
                                              const double *v, StepTape &T) {
-    accel<CYL>(G, qm, x, T.a[0]);
+    Num<FAST> num;
+    accel<CYL>(num, G, qm, x, T.a[0], T.s[0]);
     const double *a1 = T.a[0];
-    const double speed = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-    const double accn = sqrt(a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2]);
-    double dt = -1.0;
-    int branch = 0;
-    if (speed > 0.0) {
-        dt = G.h / speed;
-        branch = 1;
-    }
-    if (accn > 0.0) {
-        const double d2 = sqrt(2.0 * G.h / accn);
-        if (dt < 0.0 || d2 < dt) {
-            dt = d2;
-            branch = 2;
+    const double v2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+    const double a2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
+    double y;
+    const double speed = num.root(v2, y);
+    double dt = num.over(G.h, speed, num.inverse(speed, y));
+    int branch = 1;
+    if (FAST) {
+        num.flag |= !((a2 * G.h) * G.h < (4.0 - 4e-9) * (v2 * v2)) || !(dt > 0.0);
+    } else {
+        const double accn = sqrt(a2);
+        if (!(speed > 0.0)) {
+            dt = -1.0;
+            branch = 0;
+        }
+        if (accn > 0.0) {
+            const double d2 = sqrt(2.0 * G.h / accn);
+            if (dt < 0.0 || d2 < dt) {
+                dt = d2;
+                branch = 2;
+            }
+        }
+        if (dt < 0.0) {
+            dt = G.h;
+            branch = 0;
         }
     }
-    if (dt < 0.0) {
-        dt = G.h;
-        branch = 0;
-    }
     dt = f * dt;
+    T.dt = dt;
+    T.branch = branch;
+    // (of the step size alone: rounding apart, y^2 is 1 / v^2)
+    T.rate = FAST ? -dt * (y * y) : branch == 1 ? -dt / v2 : branch == 2 ? -0.5 * dt / a2 : 0.0;
     const double hdt = 0.5 * dt;
-    const double dt6 = div_known(dt, 6.0, 1.0 / 6.0);
+    const double dt6 = num.known(dt, 6.0, 1.0 / 6.0);
     double sx[3], sv[3], kx[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -160,7 +184,7 @@ __device__ __forceinline__ void step_forward(const Grid &G, double qm, double f,
         kx[c] = v[c] + hdt * a1[c];
         T.u[0][c] = kx[c];
     }
-    accel<CYL>(G, qm, T.q[0], T.a[1]);
+    accel<CYL>(num, G, qm, T.q[0], T.a[1], T.s[1]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + 2.0 * kx[c];
@@ -169,7 +193,7 @@ __device__ __forceinline__ void step_forward(const Grid &G, double qm, double f,
         kx[c] = v[c] + hdt * T.a[1][c];
         T.u[1][c] = kx[c];
     }
-    accel<CYL>(G, qm, T.q[1], T.a[2]);
+    accel<CYL>(num, G, qm, T.q[1], T.a[2], T.s[2]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + 2.0 * kx[c];
@@ -178,7 +202,7 @@ __device__ __forceinline__ void step_forward(const Grid &G, double qm, double f,
         kx[c] = v[c] + dt * T.a[2][c];
         T.u[2][c] = kx[c];
     }
-    accel<CYL>(G, qm, T.q[2], T.a[3]);
+    accel<CYL>(num, G, qm, T.q[2], T.a[3], T.s[3]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + kx[c];
@@ -186,10 +210,31 @@ __device__ __forceinline__ void step_forward(const Grid &G, double qm, double f,
         T.y[c] = x[c] + dt6 * sx[c];
         T.w[c] = v[c] + dt6 * sv[c];
     }
-    T.dt = dt;
-    T.speed = speed;
-    T.accn = accn;
-    T.branch = branch;
+    // (an intermediate value out of range leaves the end state out of range)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) num.in_range(T.y[c] - 1.0);
+    num.in_range(T.w[0] * T.w[0] + T.w[1] * T.w[1] + T.w[2] * T.w[2]);
+    return !num.odd();
+}
+
+template <int CYL>
+__device__ __noinline__ void step_plain(const Grid &G, double qm, double f, const double *x,
+                                        const double *v, StepTape &T) {
+    step_forward<CYL, false>(G, qm, f, x, v, T);
+}
+
+// The straight-line step, or the IEEE one where it may not hold.
+template <int CYL>
+__device__ __forceinline__ void step(const Grid &G, double qm, double f, const double *x,
+                                     const double *v, StepTape &T) {
+    if (!step_forward<CYL, true>(G, qm, f, x, v, T) || G.rh == 0.0) {
+        // copies, so that only this branch keeps anything in memory
+        const Grid g = G;
+        const double x0[3] = {x[0], x[1], x[2]}, v0[3] = {v[0], v[1], v[2]};
+        StepTape plain;
+        step_plain<CYL>(g, qm, f, x0, v0, plain);
+        T = plain;
+    }
 }
 
 // The edge fields' adjoint, added run by run: consecutive lookups in one cell add into
@@ -216,7 +261,7 @@ struct Scatter {
         kx = ky = -1;
     }
 
-    __device__ __forceinline__ void add(const Lookup &g, double exb, double eyb) {
+    __device__ __forceinline__ void add(const Stage &g, double exb, double eyb) {
         const i64 key_x = (i64)g.ix * ny + g.jx;
         if (key_x != kx) {
             if (kx >= 0) {
@@ -250,38 +295,31 @@ struct Scatter {
     }
 };
 
-// The reverse of accel: ab the adjoint of q/m E at q; adds the point's adjoint to qb and
-// the field's to the scatter.
+// The reverse of accel: ab the adjoint of q/m E at q; adds the point's adjoint to qb, and
+// exb, eyb get the field's.  Everything but the adjoint is the stage's: no lookup, root or
+// quotient stands in the chain of a step's four.
 template <int CYL>
 __device__ __forceinline__ void accel_reverse(const Grid &G, double qm, const double *q,
-                                              const double *ab, double *qb, Scatter &sc) {
-    double qy = q[1], cy = 0.0, cz = 0.0, r = 0.0;
+                                              const Stage &g, const double *ab, double *qb,
+                                              double &exb, double &eyb) {
+    const double ih = G.ih;
+    exb = qm * ab[0];
+    eyb = CYL == 1 ? qm * fma(ab[1], g.cy, ab[2] * g.cz) : qm * ab[1];
+    const double sxb = fma(exb, g.dex_du, eyb * g.dey_du);  // along x (u of either lookup)
+    const double syb = fma(exb, g.dex_dw, eyb * g.dey_dw);  // along y / r
+    qb[0] = fma(sxb, ih, qb[0]);
     if (CYL == 1) {
-        r = radius(q[1], q[2]);
-        if (r > 0.0) {
-            cy = q[1] / r;
-            cz = q[2] / r;
-        }
-        qy = r;
-    }
-    Lookup g;
-    lookup(G, div_known(q[0] - G.ox, G.h, G.rh), div_known(qy - G.oy, G.h, G.rh), g);
-    const double exb = qm * ab[0];
-    const double eyb = CYL == 1 ? qm * (ab[1] * cy + ab[2] * cz) : qm * ab[1];
-    sc.add(g, exb, eyb);
-    const double sxb = exb * g.dex_du + eyb * g.dey_du;  // along x (u of either lookup)
-    const double syb = exb * g.dex_dw + eyb * g.dey_dw;  // along y / r
-    qb[0] += sxb / G.h;
-    if (CYL == 1) {
-        if (r > 0.0) {
-            const double cyb = qm * g.ey * ab[1], czb = qm * g.ey * ab[2];
-            const double rb = syb / G.h - (cyb * q[1] + czb * q[2]) / (r * r);
-            qb[1] += cyb / r + rb * (q[1] / r);
-            qb[2] += czb / r + rb * (q[2] / r);
-        }
+        // the unit vector (cy, cz) = (q1, q2) / r
+        const double k = qm * g.ey * g.ir;
+        const double cyb = k * ab[1], czb = k * ab[2];
+        const double rb = syb * ih - fma(cyb, g.cy, czb * g.cz);
+        const bool off_axis = g.ir > 0.0;
+        qb[1] += off_axis ? fma(rb, g.cy, cyb) : 0.0;
+        qb[2] += off_axis ? fma(rb, g.cz, czb) : 0.0;
     } else {
-        qb[1] += syb / G.h;
+        qb[1] = fma(syb, ih, qb[1]);
     }
+    (void)q;
 }
 
 struct Adj {
@@ -311,7 +349,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_checkpoints(Adj A, double
                 c[(3 + q) * n] = v[q];
             }
         }
-        step_forward<CYL>(A.G, qm, a.step_fraction, x, v, T);
+        step<CYL>(A.G, qm, a.step_fraction, x, v, T);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             x[q] = T.y[q];
@@ -327,6 +365,39 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_checkpoints(Adj A, double
     }
 }
 
+// A deposit's place: its radius and the reciprocal, the cell the forward found, the weights
+// in it and the radial weight's derivative.
+struct Midpoint {
+    int i, j;
+    double r, ir, u, w, dw_dr;
+};
+
+template <int CYL, class N>
+__device__ __forceinline__ Midpoint midpoint(N &num, const Grid &G, const double *m) {
+    Midpoint M;
+    M.r = m[1];
+    M.ir = 0.0;
+    if (CYL == 1) {
+        double y;
+        M.r = num.root(m[1] * m[1] + m[2] * m[2], y);
+        M.ir = N::fast ? y : 1.0 / M.r;  // used off the axis only
+    }
+    M.i = __double2int_rd(num.known(m[0] - G.ox, G.h, G.rh));
+    M.j = __double2int_rd(num.known(M.r - G.oy, G.h, G.rh));
+    M.u = num.known(m[0] - (G.ox + G.h * (double)M.i), G.h, G.rh);
+    const double low = G.oy + G.h * (double)M.j;
+    if (CYL == 1) {
+        const double high = low + G.h;
+        const double rs = num.div(1.0, high * high - low * low);
+        M.w = (M.r * M.r - low * low) * rs;
+        M.dw_dr = 2.0 * M.r * rs;
+    } else {
+        M.w = num.known(M.r - low, G.h, G.rh);
+        M.dw_dr = G.ih;
+    }
+    return M;
+}
+
 // The reverse of one step from (x, v): xb, vb hold the adjoint of its end state on entry
 // and of its start state on return.  charge_seed: the node charges' adjoint; the hits'
 // adjoints of this step's crossings come through hit_seed at the counters cnt.
@@ -338,7 +409,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
     const bt_adjoint_args &a = A.a;
     const Grid &G = A.G;
     StepTape T;
-    step_forward<CYL>(G, qm, a.step_fraction, x, v, T);
+    step<CYL>(G, qm, a.step_fraction, x, v, T);
     const double dt = T.dt, hdt = 0.5 * T.dt;
     double yb[3] = {xb[0], xb[1], xb[2]}, wb[3] = {vb[0], vb[1], vb[2]};
     double xs[3] = {0, 0, 0}, vs[3] = {0, 0, 0};  // the start state's adjoint so far
@@ -349,22 +420,19 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         double m[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) m[c] = 0.5 * (x[c] + T.y[c]) + dt * (v[c] - T.w[c]) * 0.125;
-        const double mr = CYL == 1 ? radius(m[1], m[2]) : m[1];
-        int i = __double2int_rd(div_known(m[0] - G.ox, G.h, G.rh));
-        int j = __double2int_rd(div_known(mr - G.oy, G.h, G.rh));
-        double u = div_known(m[0] - (G.ox + G.h * (double)i), G.h, G.rh);
-        double w, dw_dr;
-        if (CYL == 1) {
-            const double low = G.oy + G.h * (double)j;
-            const double high = low + G.h;
-            const double span = high * high - low * low;
-            w = (mr * mr - low * low) / span;
-            dw_dr = 2.0 * mr / span;
-        } else {
-            w = div_known(mr - (G.oy + G.h * (double)j), G.h, G.rh);
-            dw_dr = 1.0 / G.h;
+        Midpoint M;
+        {
+            Num<true> num;
+            M = midpoint<CYL>(num, G, m);
+            if (num.odd() || G.rh == 0.0) {
+                Num<false> plain;
+                M = midpoint<CYL>(plain, G, m);
+            }
         }
-        double du_dx = 1.0 / G.h;
+        int i = M.i, j = M.j;
+        double u = M.u, w = M.w, dw_dr = M.dw_dr;
+        const double mr = M.r;
+        double du_dx = G.ih;
         if (i < 0) {
             u = 0.0;
             i = 0;
@@ -396,8 +464,8 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         const double mrb = wbar * dw_dr;
         if (CYL == 1) {
             if (mr > 0.0) {
-                mb[1] = mrb * (m[1] / mr);
-                mb[2] = mrb * (m[2] / mr);
+                mb[1] = mrb * (m[1] * M.ir);
+                mb[2] = mrb * (m[2] * M.ir);
             }
         } else {
             mb[1] = mrb;
@@ -473,8 +541,9 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
     }
     double hdtb = 0.0;
     double qb[3] = {0, 0, 0};
+    double exb[4], eyb[4];
     // a4 = acc(q4), q4 = x + dt u3, u4 = v + dt a3
-    accel_reverse<CYL>(G, qm, T.q[2], a4b, qb, sc);
+    accel_reverse<CYL>(G, qm, T.q[2], T.s[3], a4b, qb, exb[3], eyb[3]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u4b[c];
@@ -486,7 +555,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         qb[c] = 0.0;
     }
     // a3 = acc(q3), q3 = x + hdt u2, u3 = v + hdt a2
-    accel_reverse<CYL>(G, qm, T.q[1], a3b, qb, sc);
+    accel_reverse<CYL>(G, qm, T.q[1], T.s[2], a3b, qb, exb[2], eyb[2]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u3b[c];
@@ -498,7 +567,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         qb[c] = 0.0;
     }
     // a2 = acc(q2), q2 = x + hdt v, u2 = v + hdt a1
-    accel_reverse<CYL>(G, qm, T.q[0], a2b, qb, sc);
+    accel_reverse<CYL>(G, qm, T.q[0], T.s[1], a2b, qb, exb[1], eyb[1]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u2b[c];
@@ -512,16 +581,16 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
     dtb += 0.5 * hdtb;
     // the step size: f h / |v| or f sqrt(2 h / |a1|)
     if (T.branch == 1) {
-        const double coef = -dt / (T.speed * T.speed);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) vs[c] += dtb * coef * v[c];
+        for (int c = 0; c < 3; ++c) vs[c] += dtb * T.rate * v[c];
     } else if (T.branch == 2) {
-        const double coef = -0.5 * dt / (T.accn * T.accn);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) a1b[c] += dtb * coef * T.a[0][c];
+        for (int c = 0; c < 3; ++c) a1b[c] += dtb * T.rate * T.a[0][c];
     }
     // a1 = acc(x)
-    accel_reverse<CYL>(G, qm, x, a1b, xs, sc);
+    accel_reverse<CYL>(G, qm, x, T.s[0], a1b, xs, exb[0], eyb[0]);
+#pragma unroll
+    for (int k4 = 3; k4 >= 0; --k4) sc.add(T.s[k4], exb[k4], eyb[k4]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         xb[c] = xs[c];
@@ -529,7 +598,12 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
     }
 }
 
-// The sweep: every trajectory's steps reversed, from its last to its first.
+// The sweep: every trajectory's steps reversed, from its last to its first.  Bound by the
+// latency of one warp a scheduler (250 warps of a design's 8,000 rings): a step's forward
+// evaluations keep what their reverse needs, so that the reverse itself is products and sums,
+// and run straight-line as the trace's.  8,000 rings of 790 steps at 401 x 101: 3.4 ms with
+// the replay (9.7 with a second lookup, IEEE roots and quotients in the reverse, up to 17 for
+// a beam whose lengths differ); the checkpoints 1.1 ms (2.1).
 template <int CYL>
 __global__ void __launch_bounds__(kAdjThreads) adjoint_sweep(Adj A, const double *__restrict__ charge_seed,
                                                              const double *__restrict__ hit_seed,
@@ -537,42 +611,58 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_sweep(Adj A, const double
                                                              double *__restrict__ fy_bar) {
     const i64 k = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     const bt_adjoint_args &a = A.a;
-    if (k >= a.n) return;
     const i64 n = a.n;
-    const i64 steps = a.steps[k];
-    if (steps <= 0) return;
+    const bool mine = k < n;
+    const i64 steps = mine ? a.steps[k] : 0;
     int cnt[kMaxPlanes];
-    for (int p = 0; p < (int)a.n_planes; ++p) cnt[p] = (int)a.counts[k * a.n_planes + p];
-    const double qm = a.qm[k], dq = a.dq[k];
+    for (int p = 0; p < (int)a.n_planes; ++p) cnt[p] = mine ? (int)a.counts[k * a.n_planes + p] : 0;
+    const double qm = mine ? a.qm[k] : 0.0, dq = mine ? a.dq[k] : 0.0;
     Scatter sc{fx_bar, fy_bar, A.G.ny};
     double xb[3] = {0, 0, 0}, vb[3] = {0, 0, 0};
     double tape[kSegment][6];  // the segment's start states
-    const i64 segments = (steps + kSegment - 1) / kSegment;
-    for (i64 seg = segments - 1; seg >= 0; --seg) {
-        const double *c = a.checkpoints + seg * 6 * n + k;
-        double x[3] = {c[0], c[n], c[2 * n]};
-        double v[3] = {c[3 * n], c[4 * n], c[5 * n]};
-        const int len = (int)min((i64)kSegment, steps - seg * kSegment);
-        StepTape T;
-        for (int s = 0; s < len; ++s) {
+    // The warp walks its longest trajectory's segments together, step by step: lanes whose
+    // trajectories have ended wait.  Trip counts of their own let a lane with one segment
+    // more replay while its neighbours reversed, each part of the loop run for each: twice
+    // the instructions for beams whose step counts straddle a multiple of 64.
+    const int segments = (int)((steps + kSegment - 1) / kSegment);
+    for (int seg = (int)__reduce_max_sync(0xffffffffu, (unsigned)segments) - 1; seg >= 0; --seg) {
+        const int len = (int)max((i64)0, min((i64)kSegment, steps - (i64)seg * kSegment));
+        const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)len);
+        double x[3], v[3];
+        if (len > 0) {
+            const double *c = a.checkpoints + (i64)seg * 6 * n + k;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                tape[s][q] = x[q];
-                tape[s][3 + q] = v[q];
-            }
-            if (s + 1 < len) {
-                step_forward<CYL>(A.G, qm, a.step_fraction, x, v, T);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    x[q] = T.y[q];
-                    v[q] = T.w[q];
-                }
+                x[q] = c[q * n];
+                v[q] = c[(3 + q) * n];
             }
         }
-        for (int s = len - 1; s >= 0; --s) {
-            const double xs[3] = {tape[s][0], tape[s][1], tape[s][2]};
-            const double vs[3] = {tape[s][3], tape[s][4], tape[s][5]};
-            step_reverse<CYL>(A, k, qm, dq, xs, vs, xb, vb, charge_seed, hit_seed, cnt, sc);
+        for (int s = 0; s < longest; ++s) {
+            if (s < len) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    tape[s][q] = x[q];
+                    tape[s][3 + q] = v[q];
+                }
+                if (s + 1 < len) {
+                    StepTape T;
+                    step<CYL>(A.G, qm, a.step_fraction, x, v, T);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        x[q] = T.y[q];
+                        v[q] = T.w[q];
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        for (int s = longest - 1; s >= 0; --s) {
+            if (s < len) {
+                const double xs[3] = {tape[s][0], tape[s][1], tape[s][2]};
+                const double vs[3] = {tape[s][3], tape[s][4], tape[s][5]};
+                step_reverse<CYL>(A, k, qm, dq, xs, vs, xb, vb, charge_seed, hit_seed, cnt, sc);
+            }
+            __syncwarp();
         }
     }
     sc.flush();
@@ -582,7 +672,7 @@ Adj adj_of(const bt_adjoint_args *a) {
     Adj A{};
     A.a = *a;
     A.G = Grid{a->fx, a->fy, (int)a->nx, (int)a->ny, a->origin_x, a->origin_y, a->h,
-               known_reciprocal(a->h)};
+               known_reciprocal(a->h), 1.0 / a->h};
     return A;
 }
 
