@@ -405,6 +405,14 @@ struct Phases {
     int colour[kMaxPhases];
 };
 
+// Where a V-cycle reads its right-hand side and leaves its result: held on the device, so
+// that one captured graph serves every vector (a Krylov step sets them to its basis vector
+// and its image) without a copy in and out of the level's own.
+struct CycleIo {
+    const double *b;
+    double *z;
+};
+
 // The halo of `count` phases: rounded up to even, so the tile's origin has even (i, j)
 // and a node's colour follows from its place in the tile.
 __host__ __device__ inline int stage_halo(int count) { return (count + 1) & ~1; }
@@ -565,10 +573,13 @@ template <bool NINE, int R>
 __global__ void __launch_bounds__(kStageThreads) smooth_staged(
     i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ rdiag,
     const double *__restrict__ a9, const uint8_t *__restrict__ active,
-    const double *__restrict__ b, const double *__restrict__ xin, double *__restrict__ xout,
-    int tx, int ty, Phases ph, Fine F, const double *__restrict__ xc) {
+    const double *b, const double *__restrict__ xin, double *xout, int tx, int ty, Phases ph, Fine F,
+    const double *__restrict__ xc, const CycleIo *__restrict__ io, bool first, bool last) {
+    // io: the finest level's smoothing, which starts the cycle from zero and ends it in z
+    if (io) b = io->b;
+    if (io && last) xout = io->z;
     smooth_staged_tile<NINE, R>(nx, ny, c4, rdiag, a9, active, b, xin, xout, tx, ty, ph, F, xc,
-                                blockIdx.x, blockIdx.y);
+                                blockIdx.x, blockIdx.y, first);
 }
 
 // y = A x (level 0, 5-point) on active rows, 0 elsewhere; with b: r = b - A x.  Node f of
@@ -597,10 +608,11 @@ __device__ __forceinline__ double apply5_item(i64 f, i64 nx, i64 ny, const doubl
 
 __global__ void apply5(i64 nx, i64 ny, const double *__restrict__ c4,
                        const double *__restrict__ diag, const uint8_t *__restrict__ active,
-                       const double *__restrict__ x, const double *__restrict__ b,
-                       double *__restrict__ y) {
+                       const double *__restrict__ x, const double *b, double *__restrict__ y,
+                       const CycleIo *__restrict__ io) {
     const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nx * ny) return;
+    if (io) b = io->b;
     apply5_item(f, nx, ny, c4, diag, active, x, b, y);
 }
 
@@ -938,9 +950,13 @@ __global__ void __launch_bounds__(kInvertThreads) coarsest_invert(
 // x = inv b on the active rows, 0 on held ones (the inverse's held rows are unit rows up to
 // the rounding that pivoting mixes into them; a correction never moves a held node).
 __global__ void coarsest_apply(int n, const double *__restrict__ inv, const uint8_t *__restrict__ active,
-                               const double *__restrict__ b, double *__restrict__ x) {
+                               const double *b, double *x, const CycleIo *__restrict__ io) {
     const int r = threadIdx.x;
     if (r >= n) return;
+    if (io) {
+        b = io->b;
+        x = io->z;
+    }
     double s = 0.0;
     for (int c = 0; c < n; ++c) s += inv[r * n + c] * b[c];
     x[r] = active[r] ? s : 0.0;
@@ -1246,56 +1262,25 @@ TailLayout tail_layout(const std::vector<Level> &levels, int first) {
     return T;
 }
 
-// -- dot products: partial sums per block, the last block adds them in block order --------
+// -- sums over a vector: partial sums per block, the last block adds them in block order ----
 
-constexpr int kDotMax = 32;      // at most this many vectors against one
-constexpr int kDotBlocks = 296;  // two per SM
-constexpr int kDotThreads = 256;
+constexpr int kDotMax = 32;       // at most this many vectors against one
+constexpr int kDotBlocks = 148;   // one per SM, of at least an element a thread
+constexpr int kDotThreads = 512;
 
-// What a dot pass does: the sums out[q] = <V_q, w> (kPlain), or first w -= sum_q h[q] V_q
-// (classical Gram-Schmidt's orthogonalisation, written back to w) and then the sums
-// <V_q, w> (kOrthDots) or <w, w> (kOrthNorm) of the new w, q < m.  Every thread adds its
-// grid-stride elements in order, the warps and blocks are added in a fixed order, and the
-// block that finishes last (a ticket counter, reset by it) adds the blocks' partials in
-// block order: the same bits on every run, in one launch.
-enum DotMode { kPlain = 0, kOrthDots = 1, kOrthNorm = 2 };
+int dot_blocks(i64 n) { return (int)std::min<i64>(kDotBlocks, (n + kDotThreads - 1) / kDotThreads); }
 
-template <int MQ, int MODE>
-__global__ void __launch_bounds__(kDotThreads) dot_pass(
-    const double *__restrict__ V, const double *__restrict__ h, double *w, i64 n, int m,
-    double *__restrict__ partial, unsigned *__restrict__ ticket, double *__restrict__ out) {
-    constexpr int NACC = MODE == kOrthNorm ? 1 : MQ;
-    __shared__ double warp_part[kDotThreads / 32][NACC];
+// out[q] = the sum of every thread's acc[q], q < sums <= NACC: the threads of a warp, the warps
+// of a block and the blocks are added in a fixed order, the blocks' partials by the block
+// that finishes last (a ticket counter, reset by it): the same bits on every run, in one
+// launch.  True in the last block, whose threads may then read `out` (after its barrier).
+template <int NACC>
+__device__ __forceinline__ bool grid_sums(const double (&acc)[NACC], int sums,
+                                          double *__restrict__ partial,
+                                          unsigned *__restrict__ ticket, double *out) {
+    constexpr int kWarps = kDotThreads / 32;
+    __shared__ double warp_part[kWarps][NACC];
     __shared__ bool is_last;
-    const int sums = MODE == kOrthNorm ? 1 : m;
-    double acc[NACC];
-#pragma unroll
-    for (int q = 0; q < NACC; ++q) acc[q] = 0.0;
-    for (i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x; f < n;
-         f += (i64)gridDim.x * blockDim.x) {
-        double s = w[f];
-        if (MODE == kPlain) {
-#pragma unroll
-            for (int q = 0; q < MQ; ++q)
-                if (q < m) acc[q] += V[(i64)q * n + f] * s;
-        } else {
-            double vq[MQ];
-#pragma unroll
-            for (int q = 0; q < MQ; ++q)
-                if (q < m) {
-                    vq[q] = V[(i64)q * n + f];
-                    s -= h[q] * vq[q];
-                }
-            w[f] = s;
-            if (MODE == kOrthDots) {
-#pragma unroll
-                for (int q = 0; q < MQ; ++q)
-                    if (q < m) acc[q] += vq[q] * s;
-            } else {
-                acc[0] += s * s;
-            }
-        }
-    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < NACC; ++q) {
@@ -1307,21 +1292,20 @@ __global__ void __launch_bounds__(kDotThreads) dot_pass(
     __syncthreads();
     if (threadIdx.x < sums) {
         double v = 0.0;
-        for (int wi = 0; wi < kDotThreads / 32; ++wi) v += warp_part[wi][threadIdx.x];
+#pragma unroll
+        for (int wi = 0; wi < kWarps; ++wi) v += warp_part[wi][threadIdx.x];
         partial[(i64)blockIdx.x * kDotMax + threadIdx.x] = v;
     }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
-    if (!is_last) return;
+    if (!is_last) return false;
     __threadfence();
-    // the last block: warp w adds the blocks' partials of q = w, w + 8, ... (lanes stride
-    // the blocks, then a fixed tree)
-    // the blocks' partials are read together, then added in block order
+    // a warp a sum: its lanes read the blocks' partials together, then add them
     constexpr int kPer = (kDotBlocks + 31) / 32;
     const int blocks = (int)gridDim.x;
-    for (int q = warp; q < sums; q += kDotThreads / 32) {
+    for (int q = warp; q < sums; q += kWarps) {
         double part[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
@@ -1336,6 +1320,8 @@ __global__ void __launch_bounds__(kDotThreads) dot_pass(
         if (lane == 0) out[q] = v;
     }
     if (threadIdx.x == 0) *ticket = 0u;
+    __syncthreads();
+    return true;
 }
 
 // -- vector kernels of GMRES and Newton ----------------------------------------------------
@@ -1351,39 +1337,61 @@ struct Arnoldi {
     double resid[kDotMax + 1];  // |g[j]| after step j
 };
 
-__global__ void arnoldi_begin(Arnoldi *__restrict__ a, double *__restrict__ g, int m,
-                              double beta, double tol) {
-    if (threadIdx.x != 0) return;
+__global__ void set_cycle(CycleIo *__restrict__ io, const double *b, double *z) {
+    io->b = b;
+    io->z = z;
+}
+
+__global__ void cycle_begin(const CycleIo *__restrict__ io, i64 n, double *__restrict__ b,
+                            double *__restrict__ x) {
+    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= n) return;
+    b[f] = io->b[f];
+    x[f] = 0.0;
+}
+
+__global__ void cycle_end(const CycleIo *__restrict__ io, i64 n, const double *__restrict__ x) {
+    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < n) io->z[f] = x[f];
+}
+
+// A cycle begins: V_0 = r / beta, the state empty, the V-cycle's vectors the first.
+__global__ void arnoldi_begin(Arnoldi *__restrict__ a, double *__restrict__ g, int m, double beta,
+                              double tol, const double *__restrict__ r, i64 n,
+                              double *__restrict__ V, double *__restrict__ Z,
+                              CycleIo *__restrict__ io) {
+    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < n) V[f] = (1.0 / beta) * r[f];
+    if (f != 0) return;
     a->j = 0;
     a->done = 0;
     a->tol = tol;
     a->resid[0] = beta;
     g[0] = beta;
     for (int q = 1; q <= m; ++q) g[q] = 0.0;
+    io->b = V;
+    io->z = Z;
 }
 
 // Step j: the new Hessenberg column from the two Gram-Schmidt passes' coefficients h1, h2
 // and the new vector's squared norm, rotated by the earlier rotations; the new rotation and
-// g, whose last entry is the residual norm up to its sign.
-__global__ void arnoldi_step(Arnoldi *__restrict__ a, double *__restrict__ H,
-                             double *__restrict__ cs, double *__restrict__ sn,
-                             double *__restrict__ g, const double *__restrict__ h1,
-                             const double *__restrict__ h2, const double *__restrict__ norm2,
-                             int j, int m) {
+// g, whose last entry is the residual norm up to its sign.  A block's first warp.
+__device__ __forceinline__ void arnoldi_step(Arnoldi *__restrict__ a, double *__restrict__ H,
+                                             double *__restrict__ cs, double *__restrict__ sn,
+                                             double *__restrict__ g, const double *__restrict__ h1,
+                                             const double *__restrict__ h2, const double *norm2,
+                                             int j, int m) {
     // the warp reads the column's coefficients and the rotations together; one thread then
     // rotates the column in shared memory and writes it out
     __shared__ double col[kDotMax + 2], c[kDotMax], sv[kDotMax];
-    __shared__ int skip;
     const int t = threadIdx.x;
-    if (t == 0) skip = a->done || a->j != j;
-    __syncthreads();
-    if (skip) return;
-    for (int q = t; q <= j; q += blockDim.x) col[q] = h1[q] + h2[q];
-    for (int q = t; q < j; q += blockDim.x) {
+    if (t >= 32 || a->done || a->j != j) return;
+    for (int q = t; q <= j; q += 32) col[q] = h1[q] + h2[q];
+    for (int q = t; q < j; q += 32) {
         c[q] = cs[q];
         sv[q] = sn[q];
     }
-    __syncthreads();
+    __syncwarp();
     if (t != 0) return;
     const double hn = sqrt(norm2[0]);
     col[j + 1] = hn;
@@ -1409,6 +1417,108 @@ __global__ void arnoldi_step(Arnoldi *__restrict__ a, double *__restrict__ H,
     if (fabs(g[j + 1]) <= a->tol || hn == 0.0) a->done = 1;
 }
 
+// The rows of the finest operator, for the kernels that apply it as they go.
+struct Rows5 {
+    i64 nx, ny;
+    const double *c4, *diag;
+    const uint8_t *active;
+};
+
+__device__ __forceinline__ double apply_row(const Rows5 &A, i64 f, const double *__restrict__ x) {
+    if (!A.active[f]) return 0.0;
+    const i64 n = A.nx * A.ny;
+    const int ny = (int)A.ny, i = (int)((unsigned)f / (unsigned)ny), j = (int)f - i * ny;
+    double s = A.diag[f] * x[f];
+    if (i > 0) s -= A.c4[f] * x[f - ny];
+    if (i < (int)A.nx - 1) s -= A.c4[n + f] * x[f + ny];
+    if (j > 0) s -= A.c4[2 * n + f] * x[f - 1];
+    if (j < ny - 1) s -= A.c4[3 * n + f] * x[f + 1];
+    return s;
+}
+
+// A Krylov step's three passes over the new vector w and the basis V (m = j + 1 rows):
+// kApply: w = A z and h1[q] = <V_q, w>; kOrthDots: w -= sum_q h1[q] V_q (classical
+// Gram-Schmidt) and h2[q] = <V_q, w>; kOrthNorm: w -= sum_q h2[q] V_q, its squared norm, and in
+// the last block the step's Hessenberg column and rotation (arnoldi_step).  Three launches and
+// the scaling of the next basis vector, where the product, three passes, the scaling, the
+// column and the V-cycle's copies in and out took nine: KRYLOV_US.
+enum PassMode { kApply = 0, kOrthDots = 1, kOrthNorm = 2 };
+
+struct ArnoldiState {
+    Arnoldi *a;
+    double *H, *cs, *sn, *g, *h1, *h2, *hn;
+    int j, m;  // the step and the cycle's length
+};
+
+template <int MQ, int MODE>
+__global__ void __launch_bounds__(kDotThreads) krylov_pass(
+    Rows5 A, const double *__restrict__ V, const double *__restrict__ z, double *w, i64 n, int m,
+    ArnoldiState S, double *__restrict__ partial, unsigned *__restrict__ ticket) {
+    constexpr int NACC = MODE == kOrthNorm ? 1 : MQ;
+    double acc[NACC];
+#pragma unroll
+    for (int q = 0; q < NACC; ++q) acc[q] = 0.0;
+    const double *h = MODE == kOrthNorm ? S.h2 : S.h1;
+    for (i64 f = (i64)blockIdx.x * kDotThreads + threadIdx.x; f < n;
+         f += (i64)gridDim.x * kDotThreads) {
+        double vq[MQ];
+#pragma unroll
+        for (int q = 0; q < MQ; ++q)
+            if (q < m) vq[q] = V[(i64)q * n + f];
+        double s;
+        if (MODE == kApply) {
+            s = apply_row(A, f, z);
+        } else {
+            s = w[f];
+#pragma unroll
+            for (int q = 0; q < MQ; ++q)
+                if (q < m) s -= h[q] * vq[q];
+        }
+        w[f] = s;
+        if (MODE == kOrthNorm) {
+            acc[0] += s * s;
+        } else {
+#pragma unroll
+            for (int q = 0; q < MQ; ++q)
+                if (q < m) acc[q] += vq[q] * s;
+        }
+    }
+    double *out = MODE == kApply ? S.h1 : (MODE == kOrthDots ? S.h2 : S.hn);
+    const bool last = grid_sums(acc, MODE == kOrthNorm ? 1 : m, partial, ticket, out);
+    if (MODE == kOrthNorm && last)
+        arnoldi_step(S.a, S.H, S.cs, S.sn, S.g, S.h1, S.h2, S.hn, S.j, S.m);
+}
+
+// out[0] = |u|^2, out[1] = |r|^2 of r = u - A x (r also written)
+__global__ void __launch_bounds__(kDotThreads) residual_norms(Rows5 A, const double *__restrict__ u,
+                                                              const double *__restrict__ x, i64 n,
+                                                              double *__restrict__ r,
+                                                              double *__restrict__ partial,
+                                                              unsigned *__restrict__ ticket,
+                                                              double *__restrict__ out) {
+    double acc[2] = {0.0, 0.0};
+    for (i64 f = (i64)blockIdx.x * kDotThreads + threadIdx.x; f < n;
+         f += (i64)gridDim.x * kDotThreads) {
+        const double b = u[f], v = A.active[f] ? b - apply_row(A, f, x) : 0.0;
+        r[f] = v;
+        acc[0] += b * b;
+        acc[1] += v * v;
+    }
+    grid_sums(acc, 2, partial, ticket, out);
+}
+
+// out[0] = |v|^2
+__global__ void __launch_bounds__(kDotThreads) vector_norm(const double *__restrict__ v, i64 n,
+                                                           double *__restrict__ partial,
+                                                           unsigned *__restrict__ ticket,
+                                                           double *__restrict__ out) {
+    double acc[1] = {0.0};
+    for (i64 f = (i64)blockIdx.x * kDotThreads + threadIdx.x; f < n;
+         f += (i64)gridDim.x * kDotThreads)
+        acc[0] += v[f] * v[f];
+    grid_sums(acc, 1, partial, ticket, out);
+}
+
 // y = H^-1 g on the leading j x j upper triangle (j the steps taken)
 __global__ void arnoldi_solve(const Arnoldi *__restrict__ a, const double *__restrict__ H,
                               const double *__restrict__ g, double *__restrict__ y, int m) {
@@ -1421,18 +1531,18 @@ __global__ void arnoldi_solve(const Arnoldi *__restrict__ a, const double *__res
     }
 }
 
-// v = w / sqrt(norm2[0]) (zero for a zero norm: GMRES stops there)
+// V_{j+1} = w / sqrt(norm2[0]) (zero for a zero norm: GMRES stops there), the next V-cycle's
+// vectors with it.
 __global__ void scale_by_norm(const double *__restrict__ w, const double *__restrict__ norm2, i64 n,
-                              double *__restrict__ v) {
+                              double *__restrict__ v, double *z, CycleIo *__restrict__ io) {
     const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f == 0) {
+        io->b = v;
+        io->z = z;
+    }
     if (f >= n) return;
     const double s = norm2[0];
     v[f] = s > 0.0 ? w[f] / sqrt(s) : 0.0;
-}
-
-__global__ void scale_into(const double *__restrict__ w, double a, i64 n, double *__restrict__ v) {
-    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f < n) v[f] = a * w[f];
 }
 
 // x += sum_q y[q] Z[q], q below the cycle's steps
@@ -1454,8 +1564,8 @@ __device__ __forceinline__ double max_nan(double m, double v) {
 // x += d and *out = max |d| (NaN if any entry is NaN): Newton's update and its size in one
 // pass over the vectors.  Every block leaves its maximum, the block that finishes last (a
 // ticket counter, reset by it) takes theirs; a maximum does not depend on the order.  One
-// block alone took 307 us for 525,825 nodes; the grid's 296 blocks 9 us with the
-// addition.
+// block alone took 307 us for 525,825 nodes; a grid of a block a multiprocessor 9 us
+// with the addition.
 __global__ void __launch_bounds__(kDotThreads) add_max(const double *__restrict__ d, i64 n,
                                                        double *__restrict__ x,
                                                        double *__restrict__ partial,
@@ -1545,12 +1655,6 @@ __global__ void add_into(const double *__restrict__ d, i64 n, double *__restrict
     if (f < n) x[f] += d[f];
 }
 
-// w = r - w
-__global__ void subtract_from(const double *__restrict__ r, i64 n, double *__restrict__ w) {
-    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f < n) w[f] = r[f] - w[f];
-}
-
 void build_axis(Axis &A, i64 n) {
     A.n = n;
     A.coarsened = n > 3;
@@ -1626,6 +1730,7 @@ struct bt_poisson {
     bt::Buffer dot_ticket;   // the dot passes' finishing-block counter (zero between passes)
     bool ticket_ready = false;
     bt::Buffer arnoldi;      // the device Arnoldi state of GMRES (bt::Arnoldi, H, rotations)
+    bt::Buffer cycle_io;     // the V-cycle's vectors (bt::CycleIo)
     // the V-cycle from a zero guess on level 0's b into its x, captured once as a graph
     cudaGraph_t vgraph = nullptr;
     cudaGraphExec_t vexec = nullptr;
@@ -1886,18 +1991,21 @@ void smooth(bt_poisson *p, size_t l, bool pre, const Fine *pf = nullptr,
             double *in = L.cur, *out = L.cur == x ? L.x2.as<double>(L.n) : x;
             const Fine F = start == 0 && xc ? *pf : Fine{};
             const double *add = start == 0 ? xc : nullptr;
+            const CycleIo *io = five ? p->cycle_io.as<CycleIo>(1) : nullptr;
+            const bool first = five && pre && start == 0;
+            const bool last = five && !pre && start + ph.count == order.size();
             if (five && own <= 2)
                 BT_LAUNCH(p->ctx, (smooth_staged<false, 2>), tiles, kStageThreads, smem, st, L.nx,
                           L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
-                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add);
+                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add, io, first, last);
             else if (five && own == 3)
                 BT_LAUNCH(p->ctx, (smooth_staged<false, 3>), tiles, kStageThreads, smem, st, L.nx,
                           L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
-                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add);
+                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add, io, first, last);
             else if (!five && own == 1)
                 BT_LAUNCH(p->ctx, (smooth_staged<true, 1>), tiles, kStageThreads, smem, st, L.nx,
                           L.ny, (const double *)nullptr, L.rdiag.as<double>(L.n),
-                          L.a9.as<double>(9 * L.n), act, b, in, out, tx, ty, ph, F, add);
+                          L.a9.as<double>(9 * L.n), act, b, in, out, tx, ty, ph, F, add, io, first, last);
             else
                 BT_REQUIRE(false, "poisson: staged smoothing tile too large for its block");
             L.cur = out;
@@ -1919,9 +2027,9 @@ void smooth(bt_poisson *p, size_t l, bool pre, const Fine *pf = nullptr,
     }
 }
 
-// x = V-cycle(b) on level l (x starts at zero on entry for l > 0; level 0's x given).  The
-// staged smoother moves a level's x between its two buffers; the cycle leaves it in the
-// first.
+// x = V-cycle(b) on level l (x starts at zero on entry for l > 0; level 0 takes b from, and
+// leaves x in, the vectors the solver's CycleIo names).  The staged smoother moves a level's
+// x between its two buffers; the cycle leaves it in the first.
 void vcycle(bt_poisson *p, size_t l) {
     cudaStream_t st = p->ctx->stream;
     Level &L = p->levels[l];
@@ -1938,17 +2046,21 @@ void vcycle(bt_poisson *p, size_t l) {
     }
     if (l + 1 == p->levels.size()) {
         BT_LAUNCH(p->ctx, coarsest_apply, 1, kCoarsest, 0, st, (int)L.n, p->inv.as<double>(L.n * L.n),
-                  L.active.as<uint8_t>(L.n), L.b.as<double>(L.n), L.x.as<double>(L.n));
+                  L.active.as<uint8_t>(L.n), L.b.as<double>(L.n), L.x.as<double>(L.n),
+                  l == 0 ? p->cycle_io.as<CycleIo>(1) : nullptr);
         return;
     }
     Level &C = p->levels[l + 1];
     double *b = L.b.as<double>(L.n), *r = L.r.as<double>(L.n);
     const uint8_t *act = L.active.as<uint8_t>(L.n);
     L.cur = L.x.as<double>(L.n);
+    const CycleIo *io = l == 0 ? p->cycle_io.as<CycleIo>(1) : nullptr;
+    if (io && !p->staged)
+        BT_LAUNCH(p->ctx, cycle_begin, blocks_for(L.n, T), T, 0, st, io, L.n, b, L.cur);
     smooth(p, l, true);
     if (l == 0)
         BT_LAUNCH(p->ctx, apply5, blocks_for(L.n, T), T, 0, st, L.nx, L.ny, L.c4.as<double>(4 * L.n),
-                  L.diag.as<double>(L.n), act, L.cur, b, r);
+                  L.diag.as<double>(L.n), act, L.cur, b, r, io);
     else
         BT_LAUNCH(p->ctx, residual9, blocks_for(L.n, T), T, 0, st, L.nx, L.ny,
                   L.a9.as<double>(9 * L.n), act, L.cur, b, r);
@@ -1957,6 +2069,11 @@ void vcycle(bt_poisson *p, size_t l) {
                                                           C.x.as<double>(C.n));
     vcycle(p, l + 1);
     smooth(p, l, false, &F, C.x.as<double>(C.n));
+    if (io) {
+        if (!p->staged) BT_LAUNCH(p->ctx, cycle_end, blocks_for(L.n, T), T, 0, st, io, L.n, L.cur);
+        BT_CHECK_LAUNCH();
+        return;
+    }
     if (L.cur != L.x.as<double>(L.n))
         BT_CUDA(cudaMemcpyAsync(L.x.as<double>(L.n), L.cur, sizeof(double) * L.n,
                                 cudaMemcpyDeviceToDevice, st));
@@ -1964,7 +2081,7 @@ void vcycle(bt_poisson *p, size_t l) {
     BT_CHECK_LAUNCH();
 }
 
-// Capture the V-cycle (level 0's x zeroed, then the cycle on its b) as a graph: every
+// Capture the V-cycle (from the vector CycleIo::b to CycleIo::z) as a graph: every other
 // buffer it touches keeps its address for the solver's life, so one capture serves every
 // solve and every Newton Jacobian (whose coefficients change in place).
 void capture_vcycle(bt_poisson *p) {
@@ -1972,12 +2089,11 @@ void capture_vcycle(bt_poisson *p) {
     // graph then runs on whichever stream the context queues on
     cudaStream_t st = p->ctx->own_stream;
     cudaStream_t queue = p->ctx->stream;
-    Level &L = p->levels[0];
+    p->cycle_io.as<CycleIo>(1);  // (allocated before the capture)
     const i64 before = p->ctx->launch_count;
     p->ctx->stream = st;
     BT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     try {
-        BT_CUDA(cudaMemsetAsync(L.x.as<double>(L.n), 0, sizeof(double) * L.n, st));
         vcycle(p, 0);
     } catch (...) {
         cudaGraph_t broken = nullptr;
@@ -1993,34 +2109,32 @@ void capture_vcycle(bt_poisson *p) {
     p->ctx->launch_count = before;  // counted when the graph runs
 }
 
-// z = M v: one V-cycle from zero
-void precondition(bt_poisson *p, const double *v, double *z) {
-    Level &L = p->levels[0];
-    cudaStream_t st = p->ctx->stream;
+// One V-cycle from zero, from CycleIo::b to CycleIo::z.
+void run_cycle(bt_poisson *p) {
     if (!p->vexec) capture_vcycle(p);
-    BT_CUDA(cudaMemcpyAsync(L.b.as<double>(L.n), v, sizeof(double) * L.n, cudaMemcpyDeviceToDevice, st));
     {
         Timed timed(p->ctx, "vcycle");
-        BT_CUDA(cudaGraphLaunch(p->vexec, st));
+        BT_CUDA(cudaGraphLaunch(p->vexec, p->ctx->stream));
     }
     p->ctx->launch_count += p->vgraph_kernels;
-    BT_CUDA(cudaMemcpyAsync(z, L.x.as<double>(L.n), sizeof(double) * L.n, cudaMemcpyDeviceToDevice, st));
 }
 
-void apply(bt_poisson *p, const double *x, double *y) {
-    Level &L = p->levels[0];
-    BT_LAUNCH(p->ctx, apply5, blocks_for(L.n, 256), 256, 0, p->ctx->stream, L.nx, L.ny, L.c4.as<double>(4 * L.n), L.diag.as<double>(L.n),
-        L.active.as<uint8_t>(L.n), x, nullptr, y);
+// z = M v: one V-cycle from zero
+void precondition(bt_poisson *p, const double *v, double *z) {
+    BT_LAUNCH(p->ctx, set_cycle, 1, 1, 0, p->ctx->stream, p->cycle_io.as<CycleIo>(1), v, z);
+    run_cycle(p);
 }
 
-double read_scalar(bt_poisson *p, const double *dev) {
+// `count` device doubles, read after the queued work.
+const double *read_scalars(bt_poisson *p, const double *dev, int count) {
     double *host = static_cast<double *>(p->ctx->host.get(sizeof(double) * 64));
-    BT_CUDA(cudaMemcpyAsync(host, dev, sizeof(double), cudaMemcpyDeviceToHost, p->ctx->stream));
+    BT_CUDA(cudaMemcpyAsync(host, dev, sizeof(double) * count, cudaMemcpyDeviceToHost, p->ctx->stream));
     BT_CUDA(cudaStreamSynchronize(p->ctx->stream));
-    return host[0];
+    return host;
 }
 
-// The finishing-block counter of the passes over vectors (zero between them).
+// The finishing-block counter of the passes over vectors (zero between them) and the blocks'
+// partial sums.
 unsigned *dot_ticket(bt_poisson *p) {
     unsigned *ticket = p->dot_ticket.as<unsigned>(1);
     if (!p->ticket_ready) {
@@ -2029,37 +2143,58 @@ unsigned *dot_ticket(bt_poisson *p) {
     }
     return ticket;
 }
-
-// One dot pass (dot_pass) over the n-vectors w and V's rows q < m; out gets its sums.
-template <int MODE>
-void dot_launch(bt_poisson *p, const double *V, const double *h, double *w, int m, double *out) {
-    double *partial = p->dot_partial.as<double>((size_t)kDotBlocks * kDotMax);
-    unsigned *ticket = dot_ticket(p);
-    cudaStream_t st = p->ctx->stream;
-    BT_REQUIRE(m >= 1 && m <= kDotMax, "poisson: a dot pass takes 1 to 32 vectors");
-#define BT_DOT(MQ)                                                                              \
-    BT_LAUNCH(p->ctx, (dot_pass<MQ, MODE>), kDotBlocks, kDotThreads, 0, st, V, h, w, p->n, m,  \
-              partial, ticket, out)
-    if (m <= 1)
-        BT_DOT(1);
-    else if (m <= 8)
-        BT_DOT(8);
-    else if (m <= 16)
-        BT_DOT(16);
-    else
-        BT_DOT(32);
-#undef BT_DOT
+double *dot_partial(bt_poisson *p) {
+    return p->dot_partial.as<double>((size_t)kDotBlocks * kDotMax);
 }
 
-// out[q] = <V_q, w> for q < m (V's rows of n values), deterministic
-void dots(bt_poisson *p, const double *V, const double *w, int m, double *out) {
-    dot_launch<kPlain>(p, V, nullptr, const_cast<double *>(w), m, out);
+Rows5 rows_of(bt_poisson *p) {
+    Level &L = p->levels[0];
+    return Rows5{L.nx, L.ny, L.c4.as<double>(4 * L.n), L.diag.as<double>(L.n),
+                 L.active.as<uint8_t>(L.n)};
+}
+
+// One pass of Krylov step S.j.
+template <int MODE>
+void krylov_launch(bt_poisson *p, const ArnoldiState &S, const double *V, const double *z, double *w) {
+    const int m = S.j + 1;
+    cudaStream_t st = p->ctx->stream;
+    double *partial = dot_partial(p);
+    unsigned *ticket = dot_ticket(p);
+    const Rows5 A = rows_of(p);
+    BT_REQUIRE(m >= 1 && m <= kDotMax, "poisson: a Krylov pass takes 1 to 32 vectors");
+#define BT_PASS(MQ)                                                                             \
+    BT_LAUNCH(p->ctx, (krylov_pass<MQ, MODE>), dot_blocks(p->n), kDotThreads, 0, st, A, V, z, w,  \
+              p->n, m, S, partial, ticket)
+    if (m <= 4)
+        BT_PASS(4);
+    else if (m <= 8)
+        BT_PASS(8);
+    else if (m <= 16)
+        BT_PASS(16);
+    else
+        BT_PASS(32);
+#undef BT_PASS
+}
+
+// r = u - A x and the norms of u and r (one launch and one read)
+struct Norms {
+    double u, r;
+};
+Norms residual(bt_poisson *p, const double *u, const double *x, double *r) {
+    double *s = p->scalars.as<double>(16);
+    BT_LAUNCH(p->ctx, residual_norms, dot_blocks(p->n), kDotThreads, 0, p->ctx->stream, rows_of(p), u,
+              x, p->n, r, dot_partial(p), dot_ticket(p), s);
+    BT_CHECK_LAUNCH();
+    const double *host = read_scalars(p, s, 2);
+    return {std::sqrt(host[0]), std::sqrt(host[1])};
 }
 
 double norm2(bt_poisson *p, const double *v) {
-    double *s = p->scalars.as<double>(8);
-    dots(p, v, v, 1, s);
-    return std::sqrt(read_scalar(p, s));
+    double *s = p->scalars.as<double>(16);
+    BT_LAUNCH(p->ctx, vector_norm, dot_blocks(p->n), kDotThreads, 0, p->ctx->stream, v, p->n,
+              dot_partial(p), dot_ticket(p), s);
+    BT_CHECK_LAUNCH();
+    return std::sqrt(read_scalars(p, s, 1)[0]);
 }
 
 // The steps a cycle still needs by the rate of its last (up to three) steps, one fewer so
@@ -2076,68 +2211,72 @@ int steps_to_queue(const Arnoldi &a) {
     return std::max(1, (int)std::ceil(left) - 1);
 }
 
-// Solve A d = r0 for d (d zero on entry) by restarted right-preconditioned GMRES until
-// ||r0 - A d|| <= abs_tol or max_iter V-cycles; returns the V-cycles run and the final
+// Solve A d = r0 for d (d zero on entry, beta = |r0|) by restarted right-preconditioned GMRES
+// until ||r0 - A d|| <= abs_tol or max_iter V-cycles; returns the V-cycles run and the final
 // residual norm.  The Arnoldi process runs on the device (Gram-Schmidt twice, the Givens
 // rotations in arnoldi_step); the host queues steps in batches sized by the residual's
 // rate and reads the state between them, and the cycle's solution is the same as if it
 // read it after every step.
-int gmres(bt_poisson *p, const double *r0, double *d, double abs_tol, int max_iter,
+int gmres(bt_poisson *p, const double *r0, double *d, double beta, double abs_tol, int max_iter,
           double *final_norm) {
     const i64 n = p->n;
     const int m = p->restart;  // at most kDotMax - 1: a basis of m + 1 vectors
     cudaStream_t st = p->ctx->stream;
     double *V = p->V.as<double>((size_t)(m + 1) * n);
-    double *Z = p->Z.as<double>((size_t)m * n);
+    double *Z = p->Z.as<double>((size_t)(m + 1) * n);
     double *w = p->work.as<double>(n);
+    CycleIo *io = p->cycle_io.as<CycleIo>(1);
     // the device state: Arnoldi, H, cs, sn, g, y and the passes' coefficients and norm
     const size_t head = (sizeof(Arnoldi) + 255) / 256 * 256;
     const size_t doubles = (size_t)(m + 1) * m + 3 * m + 1 + 2 * (m + 2) + 1;
     unsigned char *state = p->arnoldi.as<unsigned char>(head + sizeof(double) * doubles);
-    Arnoldi *a = reinterpret_cast<Arnoldi *>(state);
-    double *H = reinterpret_cast<double *>(state + head);
-    double *cs = H + (size_t)(m + 1) * m, *sn = cs + m, *g = sn + m, *y = g + m + 1;
-    double *h1 = y + m, *h2 = h1 + (m + 2), *hn = h2 + (m + 2);
-    Arnoldi *host = static_cast<Arnoldi *>(p->ctx->host.get(sizeof(Arnoldi)));
+    ArnoldiState S{};
+    S.a = reinterpret_cast<Arnoldi *>(state);
+    S.H = reinterpret_cast<double *>(state + head);
+    S.cs = S.H + (size_t)(m + 1) * m;
+    S.sn = S.cs + m;
+    S.g = S.sn + m;
+    double *y = S.g + m + 1;
+    S.h1 = y + m;
+    S.h2 = S.h1 + (m + 2);
+    S.hn = S.h2 + (m + 2);
+    S.m = m;
+    Arnoldi *host = static_cast<Arnoldi *>(p->ctx->host.get(std::max(sizeof(Arnoldi), 64 * sizeof(double))));
     int total = 0;
-    BT_CUDA(cudaMemcpyAsync(w, r0, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-    double beta = norm2(p, w);
+    const double *r = r0;
     double previous = INFINITY;
     // stop at the tolerance, or where a whole restart cycle no longer halves the true
     // residual: the rounding floor of the residual itself
     while (beta > abs_tol && total < max_iter && beta < 0.5 * previous) {
         previous = beta;
         if (!std::isfinite(beta)) throw Error{BT_ERR_NOCONV, "field solve: the residual is not finite"};
-        BT_LAUNCH(p->ctx, scale_into, blocks_for(n, 256), 256, 0, st, w, 1.0 / beta, n, V);
-        BT_LAUNCH(p->ctx, arnoldi_begin, 1, 32, 0, st, a, g, m, beta, abs_tol);
+        BT_LAUNCH(p->ctx, arnoldi_begin, blocks_for(n, 256), 256, 0, st, S.a, S.g, m, beta, abs_tol, r,
+                  n, V, Z, io);
         int j = 0, batch = 2;
         for (;;) {
             const int count = std::min(batch, std::min(m - j, max_iter - total));
             for (int b = 0; b < count; ++b, ++j, ++total) {
-                double *v = V + (i64)j * n, *z = Z + (i64)j * n;
-                precondition(p, v, z);
-                apply(p, z, w);
-                dot_launch<kPlain>(p, V, nullptr, w, j + 1, h1);
-                dot_launch<kOrthDots>(p, V, h1, w, j + 1, h2);
-                dot_launch<kOrthNorm>(p, V, h2, w, j + 1, hn);
-                BT_LAUNCH(p->ctx, scale_by_norm, blocks_for(n, 256), 256, 0, st, w, hn, n,
-                          V + (i64)(j + 1) * n);
-                BT_LAUNCH(p->ctx, arnoldi_step, 1, 32, 0, st, a, H, cs, sn, g, h1, h2, hn, j, m);
+                S.j = j;
+                const double *z = Z + (i64)j * n;
+                run_cycle(p);
+                krylov_launch<kApply>(p, S, V, z, w);
+                krylov_launch<kOrthDots>(p, S, V, z, w);
+                krylov_launch<kOrthNorm>(p, S, V, z, w);
+                BT_LAUNCH(p->ctx, scale_by_norm, blocks_for(n, 256), 256, 0, st, w, S.hn, n,
+                          V + (i64)(j + 1) * n, Z + (i64)(j + 1) * n, io);
             }
             BT_CHECK_LAUNCH();
-            BT_CUDA(cudaMemcpyAsync(host, a, sizeof(Arnoldi), cudaMemcpyDeviceToHost, st));
+            BT_CUDA(cudaMemcpyAsync(host, S.a, sizeof(Arnoldi), cudaMemcpyDeviceToHost, st));
             BT_CUDA(cudaStreamSynchronize(st));
             if (host->done || j >= m || total >= max_iter) break;
             batch = steps_to_queue(*host);
         }
         // d += Z y, y = H^-1 g over the steps taken
-        BT_LAUNCH(p->ctx, arnoldi_solve, 1, 32, 0, st, a, H, g, y, m);
-        BT_LAUNCH(p->ctx, combine, blocks_for(n, 256), 256, 0, st, Z, y, a, n, d);
+        BT_LAUNCH(p->ctx, arnoldi_solve, 1, 32, 0, st, S.a, S.H, S.g, y, m);
+        BT_LAUNCH(p->ctx, combine, blocks_for(n, 256), 256, 0, st, Z, y, S.a, n, d);
         // the true residual r0 - A d
-        apply(p, d, w);
-        BT_LAUNCH(p->ctx, subtract_from, blocks_for(n, 256), 256, 0, st, r0, n, w);
-        BT_CHECK_LAUNCH();
-        beta = norm2(p, w);
+        beta = residual(p, r0, d, w).r;
+        r = w;
     }
     if (final_norm) *final_norm = beta;
     return total;
@@ -2280,14 +2419,12 @@ extern "C" int bt_poisson_solve(bt_poisson *p, double *phi, const double *rho, d
         if (!(amplitude > 0.0)) {
             if (!p->built || p->reaction_on) bt::build_hierarchy(p, nullptr);
             // r0 = b - A phi; the tolerance is relative to the larger of |b| and |r0|
-            BT_LAUNCH(p->ctx, bt::apply5, bt::blocks_for(n, 256), 256, 0, st, p->nx, p->ny, L0.c4.as<double>(4 * n), L0.diag.as<double>(n),
-                L0.active.as<uint8_t>(n), phi, b, r0);
-            BT_CHECK_LAUNCH();
-            const double scale = std::max(bt::norm2(p, b), bt::norm2(p, r0));
+            const bt::Norms norms = bt::residual(p, b, phi, r0);
+            const double scale = std::max(norms.u, norms.r);
             BT_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
             double left = 0.0;
             const double goal = tol * (scale > 0.0 ? scale : 1.0);
-            total_cycles = bt::gmres(p, r0, d, goal, max_cycles, &left);
+            total_cycles = bt::gmres(p, r0, d, norms.r, goal, max_cycles, &left);
             BT_LAUNCH(p->ctx, bt::add_into, bt::blocks_for(n, 256), 256, 0, st, d, n, phi);
             if (p->transposed)
                 BT_LAUNCH(p->ctx, bt::scale_by_weight, bt::blocks_for(n, 256), 256, 0, st, n, weight, active, 0, phi);
@@ -2309,13 +2446,12 @@ extern "C" int bt_poisson_solve(bt_poisson *p, double *phi, const double *rho, d
                 const double fnorm = bt::norm2(p, r0);
                 BT_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
                 double left = 0.0;
-                total_cycles += bt::gmres(p, r0, d, tol * (fnorm > 0.0 ? fnorm : 1.0),
+                total_cycles += bt::gmres(p, r0, d, fnorm, tol * (fnorm > 0.0 ? fnorm : 1.0),
                                           max_cycles, &left);
-                BT_LAUNCH(p->ctx, bt::add_max, bt::kDotBlocks, bt::kDotThreads, 0, st, d, n, phi,
-                          p->dot_partial.as<double>((size_t)bt::kDotBlocks * bt::kDotMax),
-                          bt::dot_ticket(p), scal + 8);
+                BT_LAUNCH(p->ctx, bt::add_max, bt::dot_blocks(n), bt::kDotThreads, 0, st, d, n, phi,
+                          bt::dot_partial(p), bt::dot_ticket(p), scal + 8);
                 BT_CHECK_LAUNCH();
-                const double change = bt::read_scalar(p, scal + 8);
+                const double change = bt::read_scalars(p, scal + 8, 1)[0];
                 if (!std::isfinite(change))
                     throw bt::Error{BT_ERR_NOCONV, "field solve: Newton's update is not finite"};
                 if (change < newton_tol) {
@@ -2391,14 +2527,12 @@ extern "C" int bt_poisson_solve_reaction(bt_poisson *p, double *phi, const doubl
         BT_LAUNCH(p->ctx, bt::prepare, bt::blocks_for(n, 256), 256, 0, st, n, rho, p->src.as<double>(n),
                   L0.active.as<uint8_t>(n), p->value_eff.as<double>(n), b, phi);
         bt::build_hierarchy(p, reaction);
-        BT_LAUNCH(p->ctx, bt::apply5, bt::blocks_for(n, 256), 256, 0, st, p->nx, p->ny, L0.c4.as<double>(4 * n),
-                  L0.diag.as<double>(n), L0.active.as<uint8_t>(n), phi, b, r0);
-        BT_CHECK_LAUNCH();
-        const double scale = std::max(bt::norm2(p, b), bt::norm2(p, r0));
+        const bt::Norms norms = bt::residual(p, b, phi, r0);
+        const double scale = std::max(norms.u, norms.r);
         BT_CUDA(cudaMemsetAsync(d, 0, sizeof(double) * n, st));
         double left = 0.0;
         const double goal = tol * (scale > 0.0 ? scale : 1.0);
-        const int total = bt::gmres(p, r0, d, goal, 4000, &left);
+        const int total = bt::gmres(p, r0, d, norms.r, goal, 4000, &left);
         BT_LAUNCH(p->ctx, bt::add_into, bt::blocks_for(n, 256), 256, 0, st, d, n, phi);
         BT_CHECK_LAUNCH();
         if (!(left <= 1e4 * goal))
