@@ -569,17 +569,151 @@ __device__ __forceinline__ void smooth_staged_tile(
     }
 }
 
-template <bool NINE, int R>
-__global__ void __launch_bounds__(kStageThreads) smooth_staged(
-    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ rdiag,
-    const double *__restrict__ a9, const uint8_t *__restrict__ active,
-    const double *b, const double *__restrict__ xin, double *xout, int tx, int ty, Phases ph, Fine F,
-    const double *__restrict__ xc, const CycleIo *__restrict__ io, bool first, bool last) {
-    // io: the finest level's smoothing, which starts the cycle from zero and ends it in z
-    if (io) b = io->b;
-    if (io && last) xout = io->z;
-    smooth_staged_tile<NINE, R>(nx, ny, c4, rdiag, a9, active, b, xin, xout, tx, ty, ph, F, xc,
-                                blockIdx.x, blockIdx.y, first);
+// -- the same smoothing with the coefficients in registers ----------------------------------
+//
+// A tile whose sizes the compiler knows.  A thread has one node of each colour (R of them),
+// whose coefficients, right-hand side and reciprocal diagonal it loads straight into
+// registers -- all of its nodes' loads in flight together, no index that is not a shift --
+// and only x goes through shared memory: a phase is eight (four) shared loads, the update and
+// a store.  Staging the coefficients through shared memory at sizes known at run time spent
+// 1,760 instructions a warp, most on indices, for some 300 of arithmetic: 10.3 us a launch of
+// a 9-point level, whatever its size, against REG9_US, and 12.0 for the finest level of
+// 801 x 201 against REG5_US.
+
+// One side of a fine-coarse pair's prolongation, as build_axis lays it out: the lower coarse
+// neighbour of fine node k and its weight.
+struct CoarseAxis {
+    int n, nc;
+};
+__device__ __forceinline__ int coarse_low(const CoarseAxis &A, int k, double &w) {
+    if (A.n <= 3) {
+        w = 1.0;
+        return k;
+    }
+    const int I = min(k >> 1, A.nc - 2);
+    const int c1 = min(2 * I + 2, A.n - 1);
+    w = c1 - 2 * I == 2 ? 0.5 * (double)(c1 - k) : (double)(c1 - k);
+    return I;
+}
+
+// A level as the smoother reads it.
+struct SmoothView {
+    int nx, ny;
+    i64 n;
+    const double *c4, *rdiag, *a9, *b, *xin, *xc;  // xin NULL: from zero; xc NULL: no correction
+    const uint8_t *active;
+    double *xout;
+    CoarseAxis ax, ay;  // to the next level (with xc)
+};
+
+template <bool NINE, int TX, int TY, int COUNT>
+struct Tile {
+    static constexpr int halo = (COUNT + 1) & ~1;
+    static constexpr int wx = TX + 2 * halo, wy = TY + 2 * halo;
+    static constexpr int colours = NINE ? 4 : 2;
+    static constexpr int per = wx * wy / colours;       // nodes of a colour
+    static constexpr int r = (per + 511) / 512;         // a thread's nodes of a colour
+    static constexpr int threads = ((per + r - 1) / r + 31) / 32 * 32;
+};
+
+template <bool NINE, int TX, int TY, int COUNT, bool REVERSE>
+__device__ __forceinline__ void smooth_tile(const SmoothView &L, int bx, int by) {
+    using S = Tile<NINE, TX, TY, COUNT>;
+    constexpr int K = S::colours, R = S::r, WX = S::wx, WY = S::wy, HY = WY / 2;
+    constexpr int Q = NINE ? 8 : 4;
+    __shared__ double xs[WX * WY];
+    const int tid = threadIdx.x, i0 = bx * TX - S::halo, j0 = by * TY - S::halo;
+    double coef[K][R][Q], b[K][R], rd[K][R], x[K][R];
+    int at[K][R], ring[K][R];  // the node's place in xs; its distance from the tile's edge, or
+                               // -1 where it is never updated (held, or outside the mesh)
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int u = tid + r * S::threads;
+            const int ua = u / HY, uc = u - ua * HY;
+            const int a = NINE ? 2 * ua + (k >> 1) : ua;
+            const int c = NINE ? 2 * uc + (k & 1) : 2 * uc + ((a + k) & 1);
+            const int i = i0 + a, j = j0 + c;
+            const bool in = u < S::per && i >= 0 && i < L.nx && j >= 0 && j < L.ny;
+            const int f = in ? i * L.ny + j : 0;
+            at[k][r] = a * WY + c;
+            const uint8_t act = L.active[f];
+            ring[k][r] = in && act ? min(min(a, WX - 1 - a), min(c, WY - 1 - c)) : -1;
+            if (NINE) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) coef[k][r][q] = L.a9[(q < 4 ? q : q + 1) * L.n + f];
+            } else {
+#pragma unroll
+                for (int q = 0; q < Q; ++q) coef[k][r][q] = L.c4[q * L.n + f];
+            }
+            rd[k][r] = L.rdiag[f];
+            b[k][r] = L.b[f];
+            x[k][r] = in && L.xin ? L.xin[f] : 0.0;
+            if (L.xc && in && act) {
+                // the prolonged correction, in the order prolong_sum adds it
+                double wx, wy;
+                const int I = coarse_low(L.ax, i, wx), J = coarse_low(L.ay, j, wy);
+                double sum = 0.0;
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    const double px = d ? 1.0 - wx : wx;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const double py = e ? 1.0 - wy : wy;
+                        if (px != 0.0 && py != 0.0) sum += px * py * L.xc[(I + d) * L.ay.nc + J + e];
+                    }
+                }
+                x[k][r] += sum;
+            }
+            if (u < S::per) xs[at[k][r]] = x[k][r];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < COUNT; ++kk) {
+        const int k = REVERSE ? K - 1 - kk % K : kk % K;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (ring[k][r] > kk) {  // phase kk is exact from ring kk + 1 inward
+                const double *q = xs + at[k][r];
+                const double(&c)[Q] = coef[k][r];
+                if constexpr (NINE) {
+                    const double v[8] = {q[-WY - 1], q[-WY], q[-WY + 1], q[-1],
+                                         q[1],       q[WY - 1], q[WY],   q[WY + 1]};
+                    x[k][r] = update9(b[k][r], c, v, rd[k][r]);
+                } else {
+                    x[k][r] = update5(b[k][r], c[0], c[1], c[2], c[3], q[-WY], q[WY], q[-1], q[1],
+                                      rd[k][r]);
+                }
+                xs[at[k][r]] = x[k][r];
+            }
+        }
+        if (kk + 1 < COUNT) __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int a = at[k][r] / WY, c = at[k][r] - a * WY;
+            const int i = i0 + a, j = j0 + c;
+            if (tid + r * S::threads < S::per && a >= S::halo && a < S::halo + TX && c >= S::halo &&
+                c < S::halo + TY && i < L.nx && j < L.ny)
+                L.xout[i * L.ny + j] = x[k][r];
+        }
+    }
+}
+
+template <bool NINE, int TX, int TY, int COUNT, bool REVERSE>
+__global__ void __launch_bounds__(Tile<NINE, TX, TY, COUNT>::threads)
+    smooth_level(SmoothView L, const CycleIo *__restrict__ io, bool first, bool last) {
+    // io: the finest level's smoothing, which starts the cycle from its b and ends it in z
+    if (io) {
+        L.b = io->b;
+        if (last) L.xout = io->z;
+    }
+    if (first) L.xin = nullptr;
+    smooth_tile<NINE, TX, TY, COUNT, REVERSE>(L, blockIdx.x, blockIdx.y);
 }
 
 // y = A x (level 0, 5-point) on active rows, 0 elsewhere; with b: r = b - A x.  Node f of
@@ -646,7 +780,7 @@ __global__ void residual9(i64 nx, i64 ny, const double *__restrict__ a9,
 }
 
 // bc[t] = (R r)[t] over the active fine nodes (weighted by the control volumes on level 0),
-// xc[t] = 0.  The terms are those of the fine nodes with a nonzero prolongation weight, in
+// xc[t] = 0 (where xc is not NULL: the staged smoothing starts from zero by itself).  The terms are those of the fine nodes with a nonzero prolongation weight, in
 // ascending (k, l) order; the weights and the fine values are independent loads.
 template <class Load>
 __device__ __forceinline__ void restrict_item(i64 t, const Fine &F, const double *r, double *bc,
@@ -672,7 +806,7 @@ __device__ __forceinline__ void restrict_item(i64 t, const Fine &F, const double
         }
     }
     bc[t] = s;
-    xc[t] = 0.0;
+    if (xc) xc[t] = 0.0;
 }
 
 __global__ void restrict_residual(Fine F, const double *__restrict__ r, double *__restrict__ bc,
@@ -1441,7 +1575,7 @@ __device__ __forceinline__ double apply_row(const Rows5 &A, i64 f, const double 
 // Gram-Schmidt) and h2[q] = <V_q, w>; kOrthNorm: w -= sum_q h2[q] V_q, its squared norm, and in
 // the last block the step's Hessenberg column and rotation (arnoldi_step).  Three launches and
 // the scaling of the next basis vector, where the product, three passes, the scaling, the
-// column and the V-cycle's copies in and out took nine: KRYLOV_US.
+// column and the V-cycle's copies in and out took nine: 9 to 13 us a pass at 801 x 201.
 enum PassMode { kApply = 0, kOrthDots = 1, kOrthNorm = 2 };
 
 struct ArnoldiState {
@@ -1870,11 +2004,6 @@ void setup_tail(bt_poisson *p) {
             break;
         p->tail_start = l;
     }
-    const int big5 = (int)stage_smem(false, kStage5X, kStage5Y, kMaxPhases);
-    const int big9 = (int)stage_smem(true, kStage9X, kStage9Y, kMaxPhases);
-    BT_CUDA(cudaFuncSetAttribute(smooth_staged<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big5));
-    BT_CUDA(cudaFuncSetAttribute(smooth_staged<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big5));
-    BT_CUDA(cudaFuncSetAttribute(smooth_staged<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big9));
     // the largest band any solver's coarsest level needs (the attribute is the kernel's,
     // shared by every solver of the process: never set it to one mesh's own size)
     BT_CUDA(cudaFuncSetAttribute(coarsest_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1973,45 +2102,56 @@ void smooth(bt_poisson *p, size_t l, bool pre, const Fine *pf = nullptr,
     const bool five = l == 0;
     const int colours = five ? 2 : 4;
     const int sweeps = five ? p->fine_sweeps : p->coarse_sweeps;
-    std::vector<int> order;
-    for (int sw = 0; sw < sweeps; ++sw)
-        for (int c = 0; c < colours; ++c) order.push_back(pre ? c : colours - 1 - c);
     if (p->staged) {
         const int tx = five ? kStage5X : kStage9X, ty = five ? kStage5Y : kStage9Y;
         const dim3 tiles((unsigned)((L.nx + tx - 1) / tx), (unsigned)((L.ny + ty - 1) / ty));
-        for (size_t start = 0; start < order.size(); start += kMaxPhases) {
-            Phases ph{};
-            ph.count = (int)std::min<size_t>(kMaxPhases, order.size() - start);
-            for (int k = 0; k < ph.count; ++k) ph.colour[k] = order[start + k];
-            const int halo = stage_halo(ph.count);
-            const size_t smem = stage_smem(!five, tx, ty, halo);
-            const int per = (tx + 2 * halo) * (ty + 2 * halo) / colours;
-            const int own = (per + kStageThreads - 1) / kStageThreads;
+        const int phases = sweeps * colours;
+        for (int start = 0; start < phases; start += kMaxPhases) {
+            const int count = std::min(kMaxPhases, phases - start);
             double *x = L.x.as<double>(L.n);
-            double *in = L.cur, *out = L.cur == x ? L.x2.as<double>(L.n) : x;
-            const Fine F = start == 0 && xc ? *pf : Fine{};
-            const double *add = start == 0 ? xc : nullptr;
+            double *out = L.cur == x ? L.x2.as<double>(L.n) : x;
+            SmoothView V{};
+            V.nx = (int)L.nx;
+            V.ny = (int)L.ny;
+            V.n = L.n;
+            V.c4 = five ? L.c4.as<double>(4 * L.n) : nullptr;
+            V.a9 = five ? nullptr : L.a9.as<double>(9 * L.n);
+            V.rdiag = L.rdiag.as<double>(L.n);
+            V.b = b;
+            V.active = act;
+            V.xin = L.cur;
+            V.xout = out;
+            if (start == 0 && xc) {
+                V.xc = xc;
+                V.ax = CoarseAxis{(int)L.nx, (int)pf->ncx};
+                V.ay = CoarseAxis{(int)L.ny, (int)pf->ncy};
+            }
             const CycleIo *io = five ? p->cycle_io.as<CycleIo>(1) : nullptr;
-            const bool first = five && pre && start == 0;
-            const bool last = five && !pre && start + ph.count == order.size();
-            if (five && own <= 2)
-                BT_LAUNCH(p->ctx, (smooth_staged<false, 2>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
-                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add, io, first, last);
-            else if (five && own == 3)
-                BT_LAUNCH(p->ctx, (smooth_staged<false, 3>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, L.c4.as<double>(4 * L.n), L.rdiag.as<double>(L.n),
-                          (const double *)nullptr, act, b, in, out, tx, ty, ph, F, add, io, first, last);
-            else if (!five && own == 1)
-                BT_LAUNCH(p->ctx, (smooth_staged<true, 1>), tiles, kStageThreads, smem, st, L.nx,
-                          L.ny, (const double *)nullptr, L.rdiag.as<double>(L.n),
-                          L.a9.as<double>(9 * L.n), act, b, in, out, tx, ty, ph, F, add, io, first, last);
-            else
-                BT_REQUIRE(false, "poisson: staged smoothing tile too large for its block");
+            const bool first = pre && start == 0;  // every level's cycle starts from zero
+            const bool last = five && !pre && start + count == phases;
+#define BT_SMOOTH(N, X, Y, C)                                                                   \
+    if (five != N && count == C) {                                                                \
+        if (pre)                                                                                   \
+            BT_LAUNCH(p->ctx, (smooth_level<N, X, Y, C, false>), tiles, (Tile<N, X, Y, C>::threads), \
+                      0, st, V, io, first, last);                                                  \
+        else                                                                                       \
+            BT_LAUNCH(p->ctx, (smooth_level<N, X, Y, C, true>), tiles, (Tile<N, X, Y, C>::threads),  \
+                      0, st, V, io, first, last);                                                  \
+    }
+            BT_SMOOTH(false, kStage5X, kStage5Y, 2)
+            BT_SMOOTH(false, kStage5X, kStage5Y, 4)
+            BT_SMOOTH(false, kStage5X, kStage5Y, 6)
+            BT_SMOOTH(false, kStage5X, kStage5Y, 8)
+            BT_SMOOTH(true, kStage9X, kStage9Y, 4)
+            BT_SMOOTH(true, kStage9X, kStage9Y, 8)
+#undef BT_SMOOTH
             L.cur = out;
         }
         return;
     }
+    std::vector<int> order;
+    for (int sw = 0; sw < sweeps; ++sw)
+        for (int c = 0; c < colours; ++c) order.push_back(pre ? c : colours - 1 - c);
     double *x = L.cur;
     if (xc) BT_LAUNCH(p->ctx, prolong_add, blocks_for(L.n, T), T, 0, st, *pf, xc, x);
     for (int c : order) {
@@ -2066,7 +2206,7 @@ void vcycle(bt_poisson *p, size_t l) {
                   L.a9.as<double>(9 * L.n), act, L.cur, b, r);
     Fine F = fine_of(L, C, l == 0);
     BT_LAUNCH(p->ctx, restrict_residual, blocks_for(C.n, T), T, 0, st, F, r, C.b.as<double>(C.n),
-                                                          C.x.as<double>(C.n));
+              p->staged ? nullptr : C.x.as<double>(C.n));
     vcycle(p, l + 1);
     smooth(p, l, false, &F, C.x.as<double>(C.n));
     if (io) {
@@ -2688,6 +2828,35 @@ __global__ void __launch_bounds__(kStageThreads)
                                 zero_in != 0);
 }
 
+// The same in the register form, for the tiles the compiler knows (smooth_tile).
+template <bool NINE, int TX, int TY, int COUNT, bool REVERSE>
+__global__ void __launch_bounds__(Tile<NINE, TX, TY, COUNT>::threads)
+    batch_smooth_tile(const BatchLevel *__restrict__ E, const int *__restrict__ ids,
+                      const int *__restrict__ start, int ne, const uint8_t *__restrict__ live,
+                      int from, int prolong, int zero_in) {
+    const int slot = find_entry(start, ne, blockIdx.x);
+    const BatchLevel &L = E[ids[slot]];
+    if (!live[L.cand]) return;
+    const int local = (int)blockIdx.x - start[slot];
+    const int tiles_y = ((int)L.ny + TY - 1) / TY;
+    const int bx = local / tiles_y, by = local - bx * tiles_y;
+    SmoothView V{};
+    V.nx = (int)L.nx;
+    V.ny = (int)L.ny;
+    V.n = L.n;
+    V.c4 = L.c4;
+    V.a9 = L.a9;
+    V.rdiag = L.rdiag;
+    V.b = L.b;
+    V.active = L.active;
+    V.xin = zero_in ? nullptr : (from ? L.x2 : L.x);
+    V.xout = from ? L.x : L.x2;
+    V.xc = prolong ? L.xc : nullptr;
+    V.ax = CoarseAxis{V.nx, (int)L.F.ncx};
+    V.ay = CoarseAxis{V.ny, (int)L.F.ncy};
+    smooth_tile<NINE, TX, TY, COUNT, REVERSE>(V, bx, by);
+}
+
 // r = b - A x on every entry's level (x in the buffer `from` names: 0 x, 1 x2), then
 // (after the launch) its restriction.
 template <bool NINE>
@@ -2706,7 +2875,7 @@ __global__ void batch_residual(const BatchLevel *__restrict__ E, const int *__re
         apply5_item(f, L.nx, L.ny, L.c4, L.diag, L.active, x, L.b, L.r);
 }
 
-// b of the next level = R r, its x = 0.
+// b of the next level = R r (its smoothing starts from zero).
 __global__ void batch_restrict(const BatchLevel *__restrict__ E, const int *__restrict__ ids,
                                const int *__restrict__ start,
                                int ne, const uint8_t *__restrict__ live) {
@@ -2715,7 +2884,7 @@ __global__ void batch_restrict(const BatchLevel *__restrict__ E, const int *__re
     if (!live[L.cand]) return;
     const i64 t = ((i64)blockIdx.x - start[slot]) * kBatchThreads + threadIdx.x;
     if (t >= L.ncn) return;
-    restrict_item(t, L.F, L.r, L.bc, L.xc, PlainLoad{});
+    restrict_item(t, L.F, L.r, L.bc, (double *)nullptr, PlainLoad{});
 }
 
 // Every candidate's coarse levels, one block each.
@@ -3016,6 +3185,29 @@ void batch_smooth_launch(bt_poisson_batch *B, int l, bool pre, int first, int co
     const BatchLevel *E = S.entries.as<BatchLevel>(S.cand.size());
     const int *ids = S.ids.as<int>(S.n), *start = S.smooth_start.as<int>(S.n);
     const int tx = nine ? B->tile9[0] : B->tile5[0], ty = nine ? B->tile9[1] : B->tile5[1];
+    // the register form for the tiles of the tuner's list
+#define BT_BATCH_TILE(N, X, Y, C)                                                              \
+    if (nine == N && tx == X && ty == Y && count == C && first % (N ? 4 : 2) == 0) {             \
+        if (pre)                                                                                   \
+            BT_LAUNCH(ctx, (batch_smooth_tile<N, X, Y, C, false>), S.smooth_blocks,                \
+                      (Tile<N, X, Y, C>::threads), 0, ctx->stream, E, ids, start, S.n, live, from, \
+                      prolong, zero_in);                                                           \
+        else                                                                                       \
+            BT_LAUNCH(ctx, (batch_smooth_tile<N, X, Y, C, true>), S.smooth_blocks,                 \
+                      (Tile<N, X, Y, C>::threads), 0, ctx->stream, E, ids, start, S.n, live, from, \
+                      prolong, zero_in);                                                           \
+        return;                                                                                    \
+    }
+    BT_BATCH_TILE(false, 32, 32, 4)
+    BT_BATCH_TILE(false, 32, 16, 4)
+    BT_BATCH_TILE(false, 16, 32, 4)
+    BT_BATCH_TILE(false, 64, 16, 4)
+    BT_BATCH_TILE(true, 16, 32, 8)
+    BT_BATCH_TILE(true, 16, 32, 4)
+    BT_BATCH_TILE(true, 16, 16, 4)
+    BT_BATCH_TILE(true, 32, 16, 4)
+    BT_BATCH_TILE(true, 32, 32, 4)
+#undef BT_BATCH_TILE
     const Phases ph = batch_phases(nine ? B->coarse_sweeps : B->fine_sweeps, nine ? 4 : 2, pre,
                                    first, count);
     const size_t smem = stage_smem(nine, tx, ty, stage_halo(count));
@@ -3039,8 +3231,8 @@ void batch_smooth_launch(bt_poisson_batch *B, int l, bool pre, int first, int co
 }
 
 // The smoothing of step l's live entries before (pre) or after the coarse correction;
-// returns the buffer that holds the result (0: x, 1: x2).  Level 0's pre-smoothing starts
-// from zero; the post-smoothing adds the prolonged correction as it reads.  Before the
+// returns the buffer that holds the result (0: x, 1: x2).  The pre-smoothing starts from
+// zero; the post-smoothing adds the prolonged correction as it reads.  Before the
 // correction the input is the pre-smoothing's result `from`.
 int batch_smooth_step(bt_poisson_batch *B, int l, bool pre, int from = 0) {
     auto &S = B->level[l];
@@ -3053,7 +3245,7 @@ int batch_smooth_step(bt_poisson_batch *B, int l, bool pre, int from = 0) {
     for (int first = 0, k = 0; first < phases; first += per, ++k) {
         const int count = std::min(per, phases - first);
         batch_smooth_launch(B, l, pre, first, count, in, (!pre && k == 0) ? 1 : 0,
-                            (pre && k == 0 && !nine) ? 1 : 0);
+                            (pre && k == 0) ? 1 : 0);
         in ^= 1;
     }
     return in;
