@@ -44,7 +44,7 @@ struct Level {
     Buffer weight;  // level 0: the control volumes W
     Buffer a9;      // coarse levels: 9 coefficients per node, (dI + 1) * 3 + (dJ + 1)
     Buffer active;  // uint8: free (level 0) or a nonzero row (coarse)
-    Buffer x, b, r;
+    Buffer x, b;
     Buffer x2;              // the second x of staged smoothing (it writes the other buffer)
     double *cur = nullptr;  // which of x, x2 holds the level's x while a V-cycle is recorded
     Axis ax, ay;            // the map to the next coarser level
@@ -351,12 +351,6 @@ __global__ void smooth5(i64 nx, i64 ny, const double *__restrict__ c4,
                    j < ny - 1 ? x[f + 1] : 0.0, rdiag[f]);
 }
 
-// How the item functions load the vectors they read (plain loads; a kernel whose blocks
-// shared vectors through global memory within one launch would bypass L1 here).
-struct PlainLoad {
-    __device__ __forceinline__ double operator()(const double *p) const { return *p; }
-};
-
 // The nodes of one of four colours (i % 2, j % 2) of a 9-point level: item t of `count`.
 __host__ __device__ __forceinline__ i64 colour_count(i64 nx, i64 ny, int colour) {
     const int ci = colour >> 1, cj = colour & 1;
@@ -419,8 +413,7 @@ __host__ __device__ inline int stage_halo(int count) { return (count + 1) & ~1; 
 
 // (P xc)[f], the prolongation of the coarse correction xc to the fine node f of an active
 // fine node (the bilinear weights of the fine node's coarse neighbours, in (sx, sy) order).
-template <class Load>
-__device__ __forceinline__ double prolong_sum(const Fine &F, i64 f, const double *xc, Load load) {
+__device__ __forceinline__ double prolong_sum(const Fine &F, i64 f, const double *xc) {
     const i64 k = f / F.ny, l = f - k * F.ny;
     const i64 ix = F.lox[k], iy = F.loy[l];
     const double wx = F.wx[k], wy = F.wy[l];
@@ -431,7 +424,7 @@ __device__ __forceinline__ double prolong_sum(const Fine &F, i64 f, const double
         for (int sy = 0; sy < 2; ++sy) {
             const double py = sy ? 1.0 - wy : wy;
             if (py == 0.0 || iy + sy >= F.ncy) continue;
-            s += px * py * load(xc + (ix + sx) * F.ncy + iy + sy);
+            s += px * py * xc[(ix + sx) * F.ncy + iy + sy];
         }
     }
     return s;
@@ -502,7 +495,7 @@ __device__ __forceinline__ void smooth_staged_tile(
                 for (int q = 0; q < 5; ++q) coef[q * m + pos] = q5[q];
             }
             if (av) {
-                if (xc) xv = xv + prolong_sum(F, f, xc, PlainLoad{});
+                if (xc) xv = xv + prolong_sum(F, f, xc);
                 bv = bf;
             }
         }
@@ -740,93 +733,111 @@ __device__ __forceinline__ double apply5_item(i64 f, i64 nx, i64 ny, const doubl
     return out;
 }
 
-__global__ void apply5(i64 nx, i64 ny, const double *__restrict__ c4,
-                       const double *__restrict__ diag, const uint8_t *__restrict__ active,
-                       const double *__restrict__ x, const double *b, double *__restrict__ y,
-                       const CycleIo *__restrict__ io) {
-    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nx * ny) return;
-    if (io) b = io->b;
-    apply5_item(f, nx, ny, c4, diag, active, x, b, y);
+// -- the residual and its restriction -----------------------------------------------------
+//
+// One launch a level: a block forms the residual of the fine nodes around kRestrictX x
+// kRestrictY coarse nodes, a thread a fine node with its row's loads all in flight, weighs
+// it (by the control volumes on level 0) into shared memory, and adds up each coarse node's
+// nine from there, the weights from build_axis's rule.  The blocks' edges are computed twice
+// (10 % of the rows); the residual never goes to memory and there is one launch of RESTRICT_US
+// where the two took 8 (the restriction alone 4.8: its nine loads waited for table entries).
+constexpr int kRestrictX = 8, kRestrictY = 16;
+constexpr int kRestrictFineX = 2 * kRestrictX + 1, kRestrictFineY = 2 * kRestrictY + 1;
+constexpr int kRestrictThreads = (kRestrictFineX * kRestrictFineY + 31) / 32 * 32;
+
+struct RestrictView {
+    int nx, ny, ncx, ncy;
+    i64 n;
+    const double *c4, *diag, *a9, *weight;  // level 0: c4, diag and weight; else a9
+    const uint8_t *active;
+    const double *x, *b;
+    double *bc;
+};
+
+// The weight of coarse node I at fine node k of an axis.
+__device__ __forceinline__ double coarse_weight(const CoarseAxis &A, int k, int I) {
+    double w;
+    const int lo = coarse_low(A, k, w);
+    return I == lo ? w : (I == lo + 1 ? 1.0 - w : 0.0);
 }
 
-template <class Load>
-__device__ __forceinline__ void residual9_item(i64 f, i64 nx, i64 ny, const double *__restrict__ a9,
-                                               const uint8_t *__restrict__ active,
-                                               const double *x, const double *b, double *r,
-                                               Load load) {
-    const i64 n = nx * ny;
-    if (!active[f]) {
-        r[f] = 0.0;
-        return;
-    }
-    const i64 i = f / ny, j = f - i * ny;
-    double s = load(b + f);
-    for (int di = -1; di <= 1; ++di)
-        for (int dj = -1; dj <= 1; ++dj) {
-            const i64 i2 = i + di, j2 = j + dj;
-            if (i2 < 0 || i2 >= nx || j2 < 0 || j2 >= ny) continue;
-            s -= a9[(i64)((di + 1) * 3 + (dj + 1)) * n + f] * load(x + i2 * ny + j2);
+template <bool NINE>
+__device__ __forceinline__ void restrict_tile(const RestrictView &L, int bx, int by) {
+    __shared__ double rs[kRestrictFineX * kRestrictFineY];
+    const int tid = threadIdx.x, nx = L.nx, ny = L.ny;
+    const int I0 = bx * kRestrictX, J0 = by * kRestrictY;
+    const int k0 = nx > 3 ? 2 * I0 - 1 : I0 - 1, l0 = ny > 3 ? 2 * J0 - 1 : J0 - 1;
+    if (tid < kRestrictFineX * kRestrictFineY) {
+        const int i = k0 + tid / kRestrictFineY, j = l0 + tid % kRestrictFineY;
+        double r = 0.0;
+        if (i >= 0 && i < nx && j >= 0 && j < ny) {
+            const int f = i * ny + j;
+            const bool w = i > 0, e = i < nx - 1, s = j > 0, n = j < ny - 1;
+            const double *x = L.x + f;
+            if (NINE) {
+                double a[9];
+#pragma unroll
+                for (int q = 0; q < 9; ++q) a[q] = L.a9[q * L.n + f];
+                const double v[9] = {w && s ? x[-ny - 1] : 0.0, w ? x[-ny] : 0.0,
+                                     w && n ? x[-ny + 1] : 0.0, s ? x[-1] : 0.0,
+                                     x[0],                      n ? x[1] : 0.0,
+                                     e && s ? x[ny - 1] : 0.0,  e ? x[ny] : 0.0,
+                                     e && n ? x[ny + 1] : 0.0};
+                double p = L.b[f], q = a[5] * v[5];
+#pragma unroll
+                for (int k = 0; k < 5; ++k) p = fma(-a[k], v[k], p);
+#pragma unroll
+                for (int k = 6; k < 9; ++k) q = fma(a[k], v[k], q);
+                r = p - q;
+            } else {
+                const double p = fma(-L.diag[f], x[0], L.b[f]);
+                const double q = fma(L.c4[f], w ? x[-ny] : 0.0, L.c4[L.n + f] * (e ? x[ny] : 0.0));
+                const double u = fma(L.c4[2 * L.n + f], s ? x[-1] : 0.0,
+                                     L.c4[3 * L.n + f] * (n ? x[1] : 0.0));
+                r = (p + (q + u)) * L.weight[f];
+            }
+            if (!L.active[f]) r = 0.0;
         }
-    r[f] = s;
-}
-
-__global__ void residual9(i64 nx, i64 ny, const double *__restrict__ a9,
-                          const uint8_t *__restrict__ active, const double *__restrict__ x,
-                          const double *__restrict__ b, double *__restrict__ r) {
-    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nx * ny) return;
-    residual9_item(f, nx, ny, a9, active, x, b, r, PlainLoad{});
-}
-
-// bc[t] = (R r)[t] over the active fine nodes (weighted by the control volumes on level 0),
-// xc[t] = 0 (where xc is not NULL: the staged smoothing starts from zero by itself).  The terms are those of the fine nodes with a nonzero prolongation weight, in
-// ascending (k, l) order; the weights and the fine values are independent loads.
-template <class Load>
-__device__ __forceinline__ void restrict_item(i64 t, const Fine &F, const double *r, double *bc,
-                                              double *xc, Load load) {
-    const i64 I = t / F.ncy, J = t - I * F.ncy;
-    const i64 k0 = F.rx0[I], l0 = F.ry0[J];
-    double px[kRestrict], py[kRestrict];
-#pragma unroll
-    for (int a = 0; a < kRestrict; ++a) {
-        px[a] = F.rxw[kRestrict * I + a];
-        py[a] = F.ryw[kRestrict * J + a];
+        rs[tid] = r;
     }
-    double s = 0.0;
+    __syncthreads();
+    if (tid >= kRestrictX * kRestrictY) return;
+    const int I = I0 + tid / kRestrictY, J = J0 + tid % kRestrictY;
+    if (I >= L.ncx || J >= L.ncy) return;
+    const CoarseAxis ax{nx, L.ncx}, ay{ny, L.ncy};
+    const int ki = nx > 3 ? 2 * I : I, li = ny > 3 ? 2 * J : J;  // the middle of the nine
+    double sum = 0.0;
 #pragma unroll
-    for (int a = 0; a < kRestrict; ++a) {
-        if (px[a] == 0.0) continue;
+    for (int d = -1; d <= 1; ++d) {
+        const double pk = ki + d >= 0 && ki + d < nx ? coarse_weight(ax, ki + d, I) : 0.0;
+        double row = 0.0;
 #pragma unroll
-        for (int c = 0; c < kRestrict; ++c) {
-            if (py[c] == 0.0) continue;
-            const i64 f = (k0 + a) * F.ny + l0 + c;
-            if (!F.active[f]) continue;
-            s += px[a] * py[c] * (F.weight ? F.weight[f] : 1.0) * load(r + f);
+        for (int e = -1; e <= 1; ++e) {
+            const double pl = li + e >= 0 && li + e < ny ? coarse_weight(ay, li + e, J) : 0.0;
+            if (pl != 0.0 && pk != 0.0)
+                row = fma(pl, rs[(ki + d - k0) * kRestrictFineY + (li + e - l0)], row);
         }
+        sum = fma(pk, row, sum);
     }
-    bc[t] = s;
-    if (xc) xc[t] = 0.0;
+    L.bc[I * L.ncy + J] = sum;
 }
 
-__global__ void restrict_residual(Fine F, const double *__restrict__ r, double *__restrict__ bc,
-                                  double *__restrict__ xc) {
-    const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= F.ncx * F.ncy) return;
-    restrict_item(t, F, r, bc, xc, PlainLoad{});
+template <bool NINE>
+__global__ void __launch_bounds__(kRestrictThreads)
+    restrict_level(RestrictView L, const CycleIo *__restrict__ io) {
+    if (io) L.b = io->b;
+    restrict_tile<NINE>(L, blockIdx.x, blockIdx.y);
 }
 
-template <class Load>
-__device__ __forceinline__ void prolong_item(i64 f, const Fine &F, const double *xc, double *x,
-                                             Load load) {
-    if (!F.active[f]) return;
-    x[f] = load(x + f) + prolong_sum(F, f, xc, load);
+__global__ void fill_zero(i64 n, double *__restrict__ x) {
+    const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (f < n) x[f] = 0.0;
 }
 
 __global__ void prolong_add(Fine F, const double *__restrict__ xc, double *__restrict__ x) {
     const i64 f = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= F.nx * F.ny) return;
-    prolong_item(f, F, xc, x, PlainLoad{});
+    if (F.active[f]) x[f] = x[f] + prolong_sum(F, f, xc);
 }
 
 // The coarsest level: the dense matrix of its 9-point operator, inverted in place in `M`
@@ -2191,22 +2202,36 @@ void vcycle(bt_poisson *p, size_t l) {
         return;
     }
     Level &C = p->levels[l + 1];
-    double *b = L.b.as<double>(L.n), *r = L.r.as<double>(L.n);
+    double *b = L.b.as<double>(L.n);
     const uint8_t *act = L.active.as<uint8_t>(L.n);
     L.cur = L.x.as<double>(L.n);
     const CycleIo *io = l == 0 ? p->cycle_io.as<CycleIo>(1) : nullptr;
     if (io && !p->staged)
         BT_LAUNCH(p->ctx, cycle_begin, blocks_for(L.n, T), T, 0, st, io, L.n, b, L.cur);
     smooth(p, l, true);
-    if (l == 0)
-        BT_LAUNCH(p->ctx, apply5, blocks_for(L.n, T), T, 0, st, L.nx, L.ny, L.c4.as<double>(4 * L.n),
-                  L.diag.as<double>(L.n), act, L.cur, b, r, io);
-    else
-        BT_LAUNCH(p->ctx, residual9, blocks_for(L.n, T), T, 0, st, L.nx, L.ny,
-                  L.a9.as<double>(9 * L.n), act, L.cur, b, r);
     Fine F = fine_of(L, C, l == 0);
-    BT_LAUNCH(p->ctx, restrict_residual, blocks_for(C.n, T), T, 0, st, F, r, C.b.as<double>(C.n),
-              p->staged ? nullptr : C.x.as<double>(C.n));
+    RestrictView R{};
+    R.nx = (int)L.nx;
+    R.ny = (int)L.ny;
+    R.ncx = (int)C.nx;
+    R.ncy = (int)C.ny;
+    R.n = L.n;
+    R.c4 = F.c4;
+    R.diag = F.diag;
+    R.a9 = F.a9;
+    R.weight = F.weight;
+    R.active = act;
+    R.x = L.cur;
+    R.b = b;
+    R.bc = C.b.as<double>(C.n);
+    const dim3 tiles((unsigned)((C.nx + kRestrictX - 1) / kRestrictX),
+                     (unsigned)((C.ny + kRestrictY - 1) / kRestrictY));
+    if (l == 0)
+        BT_LAUNCH(p->ctx, restrict_level<false>, tiles, kRestrictThreads, 0, st, R, io);
+    else
+        BT_LAUNCH(p->ctx, restrict_level<true>, tiles, kRestrictThreads, 0, st, R, io);
+    if (!p->staged)  // (the staged smoothing starts from zero by itself)
+        BT_LAUNCH(p->ctx, fill_zero, blocks_for(C.n, T), T, 0, st, C.n, C.x.as<double>(C.n));
     vcycle(p, l + 1);
     smooth(p, l, false, &F, C.x.as<double>(C.n));
     if (io) {
@@ -2466,7 +2491,6 @@ extern "C" int bt_poisson_create(bt_ctx *ctx, const bt_mesh_desc *m, bt_poisson 
                 L.x.as<double>(L.n);
                 L.x2.as<double>(L.n);
                 L.b.as<double>(L.n);
-                L.r.as<double>(L.n);
                 L.active.as<uint8_t>(L.n);
                 L.rdiag.as<double>(L.n);
                 if (p->levels.size() == 1) {
@@ -2764,10 +2788,9 @@ struct BatchLevel {
     const double *c4, *diag, *a9;  // level 0: c4, diag; coarse levels: a9
     const double *rdiag;
     const uint8_t *active;
-    double *x, *x2, *b, *r;
+    double *x, *x2, *b;
     Fine F;           // to the next level
     double *xc, *bc;  // the next level's x and b
-    i64 ncn;          // the next level's nodes
 };
 
 // One candidate's finest level for the outer iteration.
@@ -2857,34 +2880,34 @@ __global__ void __launch_bounds__(Tile<NINE, TX, TY, COUNT>::threads)
     smooth_tile<NINE, TX, TY, COUNT, REVERSE>(V, bx, by);
 }
 
-// r = b - A x on every entry's level (x in the buffer `from` names: 0 x, 1 x2), then
-// (after the launch) its restriction.
+// b of the next level = R (b - A x) on every entry's level (x in the buffer `from` names:
+// 0 x, 1 x2).
 template <bool NINE>
-__global__ void batch_residual(const BatchLevel *__restrict__ E, const int *__restrict__ ids,
-                               const int *__restrict__ start,
-                               int ne, const uint8_t *__restrict__ live, int from) {
+__global__ void __launch_bounds__(kRestrictThreads)
+    batch_restrict(const BatchLevel *__restrict__ E, const int *__restrict__ ids,
+                   const int *__restrict__ start, int ne, const uint8_t *__restrict__ live,
+                   int from) {
     const int slot = find_entry(start, ne, blockIdx.x);
     const BatchLevel &L = E[ids[slot]];
     if (!live[L.cand]) return;
-    const i64 f = ((i64)blockIdx.x - start[slot]) * kBatchThreads + threadIdx.x;
-    if (f >= L.n) return;
-    const double *x = from ? L.x2 : L.x;
-    if (NINE)
-        residual9_item(f, L.nx, L.ny, L.a9, L.active, x, L.b, L.r, PlainLoad{});
-    else
-        apply5_item(f, L.nx, L.ny, L.c4, L.diag, L.active, x, L.b, L.r);
-}
-
-// b of the next level = R r (its smoothing starts from zero).
-__global__ void batch_restrict(const BatchLevel *__restrict__ E, const int *__restrict__ ids,
-                               const int *__restrict__ start,
-                               int ne, const uint8_t *__restrict__ live) {
-    const int slot = find_entry(start, ne, blockIdx.x);
-    const BatchLevel &L = E[ids[slot]];
-    if (!live[L.cand]) return;
-    const i64 t = ((i64)blockIdx.x - start[slot]) * kBatchThreads + threadIdx.x;
-    if (t >= L.ncn) return;
-    restrict_item(t, L.F, L.r, L.bc, (double *)nullptr, PlainLoad{});
+    const int local = (int)blockIdx.x - start[slot];
+    RestrictView R{};
+    R.nx = (int)L.nx;
+    R.ny = (int)L.ny;
+    R.ncx = (int)L.F.ncx;
+    R.ncy = (int)L.F.ncy;
+    R.n = L.n;
+    R.c4 = L.F.c4;
+    R.diag = L.F.diag;
+    R.a9 = L.F.a9;
+    R.weight = L.F.weight;
+    R.active = L.active;
+    R.x = from ? L.x2 : L.x;
+    R.b = L.b;
+    R.bc = L.bc;
+    const int tiles_y = (R.ncy + kRestrictY - 1) / kRestrictY;
+    const int bx = local / tiles_y;
+    restrict_tile<NINE>(R, bx, local - bx * tiles_y);
 }
 
 // Every candidate's coarse levels, one block each.
@@ -3070,9 +3093,9 @@ struct bt_poisson_batch {
     // per kind of launch, each one's first block.
     struct Step {
         bt::Buffer entries;
-        std::vector<int> cand, nx, ny, nodes, coarse;
-        bt::Buffer ids, smooth_start, node_start, coarse_start;
-        int n = 0, smooth_blocks = 0, node_blocks = 0, coarse_blocks = 0;
+        std::vector<int> cand, nx, ny, coarse;
+        bt::Buffer ids, smooth_start, coarse_start;
+        int n = 0, smooth_blocks = 0, coarse_blocks = 0;
     };
     std::vector<Step> level;
     bt::Buffer tails, tail_ids;  // one block per live candidate
@@ -3114,27 +3137,23 @@ void compact(bt_poisson_batch *B, const uint8_t *alive) {
     cudaStream_t st = B->ctx->stream;
     const int count = (int)B->solvers.size();
     for (auto &S : B->level) {
-        std::vector<int> ids, smooth, node, coarse;
-        int sb = 0, nb = 0, cb = 0;
+        std::vector<int> ids, smooth, coarse;
+        int sb = 0, cb = 0;
         const bool five = &S == &B->level[0];
         const int tx = five ? B->tile5[0] : B->tile9[0], ty = five ? B->tile5[1] : B->tile9[1];
         for (int e = 0; e < (int)S.cand.size(); ++e) {
             if (!alive[S.cand[e]]) continue;
             ids.push_back(e);
             smooth.push_back(sb);
-            node.push_back(nb);
             coarse.push_back(cb);
             sb += ((S.nx[e] + tx - 1) / tx) * ((S.ny[e] + ty - 1) / ty);
-            nb += S.nodes[e];
             cb += S.coarse[e];
         }
         S.n = (int)ids.size();
         S.smooth_blocks = sb;
-        S.node_blocks = nb;
         S.coarse_blocks = cb;
         upload(S.ids, ids, st);
         upload(S.smooth_start, smooth, st);
-        upload(S.node_start, node, st);
         upload(S.coarse_start, coarse, st);
     }
     std::vector<int> tails, fine, start;
@@ -3264,13 +3283,11 @@ void batch_vcycle(bt_poisson_batch *B) {
         const int *ids = S.ids.as<int>(S.n);
         held[l] = batch_smooth_step(B, l, true);
         if (l == 0)
-            BT_LAUNCH(ctx, batch_residual<false>, S.node_blocks, kBatchThreads, 0, st, E, ids,
-                      S.node_start.as<int>(S.n), S.n, live, held[l]);
+            BT_LAUNCH(ctx, batch_restrict<false>, S.coarse_blocks, kRestrictThreads, 0, st, E, ids,
+                      S.coarse_start.as<int>(S.n), S.n, live, held[l]);
         else
-            BT_LAUNCH(ctx, batch_residual<true>, S.node_blocks, kBatchThreads, 0, st, E, ids,
-                      S.node_start.as<int>(S.n), S.n, live, held[l]);
-        BT_LAUNCH(ctx, batch_restrict, S.coarse_blocks, kBatchThreads, 0, st, E, ids,
-                  S.coarse_start.as<int>(S.n), S.n, live);
+            BT_LAUNCH(ctx, batch_restrict<true>, S.coarse_blocks, kRestrictThreads, 0, st, E, ids,
+                      S.coarse_start.as<int>(S.n), S.n, live, held[l]);
     }
     if (B->n_tails)
         BT_LAUNCH(ctx, batch_tail, (unsigned)B->n_tails, kTailThreads, B->tail_smem, st,
@@ -3412,17 +3429,15 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                     e.x = L.x.as<double>(L.n);
                     e.x2 = L.x2.as<double>(L.n);
                     e.b = L.b.as<double>(L.n);
-                    e.r = L.r.as<double>(L.n);
                     e.F = bt::fine_of(L, C, five);
                     e.xc = C.x.as<double>(C.n);
                     e.bc = C.b.as<double>(C.n);
-                    e.ncn = C.n;
                     E.push_back(e);
                     S.cand.push_back((int)c);
                     S.nx.push_back((int)L.nx);
                     S.ny.push_back((int)L.ny);
-                    S.nodes.push_back((int)bt::blocks_for(L.n, bt::kBatchThreads));
-                    S.coarse.push_back((int)bt::blocks_for(C.n, bt::kBatchThreads));
+                    S.coarse.push_back((int)(((C.nx + bt::kRestrictX - 1) / bt::kRestrictX) *
+                                             ((C.ny + bt::kRestrictY - 1) / bt::kRestrictY)));
                 }
                 bt::upload(S.entries, E, st);
             }
