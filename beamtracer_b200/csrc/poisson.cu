@@ -570,8 +570,8 @@ __device__ __forceinline__ void smooth_staged_tile(
 // and only x goes through shared memory: a phase is eight (four) shared loads, the update and
 // a store.  Staging the coefficients through shared memory at sizes known at run time spent
 // 1,760 instructions a warp, most on indices, for some 300 of arithmetic: 10.3 us a launch of
-// a 9-point level, whatever its size, against REG9_US, and 12.0 for the finest level of
-// 801 x 201 against REG5_US.
+// a 9-point level, whatever its size, against 5.5 before the coarse correction and 6.3 after
+// it, and 12.0 for the finest level of 801 x 201 against 7.9 and 10.0.
 
 // One side of a fine-coarse pair's prolongation, as build_axis lays it out: the lower coarse
 // neighbour of fine node k and its weight.
@@ -739,8 +739,8 @@ __device__ __forceinline__ double apply5_item(i64 f, i64 nx, i64 ny, const doubl
 // kRestrictY coarse nodes, a thread a fine node with its row's loads all in flight, weighs
 // it (by the control volumes on level 0) into shared memory, and adds up each coarse node's
 // nine from there, the weights from build_axis's rule.  The blocks' edges are computed twice
-// (10 % of the rows); the residual never goes to memory and there is one launch of RESTRICT_US
-// where the two took 8 (the restriction alone 4.8: its nine loads waited for table entries).
+// (10 % of the rows); the residual never goes to memory and there is one launch of 4.2 us (5.1
+// for the finest level) where the two took 8 (the restriction alone 4.8: its nine loads waited for table entries).
 constexpr int kRestrictX = 8, kRestrictY = 16;
 constexpr int kRestrictFineX = 2 * kRestrictX + 1, kRestrictFineY = 2 * kRestrictY + 1;
 constexpr int kRestrictThreads = (kRestrictFineX * kRestrictFineY + 31) / 32 * 32;
@@ -1129,12 +1129,14 @@ __global__ void five_to_nine(i64 n, const double *__restrict__ c4, const double 
 // -- the small levels in one launch, in shared memory ---------------------------------------
 
 constexpr int kTailThreads = 1024;
+constexpr int kTailRegThreads = 512;
+constexpr int kTailRows = 2;  // rows of the inverse a warp applies at a time
 constexpr int kTailMaxLevels = 16;
 constexpr size_t kTailSmemMax = 200 * 1024;
 
 struct TailLevel {
     i64 nx, ny, n;
-    const double *a9;
+    const double *a9, *rdiag;
     const uint8_t *active;
     double *x, *b;  // the level's global vectors (read: b of the first, written: x of the first)
     Fine next;      // the map to the next coarser level (unused on the coarsest)
@@ -1167,16 +1169,37 @@ struct TailLayout {
     size_t total() const { return image() + sizeof(double) * (size_t)dynamic; }
 };
 
-__device__ __forceinline__ void tail_smooth(const TailPlan &P, const double *sm, double *smd,
-                                            const uint8_t *act, int colour, int tid, int nt) {
+// A thread's place among the nodes of a colour of a level: rows and columns of the even and
+// the odd columns' lists, found once for all of a level's phases.
+struct TailPlace {
+    int row[2], col[2];
+};
+__device__ __forceinline__ TailPlace tail_place(const TailPlan &P, int tid) {
+    TailPlace T;
+#pragma unroll
+    for (int cj = 0; cj < 2; ++cj) {
+        const int hy = (P.ny - cj + 1) >> 1;
+        T.row[cj] = tid / hy;
+        T.col[cj] = tid - T.row[cj] * hy;
+    }
+    return T;
+}
+
+__device__ __forceinline__ void tail_smooth(const TailPlan &P, const TailPlace &T, const double *sm,
+                                            double *smd, const uint8_t *act, int colour, int tid,
+                                            int nt) {
     const int nx = P.nx, ny = P.ny, n = P.n, W = ny + 2;
     const int ci = colour >> 1, cj = colour & 1;
     const int hx = (nx - ci + 1) >> 1, hy = (ny - cj + 1) >> 1;
     double *x = smd + P.x;
     const double *b = smd + P.b, *a9 = sm + P.a9, *rd = sm + P.rd;
+    int ti = cj ? T.row[1] : T.row[0], tj = cj ? T.col[1] : T.col[0];
     for (int t = tid; t < hx * hy; t += nt) {
-        const int ti = t / hy;
-        const int i = 2 * ti + ci, j = 2 * (t - ti * hy) + cj;
+        if (t != tid) {
+            ti = t / hy;
+            tj = t - ti * hy;
+        }
+        const int i = 2 * ti + ci, j = 2 * tj + cj;
         const int f = i * ny + j;
         if (!act[f]) continue;
         const int q = (i + 1) * W + j + 1;
@@ -1271,9 +1294,114 @@ __device__ __forceinline__ void tail_prolong(const TailPlan &P, const TailPlan &
     }
 }
 
+// The tail's first level in registers: a thread has one node of each colour, its row, b and
+// place in x's layout.  Read from shared memory instead, a phase of 180 nodes was 18 strided
+// loads a thread and took 1,175 cycles; 465 so.
+struct TailRegisters {
+    double coef[4][8], diag[4], rd[4], b[4];
+    int at[4], node[4];  // node -1: none, or a held one
+};
+
+__device__ __forceinline__ void tail_load(const TailLevel &L, TailRegisters &R, int tid) {
+    const int nx = (int)L.nx, ny = (int)L.ny, W = ny + 2;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int ci = k >> 1, cj = k & 1;
+        const int hx = (nx - ci + 1) >> 1, hy = (ny - cj + 1) >> 1;
+        const int ti = tid / hy, tj = tid - ti * hy;
+        const int i = 2 * ti + ci, j = 2 * tj + cj;
+        const bool in = tid < hx * hy;
+        const int f = in ? i * ny + j : 0;
+        const bool on = in && L.active[f] != 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) R.coef[k][q] = L.a9[(i64)(q < 4 ? q : q + 1) * L.n + f];
+        R.diag[k] = L.a9[4 * L.n + f];
+        R.rd[k] = L.rdiag[f];
+        R.b[k] = L.b[f];
+        R.at[k] = in ? (i + 1) * W + j + 1 : W + 1;
+        R.node[k] = on ? f : (in ? -2 - f : -1);  // -2 - f: held
+    }
+}
+
+// The eight neighbours of place q in x.
+__device__ __forceinline__ void tail_neighbours(const double *x, int W, double (&v)[8]) {
+    v[0] = x[-W - 1];
+    v[1] = x[-W];
+    v[2] = x[-W + 1];
+    v[3] = x[-1];
+    v[4] = x[1];
+    v[5] = x[W - 1];
+    v[6] = x[W];
+    v[7] = x[W + 1];
+}
+
+// A block's number in its cluster, the address of a shared variable in block `rank` of it, a
+// store there, and the cluster's barrier (which completes such stores).
+__device__ __forceinline__ int cluster_rank() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+__device__ __forceinline__ void remote_store(const double *p, int rank, double v) {
+    uint32_t at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(at)
+        : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+            : "memory");
+}
+
+// The coarsest level's inverse is applied by the other seven blocks of the tail's cluster,
+// their rows of it in registers from the launch on: one block alone read the inverse's 346 KB
+// (208 nodes) at 20 bytes a cycle, 18,000 of the tail's 39,000 cycles.  The first block sends
+// every helper b, the helpers send it x; a barrier each.
+constexpr int kTailCluster = 8;
+constexpr int kHelperRows = 3;  // rows a helper's warp: 256 / 7 blocks / 16 warps, rounded up
+
+__device__ __forceinline__ void tail_helper(const TailLevel &L, const TailPlan &C,
+                                            const double *__restrict__ inv, double *smd, int rank) {
+    const int n = C.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int warps = kTailRegThreads / 32 * (kTailCluster - 1);
+    const int first = (rank - 1) * (kTailRegThreads / 32) + warp;  // rows first, first + warps, ..
+    constexpr int kChunks = kCoarsest / 32;
+    double m[kHelperRows][kChunks];
+    bool on[kHelperRows];
+#pragma unroll
+    for (int k = 0; k < kHelperRows; ++k) {
+        const int row = first + k * warps;
+        on[k] = row < n && L.active[row] != 0;
+#pragma unroll
+        for (int e = 0; e < kChunks; ++e) {
+            const int c = lane + 32 * e;
+            m[k][e] = row < n && c < n ? __ldg(inv + (i64)row * n + c) : 0.0;
+        }
+    }
+    cluster_barrier();  // b is here
+    const double *b = smd + C.b;
+#pragma unroll
+    for (int k = 0; k < kHelperRows; ++k) {
+        const int row = first + k * warps;
+        double s = 0.0;
+#pragma unroll
+        for (int e = 0; e < kChunks; ++e)
+            s = fma(m[k][e], lane + 32 * e < n ? b[lane + 32 * e] : 0.0, s);
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+        if (lane == 0 && row < n)
+            remote_store(smd + C.x + row + 2 * (row / C.ny) + C.ny + 3, 0, on[k] ? s : 0.0);
+    }
+    cluster_barrier();  // x is there
+}
+
 // levels[0] reads b from, and writes x to, global memory; `image` holds the static part
 // of the shared memory (image_words 16-byte words); inv is the coarsest level's inverse.
+// REG: a colour of the first level fits the block's threads, which hold it in registers;
+// CLUSTER: the blocks of a cluster, whose other blocks are tail_helpers.
 // (The body of vcycle_tail and of its batched form.)
+template <bool REG, bool CLUSTER>
 __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ levels,
                                                 const TailPlan *__restrict__ plans, int count,
                                                 const uint4 *__restrict__ image,
@@ -1285,50 +1413,129 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     uint8_t *smb = reinterpret_cast<uint8_t *>(smi + ints);
     double *smd = sm + 2 * image_words;  // the dynamic doubles follow the image
     const int tid = threadIdx.x, nt = blockDim.x;
+    if (CLUSTER) {
+        const int rank = cluster_rank();
+        if (rank != 0) {
+            tail_helper(levels[count - 1], plans[count - 1], inv, smd, rank);
+            return;
+        }
+    }
+    TailRegisters R;
+    if (REG && count > 1) tail_load(levels[0], R, tid);
     {
         const int *src = reinterpret_cast<const int *>(plans);
         int *dst = reinterpret_cast<int *>(plan);
         const int words = count * (int)(sizeof(TailPlan) / sizeof(int));
         for (int e = tid; e < words; e += nt) dst[e] = src[e];
     }
-    // the static image in one piece, x zero, level 0's b
+    // the static image in one piece (its first doubles are the first level's ten coefficients
+    // a node, held in registers with REG), x zero, level 0's b
     uint4 *dst = reinterpret_cast<uint4 *>(sm);
+    const int skip = REG && count > 1 ? 5 * plans[0].n : 0;
 #pragma unroll 4
-    for (int e = tid; e < image_words; e += nt) dst[e] = image[e];
+    for (int e = skip + tid; e < image_words; e += nt) dst[e] = image[e];
     for (int l = 0; l < count; ++l) {
         const TailPlan &P = plans[l];
         for (int e = tid; e < (P.nx + 2) * (P.ny + 2); e += nt) smd[P.x + e] = 0.0;
     }
-    {
+    if (!REG || count == 1) {
         const TailPlan &P = plans[0];
         const double *b0 = levels[0].b;
         for (int f = tid; f < P.n; f += nt) smd[P.b + f] = b0[f];
     }
     __syncthreads();
+    // one colour phase of the first level
+    auto phase = [&](double *x, int W, int k) {
+        if (R.node[k] >= 0) {
+            double v[8];
+            tail_neighbours(x + R.at[k], W, v);
+            x[R.at[k]] = update9(R.b[k], R.coef[k], v, R.rd[k]);
+        }
+        __syncthreads();
+    };
     for (int l = 0; l + 1 < count; ++l) {
         const TailPlan &P = plan[l];
         const uint8_t *act = smb + P.act;
-        for (int s = 0; s < sweeps; ++s)
-            for (int c = 0; c < 4; ++c) {
-                tail_smooth(P, sm, smd, act, c, tid, nt);
-                __syncthreads();
+        if (REG && l == 0) {
+            double *x = smd + P.x, *r = smd + P.r;
+            const int W = P.ny + 2;
+            for (int s = 0; s < sweeps; ++s) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) phase(x, W, c);
             }
-        tail_residual(P, sm, smd, act, tid, nt);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (R.node[k] >= 0) {
+                    double v[8];
+                    tail_neighbours(x + R.at[k], W, v);
+                    double p = fma(-R.diag[k], x[R.at[k]], R.b[k]), q = R.coef[k][7] * v[7];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) p = fma(-R.coef[k][e], v[e], p);
+#pragma unroll
+                    for (int e = 4; e < 7; ++e) q = fma(R.coef[k][e], v[e], q);
+                    r[R.node[k]] = p - q;
+                } else if (R.node[k] <= -2) {
+                    r[-2 - R.node[k]] = 0.0;
+                }
+            }
+        } else {
+            const TailPlace T = tail_place(P, tid);
+            for (int s = 0; s < sweeps; ++s)
+                for (int c = 0; c < 4; ++c) {
+                    tail_smooth(P, T, sm, smd, act, c, tid, nt);
+                    __syncthreads();
+                }
+            tail_residual(P, sm, smd, act, tid, nt);
+        }
         __syncthreads();
         tail_restrict(P, plan[l + 1], sm, smd, smi, act, tid, nt);
         __syncthreads();
     }
-    {
-        // the coarsest level: x = inv b, a warp per row, its lanes over the columns
+    if (CLUSTER) {
         const TailPlan &C = plan[count - 1];
-        const int n = C.n, W = C.ny + 2, lane = tid & 31;
+        for (int e = tid; e < C.n * (kTailCluster - 1); e += nt) {
+            const int rank = 1 + e / C.n, f = e - (rank - 1) * C.n;
+            remote_store(smd + C.b + f, rank, smd[C.b + f]);
+        }
+        cluster_barrier();
+        cluster_barrier();
+    } else {
+        // the coarsest level: x = inv b, a warp kTailRows rows at a time, its lanes over the
+        // columns
+        const TailPlan &C = plan[count - 1];
+        const int n = C.n, W = C.ny + 2, lane = tid & 31, warps = nt >> 5;
         const double *b = smd + C.b;
         const uint8_t *act = smb + C.act;
-        for (int row = tid >> 5; row < n; row += nt >> 5) {
-            double s = 0.0;
-            for (int c = lane; c < n; c += 32) s += __ldg(inv + (i64)row * n + c) * b[c];
-            for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-            if (lane == 0) smd[C.x + row + 2 * (row / C.ny) + W + 1] = act[row] ? s : 0.0;
+        constexpr int kChunks = kCoarsest / 32;
+        for (int row = tid >> 5; row < n; row += kTailRows * warps) {
+            double s[kTailRows], m[kTailRows][kChunks];
+#pragma unroll
+            for (int e = 0; e < kChunks; ++e) {
+                const int c = lane + 32 * e;
+#pragma unroll
+                for (int k = 0; k < kTailRows; ++k)
+                    m[k][e] = c < n && row + k * warps < n
+                                  ? __ldg(inv + (i64)(row + k * warps) * n + c) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kTailRows; ++k) s[k] = 0.0;
+#pragma unroll
+            for (int e = 0; e < kChunks; ++e) {
+                const double v = lane + 32 * e < n ? b[lane + 32 * e] : 0.0;
+#pragma unroll
+                for (int k = 0; k < kTailRows; ++k) s[k] = fma(m[k][e], v, s[k]);
+            }
+            for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+                for (int k = 0; k < kTailRows; ++k) s[k] += __shfl_down_sync(0xffffffffu, s[k], off);
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int k = 0; k < kTailRows; ++k) {
+                    const int r = row + k * warps;
+                    if (r < n) smd[C.x + r + 2 * (r / C.ny) + W + 1] = act[r] ? s[k] : 0.0;
+                }
+            }
         }
         __syncthreads();
     }
@@ -1337,11 +1544,20 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         const uint8_t *act = smb + P.act;
         tail_prolong(P, plan[l + 1], sm, smd, smi, act, tid, nt);
         __syncthreads();
-        for (int s = 0; s < sweeps; ++s)
-            for (int c = 3; c >= 0; --c) {
-                tail_smooth(P, sm, smd, act, c, tid, nt);
-                __syncthreads();
+        if (REG && l == 0) {
+            double *x = smd + P.x;
+            for (int s = 0; s < sweeps; ++s) {
+#pragma unroll
+                for (int c = 3; c >= 0; --c) phase(x, P.ny + 2, c);
             }
+        } else {
+            const TailPlace T = tail_place(P, tid);
+            for (int s = 0; s < sweeps; ++s)
+                for (int c = 3; c >= 0; --c) {
+                    tail_smooth(P, T, sm, smd, act, c, tid, nt);
+                    __syncthreads();
+                }
+        }
     }
     {
         const TailPlan &P = plan[0];
@@ -1351,12 +1567,24 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     }
 }
 
+__global__ void __launch_bounds__(kTailRegThreads, 1) __cluster_dims__(kTailCluster, 1, 1)
+    vcycle_tail_cluster(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans,
+                        int count, const uint4 *__restrict__ image, int image_words, int doubles,
+                        int ints, const double *__restrict__ inv, int sweeps) {
+    vcycle_tail_run<true, true>(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
+}
+
 __global__ void __launch_bounds__(kTailThreads, 1)
 vcycle_tail(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans, int count,
             const uint4 *__restrict__ image, int image_words, int doubles, int ints,
             const double *__restrict__ inv, int sweeps) {
-    vcycle_tail_run(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
+    vcycle_tail_run<false, false>(levels, plans, count, image, image_words, doubles, ints, inv,
+                                  sweeps);
 }
+
+// Whether a tail of this first level takes the register form: a colour of it fits 512 threads,
+// which have the registers for four rows each.
+bool tail_in_registers(i64 nx, i64 ny) { return ((nx + 1) / 2) * ((ny + 1) / 2) <= kTailRegThreads; }
 
 // The shared-memory layout of tail levels first .. (the coarsest): the static image
 // (coefficients of every level but the coarsest, transfer tables, active flags), then the
@@ -2038,6 +2266,7 @@ void setup_tail(bt_poisson *p) {
         t.ny = L.ny;
         t.n = L.n;
         t.a9 = L.a9.as<double>(9 * L.n);
+        t.rdiag = L.rdiag.as<double>(L.n);
         t.active = L.active.as<uint8_t>(L.n);
         t.x = L.x.as<double>(L.n);
         t.b = L.b.as<double>(L.n);
@@ -2045,6 +2274,8 @@ void setup_tail(bt_poisson *p) {
         tail.push_back(t);
     }
     // the largest any solver asks for: solvers of other meshes may launch concurrently
+    BT_CUDA(cudaFuncSetAttribute(vcycle_tail_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kTailSmemMax));
     BT_CUDA(cudaFuncSetAttribute(vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTailSmemMax));
     BT_CUDA(cudaMemcpy(p->tail_levels.as<TailLevel>(tail.size()), tail.data(),
@@ -2188,11 +2419,17 @@ void vcycle(bt_poisson *p, size_t l) {
     if ((int)l == p->tail_start) {
         const int count = (int)(p->levels.size() - l);
         const Level &Lc = p->levels.back();
-        BT_LAUNCH(p->ctx, vcycle_tail, 1, kTailThreads, p->tail_smem, st,
-                  p->tail_levels.as<TailLevel>(count), p->tail_plans.as<TailPlan>(count), count,
-                  static_cast<const uint4 *>(p->tail_image.get(16 * (size_t)p->tail_words)),
-                  p->tail_words, p->tail_doubles, p->tail_ints, p->inv.as<double>(Lc.n * Lc.n),
-                  p->coarse_sweeps);
+        const auto launch = [&](auto kernel, int blocks, int threads) {
+            BT_LAUNCH(p->ctx, kernel, blocks, threads, p->tail_smem, st,
+                      p->tail_levels.as<TailLevel>(count), p->tail_plans.as<TailPlan>(count), count,
+                      static_cast<const uint4 *>(p->tail_image.get(16 * (size_t)p->tail_words)),
+                      p->tail_words, p->tail_doubles, p->tail_ints, p->inv.as<double>(Lc.n * Lc.n),
+                      p->coarse_sweeps);
+        };
+        if (tail_in_registers(L.nx, L.ny))
+            launch(vcycle_tail_cluster, kTailCluster, kTailRegThreads);
+        else
+            launch(vcycle_tail, 1, kTailThreads);
         return;
     }
     if (l + 1 == p->levels.size()) {
@@ -2911,12 +3148,13 @@ __global__ void __launch_bounds__(kRestrictThreads)
 }
 
 // Every candidate's coarse levels, one block each.
-__global__ void __launch_bounds__(kTailThreads, 1)
+template <bool REG>
+__global__ void __launch_bounds__(REG ? kTailRegThreads : kTailThreads, 1)
     batch_tail(const BatchTail *__restrict__ T, const int *__restrict__ ids,
                const uint8_t *__restrict__ live) {
     const BatchTail &t = T[ids[blockIdx.x]];
     if (!live[t.cand]) return;
-    vcycle_tail_run(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
+    vcycle_tail_run<REG, false>(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
                     t.sweeps);
 }
 
@@ -3100,6 +3338,7 @@ struct bt_poisson_batch {
     std::vector<Step> level;
     bt::Buffer tails, tail_ids;  // one block per live candidate
     int n_tails = 0;
+    bool tail_reg = true;        // every candidate's tail takes the register form
     size_t tail_smem = 0;
     bt::Buffer fine, fine_ids, fine_start;
     std::vector<bt::BatchFine> fine_host;  // the device table's copy
@@ -3289,8 +3528,12 @@ void batch_vcycle(bt_poisson_batch *B) {
             BT_LAUNCH(ctx, batch_restrict<true>, S.coarse_blocks, kRestrictThreads, 0, st, E, ids,
                       S.coarse_start.as<int>(S.n), S.n, live, held[l]);
     }
-    if (B->n_tails)
-        BT_LAUNCH(ctx, batch_tail, (unsigned)B->n_tails, kTailThreads, B->tail_smem, st,
+    if (B->n_tails && B->tail_reg)
+        BT_LAUNCH(ctx, batch_tail<true>, (unsigned)B->n_tails, kTailRegThreads, B->tail_smem, st,
+                  B->tails.as<BatchTail>(B->solvers.size()), B->tail_ids.as<int>(B->n_tails),
+                  live);
+    else if (B->n_tails)
+        BT_LAUNCH(ctx, batch_tail<false>, (unsigned)B->n_tails, kTailThreads, B->tail_smem, st,
                   B->tails.as<BatchTail>(B->solvers.size()), B->tail_ids.as<int>(B->n_tails),
                   live);
     for (int l = B->steps - 1; l >= 0; --l) {
@@ -3403,6 +3646,8 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                            "poisson batch: a candidate's mesh is too small for the batched cycle");
                 B->steps = std::max(B->steps, p->tail_start);
                 B->tail_smem = std::max(B->tail_smem, p->tail_smem);
+                B->tail_reg &= bt::tail_in_registers(p->levels[p->tail_start].nx,
+                                                     p->levels[p->tail_start].ny);
             }
             B->level.resize(B->steps);
             for (int l = 0; l < B->steps; ++l) {
@@ -3493,7 +3738,9 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)bt::kTailSmemMax));
+                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)bt::kTailSmemMax));
             }
             for (auto &e : B->ev) BT_CUDA(cudaEventCreate(&e));
