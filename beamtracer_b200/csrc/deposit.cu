@@ -17,8 +17,13 @@ namespace bt {
 namespace {
 
 constexpr int kThreads = 256;  // = the radix (one thread per digit in the scans)
-constexpr int kItems = 16;
-constexpr int kTile = kThreads * kItems;
+// A tile's records a thread.  A sort of up to kSmallSort records takes half the tile: its few
+// blocks leave most of the chip idle and a block's time is the latency of ranking its items
+// one after another (a deposit of 20,000 charges 53 us against 60).  A larger one keeps the
+// longer tile, whose histograms are half as many (a million charges 99 us against 102).
+constexpr int kItems = 16, kSmallItems = 8;
+constexpr i64 kSmallSort = (i64)1 << 18;
+__host__ __device__ constexpr int tile_of(int items) { return kThreads * items; }
 constexpr int kRadix = 256;      // 8-bit digits
 constexpr int kRadixMax = 1024;  // up to 10-bit digits, when they save a pass
 constexpr int kWarps = kThreads / 32;
@@ -32,7 +37,7 @@ __device__ __forceinline__ i64 record_count(i64 n, const i64 *n_dev) { return n_
 // the counts and the output; kNoSkip leaves none out.
 constexpr uint32_t kNoSkip = 0xffffffffu;
 
-template <int R>
+template <int R, int ITEMS>
 __global__ void radix_hist(const uint32_t *__restrict__ keys, i64 n_host,
                            const i64 *__restrict__ n_dev, uint32_t skip, int shift,
                            uint32_t *__restrict__ hist, int nblocks) {
@@ -40,15 +45,15 @@ __global__ void radix_hist(const uint32_t *__restrict__ keys, i64 n_host,
     const i64 n = record_count(n_host, n_dev);
     for (int d = threadIdx.x; d < R; d += kThreads) h[d] = 0;
     __syncthreads();
-    const i64 base = (i64)blockIdx.x * kTile;
-    uint32_t key[kItems];
+    const i64 base = (i64)blockIdx.x * tile_of(ITEMS);
+    uint32_t key[ITEMS];
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {  // the loads first, all in flight
+    for (int i = 0; i < ITEMS; ++i) {  // the loads first, all in flight
         const i64 r = base + (i64)i * kThreads + threadIdx.x;
         key[i] = r < n ? keys[r] : skip;
     }
 #pragma unroll
-    for (int i = 0; i < kItems; ++i)
+    for (int i = 0; i < ITEMS; ++i)
         if (key[i] != skip) atomicAdd(&h[(key[i] >> shift) & (R - 1)], 1u);
     __syncthreads();
     for (int d = threadIdx.x; d < R; d += kThreads) hist[(i64)d * nblocks + blockIdx.x] = h[d];
@@ -79,11 +84,18 @@ __device__ uint32_t block_inclusive_scan(uint32_t v, uint32_t *warp_sums) {
     return out;
 }
 
-// Row d of hist (one digit over all blocks) to its exclusive prefix; the row total.
-__global__ void radix_row_scan(const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs,
-                               uint32_t *__restrict__ totals, int nblocks) {
+// Row d of hist (one digit over all blocks) to its exclusive prefix, the row's total; then, in
+// the block that finishes last (a ticket counter, reset by it), the exclusive prefix of the R
+// totals, thread t scanning digits t * R / kThreads onwards.  `count`, when not NULL, gets the
+// number of records the pass sorts.
+template <int R>
+__global__ void __launch_bounds__(kThreads) radix_row_scan(
+    const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs, uint32_t *__restrict__ totals,
+    int nblocks, uint32_t *__restrict__ base, i64 *__restrict__ count,
+    unsigned *__restrict__ ticket) {
     __shared__ uint32_t warp_sums[kWarps];
     __shared__ uint32_t carry;
+    __shared__ bool is_last;
     const i64 row = (i64)blockIdx.x * nblocks;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -97,21 +109,20 @@ __global__ void radix_row_scan(const uint32_t *__restrict__ hist, uint32_t *__re
         if (threadIdx.x == kThreads - 1) carry = c + incl;
         __syncthreads();
     }
-    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
-}
-
-// Exclusive prefix of the R digit totals; thread t scans digits t * R / kThreads onwards.
-// `count`, when not NULL, gets the number of records the pass sorts.
-template <int R>
-__global__ void radix_digit_base(const uint32_t *__restrict__ totals, uint32_t *__restrict__ base,
-                                 i64 *__restrict__ count) {
-    __shared__ uint32_t warp_sums[kWarps];
+    if (threadIdx.x == 0) {
+        totals[blockIdx.x] = carry;
+        __threadfence();
+        is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
     constexpr int D = R / kThreads;
     uint32_t mine[D];
     uint32_t v = 0;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        mine[k] = totals[threadIdx.x * D + k];
+        mine[k] = __ldcg(totals + threadIdx.x * D + k);
         v += mine[k];
     }
     const uint32_t inclusive = block_inclusive_scan(v, warp_sums);
@@ -121,26 +132,43 @@ __global__ void radix_digit_base(const uint32_t *__restrict__ totals, uint32_t *
         base[threadIdx.x * D + k] = run;
         run += mine[k];
     }
+    if (threadIdx.x == 0) *ticket = 0u;
     if (count && threadIdx.x == kThreads - 1) *count = inclusive;
 }
 
-// Stable scatter of one tile of kTile records.  Warp w ranks the tile's items
-// [w * kTile / kWarps, (w + 1) * kTile / kWarps) in order, 32 at a time (peers of a digit
-// by __match_any_sync, a running count per warp and digit in shared memory: no block
+// The lanes whose valid digit (of R values) is this lane's: a vote a bit, independent of one
+// another.  With the warp's match instruction, which is a chain of its own for every item, a
+// deposit of four million charges took 287 us; 254 so.
+template <int R>
+__device__ __forceinline__ unsigned digit_peers(uint32_t d, bool valid) {
+    unsigned peers = __ballot_sync(kFull, valid);
+#pragma unroll
+    for (int b = 1; b < R; b <<= 1) {
+        const bool bit = (d & b) != 0;
+        const unsigned v = __ballot_sync(kFull, bit);
+        peers &= bit ? v : ~v;
+    }
+    return peers;
+}
+
+// Stable scatter of one tile of records.  Warp w ranks the tile's items
+// [w * tile / kWarps, (w + 1) * tile / kWarps) in order, 32 at a time (peers of a digit
+// by votes, a running count per warp and digit in shared memory: no block
 // barrier in the loop); the counts are then turned into per-warp offsets in warp order and
 // the tile's digit starts, the tile is sorted by digit in shared memory, and written out in
 // order, so that the records of one digit go to consecutive addresses (coalesced runs).
 // The shared array first holds the counts, then the sorted tile.
-template <int R>
+template <int R, int ITEMS>
 __global__ void __launch_bounds__(kThreads) radix_scatter(
     const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in, i64 n_host,
     const i64 *__restrict__ n_dev, uint32_t skip, int shift, const uint32_t *__restrict__ offs,
     const uint32_t *__restrict__ base, int nblocks, uint32_t *__restrict__ keys_out,
     uint32_t *__restrict__ vals_out) {
-    static_assert(kWarps * R * 4 <= kTile * 8, "the counts must fit the tile's space");
+    constexpr int kTileSize = tile_of(ITEMS);
+    constexpr int kSpace = kWarps * R > 2 * kTileSize ? kWarps * R : 2 * kTileSize;
     constexpr int D = R / kThreads;             // digits a thread scans
-    constexpr int kPerWarp = kTile / kWarps;    // items a warp ranks
-    __shared__ __align__(16) uint32_t space[2 * kTile];  // counts [kWarps][R], then the tile
+    constexpr int kPerWarp = kTileSize / kWarps;    // items a warp ranks
+    __shared__ __align__(16) uint32_t space[kSpace];  // counts [kWarps][R], then the tile
     __shared__ uint32_t start[R];               // the tile's first slot of each digit
     __shared__ uint32_t run[R];                 // the digit's first global slot for this tile
     __shared__ uint32_t warp_sums[kWarps];
@@ -150,25 +178,25 @@ __global__ void __launch_bounds__(kThreads) radix_scatter(
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int d = t; d < kWarps * R; d += kThreads) count[d] = 0;
     __syncthreads();
-    const i64 tile = (i64)blockIdx.x * kTile;
+    const i64 tile = (i64)blockIdx.x * kTileSize;
     const unsigned below = (1u << lane) - 1u;
-    uint32_t key[kItems], val[kItems], pos[kItems];
+    uint32_t key[ITEMS], val[ITEMS], pos[ITEMS];
     unsigned valid_mask = 0;  // bit i: item i is sorted
     // every load of the tile first (all in flight at once), then the ranking
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const i64 r = tile + (i64)warp * kPerWarp + (i64)i * 32 + lane;
         key[i] = r < n ? keys_in[r] : skip;
         val[i] = r < n ? (vals_in ? vals_in[r] : (uint32_t)r) : 0u;
     }
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const i64 r = tile + (i64)warp * kPerWarp + (i64)i * 32 + lane;
         const bool valid = r < n && key[i] != skip;
         if (valid) valid_mask |= 1u << i;
         if (!valid) val[i] = 0u;
         const uint32_t d = (key[i] >> shift) & (R - 1);
-        const unsigned peers = __match_any_sync(kFull, valid ? d : 0xffffffffu);
+        const unsigned peers = digit_peers<R>(d, valid);
         uint32_t *c = count + warp * R + d;
         const uint32_t before = valid ? *c : 0u;
         pos[i] = before + __popc(peers & below);
@@ -206,16 +234,16 @@ __global__ void __launch_bounds__(kThreads) radix_scatter(
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         if (valid_mask & (1u << i)) {
             const uint32_t d = (key[i] >> shift) & (R - 1);
             pos[i] += start[d] + count[warp * R + d];
         }
     }
     __syncthreads();  // the counts are read: the space takes the sorted tile
-    uint32_t *skey = space, *sval = space + kTile;
+    uint32_t *skey = space, *sval = space + kTileSize;
 #pragma unroll
-    for (int i = 0; i < kItems; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         if (valid_mask & (1u << i)) {
             skey[pos[i]] = key[i];
             sval[pos[i]] = val[i];
@@ -418,17 +446,17 @@ int bits_for(uint64_t max_key) {
 
 // One stable pass on the digit of R values at `shift`.
 // `skip`: the key the pass leaves out; `count`, when not NULL, gets the records it sorted.
-template <int R>
+template <int R, int ITEMS>
 void sort_pass(bt_ctx *ctx, const uint32_t *src_k, const uint32_t *src_v, i64 n,
                const i64 *n_dev, uint32_t skip, int shift, uint32_t *hist, uint32_t *offs,
-               uint32_t *totals, uint32_t *digit, i64 *count, int nblocks, uint32_t *dst_k,
-               uint32_t *dst_v) {
+               uint32_t *totals, uint32_t *digit, unsigned *ticket, i64 *count, int nblocks,
+               uint32_t *dst_k, uint32_t *dst_v) {
     cudaStream_t st = ctx->stream;
-    BT_LAUNCH(ctx, radix_hist<R>, nblocks, kThreads, 0, st, src_k, n, n_dev, skip, shift, hist,
-              nblocks);
-    BT_LAUNCH(ctx, radix_row_scan, R, kThreads, 0, st, hist, offs, totals, nblocks);
-    BT_LAUNCH(ctx, radix_digit_base<R>, 1, kThreads, 0, st, totals, digit, count);
-    BT_LAUNCH(ctx, radix_scatter<R>, nblocks, kThreads, 0, st, src_k, src_v, n, n_dev, skip,
+    BT_LAUNCH(ctx, (radix_hist<R, ITEMS>), nblocks, kThreads, 0, st, src_k, n, n_dev, skip, shift,
+              hist, nblocks);
+    BT_LAUNCH(ctx, radix_row_scan<R>, R, kThreads, 0, st, hist, offs, totals, nblocks, digit, count,
+              ticket);
+    BT_LAUNCH(ctx, (radix_scatter<R, ITEMS>), nblocks, kThreads, 0, st, src_k, src_v, n, n_dev, skip,
               shift, offs, digit, nblocks, dst_k, dst_v);
 }
 
@@ -437,13 +465,20 @@ void radix_sort_pairs(bt_ctx *ctx, const uint32_t *keys_in, i64 n, const i64 *n_
                       const i64 **count_out) {
     BT_REQUIRE(n < (i64)0xffffffffLL, "radix sort: too many records for 32-bit indices");
     DepositScratch &s = ctx->deposit;
-    const int nblocks = (int)((n + kTile - 1) / kTile);
+    const bool small = n <= kSmallSort;
+    const i64 tile = tile_of(small ? kSmallItems : kItems);
+    const int nblocks = (int)((n + tile - 1) / tile);
     uint32_t *ka = s.keys_alt.as<uint32_t>(n), *va = s.vals.as<uint32_t>(n);
     uint32_t *kb = s.keys.as<uint32_t>(n), *vb = s.vals_alt.as<uint32_t>(n);
     uint32_t *hist = s.hist.as<uint32_t>((size_t)kRadixMax * nblocks);
     uint32_t *offs = s.row_offsets.as<uint32_t>((size_t)kRadixMax * nblocks);
-    uint32_t *digit = s.digit_base.as<uint32_t>(2 * kRadixMax);
+    uint32_t *digit = s.digit_base.as<uint32_t>(2 * kRadixMax + 1);
     uint32_t *totals = digit + kRadixMax;
+    unsigned *ticket = totals + kRadixMax;  // zero between passes
+    if (!s.ticket_ready) {
+        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), ctx->stream));
+        s.ticket_ready = true;
+    }
     i64 *sorted = s.sorted.as<i64>(1);  // the records left after the first pass
     const uint32_t *src_k = keys_in;
     const uint32_t *src_v = nullptr;
@@ -462,15 +497,16 @@ void radix_sort_pairs(bt_ctx *ctx, const uint32_t *keys_in, i64 n, const i64 *n_
         const i64 *count = p == 0 ? n_dev : sorted;
         const uint32_t leave = p == 0 ? skip : kNoSkip;
         i64 *out = p == 0 ? sorted : nullptr;
+        const auto pass = [&](auto run) {
+            run(ctx, src_k, src_v, n, count, leave, shift, hist, offs, totals, digit, ticket, out,
+                nblocks, dst_k, dst_v);
+        };
         if (bits == 10)
-            sort_pass<1024>(ctx, src_k, src_v, n, count, leave, shift, hist, offs, totals,
-                            digit, out, nblocks, dst_k, dst_v);
+            small ? pass(sort_pass<1024, kSmallItems>) : pass(sort_pass<1024, kItems>);
         else if (bits == 9)
-            sort_pass<512>(ctx, src_k, src_v, n, count, leave, shift, hist, offs, totals, digit,
-                           out, nblocks, dst_k, dst_v);
+            small ? pass(sort_pass<512, kSmallItems>) : pass(sort_pass<512, kItems>);
         else
-            sort_pass<256>(ctx, src_k, src_v, n, count, leave, shift, hist, offs, totals, digit,
-                           out, nblocks, dst_k, dst_v);
+            small ? pass(sort_pass<256, kSmallItems>) : pass(sort_pass<256, kItems>);
         BT_CHECK_LAUNCH();
         src_k = dst_k;
         src_v = dst_v;
@@ -579,7 +615,7 @@ namespace {
 
 constexpr i64 kNoallocPoints = 65536;  // at most this many charges per call
 constexpr i64 kNoallocNodes = 65536;   // and a mesh of at most this many nodes
-constexpr i64 kNoallocBlocks = (kNoallocPoints + kTile - 1) / kTile;
+constexpr i64 kNoallocBlocks = (kNoallocPoints + tile_of(kSmallItems) - 1) / tile_of(kSmallItems);
 constexpr i64 kNoallocWarps = (kNoallocPoints + 31) / 32;
 
 constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -589,7 +625,7 @@ constexpr size_t kOffKeys = 0;  // keys, keys_alt, vals, vals_alt (u32)
 constexpr size_t kOffPayload = kOffKeys + align256(4 * 4 * kNoallocPoints);  // records
 constexpr size_t kOffHist = kOffPayload + align256(32 * kNoallocPoints);  // hist, offs
 constexpr size_t kOffDigits = kOffHist + align256(2 * 4 * kRadix * kNoallocBlocks);
-constexpr size_t kOffCells = kOffDigits + align256(2 * 4 * kRadix);
+constexpr size_t kOffCells = kOffDigits + align256(4 * (2 * kRadix + 1));
 constexpr size_t kOffWarps = kOffCells + align256(32 * kNoallocNodes);  // first, last
 constexpr size_t kOffFlags = kOffWarps + align256(2 * 32 * kNoallocWarps);
 constexpr size_t kNoallocBytes = kOffFlags + align256(2 * kNoallocWarps);
@@ -639,6 +675,8 @@ extern "C" int bt_deposit_trajectories_2d_noalloc(void *stream, const double *px
         uint32_t *offs = hist + kRadix * kNoallocBlocks;
         uint32_t *digit = reinterpret_cast<uint32_t *>(base + kOffDigits);
         uint32_t *totals = digit + kRadix;
+        unsigned *ticket = totals + kRadix;
+        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
         double4 *cells = reinterpret_cast<double4 *>(base + kOffCells);
         double4 *first = reinterpret_cast<double4 *>(base + kOffWarps);
         double4 *last = first + kNoallocWarps;
@@ -648,20 +686,18 @@ extern "C" int bt_deposit_trajectories_2d_noalloc(void *stream, const double *px
         point_records<<<blocks_for(n, 256), 256, 0, st>>>(px, py, q, n, origin_x, origin_y, h,
                                                           cylindrical, nx, ny, keys, rec);
         // the stable radix sort, ping-ponging between the key and value arrays
-        const int nblocks = (int)((n + kTile - 1) / kTile);
+        const int nblocks = (int)((n + tile_of(kSmallItems) - 1) / tile_of(kSmallItems));
         const int passes = (bits_for(sentinel) + 7) / 8;
         const uint32_t *src_k = keys, *src_v = nullptr;
         uint32_t *dst_k = keys_alt, *dst_v = vals;
         for (int pass = 0; pass < passes; ++pass) {
             const int shift = 8 * pass;
-            radix_hist<kRadix><<<nblocks, kThreads, 0, st>>>(src_k, n, nullptr, kNoSkip, shift,
-                                                             hist, nblocks);
-            radix_row_scan<<<kRadix, kThreads, 0, st>>>(hist, offs, totals, nblocks);
-            radix_digit_base<kRadix><<<1, kThreads, 0, st>>>(totals, digit, nullptr);
-            radix_scatter<kRadix><<<nblocks, kThreads, 0, st>>>(src_k, src_v, n, nullptr, kNoSkip,
-                                                                shift,
-                                                                offs, digit, nblocks, dst_k,
-                                                                dst_v);
+            radix_hist<kRadix, kSmallItems><<<nblocks, kThreads, 0, st>>>(
+                src_k, n, nullptr, kNoSkip, shift, hist, nblocks);
+            radix_row_scan<kRadix><<<kRadix, kThreads, 0, st>>>(hist, offs, totals, nblocks, digit,
+                                                               nullptr, ticket);
+            radix_scatter<kRadix, kSmallItems><<<nblocks, kThreads, 0, st>>>(
+                src_k, src_v, n, nullptr, kNoSkip, shift, offs, digit, nblocks, dst_k, dst_v);
             src_k = dst_k;
             src_v = dst_v;
             if (dst_k == keys_alt) {
