@@ -1114,16 +1114,17 @@ void trace_all(bt_ctx *ctx, const bt_trace_args *args, const bt_magnetic *mag, i
                     // none: 255 registers let the lookups' chains run side by side (20,000
                     // rings, 157 blocks: 132 us a window against 159 with 168 registers).
                     // A larger one hides latency with a third block (40,000 rings: 7.3 ms a
-                    // trace against 8.3), as do the magnetic trace's (52 ms against 64) and a
-                    // batch's thousands of blocks.
-                    const bool wide = !mag && !batch && grid <= (unsigned)(2 * ctx->num_sms);
+                    // trace against 8.3), as do the magnetic trace's (52 ms against 64).  A
+                    // batch's windows come down to the first kind as its candidates finish.
+                    const bool wide = !mag && grid <= (unsigned)(2 * ctx->num_sms);
 #define BT_TRACE_CASE_N(C, I, G, M, B, N)                                                       \
     if (a.cylindrical == C && (a.integrator != 0) == (I != 0) && general == G &&                 \
         (mag != nullptr) == M && (batch != nullptr) == B && wide == (N == 2))                    \
         BT_LAUNCH(ctx, (bt::trace_window<C, I, G, M, B, N>), grid, 128, 0, st, tr, act_a,         \
                   live + lv, bound, S, keys[cur] + used, rec[cur] + used, sentinel,               \
                   records_end + cur, used + need, block_live, alive);
-#define BT_TRACE_CASE_B(C, I, G, M, B) BT_TRACE_CASE_N(C, I, G, M, B, 3)
+#define BT_TRACE_CASE_B(C, I, G, M, B)                                                          \
+    BT_TRACE_CASE_N(C, I, G, M, B, 3) BT_TRACE_CASE_N(C, I, G, M, B, 2)
 #define BT_TRACE_CASE(C, I, G, M)                                                               \
     BT_TRACE_CASE_N(C, I, G, M, false, 3)                                                         \
     if (!M) { BT_TRACE_CASE_N(C, I, G, false, false, 2) }
