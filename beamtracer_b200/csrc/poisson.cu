@@ -236,13 +236,14 @@ __device__ __forceinline__ void axis_weights(const int32_t *__restrict__ lo,
 // A thread a coarse node.  Its row is a product over the axes: with the weights of both
 // axes in registers, each fine row's three neighbour rows are contracted along y, then
 // along x -- some 54 multiply-adds a fine node and no branch but the fine node's own, and
-// the loads of a fine row of nodes are all in flight together.  Testing every pair of fine
+// the loads of a fine row of nodes are all in flight together.  PLAIN adds every neighbour
+// to all nine coarse nodes one after another (see update9).  Testing every pair of fine
 // neighbour and coarse node instead (a branch and an index a term) took 60 us a level of a
 // 1025 x 513 mesh, its levels of a few thousand nodes as long as the finest; so the finest
 // takes 22 us and the others 14.
 constexpr int kGalerkinThreads = 64;
 
-template <bool NINE>
+template <bool NINE, bool PLAIN>
 __global__ void __launch_bounds__(kGalerkinThreads)
     galerkin(Fine F, double *__restrict__ a9c, double *__restrict__ rdiag_c,
              uint8_t *__restrict__ active_c) {
@@ -290,6 +291,24 @@ __global__ void __launch_bounds__(kGalerkinThreads)
                 m[1][0] = -F.c4[2 * n + f] * free_at(k, l - 1);
                 m[1][2] = -F.c4[3 * n + f] * free_at(k, l + 1);
             }
+            if (PLAIN) {
+                // every neighbour (d, e), in row order, to every coarse node (p, q) it
+                // prolongs from
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+#pragma unroll
+                    for (int e = 0; e < 3; ++e) {
+                        if (!NINE && d != 1 && e != 1) continue;
+                        const double t = wgt * m[d][e];
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) {
+                            const double tp = t * px[a + d][p];
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) acc[p][q] += tp * py[c + e][q];
+                        }
+                    }
+                continue;
+            }
 #pragma unroll
             for (int e = 0; e < 3; ++e) {
                 double row[3];
@@ -320,14 +339,29 @@ __global__ void __launch_bounds__(kGalerkinThreads)
 // east, south, north) or a 9-point row (the eight neighbours' in row order).  Two chains of
 // fused multiply-adds and the diagonal's reciprocal: a colour phase is one such update a
 // thread between barriers, so its time is the update's latency -- 17 dependent roundings
-// and an IEEE quotient, some 240 cycles, before; some 56 so.  Every form of the smoothing
-// (a launch a colour, staged tiles, the coarse levels in one launch) takes these updates.
+// and an IEEE quotient, some 240 cycles, before; some 56 so.  Every form of a
+// single solve's smoothing (a launch a colour, staged tiles, the coarse levels in one
+// launch) takes these updates.
+// PLAIN: one term after another and the quotient by the diagonal (rd is the diagonal).  A
+// batch of candidates takes PLAIN throughout (smoothing, restriction, the coarse operators
+// and their inverse): some of its candidates never settle, and such a one multiplies a
+// rounding of its field by 1e5 and more over its iterations -- with the fused forms some
+// sweeps end with moments 3.5e-8 from PLAIN's (the others within 2e-12).  The batch's launches
+// are many tiles deep, so the longer chains cost it little: 360 ms a sweep for 352.
+template <bool PLAIN = false>
 __device__ __forceinline__ double update5(double b, double cw, double ce, double cs, double cn,
                                           double xw, double xe, double xs, double xn, double rd) {
+    if (PLAIN) return (b + cw * xw + ce * xe + cs * xs + cn * xn) / rd;
     return (fma(ce, xe, fma(cw, xw, b)) + fma(cn, xn, cs * xs)) * rd;
 }
+template <bool PLAIN = false>
 __device__ __forceinline__ double update9(double b, const double (&a)[8], const double (&x)[8],
                                           double rd) {
+    if (PLAIN) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) b -= a[q] * x[q];
+        return b / rd;
+    }
     const double p = fma(-a[3], x[3], fma(-a[2], x[2], fma(-a[1], x[1], fma(-a[0], x[0], b))));
     const double q = fma(a[7], x[7], fma(a[6], x[6], fma(a[5], x[5], a[4] * x[4])));
     return (p - q) * rd;
@@ -439,7 +473,7 @@ __host__ __device__ inline size_t stage_smem(bool nine, int tx, int ty, int halo
 // form).
 template <bool NINE, int R>
 __device__ __forceinline__ void smooth_staged_tile(
-    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ rdiag,
+    i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ diag,
     const double *__restrict__ a9, const uint8_t *__restrict__ active,
     const double *__restrict__ b, const double *__restrict__ xin, double *__restrict__ xout,
     int tx, int ty, const Phases &ph, const Fine &F, const double *__restrict__ xc, i64 bx,
@@ -448,7 +482,6 @@ __device__ __forceinline__ void smooth_staged_tile(
     // xc, when not NULL: the coarse correction, prolonged onto x as it is read (the values
     // prolong_add would leave in xin)
     extern __shared__ double sm[];
-    // coefficients per node, the reciprocal diagonal in the diagonal's place (5-point: last)
     constexpr int Q = NINE ? 9 : 5;
     constexpr int K = NINE ? 4 : 2;  // colours
     const int halo = stage_halo(ph.count);
@@ -483,14 +516,14 @@ __device__ __forceinline__ void smooth_staged_tile(
             if (NINE) {
                 double q9[9];
 #pragma unroll
-                for (int q = 0; q < 9; ++q) q9[q] = q == 4 ? rdiag[f] : a9[(i64)q * n + f];
+                for (int q = 0; q < 9; ++q) q9[q] = a9[(i64)q * n + f];
 #pragma unroll
                 for (int q = 0; q < 9; ++q) coef[q * m + pos] = q9[q];
             } else {
                 double q5[5];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) q5[q] = c4[(i64)q * n + f];
-                q5[4] = rdiag[f];
+                q5[4] = diag[f];
 #pragma unroll
                 for (int q = 0; q < 5; ++q) coef[q * m + pos] = q5[q];
             }
@@ -544,9 +577,9 @@ __device__ __forceinline__ void smooth_staged_tile(
                                          coef[7 * m + pos], coef[8 * m + pos]};
                     const double v[8] = {xs[q - wy - 1], xs[q - wy],     xs[q - wy + 1], xs[q - 1],
                                          xs[q + 1],      xs[q + wy - 1], xs[q + wy],     xs[q + wy + 1]};
-                    xs[q] = update9(bs[pos], c, v, coef[4 * m + pos]);
+                    xs[q] = update9<true>(bs[pos], c, v, coef[4 * m + pos]);
                 } else {
-                    xs[q] = update5(bs[pos], coef[pos], coef[m + pos], coef[2 * m + pos],
+                    xs[q] = update5<true>(bs[pos], coef[pos], coef[m + pos], coef[2 * m + pos],
                                     coef[3 * m + pos], xs[q - wy], xs[q + wy], xs[q - 1], xs[q + 1],
                                     coef[4 * m + pos]);
                 }
@@ -609,7 +642,8 @@ struct Tile {
     static constexpr int threads = ((per + r - 1) / r + 31) / 32 * 32;
 };
 
-template <bool NINE, int TX, int TY, int COUNT, bool REVERSE>
+// PLAIN: rdiag names the diagonal itself (update9).
+template <bool NINE, int TX, int TY, int COUNT, bool REVERSE, bool PLAIN = false>
 __device__ __forceinline__ void smooth_tile(const SmoothView &L, int bx, int by) {
     using S = Tile<NINE, TX, TY, COUNT>;
     constexpr int K = S::colours, R = S::r, WX = S::wx, WY = S::wy, HY = WY / 2;
@@ -674,10 +708,10 @@ __device__ __forceinline__ void smooth_tile(const SmoothView &L, int bx, int by)
                 if constexpr (NINE) {
                     const double v[8] = {q[-WY - 1], q[-WY], q[-WY + 1], q[-1],
                                          q[1],       q[WY - 1], q[WY],   q[WY + 1]};
-                    x[k][r] = update9(b[k][r], c, v, rd[k][r]);
+                    x[k][r] = update9<PLAIN>(b[k][r], c, v, rd[k][r]);
                 } else {
-                    x[k][r] = update5(b[k][r], c[0], c[1], c[2], c[3], q[-WY], q[WY], q[-1], q[1],
-                                      rd[k][r]);
+                    x[k][r] = update5<PLAIN>(b[k][r], c[0], c[1], c[2], c[3], q[-WY], q[WY], q[-1],
+                                             q[1], rd[k][r]);
                 }
                 xs[at[k][r]] = x[k][r];
             }
@@ -761,7 +795,8 @@ __device__ __forceinline__ double coarse_weight(const CoarseAxis &A, int k, int 
     return I == lo ? w : (I == lo + 1 ? 1.0 - w : 0.0);
 }
 
-template <bool NINE>
+// PLAIN: every sum one term after another, as a batch of candidates restricts.
+template <bool NINE, bool PLAIN = false>
 __device__ __forceinline__ void restrict_tile(const RestrictView &L, int bx, int by) {
     __shared__ double rs[kRestrictFineX * kRestrictFineY];
     const int tid = threadIdx.x, nx = L.nx, ny = L.ny;
@@ -783,12 +818,25 @@ __device__ __forceinline__ void restrict_tile(const RestrictView &L, int bx, int
                                      x[0],                      n ? x[1] : 0.0,
                                      e && s ? x[ny - 1] : 0.0,  e ? x[ny] : 0.0,
                                      e && n ? x[ny + 1] : 0.0};
-                double p = L.b[f], q = a[5] * v[5];
+                if (PLAIN) {
+                    r = L.b[f];
 #pragma unroll
-                for (int k = 0; k < 5; ++k) p = fma(-a[k], v[k], p);
+                    for (int k = 0; k < 9; ++k) r -= a[k] * v[k];
+                } else {
+                    double p = L.b[f], q = a[5] * v[5];
 #pragma unroll
-                for (int k = 6; k < 9; ++k) q = fma(a[k], v[k], q);
-                r = p - q;
+                    for (int k = 0; k < 5; ++k) p = fma(-a[k], v[k], p);
+#pragma unroll
+                    for (int k = 6; k < 9; ++k) q = fma(a[k], v[k], q);
+                    r = p - q;
+                }
+            } else if (PLAIN) {
+                double t = L.diag[f] * x[0];
+                t -= L.c4[f] * (w ? x[-ny] : 0.0);
+                t -= L.c4[L.n + f] * (e ? x[ny] : 0.0);
+                t -= L.c4[2 * L.n + f] * (s ? x[-1] : 0.0);
+                t -= L.c4[3 * L.n + f] * (n ? x[1] : 0.0);
+                r = (L.b[f] - t) * L.weight[f];
             } else {
                 const double p = fma(-L.diag[f], x[0], L.b[f]);
                 const double q = fma(L.c4[f], w ? x[-ny] : 0.0, L.c4[L.n + f] * (e ? x[ny] : 0.0));
@@ -814,10 +862,14 @@ __device__ __forceinline__ void restrict_tile(const RestrictView &L, int bx, int
 #pragma unroll
         for (int e = -1; e <= 1; ++e) {
             const double pl = li + e >= 0 && li + e < ny ? coarse_weight(ay, li + e, J) : 0.0;
-            if (pl != 0.0 && pk != 0.0)
-                row = fma(pl, rs[(ki + d - k0) * kRestrictFineY + (li + e - l0)], row);
+            if (pl == 0.0 || pk == 0.0) continue;
+            const double r = rs[(ki + d - k0) * kRestrictFineY + (li + e - l0)];
+            if (PLAIN)
+                sum += pk * pl * r;
+            else
+                row = fma(pl, r, row);
         }
-        sum = fma(pk, row, sum);
+        if (!PLAIN) sum = fma(pk, row, sum);
     }
     L.bc[I * L.ncy + J] = sum;
 }
@@ -882,13 +934,17 @@ __device__ __forceinline__ int band_node(int o, int nx, int ny) {
 
 // factors: column k of L below the diagonal at [k kBandPad + j - 1] (row k + j), column k of
 // U above it at [(n + k) kBandPad + j - 1] (row k - j), the reciprocal pivots after both.
+// PLAIN (see update9) divides by the pivots, keeps row k of U right of the diagonal (column
+// k + j) in the place of its column, and the pivots themselves.
+template <bool PLAIN>
 __global__ void __launch_bounds__(32 * kBandMax) coarsest_band_factor(
     int nx, int ny, const double *__restrict__ a9, double *__restrict__ factors,
     int *__restrict__ fallback) {
     extern __shared__ double band[];  // row r: band[r * W + (c - r + b)], |c - r| <= b
     const int n = nx * ny;
     const int b = band_half(nx, ny), W = 2 * b + 1;
-    double *inv = band + n * W;  // the reciprocal pivots
+    double *inv = band + n * W;  // the pivots' reciprocals; PLAIN: the pivots
+    const auto over = [](double v, double d) { return PLAIN ? v / d : v * d; };
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     for (int e = tid; e < n * W; e += nt) band[e] = 0.0;
     __syncthreads();
@@ -908,10 +964,10 @@ __global__ void __launch_bounds__(32 * kBandMax) coarsest_band_factor(
     const double *left = band + (warp + 1) * W + b - 1 - warp, *up = band + b + 1 + lane;
     const double *diag = band + b;
     for (int k = 0; k < n; ++k) {
-        const double r = 1.0 / *diag;
+        const double r = PLAIN ? *diag : 1.0 / *diag;
         if (tid == 0) inv[k] = r;
         if (lane < b && k + 1 + lane < n && k + 1 + warp < n)
-            *mine = fma(-(*left * r), *up, *mine);
+            *mine = PLAIN ? *mine - (*left / r) * *up : fma(-(*left * r), *up, *mine);
         __syncthreads();
         mine += W;
         left += W;
@@ -924,10 +980,11 @@ __global__ void __launch_bounds__(32 * kBandMax) coarsest_band_factor(
         double *L = factors + k * kBandPad, *U = factors + (n + k) * kBandPad;
         for (int j = 1; j <= kBandPad; ++j) {
             const bool below = j <= b && k + j < n, above = j <= b && k - j >= 0;
-            L[j - 1] = below ? band[(k + j) * W + b - j] * r : 0.0;
-            U[j - 1] = above ? band[(k - j) * W + b + j] : 0.0;
+            L[j - 1] = below ? over(band[(k + j) * W + b - j], r) : 0.0;
+            U[j - 1] = PLAIN ? (below ? band[k * W + b + j] : 0.0)
+                             : (above ? band[(k - j) * W + b + j] : 0.0);
             // row k's own entries: its multipliers and its part of U
-            if (above) row = fmax(row, fabs(band[k * W + b - j] * inv[k - j]));
+            if (above) row = fmax(row, fabs(over(band[k * W + b - j], inv[k - j])));
             if (below) row = fmax(row, fabs(band[k * W + b + j]));
         }
         const double piv = band[k * W + b];
@@ -938,16 +995,17 @@ __global__ void __launch_bounds__(32 * kBandMax) coarsest_band_factor(
 }
 
 // M[., col] = (L U)^-1 e_col, a thread a column: KB at least b, even.  The window w[j] holds
-// row o + j's (forward) or o - j's (backward) remaining right-hand side.  The forward
+// row o + j's (forward) or o - j's (backward) remaining right-hand side; PLAIN's backward one
+// row o + 1 + j's solution, a row's terms taken from the diagonal outwards.  The forward
 // results go through M; the backward pass reads its own column's values kAhead rows early.
-template <int KB>
+template <int KB, bool PLAIN>
 __global__ void __launch_bounds__(kSolveThreads) coarsest_band_solve(
     int nx, int ny, const double *__restrict__ factors, double *__restrict__ M,
     const int *__restrict__ fallback) {
     extern __shared__ __align__(16) double f[];
     if (*fallback) return;
     const int n = nx * ny;
-    // the first KB of every factor column, then the reciprocal pivots
+    // the first KB of every factor column (PLAIN: of U, row), then the (reciprocal) pivots
     for (int e = threadIdx.x; e < 2 * n * KB; e += kSolveThreads) {
         const int k = e / KB;
         f[e] = factors[k * kBandPad + (e - k * KB)];
@@ -966,8 +1024,8 @@ __global__ void __launch_bounds__(kSolveThreads) coarsest_band_solve(
 #pragma unroll
         for (int j = 0; j < KB / 2; ++j) {
             const double2 l = L[j];
-            w[2 * j] = fma(-l.x, y, w[2 * j + 1]);
-            w[2 * j + 1] = fma(-l.y, y, w[2 * j + 2]);
+            w[2 * j] = PLAIN ? w[2 * j + 1] - l.x * y : fma(-l.x, y, w[2 * j + 1]);
+            w[2 * j + 1] = PLAIN ? w[2 * j + 2] - l.y * y : fma(-l.y, y, w[2 * j + 2]);
         }
         w[KB] = 0.0;
         if (col < n) M[(i64)band_node(o, nx, ny) * n + col] = y;
@@ -984,17 +1042,29 @@ __global__ void __launch_bounds__(kSolveThreads) coarsest_band_solve(
         for (int q = 0; q < kAhead; ++q) {
             const int o = top - q;
             if (o < 0) break;
-            const double x = (w[0] + ahead[q]) * inv[o];
+            double x = PLAIN ? ahead[q] : (w[0] + ahead[q]) * inv[o];
             const int next = o - kAhead;
             ahead[q] = col < n && next >= 0 ? M[(i64)band_node(next, nx, ny) * n + col] : 0.0;
             const double2 *U = reinterpret_cast<const double2 *>(f + (n + o) * KB);
 #pragma unroll
             for (int j = 0; j < KB / 2; ++j) {
                 const double2 u = U[j];
-                w[2 * j] = fma(-u.x, x, w[2 * j + 1]);
-                w[2 * j + 1] = fma(-u.y, x, w[2 * j + 2]);
+                if (PLAIN) {
+                    x -= u.x * w[2 * j];
+                    x -= u.y * w[2 * j + 1];
+                } else {
+                    w[2 * j] = fma(-u.x, x, w[2 * j + 1]);
+                    w[2 * j + 1] = fma(-u.y, x, w[2 * j + 2]);
+                }
             }
-            w[KB] = 0.0;
+            if (PLAIN) {
+                x = x / inv[o];
+#pragma unroll
+                for (int j = KB; j > 0; --j) w[j] = w[j - 1];
+                w[0] = x;
+            } else {
+                w[KB] = 0.0;
+            }
             if (col < n) M[(i64)band_node(o, nx, ny) * n + col] = x;
         }
     }
@@ -1185,6 +1255,7 @@ __device__ __forceinline__ TailPlace tail_place(const TailPlan &P, int tid) {
     return T;
 }
 
+template <bool PLAIN>
 __device__ __forceinline__ void tail_smooth(const TailPlan &P, const TailPlace &T, const double *sm,
                                             double *smd, const uint8_t *act, int colour, int tid,
                                             int nt) {
@@ -1192,7 +1263,7 @@ __device__ __forceinline__ void tail_smooth(const TailPlan &P, const TailPlace &
     const int ci = colour >> 1, cj = colour & 1;
     const int hx = (nx - ci + 1) >> 1, hy = (ny - cj + 1) >> 1;
     double *x = smd + P.x;
-    const double *b = smd + P.b, *a9 = sm + P.a9, *rd = sm + P.rd;
+    const double *b = smd + P.b, *a9 = sm + P.a9, *rd = PLAIN ? a9 + 4 * n : sm + P.rd;
     int ti = cj ? T.row[1] : T.row[0], tj = cj ? T.col[1] : T.col[0];
     for (int t = tid; t < hx * hy; t += nt) {
         if (t != tid) {
@@ -1207,7 +1278,7 @@ __device__ __forceinline__ void tail_smooth(const TailPlan &P, const TailPlace &
                              a9[5 * n + f], a9[6 * n + f], a9[7 * n + f], a9[8 * n + f]};
         const double v[8] = {x[q - W - 1], x[q - W],     x[q - W + 1], x[q - 1],
                              x[q + 1],     x[q + W - 1], x[q + W],     x[q + W + 1]};
-        x[q] = update9(b[f], c, v, rd[f]);
+        x[q] = update9<PLAIN>(b[f], c, v, rd[f]);
     }
 }
 
@@ -1399,9 +1470,10 @@ __device__ __forceinline__ void tail_helper(const TailLevel &L, const TailPlan &
 // levels[0] reads b from, and writes x to, global memory; `image` holds the static part
 // of the shared memory (image_words 16-byte words); inv is the coarsest level's inverse.
 // REG: a colour of the first level fits the block's threads, which hold it in registers;
-// CLUSTER: the blocks of a cluster, whose other blocks are tail_helpers.
+// CLUSTER: the blocks of a cluster, whose other blocks are tail_helpers; PLAIN: a batch's
+// arithmetic (update9).
 // (The body of vcycle_tail and of its batched form.)
-template <bool REG, bool CLUSTER>
+template <bool REG, bool CLUSTER, bool PLAIN>
 __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ levels,
                                                 const TailPlan *__restrict__ plans, int count,
                                                 const uint4 *__restrict__ image,
@@ -1449,7 +1521,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         if (R.node[k] >= 0) {
             double v[8];
             tail_neighbours(x + R.at[k], W, v);
-            x[R.at[k]] = update9(R.b[k], R.coef[k], v, R.rd[k]);
+            x[R.at[k]] = update9<PLAIN>(R.b[k], R.coef[k], v, PLAIN ? R.diag[k] : R.rd[k]);
         }
         __syncthreads();
     };
@@ -1468,12 +1540,22 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
                 if (R.node[k] >= 0) {
                     double v[8];
                     tail_neighbours(x + R.at[k], W, v);
-                    double p = fma(-R.diag[k], x[R.at[k]], R.b[k]), q = R.coef[k][7] * v[7];
+                    if (PLAIN) {
+                        double p = R.b[k];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) p = fma(-R.coef[k][e], v[e], p);
+                        for (int e = 0; e < 4; ++e) p -= R.coef[k][e] * v[e];
+                        p -= R.diag[k] * x[R.at[k]];
 #pragma unroll
-                    for (int e = 4; e < 7; ++e) q = fma(R.coef[k][e], v[e], q);
-                    r[R.node[k]] = p - q;
+                        for (int e = 4; e < 8; ++e) p -= R.coef[k][e] * v[e];
+                        r[R.node[k]] = p;
+                    } else {
+                        double p = fma(-R.diag[k], x[R.at[k]], R.b[k]), q = R.coef[k][7] * v[7];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) p = fma(-R.coef[k][e], v[e], p);
+#pragma unroll
+                        for (int e = 4; e < 7; ++e) q = fma(R.coef[k][e], v[e], q);
+                        r[R.node[k]] = p - q;
+                    }
                 } else if (R.node[k] <= -2) {
                     r[-2 - R.node[k]] = 0.0;
                 }
@@ -1482,7 +1564,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
             const TailPlace T = tail_place(P, tid);
             for (int s = 0; s < sweeps; ++s)
                 for (int c = 0; c < 4; ++c) {
-                    tail_smooth(P, T, sm, smd, act, c, tid, nt);
+                    tail_smooth<PLAIN>(P, T, sm, smd, act, c, tid, nt);
                     __syncthreads();
                 }
             tail_residual(P, sm, smd, act, tid, nt);
@@ -1523,7 +1605,8 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
             for (int e = 0; e < kChunks; ++e) {
                 const double v = lane + 32 * e < n ? b[lane + 32 * e] : 0.0;
 #pragma unroll
-                for (int k = 0; k < kTailRows; ++k) s[k] = fma(m[k][e], v, s[k]);
+                for (int k = 0; k < kTailRows; ++k)
+                    s[k] = PLAIN ? s[k] + m[k][e] * v : fma(m[k][e], v, s[k]);
             }
             for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
@@ -1554,7 +1637,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
             const TailPlace T = tail_place(P, tid);
             for (int s = 0; s < sweeps; ++s)
                 for (int c = 3; c >= 0; --c) {
-                    tail_smooth(P, T, sm, smd, act, c, tid, nt);
+                    tail_smooth<PLAIN>(P, T, sm, smd, act, c, tid, nt);
                     __syncthreads();
                 }
         }
@@ -1571,14 +1654,14 @@ __global__ void __launch_bounds__(kTailRegThreads, 1) __cluster_dims__(kTailClus
     vcycle_tail_cluster(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans,
                         int count, const uint4 *__restrict__ image, int image_words, int doubles,
                         int ints, const double *__restrict__ inv, int sweeps) {
-    vcycle_tail_run<true, true>(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
+    vcycle_tail_run<true, true, false>(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
 }
 
 __global__ void __launch_bounds__(kTailThreads, 1)
 vcycle_tail(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans, int count,
             const uint4 *__restrict__ image, int image_words, int doubles, int ints,
             const double *__restrict__ inv, int sweeps) {
-    vcycle_tail_run<false, false>(levels, plans, count, image, image_words, doubles, ints, inv,
+    vcycle_tail_run<false, false, false>(levels, plans, count, image, image_words, doubles, ints, inv,
                                   sweeps);
 }
 
@@ -2172,7 +2255,49 @@ void build_operator(bt_poisson *p) {
     p->reaction_on = true;  // force the diagonal to be set
 }
 
-// Set the level-0 diagonal (with `reaction`, or without) and rebuild the coarse levels.
+// The coarse operators of the hierarchy, and the banded factors and inverse of the coarsest.
+template <bool PLAIN>
+void coarse_operators(bt_poisson *p) {
+    cudaStream_t st = p->ctx->stream;
+    for (size_t l = 0; l + 1 < p->levels.size(); ++l) {
+        Level &L = p->levels[l], &C = p->levels[l + 1];
+        Fine F = fine_of(L, C, l == 0);
+        const unsigned grid = blocks_for(C.n, kGalerkinThreads);
+        if (F.a9)
+            BT_LAUNCH(p->ctx, (galerkin<true, PLAIN>), grid, kGalerkinThreads, 0, st, F,
+                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
+        else
+            BT_LAUNCH(p->ctx, (galerkin<false, PLAIN>), grid, kGalerkinThreads, 0, st, F,
+                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
+    }
+}
+template <bool PLAIN>
+void coarsest_band(bt_poisson *p, const double *a9c, double *inv, int *status) {
+    cudaStream_t st = p->ctx->stream;
+    const Level &Lc = p->levels.back();
+    const int nx = (int)Lc.nx, ny = (int)Lc.ny, n = nx * ny, b = band_half(nx, ny);
+    double *factors = p->band.as<double>((size_t)n * (2 * kBandPad + 1));
+    BT_LAUNCH(p->ctx, coarsest_band_factor<PLAIN>, 1, 32 * b, band_smem(nx, ny), st, nx, ny, a9c,
+              factors, status + 1);
+    const unsigned grid = blocks_for(n, kSolveThreads);
+    const auto smem = [&](int kb) { return sizeof(double) * (size_t)n * (2 * kb + 1); };
+    if (b <= 6)
+        BT_LAUNCH(p->ctx, (coarsest_band_solve<6, PLAIN>), grid, kSolveThreads, smem(6), st, nx, ny,
+                  factors, inv, status + 1);
+    else if (b <= 10)
+        BT_LAUNCH(p->ctx, (coarsest_band_solve<10, PLAIN>), grid, kSolveThreads, smem(10), st, nx, ny,
+                  factors, inv, status + 1);
+    else if (b <= 14)
+        BT_LAUNCH(p->ctx, (coarsest_band_solve<14, PLAIN>), grid, kSolveThreads, smem(14), st, nx, ny,
+                  factors, inv, status + 1);
+    else
+        BT_LAUNCH(p->ctx, (coarsest_band_solve<18, PLAIN>), grid, kSolveThreads, smem(18), st, nx, ny,
+                  factors, inv, status + 1);
+}
+
+// Set the level-0 diagonal (with `reaction`, or without) and rebuild the coarse levels.  A
+// batch takes single solvers' operators without a reaction, so those are PLAIN's (once an
+// operator: some 0.1 ms more); a Newton step's, rebuilt at every step, are not.
 void build_hierarchy(bt_poisson *p, const double *reaction) {
     cudaStream_t st = p->ctx->stream;
     Timed timed(p->ctx, "hierarchy");
@@ -2180,17 +2305,10 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     BT_LAUNCH(p->ctx, add_diag, blocks_for(p->n, 256), 256, 0, st, p->n, L0.base.as<double>(p->n), reaction,
                                                     L0.active.as<uint8_t>(p->n),
                                                     L0.diag.as<double>(p->n), L0.rdiag.as<double>(p->n));
-    for (size_t l = 0; l + 1 < p->levels.size(); ++l) {
-        Level &L = p->levels[l], &C = p->levels[l + 1];
-        Fine F = fine_of(L, C, l == 0);
-        const unsigned grid = blocks_for(C.n, kGalerkinThreads);
-        if (F.a9)
-            BT_LAUNCH(p->ctx, galerkin<true>, grid, kGalerkinThreads, 0, st, F,
-                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
-        else
-            BT_LAUNCH(p->ctx, galerkin<false>, grid, kGalerkinThreads, 0, st, F,
-                      C.a9.as<double>(9 * C.n), C.rdiag.as<double>(C.n), C.active.as<uint8_t>(C.n));
-    }
+    if (reaction)
+        coarse_operators<false>(p);
+    else
+        coarse_operators<true>(p);
     Level &Lc = p->levels.back();
     if (p->levels.size() == 1)
         BT_LAUNCH(p->ctx, five_to_nine, blocks_for(Lc.n, 256), 256, 0, st, Lc.n,
@@ -2201,24 +2319,10 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     double *inv = p->inv.as<double>(Lc.n * Lc.n);
     const double *a9c = Lc.a9.as<double>(9 * Lc.n);
     if (band_half(Lc.nx, Lc.ny) <= kBandMax) {
-        const int nx = (int)Lc.nx, ny = (int)Lc.ny, n = nx * ny, b = band_half(nx, ny);
-        double *factors = p->band.as<double>((size_t)n * (2 * kBandPad + 1));
-        BT_LAUNCH(p->ctx, coarsest_band_factor, 1, 32 * b, band_smem(nx, ny), st, nx, ny, a9c,
-                  factors, status + 1);
-        const unsigned grid = blocks_for(n, kSolveThreads);
-        const auto smem = [&](int kb) { return sizeof(double) * (size_t)n * (2 * kb + 1); };
-        if (b <= 6)
-            BT_LAUNCH(p->ctx, coarsest_band_solve<6>, grid, kSolveThreads, smem(6), st, nx, ny,
-                      factors, inv, status + 1);
-        else if (b <= 10)
-            BT_LAUNCH(p->ctx, coarsest_band_solve<10>, grid, kSolveThreads, smem(10), st, nx, ny,
-                      factors, inv, status + 1);
-        else if (b <= 14)
-            BT_LAUNCH(p->ctx, coarsest_band_solve<14>, grid, kSolveThreads, smem(14), st, nx, ny,
-                      factors, inv, status + 1);
+        if (reaction)
+            coarsest_band<false>(p, a9c, inv, status);
         else
-            BT_LAUNCH(p->ctx, coarsest_band_solve<18>, grid, kSolveThreads, smem(18), st, nx, ny,
-                      factors, inv, status + 1);
+            coarsest_band<true>(p, a9c, inv, status);
         BT_LAUNCH(p->ctx, coarsest_invert, 1, kInvertThreads, 0, st, Lc.nx, Lc.ny, a9c, inv,
                   status, status + 1);
     } else {
@@ -2229,6 +2333,18 @@ void build_hierarchy(bt_poisson *p, const double *reaction) {
     refresh_tail_image(p);
     p->built = true;
     p->reaction_on = reaction != nullptr;
+}
+
+// The shared memory any solver's coarsest level needs.
+template <bool PLAIN>
+void coarsest_band_limits() {
+    BT_CUDA(cudaFuncSetAttribute(coarsest_band_factor<PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(sizeof(double) * kCoarsest * (2 * kBandMax + 2))));
+    const int solve = (int)(sizeof(double) * kCoarsest * (2 * kBandPad + 1));
+    BT_CUDA(cudaFuncSetAttribute((coarsest_band_solve<6, PLAIN>), cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute((coarsest_band_solve<10, PLAIN>), cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute((coarsest_band_solve<14, PLAIN>), cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    BT_CUDA(cudaFuncSetAttribute((coarsest_band_solve<18, PLAIN>), cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
 }
 
 // The tail: the longest run of coarsest levels (never level 0, whose operator is 5-point),
@@ -2245,13 +2361,8 @@ void setup_tail(bt_poisson *p) {
     }
     // the largest band any solver's coarsest level needs (the attribute is the kernel's,
     // shared by every solver of the process: never set it to one mesh's own size)
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_factor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(sizeof(double) * kCoarsest * (2 * kBandMax + 2))));
-    const int solve = (int)(sizeof(double) * kCoarsest * (2 * kBandPad + 1));
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<14>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
-    BT_CUDA(cudaFuncSetAttribute(coarsest_band_solve<18>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve));
+    coarsest_band_limits<true>();
+    coarsest_band_limits<false>();
     if (p->tail_start <= 0) return;
     const TailLayout T = tail_layout(p->levels, p->tail_start);
     p->tail_smem = T.total();
@@ -3023,7 +3134,6 @@ struct BatchLevel {
     int cand;
     i64 nx, ny, n;
     const double *c4, *diag, *a9;  // level 0: c4, diag; coarse levels: a9
-    const double *rdiag;
     const uint8_t *active;
     double *x, *x2, *b;
     Fine F;           // to the next level
@@ -3083,7 +3193,7 @@ __global__ void __launch_bounds__(kStageThreads)
     const double *in = from ? L.x2 : L.x;
     double *out = from ? L.x : L.x2;
     const Fine none{};
-    smooth_staged_tile<NINE, R>(L.nx, L.ny, L.c4, L.rdiag, L.a9, L.active, L.b, in, out, tx, ty,
+    smooth_staged_tile<NINE, R>(L.nx, L.ny, L.c4, L.diag, L.a9, L.active, L.b, in, out, tx, ty,
                                 ph, prolong ? L.F : none, prolong ? L.xc : nullptr, bx, by,
                                 zero_in != 0);
 }
@@ -3106,7 +3216,7 @@ __global__ void __launch_bounds__(Tile<NINE, TX, TY, COUNT>::threads)
     V.n = L.n;
     V.c4 = L.c4;
     V.a9 = L.a9;
-    V.rdiag = L.rdiag;
+    V.rdiag = NINE ? L.a9 + 4 * L.n : L.diag;
     V.b = L.b;
     V.active = L.active;
     V.xin = zero_in ? nullptr : (from ? L.x2 : L.x);
@@ -3114,7 +3224,7 @@ __global__ void __launch_bounds__(Tile<NINE, TX, TY, COUNT>::threads)
     V.xc = prolong ? L.xc : nullptr;
     V.ax = CoarseAxis{V.nx, (int)L.F.ncx};
     V.ay = CoarseAxis{V.ny, (int)L.F.ncy};
-    smooth_tile<NINE, TX, TY, COUNT, REVERSE>(V, bx, by);
+    smooth_tile<NINE, TX, TY, COUNT, REVERSE, true>(V, bx, by);
 }
 
 // b of the next level = R (b - A x) on every entry's level (x in the buffer `from` names:
@@ -3144,7 +3254,7 @@ __global__ void __launch_bounds__(kRestrictThreads)
     R.bc = L.bc;
     const int tiles_y = (R.ncy + kRestrictY - 1) / kRestrictY;
     const int bx = local / tiles_y;
-    restrict_tile<NINE>(R, bx, local - bx * tiles_y);
+    restrict_tile<NINE, true>(R, bx, local - bx * tiles_y);
 }
 
 // Every candidate's coarse levels, one block each.
@@ -3154,7 +3264,7 @@ __global__ void __launch_bounds__(REG ? kTailRegThreads : kTailThreads, 1)
                const uint8_t *__restrict__ live) {
     const BatchTail &t = T[ids[blockIdx.x]];
     if (!live[t.cand]) return;
-    vcycle_tail_run<REG, false>(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
+    vcycle_tail_run<REG, false, true>(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
                     t.sweeps);
 }
 
@@ -3669,7 +3779,6 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                     } else {
                         e.a9 = L.a9.as<double>(9 * L.n);
                     }
-                    e.rdiag = L.rdiag.as<double>(L.n);
                     e.active = L.active.as<uint8_t>(L.n);
                     e.x = L.x.as<double>(L.n);
                     e.x2 = L.x2.as<double>(L.n);
