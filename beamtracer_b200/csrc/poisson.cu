@@ -239,8 +239,8 @@ __device__ __forceinline__ void axis_weights(const int32_t *__restrict__ lo,
 // the loads of a fine row of nodes are all in flight together.  PLAIN adds every neighbour
 // to all nine coarse nodes one after another (see update9).  Testing every pair of fine
 // neighbour and coarse node instead (a branch and an index a term) took 60 us a level of a
-// 1025 x 513 mesh, its levels of a few thousand nodes as long as the finest; so the finest
-// takes 22 us and the others 14.
+// 1025 x 513 mesh, its levels of a few thousand nodes as long as the finest; the product
+// takes 22 us for the finest and 14 for the others.
 constexpr int kGalerkinThreads = 64;
 
 template <bool NINE, bool PLAIN>
@@ -774,7 +774,8 @@ __device__ __forceinline__ double apply5_item(i64 f, i64 nx, i64 ny, const doubl
 // it (by the control volumes on level 0) into shared memory, and adds up each coarse node's
 // nine from there, the weights from build_axis's rule.  The blocks' edges are computed twice
 // (10 % of the rows); the residual never goes to memory and there is one launch of 4.2 us (5.1
-// for the finest level) where the two took 8 (the restriction alone 4.8: its nine loads waited for table entries).
+// for the finest level) where the two took 8 (the restriction alone 4.8: its nine loads
+// waited for table entries).
 constexpr int kRestrictX = 8, kRestrictY = 16;
 constexpr int kRestrictFineX = 2 * kRestrictX + 1, kRestrictFineY = 2 * kRestrictY + 1;
 constexpr int kRestrictThreads = (kRestrictFineX * kRestrictFineY + 31) / 32 * 32;
@@ -910,7 +911,8 @@ constexpr int kInvertThreads = 1024;
 // serial chain of 3 n rows, so the time is rows times latency: with the substitutions
 // reading global memory row by row and a serial scan of every pivot row, 208 nodes
 // (b = 9, an 801 x 201 mesh) took 374 us and 153 nodes (b = 10, 1025 x 513) 284 us; now
-// 37 + 37 us and 28 + 31 us.  A pivot smaller than 1e-12 of its row (a matrix that needs pivoting, or a singular
+// 37 + 37 us and 28 + 31 us.  A pivot smaller than 1e-12 of its row (a matrix that needs
+// pivoting, or a singular
 // one) sets *fallback and the pivoting Gauss-Jordan below computes the inverse instead.
 constexpr int kBandMax = 17;
 constexpr int kBandPad = kBandMax + 1;  // a factor column's stride, in doubles (even: 16-byte loads)
@@ -2296,8 +2298,9 @@ void coarsest_band(bt_poisson *p, const double *a9c, double *inv, int *status) {
 }
 
 // Set the level-0 diagonal (with `reaction`, or without) and rebuild the coarse levels.  A
-// batch takes single solvers' operators without a reaction, so those are PLAIN's (once an
-// operator: some 0.1 ms more); a Newton step's, rebuilt at every step, are not.
+// batch takes single solvers' operators without a reaction, so those are PLAIN's
+// (once an operator); a Newton step's, rebuilt at every step, are not (some 50 us less a
+// step at 1025 x 513: a field of seven steps 12.4 ms against 12.8).
 void build_hierarchy(bt_poisson *p, const double *reaction) {
     cudaStream_t st = p->ctx->stream;
     Timed timed(p->ctx, "hierarchy");
