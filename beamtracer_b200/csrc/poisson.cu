@@ -469,8 +469,8 @@ __host__ __device__ inline size_t stage_smem(bool nine, int tx, int ty, int halo
     return m * sizeof(double) * (nine ? 11 : 7) + m;
 }
 
-// One tile (bx, by) of the staged smoothing (the body of smooth_staged and of its batched
-// form).
+// One tile (bx, by) of a batch's staged smoothing, for the tile sizes and phase counts that no
+// register tile is compiled for, in PLAIN arithmetic (update9).
 template <bool NINE, int R>
 __device__ __forceinline__ void smooth_staged_tile(
     i64 nx, i64 ny, const double *__restrict__ c4, const double *__restrict__ diag,
@@ -3267,8 +3267,8 @@ __global__ void __launch_bounds__(REG ? kTailRegThreads : kTailThreads, 1)
                const uint8_t *__restrict__ live) {
     const BatchTail &t = T[ids[blockIdx.x]];
     if (!live[t.cand]) return;
-    vcycle_tail_run<REG, false, true>(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
-                    t.sweeps);
+    vcycle_tail_run<REG, false, true>(t.levels, t.plans, t.count, t.image, t.words, t.doubles,
+                                      t.ints, t.inv, t.sweeps);
 }
 
 // The per-block partial sums of the finest levels' squares: part[2 block + q].
