@@ -1408,8 +1408,9 @@ __device__ __forceinline__ void tail_neighbours(const double *x, int W, double (
     v[7] = x[W + 1];
 }
 
-// A block's number in its cluster, the address of a shared variable in block `rank` of it, a
-// store there, and the cluster's barrier (which completes such stores).
+// A block's number in its cluster, a store to a shared variable of block `rank` of it, and the
+// cluster's barrier (which completes such stores) in two halves, of which every thread takes
+// the one and the other in turn; a warp's lanes take them together.
 __device__ __forceinline__ int cluster_rank() {
     uint32_t r;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -1422,16 +1423,26 @@ __device__ __forceinline__ void remote_store(const double *p, int rank, double v
         : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
 }
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile(
-        "barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-            : "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 
 // The coarsest level's inverse is applied by the other seven blocks of the tail's cluster,
 // their rows of it in registers from the launch on: one block alone read the inverse's 346 KB
 // (208 nodes) at 20 bytes a cycle, 18,000 of the tail's 39,000 cycles.  The first block sends
-// every helper b, the helpers send it x; a barrier each.
+// every helper b, the helpers send it x; a barrier each.  A block's shared memory may be
+// stored to only once the block has started: every block arrives at a barrier as it starts,
+// and the first waits there just before it sends (the helpers once their rows are asked for),
+// by when the others have long arrived.
 constexpr int kTailCluster = 8;
 constexpr int kHelperRows = 3;  // rows a helper's warp: 256 / 7 blocks / 16 warps, rounded up
 
@@ -1453,6 +1464,7 @@ __device__ __forceinline__ void tail_helper(const TailLevel &L, const TailPlan &
             m[k][e] = row < n && c < n ? __ldg(inv + (i64)row * n + c) : 0.0;
         }
     }
+    cluster_wait();     // (of the start's barrier)
     cluster_barrier();  // b is here
     const double *b = smd + C.b;
 #pragma unroll
@@ -1488,6 +1500,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     double *smd = sm + 2 * image_words;  // the dynamic doubles follow the image
     const int tid = threadIdx.x, nt = blockDim.x;
     if (CLUSTER) {
+        cluster_arrive();  // this block has started
         const int rank = cluster_rank();
         if (rank != 0) {
             tail_helper(levels[count - 1], plans[count - 1], inv, smd, rank);
@@ -1577,6 +1590,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     }
     if (CLUSTER) {
         const TailPlan &C = plan[count - 1];
+        cluster_wait();  // every helper has started
         for (int e = tid; e < C.n * (kTailCluster - 1); e += nt) {
             const int rank = 1 + e / C.n, f = e - (rank - 1) * C.n;
             remote_store(smd + C.b + f, rank, smd[C.b + f]);
