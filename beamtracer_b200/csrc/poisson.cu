@@ -2649,8 +2649,14 @@ void run_cycle(bt_poisson *p) {
     p->ctx->launch_count += p->vgraph_kernels;
 }
 
-// z = M v: one V-cycle from zero
+// z = M v: one V-cycle from zero.  Blocks of the cycle's last launch read v around the nodes
+// of z that others write: where the two overlap, v's copy in the level's own b is read instead.
 void precondition(bt_poisson *p, const double *v, double *z) {
+    if (v < z + p->n && z < v + p->n) {
+        double *b = p->levels[0].b.as<double>(p->n);
+        BT_CUDA(cudaMemcpyAsync(b, v, sizeof(double) * p->n, cudaMemcpyDeviceToDevice, p->ctx->stream));
+        v = b;
+    }
     BT_LAUNCH(p->ctx, set_cycle, 1, 1, 0, p->ctx->stream, p->cycle_io.as<CycleIo>(1), v, z);
     run_cycle(p);
 }

@@ -513,12 +513,12 @@ int bt_boltzmann_terms(bt_ctx *ctx, int64_t n, const uint8_t *own, const double 
                        double amplitude, double temperature, double up, int32_t sign,
                        double *r, double *reaction);
 
-/* One multigrid V-cycle from zero: z = M b (DEVICE (nx, ny); b a right-hand side of the
- * mesh's equation as the residual of bt_poisson_residual is one, zero on held nodes), the
- * operator's diagonal plus `reaction` (DEVICE, or NULL for none); the hierarchy is rebuilt
- * when `rebuild` is set, the reaction's presence changed or the held nodes did.  The
- * inexact local solve of each patch in the composite sweeps of refined boxes
- * (solver/poisson.py:169-335 through patchwork, absent here). */
+/* One multigrid V-cycle from zero: z = M b (DEVICE (nx, ny), z and b may overlap; b a
+ * right-hand side of the mesh's equation as the residual of bt_poisson_residual is one,
+ * zero on held nodes), the operator's diagonal plus `reaction` (DEVICE, or NULL for none);
+ * the hierarchy is rebuilt when `rebuild` is set, the reaction's presence changed or the
+ * held nodes did.  The inexact local solve of each patch in the composite sweeps of refined
+ * boxes (solver/poisson.py:169-335 through patchwork, absent here). */
 int bt_poisson_vcycle(bt_poisson *p, const double *b, const double *reaction, int32_t rebuild,
                       double *z);
 
