@@ -2747,6 +2747,13 @@ int steps_to_queue(const Arnoldi &a) {
     return std::max(1, (int)std::ceil(left) - 1);
 }
 
+// A residual norm, which must be finite: no comparison with a tolerance would tell that it is
+// not (one that is no number fails them all, and a tolerance relative to an infinite one is met).
+double finite_norm(double norm) {
+    if (!std::isfinite(norm)) throw Error{BT_ERR_NOCONV, "field solve: the residual is not finite"};
+    return norm;
+}
+
 // Solve A d = r0 for d (d zero on entry, beta = |r0|) by restarted right-preconditioned GMRES
 // until ||r0 - A d|| <= abs_tol or max_iter V-cycles; returns the V-cycles run and the final
 // residual norm.  The Arnoldi process runs on the device (Gram-Schmidt twice, the Givens
@@ -2780,12 +2787,12 @@ int gmres(bt_poisson *p, const double *r0, double *d, double beta, double abs_to
     Arnoldi *host = static_cast<Arnoldi *>(p->ctx->host.get(std::max(sizeof(Arnoldi), 64 * sizeof(double))));
     int total = 0;
     const double *r = r0;
+    finite_norm(beta);
     double previous = INFINITY;
     // stop at the tolerance, or where a whole restart cycle no longer halves the true
     // residual: the rounding floor of the residual itself
     while (beta > abs_tol && total < max_iter && beta < 0.5 * previous) {
         previous = beta;
-        if (!std::isfinite(beta)) throw Error{BT_ERR_NOCONV, "field solve: the residual is not finite"};
         BT_LAUNCH(p->ctx, arnoldi_begin, blocks_for(n, 256), 256, 0, st, S.a, S.g, m, beta, abs_tol, r,
                   n, V, Z, io);
         int j = 0, batch = 2;
@@ -2811,7 +2818,7 @@ int gmres(bt_poisson *p, const double *r0, double *d, double beta, double abs_to
         BT_LAUNCH(p->ctx, arnoldi_solve, 1, 32, 0, st, S.a, S.H, S.g, y, m);
         BT_LAUNCH(p->ctx, combine, blocks_for(n, 256), 256, 0, st, Z, y, S.a, n, d);
         // the true residual r0 - A d
-        beta = residual(p, r0, d, w).r;
+        beta = finite_norm(residual(p, r0, d, w).r);
         r = w;
     }
     if (final_norm) *final_norm = beta;
