@@ -71,7 +71,11 @@ __device__ __forceinline__ void accel(N &num, const Grid &G, double qm, const do
         g.cz = off_axis ? uz : 0.0;
         g.ir = off_axis ? ir : 0.0;
     }
-    const double sx = num.known(q[0] - G.ox, G.h, G.rh), sy = num.known(qy - G.oy, G.h, G.rh);
+    // (the coordinates tested, not their differences from the origin; a radius is its root's)
+    num.not_tiny(q[0]);
+    if (CYL != 1) num.not_tiny(qy);
+    const double sx = num.known_sound(q[0] - G.ox, G.h, G.rh);
+    const double sy = num.known_sound(qy - G.oy, G.h, G.rh);
     const double hx = sx + 0.5, hy = sy + 0.5;
     if (N::fast) {
         const int i = __double2int_rd(sx), j = __double2int_rd(sy);
@@ -146,7 +150,7 @@ __device__ __forceinline__ bool step_forward(const Grid &G, double qm, double f,
     const double a2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
     double y;
     const double speed = num.root(v2, y);
-    double dt = num.over(G.h, speed, num.inverse(speed, y));
+    double dt = num.over_sound(G.h, speed, num.inverse(speed, y));
     int branch = 1;
     if (FAST) {
         num.flag |= !((a2 * G.h) * G.h < (4.0 - 4e-9) * (v2 * v2)) || !(dt > 0.0);
@@ -382,17 +386,19 @@ __device__ __forceinline__ Midpoint midpoint(N &num, const Grid &G, const double
         M.r = num.root(m[1] * m[1] + m[2] * m[2], y);
         M.ir = N::fast ? y : 1.0 / M.r;  // used off the axis only
     }
-    M.i = __double2int_rd(num.known(m[0] - G.ox, G.h, G.rh));
-    M.j = __double2int_rd(num.known(M.r - G.oy, G.h, G.rh));
-    M.u = num.known(m[0] - (G.ox + G.h * (double)M.i), G.h, G.rh);
+    num.not_tiny(m[0]);
+    if (CYL != 1) num.not_tiny(M.r);
+    M.i = __double2int_rd(num.known_sound(m[0] - G.ox, G.h, G.rh));
+    M.j = __double2int_rd(num.known_sound(M.r - G.oy, G.h, G.rh));
+    M.u = num.known_sound(m[0] - (G.ox + G.h * (double)M.i), G.h, G.rh);
     const double low = G.oy + G.h * (double)M.j;
     if (CYL == 1) {
         const double high = low + G.h;
-        const double rs = num.div(1.0, high * high - low * low);
+        const double rs = num.div_sound(1.0, high * high - low * low);
         M.w = (M.r * M.r - low * low) * rs;
         M.dw_dr = 2.0 * M.r * rs;
     } else {
-        M.w = num.known(M.r - low, G.h, G.rh);
+        M.w = num.known_sound(M.r - low, G.h, G.rh);
         M.dw_dr = G.ih;
     }
     return M;
@@ -672,7 +678,8 @@ Adj adj_of(const bt_adjoint_args *a) {
     Adj A{};
     A.a = *a;
     A.G = Grid{a->fx, a->fy, (int)a->nx, (int)a->ny, a->origin_x, a->origin_y, a->h,
-               known_reciprocal(a->h), 1.0 / a->h};
+               sound_origin(a->origin_x) && sound_origin(a->origin_y) ? known_reciprocal(a->h) : 0.0,
+               1.0 / a->h};
     return A;
 }
 

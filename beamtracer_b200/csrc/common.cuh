@@ -227,9 +227,10 @@ __device__ __forceinline__ double div_known(double a, double b, double rb) {
 // routine, so no two of them, nor the loads and sums between, are scheduled into one another:
 // a chain of a dozen per trajectory step ran behind one another with one warp a scheduler.
 // Num<true> gives the same bits as straight-line code, and `odd()` afterwards is true where it
-// might not (an operand outside 2^-400 .. 2^400 other than zero, a divisor whose significand
-// is all ones); the caller then computes everything again with Num<false>, the IEEE
-// operations.  The operands' exponents are gathered in two integer extremes, tested once.
+// might not (an operand outside 2^-400 .. 2^400 other than a zero root or dividend, a divisor
+// whose significand may be all ones: its low word is); the caller then computes everything
+// again with Num<false>, the IEEE operations.  The operands' exponents are gathered in two
+// integer extremes, tested once.
 //
 // The methods are Markstein's (IBM J. Res. Develop. 34(1), 1990): a Newton step from the
 // hardware's approximations (20 bits) of third order, then corrections by exact remainders.
@@ -247,19 +248,33 @@ struct Num {
     static constexpr bool fast = FAST;
     static constexpr unsigned kLow = (1023u - 400u) << 20, kHigh = (1023u + 400u) << 20;
     bool flag = false;
-    unsigned low = 0xffffffffu, high = 0u;  // the operands' smallest and largest high words
+    // the operands' smallest magnitude (below) and largest high word
+    unsigned low = 0xffffffffu, high = 0u;
 
-    __device__ __forceinline__ bool odd() const { return flag || low < kLow - 1u || high > kHigh; }
-    // an operand that may be zero (high word 0 wraps past every exponent) but not tiny
+    __device__ __forceinline__ bool odd() const { return flag || low < 2u * kLow - 1u || high > kHigh; }
+    // twice the high word of |v|, less one where the low word is zero: a zero alone wraps past
+    // every exponent (some subnormals have bits in the low word only).  The low word's borrow,
+    // so that it takes the two additions that the high word's mask and decrement took.
+    static __device__ __forceinline__ unsigned magnitude(double v) {
+        unsigned t;
+        const unsigned twice = 2u * (unsigned)__double2hiint(v);
+        asm("{\n\t.reg .u32 w;\n\tadd.cc.u32 w, %1, -1;\n\taddc.u32 %0, %2, -1;\n\t}"
+            : "=r"(t)
+            : "r"(__double2loint(v)), "r"(twice));
+        return t;
+    }
+    __device__ __forceinline__ void not_huge(double v) {
+        high = max(high, (unsigned)(__double2hiint(v) & 0x7fffffff));
+    }
+    // an operand that may be zero but not tiny
     __device__ __forceinline__ void not_tiny(double v) {
-        if (FAST) low = min(low, (unsigned)(__double2hiint(v) & 0x7fffffff) - 1u);
+        if (FAST) low = min(low, magnitude(v));
     }
     // nor huge, infinite or not a number
     __device__ __forceinline__ void in_range(double v) {
         if (!FAST) return;
-        const unsigned t = (unsigned)(__double2hiint(v) & 0x7fffffff);
-        low = min(low, t - 1u);
-        high = max(high, t);
+        not_tiny(v);
+        not_huge(v);
     }
 
     // sqrt(s), s >= 0 or NaN, and an approximation y of its reciprocal for `inverse` (no
@@ -293,29 +308,49 @@ struct Num {
     }
     __device__ __forceinline__ double inverse(double b) {
         if (!FAST) return 0.0;
-        in_range(b);
+        low = min(low, 2u * (unsigned)__double2hiint(b));  // in range, and not zero
+        not_huge(b);
         double y;
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
         // e = 1 - b y to third order: y (1 + e + e^2)
         const double e = fma(-b, y, 1.0);
         return inverse(b, fma(fma(e, e, e), y, y));
     }
-    // a / b, rb the inverse of b.  A huge or infinite a or one that is no number gives such a
-    // quotient: the caller has its results' range tested (in_range).
-    __device__ __forceinline__ double over(double a, double b, double rb) {
+    // a / b, rb the inverse of b, of an a that the caller knows to be zero or at least 2^-600
+    // (which leaves the quotient and the remainders normal).  A huge or infinite a or one that
+    // is no number gives such a quotient: the caller has its results' range tested (in_range).
+    __device__ __forceinline__ double over_sound(double a, double b, double rb) {
         if (!FAST) return a / b;
-        not_tiny(a);
         double q = a * rb;
         q = fma(fma(-q, b, a), rb, q);
         return fma(fma(-q, b, a), rb, q);
     }
+    // the same, a tested
+    __device__ __forceinline__ double over(double a, double b, double rb) {
+        not_tiny(a);
+        return over_sound(a, b, rb);
+    }
     __device__ __forceinline__ double div(double a, double b) { return over(a, b, inverse(b)); }
+    __device__ __forceinline__ double div_sound(double a, double b) {
+        return over_sound(a, b, inverse(b));
+    }
     // a / b for a divisor known in advance (div_known; FAST: rb is not 0)
     __device__ __forceinline__ double known(double a, double b, double rb) {
-        if (!FAST) return div_known(a, b, rb);
-        return over(a, b, rb);
+        not_tiny(a);
+        return known_sound(a, b, rb);
+    }
+    __device__ __forceinline__ double known_sound(double a, double b, double rb) {
+        return FAST ? over_sound(a, b, rb) : div_known(a, b, rb);
     }
 };
+
+// Whether every difference of a mesh's origin (or one of its nodes' coordinates, its spacing
+// of known_reciprocal's range) and a coordinate that is zero or at least 2^-400 is itself zero
+// or at least 2^-452: all are multiples of that, as the differences of the squares of such a
+// node and a root are of 2^-556.
+__host__ __device__ __forceinline__ bool sound_origin(double o) {
+    return o == 0.0 || (fabs(o) >= 0x1p-200 && fabs(o) <= 0x1p200);
+}
 
 // The Lorentz factor sqrt(1 + |u|^2 / c^2) of a proper velocity u (1 for inv_c2 = 0).
 __device__ __forceinline__ double lorentz(double u0, double u1, double u2, double inv_c2) {

@@ -205,7 +205,7 @@ __device__ __forceinline__ void kick(N &num, double *v, const double *e, const d
     const double f = 0.5 * tau * qm;
     const double m0 = v[0] + f * e[0], m1 = v[1] + f * e[1], m2 = v[2] + f * e[2];
     const double t0 = f * b[0], t1 = f * b[1], t2 = f * b[2];
-    const double d = num.div(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
+    const double d = num.div_sound(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
     const double s0 = d * t0, s1 = d * t1, s2 = d * t2;
     const double p0 = m0 + (m1 * t2 - m2 * t1);
     const double p1 = m1 + (m2 * t0 - m0 * t2);
@@ -223,7 +223,8 @@ __device__ __forceinline__ void kick(N &num, double *v, const double *e, const d
 template <bool GENERAL, class N>
 __device__ __forceinline__ double inv_gamma(N &num, double u0, double u1, double u2,
                                             double inv_c2) {
-    return GENERAL ? num.div(1.0, num.root(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2)) : 1.0;
+    return GENERAL ? num.div_sound(1.0, num.root(1.0 + (u0 * u0 + u1 * u1 + u2 * u2) * inv_c2))
+                   : 1.0;
 }
 
 // What a trajectory's steps share: its mesh (its candidate's in a batch), its base patch,
@@ -235,7 +236,8 @@ struct Geo {
     int P, n_x_nodes;
     bool graded;
     bool same;  // one patch, which is the mesh: cell coordinates serve both
-    bool fast;  // the straight-line arithmetic may be tried (every reciprocal is one)
+    bool fast;  // the straight-line arithmetic may be tried (every reciprocal is one, the
+                // origins are sound)
 };
 
 // A point on the mesh: its radius or distance from the axis (the mesh's second coordinate)
@@ -284,8 +286,11 @@ __device__ __forceinline__ void locate(N &num, const bt_trace_args &a, const Geo
     else if (CYL == 2)
         W.r = G.oy + fabs(q[1] - G.oy);
     W.lx = uniform_x<GENERAL>(num, a, G, q[0], hint, W.cell);
-    W.sx = num.known(W.lx - G.ox, G.h, G.rh);
-    W.sy = num.known(W.r - G.oy, G.h, G.rh);
+    // (the coordinates tested, not their differences from the origin; a radius is its root's)
+    num.not_tiny(W.lx);
+    if (CYL != 1) num.not_tiny(W.r);
+    W.sx = num.known_sound(W.lx - G.ox, G.h, G.rh);
+    W.sy = num.known_sound(W.r - G.oy, G.h, G.rh);
 }
 
 // The pace of a state at its place.
@@ -319,7 +324,8 @@ __device__ __forceinline__ void set_pace(N &num, const bt_trace_args &a, const G
     const double speed = GENERAL ? S.gv * root : root;
     S.speed2 = speed * speed;
     // (at rest the quotient is not used; Num<true> then calls the step odd)
-    const double time = GENERAL ? num.div(hloc, speed) : num.over(hloc, speed, num.inverse(speed, y));
+    const double time =
+        GENERAL ? num.div(hloc, speed) : num.over_sound(hloc, speed, num.inverse(speed, y));
     S.dt0 = speed > 0.0 ? time : -1.0;
 }
 
@@ -529,7 +535,11 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
     const PatchGeom g = one ? G.base : patch_geom(a, finest_patch(a, G.P, m0, m1));
     const double rphh = one ? g.rphh : 0.0;
     // quotients by the patch's spacing
-    auto cells_of = [&](double v) { return one ? num.known(v, g.phh, rphh) : num.div(v, g.phh); };
+    num.not_tiny(m0);
+    if (CYL != 1) num.not_tiny(m1);
+    auto cells_of = [&](double v) {
+        return one ? num.known_sound(v, g.phh, rphh) : num.div(v, g.phh);
+    };
     const int pnx = (int)g.pnx, pny = (int)g.pny;
     int i = __double2int_rd(cells_of(m0 - g.pox));
     int j = __double2int_rd(cells_of(m1 - g.poy));
@@ -538,7 +548,8 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
     if (CYL == 1) {
         const double low = g.poy + g.phh * (double)j;
         const double high = low + g.phh;
-        wr = num.div(m1 * m1 - low * low, high * high - low * low);
+        const double span = high * high - low * low, part = m1 * m1 - low * low;
+        wr = one ? num.div_sound(part, span) : num.div(part, span);
     } else {
         wr = cells_of(m1 - (g.poy + g.phh * (double)j));
     }
@@ -633,7 +644,9 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
     G.graded = GENERAL && a.graded != 0;
     G.n_x_nodes = (int)a.n_x_nodes;
     G.same = G.P == 1 && G.base.pox == G.ox && G.base.poy == G.oy && G.base.phh == G.h;
-    G.fast = G.rh != 0.0 && G.base.rphh != 0.0 && G.rhz != 0.0 && (GENERAL || G.same);
+    G.fast = G.rh != 0.0 && G.base.rphh != 0.0 && G.rhz != 0.0 && (GENERAL || G.same) &&
+             sound_origin(G.ox) && sound_origin(G.oy) && sound_origin(G.base.pox) &&
+             sound_origin(G.base.poy);
     const double upper_x = BATCH ? __ldg(a.patch_real + cand * 7 + 5) : a.upper_x;
     const double upper_y = BATCH ? __ldg(a.patch_real + cand * 7 + 6) : a.upper_y;
     const i64 *__restrict__ cells = BATCH ? a.cells + __ldg(tr.cell_off + cand) : a.cells;

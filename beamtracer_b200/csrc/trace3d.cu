@@ -176,7 +176,7 @@ __device__ __forceinline__ void boris_push(N &num, double *u, const double *e, c
     const double g = N::fast ? 1.0 : sqrt(1.0 + (m0 * m0 + m1 * m1 + m2 * m2) * inv_c2);
     const double t0 = N::fast ? b[0] : b[0] / g, t1 = N::fast ? b[1] : b[1] / g,
                  t2 = N::fast ? b[2] : b[2] / g;
-    const double f = num.div(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
+    const double f = num.div_sound(2.0, 1.0 + (t0 * t0 + t1 * t1 + t2 * t2));
     const double s0 = f * t0, s1 = f * t1, s2 = f * t2;
     const double p0 = m0 + (m1 * t2 - m2 * t1);
     const double p1 = m1 + (m2 * t0 - m0 * t2);
@@ -283,7 +283,7 @@ __device__ __forceinline__ void set_pace3(N &num, const bt_trace3d_args &a, cons
     const double root = num.root(S.v[0] * S.v[0] + S.v[1] * S.v[1] + S.v[2] * S.v[2], y);
     const double speed = N::fast ? root : S.gv * root;
     S.speed2 = speed * speed;
-    const double time = num.over(S.hloc, speed, num.inverse(speed, y));
+    const double time = num.over_sound(S.hloc, speed, num.inverse(speed, y));
     S.dt0 = speed > 0.0 ? time : -1.0;
 }
 
