@@ -114,7 +114,6 @@ struct DepositScratch {
     Buffer keys, keys_alt, vals, vals_alt, rec;
     Buffer hist, row_offsets, digit_base, sorted;
     Buffer cell_sums, warp_first, warp_last, warp_flags;
-    bool ticket_ready = false;  // the finishing-block counter in digit_base is zeroed
 };
 
 // The tracer's scratch: the live lists and two record buffers, one filled by the trace

@@ -40,10 +40,12 @@ constexpr uint32_t kNoSkip = 0xffffffffu;
 template <int R, int ITEMS>
 __global__ void radix_hist(const uint32_t *__restrict__ keys, i64 n_host,
                            const i64 *__restrict__ n_dev, uint32_t skip, int shift,
-                           uint32_t *__restrict__ hist, int nblocks) {
+                           uint32_t *__restrict__ hist, int nblocks,
+                           unsigned *__restrict__ ticket) {
     __shared__ uint32_t h[R];
     const i64 n = record_count(n_host, n_dev);
     for (int d = threadIdx.x; d < R; d += kThreads) h[d] = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0u;  // for the pass's radix_row_scan
     __syncthreads();
     const i64 base = (i64)blockIdx.x * tile_of(ITEMS);
     uint32_t key[ITEMS];
@@ -85,9 +87,10 @@ __device__ uint32_t block_inclusive_scan(uint32_t v, uint32_t *warp_sums) {
 }
 
 // Row d of hist (one digit over all blocks) to its exclusive prefix, the row's total; then, in
-// the block that finishes last (a ticket counter, reset by it), the exclusive prefix of the R
-// totals, thread t scanning digits t * R / kThreads onwards.  `count`, when not NULL, gets the
-// number of records the pass sorts.
+// the block that finishes last (a ticket counter, which the pass's radix_hist has zeroed: a
+// pass relies on nothing an earlier launch has left), the exclusive prefix of the R totals,
+// thread t scanning digits t * R / kThreads onwards.  `count`, when not NULL, gets the number
+// of records the pass sorts.
 template <int R>
 __global__ void __launch_bounds__(kThreads) radix_row_scan(
     const uint32_t *__restrict__ hist, uint32_t *__restrict__ offs, uint32_t *__restrict__ totals,
@@ -132,7 +135,6 @@ __global__ void __launch_bounds__(kThreads) radix_row_scan(
         base[threadIdx.x * D + k] = run;
         run += mine[k];
     }
-    if (threadIdx.x == 0) *ticket = 0u;
     if (count && threadIdx.x == kThreads - 1) *count = inclusive;
 }
 
@@ -453,7 +455,7 @@ void sort_pass(bt_ctx *ctx, const uint32_t *src_k, const uint32_t *src_v, i64 n,
                uint32_t *dst_k, uint32_t *dst_v) {
     cudaStream_t st = ctx->stream;
     BT_LAUNCH(ctx, (radix_hist<R, ITEMS>), nblocks, kThreads, 0, st, src_k, n, n_dev, skip, shift,
-              hist, nblocks);
+              hist, nblocks, ticket);
     BT_LAUNCH(ctx, radix_row_scan<R>, R, kThreads, 0, st, hist, offs, totals, nblocks, digit, count,
               ticket);
     BT_LAUNCH(ctx, (radix_scatter<R, ITEMS>), nblocks, kThreads, 0, st, src_k, src_v, n, n_dev, skip,
@@ -474,11 +476,7 @@ void radix_sort_pairs(bt_ctx *ctx, const uint32_t *keys_in, i64 n, const i64 *n_
     uint32_t *offs = s.row_offsets.as<uint32_t>((size_t)kRadixMax * nblocks);
     uint32_t *digit = s.digit_base.as<uint32_t>(2 * kRadixMax + 1);
     uint32_t *totals = digit + kRadixMax;
-    unsigned *ticket = totals + kRadixMax;  // zero between passes
-    if (!s.ticket_ready) {
-        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), ctx->stream));
-        s.ticket_ready = true;
-    }
+    unsigned *ticket = totals + kRadixMax;
     i64 *sorted = s.sorted.as<i64>(1);  // the records left after the first pass
     const uint32_t *src_k = keys_in;
     const uint32_t *src_v = nullptr;
@@ -676,7 +674,6 @@ extern "C" int bt_deposit_trajectories_2d_noalloc(void *stream, const double *px
         uint32_t *digit = reinterpret_cast<uint32_t *>(base + kOffDigits);
         uint32_t *totals = digit + kRadix;
         unsigned *ticket = totals + kRadix;
-        BT_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), st));
         double4 *cells = reinterpret_cast<double4 *>(base + kOffCells);
         double4 *first = reinterpret_cast<double4 *>(base + kOffWarps);
         double4 *last = first + kNoallocWarps;
@@ -693,7 +690,7 @@ extern "C" int bt_deposit_trajectories_2d_noalloc(void *stream, const double *px
         for (int pass = 0; pass < passes; ++pass) {
             const int shift = 8 * pass;
             radix_hist<kRadix, kSmallItems><<<nblocks, kThreads, 0, st>>>(
-                src_k, n, nullptr, kNoSkip, shift, hist, nblocks);
+                src_k, n, nullptr, kNoSkip, shift, hist, nblocks, ticket);
             radix_row_scan<kRadix><<<kRadix, kThreads, 0, st>>>(hist, offs, totals, nblocks, digit,
                                                                nullptr, ticket);
             radix_scatter<kRadix, kSmallItems><<<nblocks, kThreads, 0, st>>>(
