@@ -39,7 +39,7 @@ struct Trace {
 
 // The cell of x on a graded axis: the last node at or before x, within the axis (0 left of
 // it or for a NaN).  `hint` is where the search starts: a trajectory's points lie in its last
-// cell or beside it, so the walk reads two or three nodes where a bisection read eleven
+// cell or beside it, so the walk reads two or three nodes where a bisection reads eleven
 // of 1025, each waiting for the one before.
 __device__ __forceinline__ int node_cell(double x, const double *__restrict__ nodes, int n,
                                          int hint) {
@@ -49,6 +49,19 @@ __device__ __forceinline__ int node_cell(double x, const double *__restrict__ no
     while (x < nodes[c]) --c;
     while (x >= nodes[c + 1]) ++c;
     return c;
+}
+
+// The same by bisection, for a window's first point, which has no cell to walk from.
+__device__ __forceinline__ int first_cell(double x, const double *__restrict__ nodes, int n) {
+    int lo = 0, hi = n - 1;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) / 2;
+        if (nodes[mid] <= x)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
 }
 
 __device__ __forceinline__ i64 finest_patch(const bt_trace_args &a, i64 P, double px, double py) {
@@ -659,7 +672,7 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
         now.e[c] = now.b[c] = 0.0;
     }
     now.have = false;
-    now.at.cell = 0;
+    now.at.cell = G.graded ? first_cell(now.x[0], a.x_nodes, G.n_x_nodes) : 0;
     {
         State first = now;
         const Geo g = G;
