@@ -153,8 +153,8 @@ struct bt_ctx {
     bt::Buffer anderson;        // the Anderson mixer's sums, R, Q^T f and gamma
     bt::Buffer measure;         // the FP64 peak measurement's output
     // the 3D tracer's records (charge, current), live flags and live count
-    bt::Buffer t3_keys, t3_vals, t3_jkeys, t3_jvals, t3_alive, t3_live, t3_cells, t3_jcells,
-        t3_pieces, t3_flags;
+    bt::Buffer t3_keys, t3_vals, t3_jkeys, t3_jvals, t3_alive, t3_live, t3_place, t3_pieces,
+        t3_flags;
     i64 launch_count = 0;       // kernels launched on the context since its creation
     i64 last_windows = 0, last_records = 0, last_flushes = 0;
 };

@@ -643,20 +643,23 @@ __global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__
 
 // The cells' sums: the records of a cell lie together after the sort, in runs of hundreds
 // where a beam of many trajectories moves down the mesh.  A warp adds 32 records by a
-// segmented scan in record order; a cell wholly inside a warp is written, the pieces of one
-// that crosses warps go to `first` (a leading piece, `ends` set where its cell ends in this
-// warp) and `last` (a trailing piece of a cell that begins here, `owns` set), chained in warp
-// order by cell_chains.  The sums depend on the records alone.  (One thread a run, waiting
-// for each record behind the one before, took 343 us for 1.6 M records in cells of some 500;
-// the two kernels take 50 us.)  The cells of no record hold zeros.
+// segmented scan in record order and leaves a cell's sum in the place of one of its records
+// (which no other thread reads), that place plus one in `place` (0: a cell of no record): of
+// its last record in the cell that is wholly inside the warp, of the warp's last where a cell
+// begins here and goes on (`owns` set).  The leading piece of one that began in an earlier
+// warp goes to `first` (`ends` set where its cell ends in this warp); cell_chains adds those
+// up in warp order.  The sums depend on the records alone.  (One thread a run, waiting for
+// each record behind the one before, took 343 us for 1.6 M records in cells of some 500; the
+// two kernels take 50 us.)  A window clears a word a cell, which every node reads, and no
+// more: with the sums themselves in an array of a record a cell (192 bytes of the current's)
+// a window of a hundred trajectories with the current on 257^3 nodes took 2.6 ms and 3.3 GB
+// more; 0.6 ms so.
 template <int N>
 __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K,
-                                                  const uint32_t *__restrict__ I,
-                                                  const Rec<N> *__restrict__ recs,
+                                                  const uint32_t *__restrict__ I, Rec<N> *recs,
                                                   const i64 *__restrict__ count,
-                                                  Rec<N> *__restrict__ cells,
+                                                  uint32_t *__restrict__ place,
                                                   Rec<N> *__restrict__ first,
-                                                  Rec<N> *__restrict__ last,
                                                   uint8_t *__restrict__ ends,
                                                   uint8_t *__restrict__ owns) {
     const i64 n = *count;
@@ -665,10 +668,10 @@ __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K
     const int lane = threadIdx.x & 31;
     const i64 r = w * 32 + lane;
     const bool valid = r < n;
-    const uint32_t key = valid ? K[r] : 0xffffffffu;
+    const uint32_t key = valid ? K[r] : 0xffffffffu, at = valid ? I[r] : 0u;
     Rec<N> sum;
     if (valid) {
-        sum = recs[I[r]];
+        sum = recs[at];
     } else {
 #pragma unroll
         for (int c = 0; c < N; ++c) sum.c[c] = 0.0;
@@ -686,31 +689,23 @@ __global__ void __launch_bounds__(256) cell_warps(const uint32_t *__restrict__ K
         if (lane >= off) head = head || before;
     }
     // head: the cell's first record is in this warp
-    if (tail) {
-        if (head) {
-            cells[key] = sum;
-        } else {
-            first[w] = sum;
-            ends[w] = 1;
-        }
-    }
-    if (lane == 31) {
-        const bool open = valid && !tail;
-        owns[w] = open && head ? 1 : 0;
-        if (open && head) last[w] = sum;
-        if (open && !head) {
-            first[w] = sum;
-            ends[w] = 0;
-        }
+    const bool open = valid && lane == 31 && !tail;
+    if (lane == 31) owns[w] = open && head ? 1 : 0;
+    if (!tail && !open) return;
+    if (head) {
+        recs[at] = sum;
+        place[key] = at + 1u;
+    } else {
+        first[w] = sum;
+        ends[w] = tail ? 1 : 0;
     }
 }
 
 template <int N>
-__global__ void __launch_bounds__(256) cell_chains(const uint32_t *__restrict__ K,
+__global__ void __launch_bounds__(256) cell_chains(const uint32_t *__restrict__ I,
+                                                   Rec<N> *__restrict__ recs,
                                                    const i64 *__restrict__ count,
-                                                   Rec<N> *__restrict__ cells,
                                                    const Rec<N> *__restrict__ first,
-                                                   const Rec<N> *__restrict__ last,
                                                    const uint8_t *__restrict__ ends,
                                                    const uint8_t *__restrict__ owns) {
     const i64 n_warps = (*count + 31) / 32;
@@ -719,34 +714,48 @@ __global__ void __launch_bounds__(256) cell_chains(const uint32_t *__restrict__ 
     const i64 w0 = t / N;
     const int c = (int)(t - w0 * N);
     if (w0 >= n_warps || !owns[w0]) return;
-    double s = last[w0].c[c];
+    double &sum = recs[I[w0 * 32 + 31]].c[c];
+    double s = sum;
     for (i64 w = w0 + 1; w < n_warps; ++w) {
         s = s + first[w].c[c];
         if (ends[w]) break;
     }
-    cells[K[w0 * 32 + 31]].c[c] = s;
+    sum = s;
 }
 
-// charge[node] += its shares of the eight cells it is a corner of, in a fixed order (the
+// A node's shares of the eight cells it is a corner of, added up in a fixed order (the
 // corner q = 4 di + 2 dj + dk of the cell at node - (di, dj, dk)), within a box of
-// (pnx, pny, pnz) nodes, the node's place in it `local`; `shift` selects a record's component.
+// (pnx, pny, pnz) nodes, the node's place in it `local`; a record's components in s.
 template <int N>
-__device__ __forceinline__ double corner_sum(const Rec<N> *__restrict__ cells, i64 node, i64 local,
-                                             i64 pnx, i64 pny, i64 pnz, int shift) {
+__device__ __forceinline__ bool corner_sums(const uint32_t *__restrict__ place,
+                                            const Rec<N> *__restrict__ recs, i64 node, i64 local,
+                                            i64 pnx, i64 pny, i64 pnz, double (&s)[N / 8]) {
     const i64 i = local / (pny * pnz), j = (local / pnz) % pny, k = local % pnz;
-    double s = 0.0;
+    uint32_t at[8], any = 0u;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int di = q >> 2, dj = (q >> 1) & 1, dk = q & 1;
         const i64 ci = i - di, cj = j - dj, ck = k - dk;
-        if (ci < 0 || cj < 0 || ck < 0 || ci > pnx - 2 || cj > pny - 2 || ck > pnz - 2) continue;
-        s = s + cells[node - di * pny * pnz - dj * pnz - dk].c[shift + q];
+        const bool in =
+            ci >= 0 && cj >= 0 && ck >= 0 && ci <= pnx - 2 && cj <= pny - 2 && ck <= pnz - 2;
+        at[q] = in ? place[node - di * pny * pnz - dj * pnz - dk] : 0u;
+        any |= at[q];
     }
-    return s;
+#pragma unroll
+    for (int m = 0; m < N / 8; ++m) s[m] = 0.0;
+    if (any == 0u) return false;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        if (at[q] == 0u) continue;
+#pragma unroll
+        for (int m = 0; m < N / 8; ++m) s[m] = s[m] + recs[at[q] - 1u].c[8 * m + q];
+    }
+    return true;
 }
 
-__global__ void node_gather3(const CellRec *__restrict__ cells, const i64 *__restrict__ patch_int,
-                             int n_patches, i64 n_nodes, double *__restrict__ charge) {
+__global__ void node_gather3(const uint32_t *__restrict__ place, const CellRec *__restrict__ recs,
+                             const i64 *__restrict__ patch_int, int n_patches, i64 n_nodes,
+                             double *__restrict__ charge) {
     const i64 node = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= n_nodes) return;
     int p = 0;
@@ -756,16 +765,21 @@ __global__ void node_gather3(const CellRec *__restrict__ cells, const i64 *__res
     const i64 *pi = patch_int + p * 8;
     const i64 pnx = pi[0], pny = pi[1], pnz = pi[2], local = node - pi[7];
     if (local < 0 || local >= pnx * pny * pnz) return;
-    charge[node] += corner_sum(cells, node, local, pnx, pny, pnz, 0);
+    double s[1];
+    if (corner_sums(place, recs, node, local, pnx, pny, pnz, s)) charge[node] += s[0];
 }
 
-// The current's three components on the base mesh's nodes (blockIdx.y the component).
-__global__ void node_gather_current(const CurrentRec *__restrict__ cells, i64 nx, i64 ny, i64 nz,
+// The current's three components on the base mesh's nodes.
+__global__ void node_gather_current(const uint32_t *__restrict__ place,
+                                    const CurrentRec *__restrict__ recs, i64 nx, i64 ny, i64 nz,
                                     double *__restrict__ current) {
     const i64 node = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     const i64 n = nx * ny * nz;
     if (node >= n) return;
-    current[blockIdx.y * n + node] += corner_sum(cells, node, node, nx, ny, nz, 8 * (int)blockIdx.y);
+    double s[3];
+    if (!corner_sums(place, recs, node, node, nx, ny, nz, s)) return;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) current[m * n + node] += s[m];
 }
 
 __global__ void fill_flags(uint8_t *__restrict__ flags, i64 n, uint8_t value) {
@@ -786,23 +800,26 @@ int key_bits(uint64_t max_key) {
 }
 
 // A window's records (`slots` keys, those with the sentinel left out) sorted by cell and
-// summed per cell in record order into `cells` (n_cells, zeroed first).
+// summed per cell in record order, the sums in the records' own places; the returned map of
+// n_cells says where (cell_warps).
 template <int N>
-void sum_cells(bt_ctx *ctx, const uint32_t *keys, const Rec<N> *recs, i64 slots, uint32_t sentinel,
-               Rec<N> *cells, i64 n_cells) {
+const uint32_t *sum_cells(bt_ctx *ctx, const uint32_t *keys, Rec<N> *recs, i64 slots,
+                          uint32_t sentinel, i64 n_cells) {
     cudaStream_t st = ctx->stream;
     const i64 pieces = (slots + 31) / 32;
-    Rec<N> *first = ctx->t3_pieces.as<Rec<N>>(2 * pieces), *last = first + pieces;
+    Rec<N> *first = ctx->t3_pieces.as<Rec<N>>(pieces);
     uint8_t *flags = ctx->t3_flags.as<uint8_t>(2 * pieces);
+    uint32_t *place = ctx->t3_place.as<uint32_t>(n_cells);
     uint32_t *sk = nullptr, *sv = nullptr;
     const i64 *count = nullptr;
     radix_sort_pairs(ctx, keys, slots, nullptr, key_bits(sentinel), sentinel, &sk, &sv, &count);
-    BT_CUDA(cudaMemsetAsync(cells, 0, sizeof(Rec<N>) * n_cells, st));
+    BT_CUDA(cudaMemsetAsync(place, 0, sizeof(uint32_t) * n_cells, st));
     BT_LAUNCH(ctx, cell_warps<N>, blocks_for(pieces * 32, 256), 256, 0, st, sk, sv, recs, count,
-              cells, first, last, flags, flags + pieces);
-    BT_LAUNCH(ctx, cell_chains<N>, blocks_for(pieces * N, 256), 256, 0, st, sk, count, cells, first,
-              last, flags, flags + pieces);
+              place, first, flags, flags + pieces);
+    BT_LAUNCH(ctx, cell_chains<N>, blocks_for(pieces * N, 256), 256, 0, st, sv, recs, count, first,
+              flags, flags + pieces);
     BT_CHECK_LAUNCH();
+    return place;
 }
 
 void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
@@ -859,10 +876,8 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
                "trace3d: too many records a window (use a shorter window)");
     uint32_t *keys = ctx->t3_keys.as<uint32_t>(slots);
     CellRec *recs = ctx->t3_vals.as<CellRec>(slots);
-    CellRec *cells = ctx->t3_cells.as<CellRec>(a.n_nodes);
     uint32_t *jkeys = a.has_j ? ctx->t3_jkeys.as<uint32_t>(slots) : nullptr;
     CurrentRec *jrecs = a.has_j ? ctx->t3_jvals.as<CurrentRec>(slots) : nullptr;
-    CurrentRec *jcells = a.has_j ? ctx->t3_jcells.as<CurrentRec>(nb) : nullptr;
     uint8_t *alive = ctx->t3_alive.as<uint8_t>(na);
     auto *live = ctx->t3_live.as<unsigned long long>(1);
     unsigned long long *host = static_cast<unsigned long long *>(ctx->host.get(64));
@@ -886,13 +901,13 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
         }
         BT_CHECK_LAUNCH();
         // the window's records: sorted by cell, summed per cell, gathered per node
-        sum_cells<8>(ctx, keys, recs, slots, T.sentinel, cells, a.n_nodes);
-        BT_LAUNCH(ctx, node_gather3, blocks_for(a.n_nodes, 256), 256, 0, st, cells, a.patch_int,
-                  (int)a.n_patches, a.n_nodes, a.charge);
+        const uint32_t *place = sum_cells(ctx, keys, recs, slots, T.sentinel, a.n_nodes);
+        BT_LAUNCH(ctx, node_gather3, blocks_for(a.n_nodes, 256), 256, 0, st, place, recs,
+                  a.patch_int, (int)a.n_patches, a.n_nodes, a.charge);
         if (a.has_j) {
-            sum_cells<24>(ctx, jkeys, jrecs, slots, T.jsentinel, jcells, nb);
-            BT_LAUNCH(ctx, node_gather_current, dim3(blocks_for(nb, 256), 3), 256, 0, st, jcells,
-                      T.nx, T.ny, T.nz, a.current);
+            place = sum_cells(ctx, jkeys, jrecs, slots, T.jsentinel, nb);
+            BT_LAUNCH(ctx, node_gather_current, blocks_for(nb, 256), 256, 0, st, place, jrecs, T.nx,
+                      T.ny, T.nz, a.current);
         }
         BT_CHECK_LAUNCH();
         BT_CUDA(cudaMemcpyAsync(host, live, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
