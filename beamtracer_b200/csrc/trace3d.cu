@@ -858,7 +858,6 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
     T.nz = base[2];
     BT_REQUIRE(T.nx >= 2 && T.ny >= 2 && T.nz >= 2, "trace3d: the mesh needs 2 x 2 x 2 nodes");
     const i64 nb = T.nx * T.ny * T.nz;
-    BT_REQUIRE(!a.has_j || 3 * nb < (int64_t)0xffffffffLL, "trace3d: too many current nodes");
     // one patch that is the mesh, whose spacing has a reciprocal, and no relativity
     bool fast = a.n_patches == 1 && a.inv_c2 == 0.0 && known_reciprocal(a.h) != 0.0;
     if (fast) {
@@ -872,7 +871,7 @@ void trace3d_all(bt_ctx *ctx, const bt_trace3d_args *args, int64_t window) {
     T.jsentinel = (uint32_t)nb;
     const i64 na = a.n_active;
     const i64 slots = (i64)T.S * na;
-    BT_REQUIRE(slots < (i64)0xffffffffLL && (!a.has_j || 24 * slots < (i64)0xffffffffLL),
+    BT_REQUIRE(slots < (i64)0xffffffffLL,
                "trace3d: too many records a window (use a shorter window)");
     uint32_t *keys = ctx->t3_keys.as<uint32_t>(slots);
     CellRec *recs = ctx->t3_vals.as<CellRec>(slots);

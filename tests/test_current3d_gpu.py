@@ -90,3 +90,35 @@ def test_scratch_of_few_trajectories_on_many_nodes():
     assert float(args[CHARGE].sum()) == pytest.approx(time.sum(), rel=1e-12)
     np.testing.assert_allclose(args[CURRENT].reshape(3, -1).sum(1).cpu().numpy(), moved.sum(1),
                                rtol=0, atol=1e-12 * np.abs(moved).max())  # fmt: skip
+
+
+def test_current_of_a_long_window():
+    """A window whose records are fewer than 2^32, though the shares of their current are more:
+    the outputs of the default window."""
+    import threading
+
+    import torch
+
+    from beamtracer_b200.kernels import KERNELS
+
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("the window's records take 62 GB")
+    args, _ = load_golden("trace3d_i0_r0_m1_b0_j1")
+    n = args[1].shape[1]
+    window = 2**32 // (24 * n) + 1
+    results = []
+
+    def run():  # in a thread: its context gives the scratch back
+        for steps in (0, window):
+            device = to_device(args)
+            KERNELS["trace_trajectories_3d"](*device, window=steps)
+            results.append(to_host(device))
+
+    thread = threading.Thread(target=run)
+    thread.start()
+    thread.join()
+    assert len(results) == 2
+    for short, long in zip(*results, strict=True):
+        if isinstance(short, np.ndarray):
+            scale = max(float(np.abs(short).max()), 1e-300) if short.size else 1.0
+            np.testing.assert_allclose(long, short, rtol=0, atol=1e-13 * scale)
