@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_sweep(Adj A, const double
     const bt_adjoint_args &a = A.a;
     const i64 n = a.n;
     const bool mine = k < n;
-    const i64 steps = mine ? a.steps[k] : 0;
+    const i64 steps = mine ? max(a.steps[k], (i64)0) : 0;  // (a count below zero is none)
     int cnt[kMaxPlanes];
     for (int p = 0; p < (int)a.n_planes; ++p) cnt[p] = mine ? (int)a.counts[k * a.n_planes + p] : 0;
     const double qm = mine ? a.qm[k] : 0.0, dq = mine ? a.dq[k] : 0.0;
