@@ -216,8 +216,8 @@ __device__ __forceinline__ bool step_forward(const Grid &G, double qm, double f,
     }
     // (an intermediate value out of range leaves the end state out of range)
 #pragma unroll
-    for (int c = 0; c < 3; ++c) num.in_range(T.y[c] - 1.0);
-    num.in_range(T.w[0] * T.w[0] + T.w[1] * T.w[1] + T.w[2] * T.w[2]);
+    for (int c = 0; c < 3; ++c) num.not_huge(T.y[c]);
+    num.not_huge(T.w[0] * T.w[0] + T.w[1] * T.w[1] + T.w[2] * T.w[2]);
     return !num.odd();
 }
 

@@ -262,14 +262,15 @@ struct Num {
             : "r"(__double2loint(v)), "r"(twice));
         return t;
     }
+    // an operand, or an end result, that must not be huge, infinite or no number
     __device__ __forceinline__ void not_huge(double v) {
-        high = max(high, (unsigned)(__double2hiint(v) & 0x7fffffff));
+        if (FAST) high = max(high, (unsigned)(__double2hiint(v) & 0x7fffffff));
     }
     // an operand that may be zero but not tiny
     __device__ __forceinline__ void not_tiny(double v) {
         if (FAST) low = min(low, magnitude(v));
     }
-    // nor huge, infinite or not a number
+    // an operand that must be neither
     __device__ __forceinline__ void in_range(double v) {
         if (!FAST) return;
         not_tiny(v);

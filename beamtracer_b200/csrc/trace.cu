@@ -588,8 +588,8 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
     D.c11 = u * wr * ch;
     dt_out = dt;
     // (an intermediate value out of range leaves the end state, or its root, out of range)
-    num.in_range(y[0]);
-    if (CYL != 1) num.in_range(y[1]);
+    num.not_huge(y[0]);
+    if (CYL != 1) num.not_huge(y[1]);
     return !num.odd();
 }
 

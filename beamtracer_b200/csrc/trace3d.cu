@@ -421,7 +421,7 @@ __device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G
     }
     D.dt = dt;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) num.in_range(y[c] - 1.0);
+    for (int c = 0; c < 3; ++c) num.not_huge(y[c]);
     return !num.odd();
 }
 
