@@ -130,7 +130,6 @@ __device__ __forceinline__ void accel(N &num, const Grid &G, double qm, const do
 struct StepTape {
     double y[3], w[3];     // the end state
     double a[4][3];        // the stage accelerations
-    double q[3][3];        // the stage points of stages 2-4
     double u[3][3];        // the stage velocities of stages 2-4
     Stage s[4];            // the stages' field evaluations
     double dt;
@@ -179,34 +178,34 @@ __device__ __forceinline__ bool step_forward(const Grid &G, double qm, double f,
     T.rate = FAST ? -dt * (y * y) : branch == 1 ? -dt / v2 : branch == 2 ? -0.5 * dt / a2 : 0.0;
     const double hdt = 0.5 * dt;
     const double dt6 = num.known(dt, 6.0, 1.0 / 6.0);
-    double sx[3], sv[3], kx[3];
+    double sx[3], sv[3], kx[3], q[3];  // q: the stage point
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = v[c];
         sv[c] = a1[c];
-        T.q[0][c] = x[c] + hdt * v[c];
+        q[c] = x[c] + hdt * v[c];
         kx[c] = v[c] + hdt * a1[c];
         T.u[0][c] = kx[c];
     }
-    accel<CYL>(num, G, qm, T.q[0], T.a[1], T.s[1]);
+    accel<CYL>(num, G, qm, q, T.a[1], T.s[1]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + 2.0 * kx[c];
         sv[c] = sv[c] + 2.0 * T.a[1][c];
-        T.q[1][c] = x[c] + hdt * kx[c];
+        q[c] = x[c] + hdt * kx[c];
         kx[c] = v[c] + hdt * T.a[1][c];
         T.u[1][c] = kx[c];
     }
-    accel<CYL>(num, G, qm, T.q[1], T.a[2], T.s[2]);
+    accel<CYL>(num, G, qm, q, T.a[2], T.s[2]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + 2.0 * kx[c];
         sv[c] = sv[c] + 2.0 * T.a[2][c];
-        T.q[2][c] = x[c] + dt * kx[c];
+        q[c] = x[c] + dt * kx[c];
         kx[c] = v[c] + dt * T.a[2][c];
         T.u[2][c] = kx[c];
     }
-    accel<CYL>(num, G, qm, T.q[2], T.a[3], T.s[3]);
+    accel<CYL>(num, G, qm, q, T.a[3], T.s[3]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         sx[c] = sx[c] + kx[c];
@@ -303,8 +302,8 @@ struct Scatter {
 // exb, eyb get the field's.  Everything but the adjoint is the stage's: no lookup, root or
 // quotient stands in the chain of a step's four.
 template <int CYL>
-__device__ __forceinline__ void accel_reverse(const Grid &G, double qm, const double *q,
-                                              const Stage &g, const double *ab, double *qb,
+__device__ __forceinline__ void accel_reverse(const Grid &G, double qm, const Stage &g,
+                                              const double *ab, double *qb,
                                               double &exb, double &eyb) {
     const double ih = G.ih;
     exb = qm * ab[0];
@@ -323,7 +322,6 @@ __device__ __forceinline__ void accel_reverse(const Grid &G, double qm, const do
     } else {
         qb[1] = fma(syb, ih, qb[1]);
     }
-    (void)q;
 }
 
 struct Adj {
@@ -549,7 +547,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
     double qb[3] = {0, 0, 0};
     double exb[4], eyb[4];
     // a4 = acc(q4), q4 = x + dt u3, u4 = v + dt a3
-    accel_reverse<CYL>(G, qm, T.q[2], T.s[3], a4b, qb, exb[3], eyb[3]);
+    accel_reverse<CYL>(G, qm, T.s[3], a4b, qb, exb[3], eyb[3]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u4b[c];
@@ -561,7 +559,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         qb[c] = 0.0;
     }
     // a3 = acc(q3), q3 = x + hdt u2, u3 = v + hdt a2
-    accel_reverse<CYL>(G, qm, T.q[1], T.s[2], a3b, qb, exb[2], eyb[2]);
+    accel_reverse<CYL>(G, qm, T.s[2], a3b, qb, exb[2], eyb[2]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u3b[c];
@@ -573,7 +571,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         qb[c] = 0.0;
     }
     // a2 = acc(q2), q2 = x + hdt v, u2 = v + hdt a1
-    accel_reverse<CYL>(G, qm, T.q[0], T.s[1], a2b, qb, exb[1], eyb[1]);
+    accel_reverse<CYL>(G, qm, T.s[1], a2b, qb, exb[1], eyb[1]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         vs[c] += u2b[c];
@@ -594,7 +592,7 @@ __device__ void step_reverse(const Adj &A, i64 k, double qm, double dq, const do
         for (int c = 0; c < 3; ++c) a1b[c] += dtb * T.rate * T.a[0][c];
     }
     // a1 = acc(x)
-    accel_reverse<CYL>(G, qm, x, T.s[0], a1b, xs, exb[0], eyb[0]);
+    accel_reverse<CYL>(G, qm, T.s[0], a1b, xs, exb[0], eyb[0]);
 #pragma unroll
     for (int k4 = 3; k4 >= 0; --k4) sc.add(T.s[k4], exb[k4], eyb[k4]);
 #pragma unroll

@@ -1200,8 +1200,7 @@ __global__ void five_to_nine(i64 n, const double *__restrict__ c4, const double 
 
 // -- the small levels in one launch, in shared memory ---------------------------------------
 
-constexpr int kTailThreads = 1024;
-constexpr int kTailRegThreads = 512;
+constexpr int kTailThreads = 512;
 constexpr int kTailRows = 2;  // rows of the inverse a warp applies at a time
 constexpr int kTailMaxLevels = 16;
 constexpr size_t kTailSmemMax = 200 * 1024;
@@ -1211,7 +1210,6 @@ struct TailLevel {
     const double *a9, *rdiag;
     const uint8_t *active;
     double *x, *b;  // the level's global vectors (read: b of the first, written: x of the first)
-    Fine next;      // the map to the next coarser level (unused on the coarsest)
 };
 
 // Where a tail level lives in shared memory.  The block's shared memory is a static image
@@ -1449,8 +1447,8 @@ constexpr int kHelperRows = 3;  // rows a helper's warp: 256 / 7 blocks / 16 war
 __device__ __forceinline__ void tail_helper(const TailLevel &L, const TailPlan &C,
                                             const double *__restrict__ inv, double *smd, int rank) {
     const int n = C.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int warps = kTailRegThreads / 32 * (kTailCluster - 1);
-    const int first = (rank - 1) * (kTailRegThreads / 32) + warp;  // rows first, first + warps, ..
+    const int warps = kTailThreads / 32 * (kTailCluster - 1);
+    const int first = (rank - 1) * (kTailThreads / 32) + warp;  // rows first, first + warps, ..
     constexpr int kChunks = kCoarsest / 32;
     double m[kHelperRows][kChunks];
     bool on[kHelperRows];
@@ -1483,11 +1481,10 @@ __device__ __forceinline__ void tail_helper(const TailLevel &L, const TailPlan &
 
 // levels[0] reads b from, and writes x to, global memory; `image` holds the static part
 // of the shared memory (image_words 16-byte words); inv is the coarsest level's inverse.
-// REG: a colour of the first level fits the block's threads, which hold it in registers;
-// CLUSTER: the blocks of a cluster, whose other blocks are tail_helpers; PLAIN: a batch's
-// arithmetic (update9).
-// (The body of vcycle_tail and of its batched form.)
-template <bool REG, bool CLUSTER, bool PLAIN>
+// The first block of a cluster, whose other blocks are tail_helpers; PLAIN: a batch's, in its
+// arithmetic (update9), one block a candidate.
+// (The body of vcycle_tail and of batch_tail.)
+template <bool PLAIN>
 __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ levels,
                                                 const TailPlan *__restrict__ plans, int count,
                                                 const uint4 *__restrict__ image,
@@ -1499,7 +1496,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     uint8_t *smb = reinterpret_cast<uint8_t *>(smi + ints);
     double *smd = sm + 2 * image_words;  // the dynamic doubles follow the image
     const int tid = threadIdx.x, nt = blockDim.x;
-    if (CLUSTER) {
+    if (!PLAIN) {
         cluster_arrive();  // this block has started
         const int rank = cluster_rank();
         if (rank != 0) {
@@ -1508,7 +1505,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         }
     }
     TailRegisters R;
-    if (REG && count > 1) tail_load(levels[0], R, tid);
+    if (count > 1) tail_load(levels[0], R, tid);
     {
         const int *src = reinterpret_cast<const int *>(plans);
         int *dst = reinterpret_cast<int *>(plan);
@@ -1516,16 +1513,16 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         for (int e = tid; e < words; e += nt) dst[e] = src[e];
     }
     // the static image in one piece (its first doubles are the first level's ten coefficients
-    // a node, held in registers with REG), x zero, level 0's b
+    // a node, held in registers), x zero, level 0's b
     uint4 *dst = reinterpret_cast<uint4 *>(sm);
-    const int skip = REG && count > 1 ? 5 * plans[0].n : 0;
+    const int skip = count > 1 ? 5 * plans[0].n : 0;
 #pragma unroll 4
     for (int e = skip + tid; e < image_words; e += nt) dst[e] = image[e];
     for (int l = 0; l < count; ++l) {
         const TailPlan &P = plans[l];
         for (int e = tid; e < (P.nx + 2) * (P.ny + 2); e += nt) smd[P.x + e] = 0.0;
     }
-    if (!REG || count == 1) {
+    if (count == 1) {
         const TailPlan &P = plans[0];
         const double *b0 = levels[0].b;
         for (int f = tid; f < P.n; f += nt) smd[P.b + f] = b0[f];
@@ -1543,7 +1540,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     for (int l = 0; l + 1 < count; ++l) {
         const TailPlan &P = plan[l];
         const uint8_t *act = smb + P.act;
-        if (REG && l == 0) {
+        if (l == 0) {
             double *x = smd + P.x, *r = smd + P.r;
             const int W = P.ny + 2;
             for (int s = 0; s < sweeps; ++s) {
@@ -1588,7 +1585,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         tail_restrict(P, plan[l + 1], sm, smd, smi, act, tid, nt);
         __syncthreads();
     }
-    if (CLUSTER) {
+    if (!PLAIN) {
         const TailPlan &C = plan[count - 1];
         cluster_wait();  // every helper has started
         for (int e = tid; e < C.n * (kTailCluster - 1); e += nt) {
@@ -1622,7 +1619,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
                 const double v = lane + 32 * e < n ? b[lane + 32 * e] : 0.0;
 #pragma unroll
                 for (int k = 0; k < kTailRows; ++k)
-                    s[k] = PLAIN ? s[k] + m[k][e] * v : fma(m[k][e], v, s[k]);
+                    s[k] = s[k] + m[k][e] * v;
             }
             for (int off = 16; off > 0; off >>= 1) {
 #pragma unroll
@@ -1643,7 +1640,7 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
         const uint8_t *act = smb + P.act;
         tail_prolong(P, plan[l + 1], sm, smd, smi, act, tid, nt);
         __syncthreads();
-        if (REG && l == 0) {
+        if (l == 0) {
             double *x = smd + P.x;
             for (int s = 0; s < sweeps; ++s) {
 #pragma unroll
@@ -1666,24 +1663,17 @@ __device__ __forceinline__ void vcycle_tail_run(const TailLevel *__restrict__ le
     }
 }
 
-__global__ void __launch_bounds__(kTailRegThreads, 1) __cluster_dims__(kTailCluster, 1, 1)
-    vcycle_tail_cluster(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans,
-                        int count, const uint4 *__restrict__ image, int image_words, int doubles,
-                        int ints, const double *__restrict__ inv, int sweeps) {
-    vcycle_tail_run<true, true, false>(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
+__global__ void __launch_bounds__(kTailThreads, 1) __cluster_dims__(kTailCluster, 1, 1)
+    vcycle_tail(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans, int count,
+                const uint4 *__restrict__ image, int image_words, int doubles, int ints,
+                const double *__restrict__ inv, int sweeps) {
+    vcycle_tail_run<false>(levels, plans, count, image, image_words, doubles, ints, inv, sweeps);
 }
 
-__global__ void __launch_bounds__(kTailThreads, 1)
-vcycle_tail(const TailLevel *__restrict__ levels, const TailPlan *__restrict__ plans, int count,
-            const uint4 *__restrict__ image, int image_words, int doubles, int ints,
-            const double *__restrict__ inv, int sweeps) {
-    vcycle_tail_run<false, false, false>(levels, plans, count, image, image_words, doubles, ints, inv,
-                                  sweeps);
-}
-
-// Whether a tail of this first level takes the register form: a colour of it fits 512 threads,
-// which have the registers for four rows each.
-bool tail_in_registers(i64 nx, i64 ny) { return ((nx + 1) / 2) * ((ny + 1) / 2) <= kTailRegThreads; }
+// Whether a colour of a tail's first level fits the block's threads, which hold it in
+// registers: no level with more nodes of a colour fits the shared memory (the smallest such
+// takes 260 KB), so this ends no tail earlier than that does.
+bool tail_fits_threads(i64 nx, i64 ny) { return ((nx + 1) / 2) * ((ny + 1) / 2) <= kTailThreads; }
 
 // The shared-memory layout of tail levels first .. (the coarsest): the static image
 // (coefficients of every level but the coarsest, transfer tables, active flags), then the
@@ -2372,7 +2362,9 @@ void setup_tail(bt_poisson *p) {
     p->tail_start = -1;
     p->tail_smem = 0;
     for (int l = levels - 1; l >= 1 && levels - l <= kTailMaxLevels; --l) {
-        if (p->levels[l].n > p->tail_nodes || tail_layout(p->levels, l).total() > kTailSmemMax)
+        const Level &L = p->levels[l];
+        if (L.n > p->tail_nodes || !tail_fits_threads(L.nx, L.ny) ||
+            tail_layout(p->levels, l).total() > kTailSmemMax)
             break;
         p->tail_start = l;
     }
@@ -2398,12 +2390,9 @@ void setup_tail(bt_poisson *p) {
         t.active = L.active.as<uint8_t>(L.n);
         t.x = L.x.as<double>(L.n);
         t.b = L.b.as<double>(L.n);
-        if (l + 1 < levels) t.next = fine_of(L, p->levels[l + 1], false);
         tail.push_back(t);
     }
     // the largest any solver asks for: solvers of other meshes may launch concurrently
-    BT_CUDA(cudaFuncSetAttribute(vcycle_tail_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kTailSmemMax));
     BT_CUDA(cudaFuncSetAttribute(vcycle_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kTailSmemMax));
     BT_CUDA(cudaMemcpy(p->tail_levels.as<TailLevel>(tail.size()), tail.data(),
@@ -2547,17 +2536,11 @@ void vcycle(bt_poisson *p, size_t l) {
     if ((int)l == p->tail_start) {
         const int count = (int)(p->levels.size() - l);
         const Level &Lc = p->levels.back();
-        const auto launch = [&](auto kernel, int blocks, int threads) {
-            BT_LAUNCH(p->ctx, kernel, blocks, threads, p->tail_smem, st,
-                      p->tail_levels.as<TailLevel>(count), p->tail_plans.as<TailPlan>(count), count,
-                      static_cast<const uint4 *>(p->tail_image.get(16 * (size_t)p->tail_words)),
-                      p->tail_words, p->tail_doubles, p->tail_ints, p->inv.as<double>(Lc.n * Lc.n),
-                      p->coarse_sweeps);
-        };
-        if (tail_in_registers(L.nx, L.ny))
-            launch(vcycle_tail_cluster, kTailCluster, kTailRegThreads);
-        else
-            launch(vcycle_tail, 1, kTailThreads);
+        BT_LAUNCH(p->ctx, vcycle_tail, kTailCluster, kTailThreads, p->tail_smem, st,
+                  p->tail_levels.as<TailLevel>(count), p->tail_plans.as<TailPlan>(count), count,
+                  static_cast<const uint4 *>(p->tail_image.get(16 * (size_t)p->tail_words)),
+                  p->tail_words, p->tail_doubles, p->tail_ints, p->inv.as<double>(Lc.n * Lc.n),
+                  p->coarse_sweeps);
         return;
     }
     if (l + 1 == p->levels.size()) {
@@ -3288,14 +3271,13 @@ __global__ void __launch_bounds__(kRestrictThreads)
 }
 
 // Every candidate's coarse levels, one block each.
-template <bool REG>
-__global__ void __launch_bounds__(REG ? kTailRegThreads : kTailThreads, 1)
+__global__ void __launch_bounds__(kTailThreads, 1)
     batch_tail(const BatchTail *__restrict__ T, const int *__restrict__ ids,
                const uint8_t *__restrict__ live) {
     const BatchTail &t = T[ids[blockIdx.x]];
     if (!live[t.cand]) return;
-    vcycle_tail_run<REG, false, true>(t.levels, t.plans, t.count, t.image, t.words, t.doubles,
-                                      t.ints, t.inv, t.sweeps);
+    vcycle_tail_run<true>(t.levels, t.plans, t.count, t.image, t.words, t.doubles, t.ints, t.inv,
+                          t.sweeps);
 }
 
 // The per-block partial sums of the finest levels' squares: part[2 block + q].
@@ -3478,7 +3460,6 @@ struct bt_poisson_batch {
     std::vector<Step> level;
     bt::Buffer tails, tail_ids;  // one block per live candidate
     int n_tails = 0;
-    bool tail_reg = true;        // every candidate's tail takes the register form
     size_t tail_smem = 0;
     bt::Buffer fine, fine_ids, fine_start;
     std::vector<bt::BatchFine> fine_host;  // the device table's copy
@@ -3668,12 +3649,8 @@ void batch_vcycle(bt_poisson_batch *B) {
             BT_LAUNCH(ctx, batch_restrict<true>, S.coarse_blocks, kRestrictThreads, 0, st, E, ids,
                       S.coarse_start.as<int>(S.n), S.n, live, held[l]);
     }
-    if (B->n_tails && B->tail_reg)
-        BT_LAUNCH(ctx, batch_tail<true>, (unsigned)B->n_tails, kTailRegThreads, B->tail_smem, st,
-                  B->tails.as<BatchTail>(B->solvers.size()), B->tail_ids.as<int>(B->n_tails),
-                  live);
-    else if (B->n_tails)
-        BT_LAUNCH(ctx, batch_tail<false>, (unsigned)B->n_tails, kTailThreads, B->tail_smem, st,
+    if (B->n_tails)
+        BT_LAUNCH(ctx, batch_tail, (unsigned)B->n_tails, kTailThreads, B->tail_smem, st,
                   B->tails.as<BatchTail>(B->solvers.size()), B->tail_ids.as<int>(B->n_tails),
                   live);
     for (int l = B->steps - 1; l >= 0; --l) {
@@ -3786,8 +3763,6 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                            "poisson batch: a candidate's mesh is too small for the batched cycle");
                 B->steps = std::max(B->steps, p->tail_start);
                 B->tail_smem = std::max(B->tail_smem, p->tail_smem);
-                B->tail_reg &= bt::tail_in_registers(p->levels[p->tail_start].nx,
-                                                     p->levels[p->tail_start].ny);
             }
             B->level.resize(B->steps);
             for (int l = 0; l < B->steps; ++l) {
@@ -3877,9 +3852,7 @@ extern "C" int bt_poisson_batch_create(bt_ctx *ctx, bt_poisson *const *solvers, 
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
                 BT_CUDA(cudaFuncSetAttribute(bt::batch_smooth<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)bt::kTailSmemMax));
-                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                BT_CUDA(cudaFuncSetAttribute(bt::batch_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)bt::kTailSmemMax));
             }
             for (auto &e : B->ev) BT_CUDA(cudaEventCreate(&e));
