@@ -3974,8 +3974,9 @@ extern "C" int bt_poisson_batch_solve(bt_poisson_batch *B, double *phi, const do
             if (!members[c]) continue;
             if (cycles) cycles[c] = C[c];
             if (residual) residual[c] = S[4 * c + 2];
-            // a residual stalled within 1e4 of the goal is the floor of its own rounding
-            if (!(S[4 * c + 2] <= 1e4 * S[4 * c]))
+            // a residual stalled within 1e4 of the goal is the floor of its own rounding (an
+            // infinite one meets its own relative goal)
+            if (!(S[4 * c + 2] <= 1e4 * S[4 * c]) || !std::isfinite(S[4 * c + 2]))
                 throw bt::Error{BT_ERR_NOCONV, "batched field solve: a candidate did not reach the tolerance"};
         }
     });

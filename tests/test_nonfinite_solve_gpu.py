@@ -29,3 +29,19 @@ def test_nonfinite_input_is_refused(where, value, plasma):
         solver.solve_device(arrays["phi"], arrays["rho"], plasma=species)
     expected = IonOpticsPoisson(_plates((33, 17))).solve(plasma=species)
     assert np.array_equal(solver.solve(plasma=species), expected)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_a_batch_refuses_a_nonfinite_candidate(value):
+    """The candidate's own solves are refused; the batch then solves finite densities."""
+    from beamtracer_b200._lib import ConvergenceError
+    from tests.test_batch_gpu import DESIGNS, _batch
+
+    batch = _batch(DESIGNS[:2])
+    batch.node_view(batch.rho, 1)[80, 5] = value
+    with pytest.raises(ConvergenceError):
+        batch.poisson_batch.solve(batch.phi, batch.rho, [0, 1])
+    batch.rho.zero_()
+    batch.phi.zero_()
+    batch.poisson_batch.solve(batch.phi, batch.rho, [0, 1])
+    assert bool(batch.phi.isfinite().all())
