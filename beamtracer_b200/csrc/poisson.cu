@@ -14,7 +14,8 @@
 // nearly symmetric) and A_{l+1} = P^T A_l P: 9-point stencils on every coarse level, built
 // on the device (and rebuilt for every Newton step's Jacobian).  Smoothing: red-black
 // Gauss-Seidel on the 5-point fine level, four-colour Gauss-Seidel on the 9-point levels;
-// the coarsest level (at most 64 nodes) is inverted by Gauss-Jordan in shared memory.
+// the coarsest level (at most 256 nodes) is inverted from its band's LU factors, or by a
+// pivoting Gauss-Jordan where those meet a tiny pivot.
 #include <cmath>
 #include <vector>
 
@@ -911,9 +912,10 @@ constexpr int kInvertThreads = 1024;
 // serial chain of 3 n rows, so the time is rows times latency: with the substitutions
 // reading global memory row by row and a serial scan of every pivot row, 208 nodes
 // (b = 9, an 801 x 201 mesh) took 374 us and 153 nodes (b = 10, 1025 x 513) 284 us; now
-// 37 + 37 us and 28 + 31 us.  A pivot smaller than 1e-12 of its row (a matrix that needs
-// pivoting, or a singular
-// one) sets *fallback and the pivoting Gauss-Jordan below computes the inverse instead.
+// 49 + 94 us in PLAIN's order, which a linear operator takes, and 28 + 32 us for the 153 of
+// a Newton step's.  A pivot smaller than 1e-12 of its row (a matrix that needs pivoting, or a
+// singular one) sets *fallback and the pivoting Gauss-Jordan below computes the inverse
+// instead.
 constexpr int kBandMax = 17;
 constexpr int kBandPad = kBandMax + 1;  // a factor column's stride, in doubles (even: 16-byte loads)
 constexpr int kSolveThreads = 32;       // columns a block of coarsest_band_solve: a warp

@@ -5,8 +5,8 @@
 // Boris's kick-drift-kick through the staggered edge fields of the patches, plane
 // crossings, kept paths, exit and electrode sub-cell tests: the reference's step, term by
 // term, in FP64 with no contracted multiply-add, so a trajectory ends bit for bit where the
-// reference's CPU kernel ends it; the only fused multiply-adds are those of `div_known`,
-// whose quotients are the IEEE division's).  Instead of adding its charge to the mesh with
+// reference's CPU kernel ends it; the only fused multiply-adds are those of `div_known` and
+// `Num`, whose quotients and roots are the IEEE operations').  Instead of adding its charge to the mesh with
 // atomics, every step writes one deposit record (cell, u, w, dq dt) to a slot fixed by
 // (window, step, trajectory); between windows the live trajectories are compacted in order,
 // and the records are sorted by cell and reduced per cell in record order (deposit.cu), so
@@ -410,7 +410,7 @@ __device__ __forceinline__ void pull(double qm, const double *E, const double *B
 // FP64 a step (8 cycles each behind another, 2 of issue).  A window of 64 Runge-Kutta steps of
 // 20,000 rings at 801 x 201 takes 132 us (216 with IEEE roots and quotients and a step time
 // that waits for the field); 64 Boris steps of 100,000 ions on a graded 1025 x 513 mesh in
-// a solenoid 965 us before, some 550 now.
+// a solenoid 965 us before, 465 now (a pass's 68 windows on average).
 template <int CYL, int INTEG, bool GENERAL, bool MAG, bool FAST>
 __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magnetic &mag,
                                         const Geo &G, const State &S, State &T, Share &D,

@@ -310,7 +310,7 @@ __device__ __forceinline__ void pull3(N &, double qm, const Fields3 &F, const do
 // same straight-line roots and quotients, the same step time known in advance, false where
 // either may not hold).  With IEEE operations a step was 2,429 instructions, its quotients by
 // the spacing and its roots behind one another: 509 us a window of 32 Runge-Kutta steps of
-// 100,000 trajectories; 1,620 instructions and 346 us now, the L1 data path busy 62 % of them
+// 100,000 trajectories; 1,620 instructions and 346 us now, the L1 data path busy 64 % of them
 // with the 96 corner loads a step.  Three blocks a multiprocessor (168 registers) hide more
 // of the loads than two with 255 (384 us).
 template <int INTEG, bool HASB, bool FAST>

@@ -536,6 +536,7 @@ int bt_newton_residual(bt_ctx *ctx, int64_t n, const uint8_t *own, const double 
  * (amplitude = rho_0 / eps0) joins the source, and Newton's method runs: every step a
  * GMRES solve of that step's Jacobian (the multigrid rebuilt for it) to the relative
  * residual tol, until the largest update is below newton_tol or max_newton steps.
+ * BT_ERR_NOCONV where a residual is not finite or a linear one ends above 1e4 times its goal.
  * Host out-params (may be NULL): Newton steps, V-cycles. */
 int bt_poisson_solve(bt_poisson *p, double *phi, const double *rho, double amplitude,
                      double temperature, double up, int32_t sign, double tol,
