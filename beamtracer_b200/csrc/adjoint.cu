@@ -55,7 +55,7 @@ struct Stage {
 
 // q/m E at a point, as trace.cu forms it (the radius and its unit vector in cylindrical
 // geometry).  Num<true>: straight-line roots and quotients (common.cuh), and the cells of
-// s + 1/2 from those of s, a clamped point called odd -- as the trace's own step.
+// s + 1/2 from those of s, as the trace's own step.
 template <int CYL, class N>
 __device__ __forceinline__ void accel(N &num, const Grid &G, double qm, const double *q, double *a,
                                       Stage &g) {
@@ -81,15 +81,20 @@ __device__ __forceinline__ void accel(N &num, const Grid &G, double qm, const do
         const int i = __double2int_rd(sx), j = __double2int_rd(sy);
         const double fi = (double)i, fj = (double)j;
         const bool up_i = hx >= fi + 1.0, up_j = hy >= fj + 1.0;
-        g.ix = clamp_cell(i + (up_i ? 1 : 0), 0, G.nx - 1);
+        g.ix = clamp_cell(clamp_cell(i, -1, G.nx - 1) + (up_i ? 1 : 0), 0, G.nx - 1);
         g.jx = clamp_cell(j, 0, G.ny - 2);
         g.iy = clamp_cell(i, 0, G.nx - 2);
-        g.jy = clamp_cell(j + (up_j ? 1 : 0), 0, G.ny - 1);
-        num.flag |= g.iy != i || g.jx != j;
+        g.jy = clamp_cell(clamp_cell(j, -1, G.ny - 1) + (up_j ? 1 : 0), 0, G.ny - 1);
         g.uy = sx - fi;
         g.wx = sy - fj;
         g.ux = hx - (up_i ? fi + 1.0 : fi);
         g.wy = hy - (up_j ? fj + 1.0 : fj);
+        if (g.iy != i || g.jx != j) {  // past the mesh's edge
+            g.ux = hx - (double)g.ix;
+            g.wx = sy - (double)g.jx;
+            g.uy = sx - (double)g.iy;
+            g.wy = hy - (double)g.jy;
+        }
     } else {
         g.ix = clamp_cell(__double2int_rd(hx), 0, G.nx - 1);
         g.jx = clamp_cell(__double2int_rd(sy), 0, G.ny - 2);

@@ -113,7 +113,11 @@ __device__ __forceinline__ double bilinear(const double *__restrict__ f, int str
 // E at the point (sx, sy) in cells of patch g from its origin (the finest patch holding the
 // point; trace_trajectories_2d_pyccel.py:212-269).  The straight-line form takes the cell of
 // s + 1/2 from the cell c of s -- it is c, or c + 1 where s + 1/2, as rounded, has reached
-// it -- without a second pair of conversions, and calls a point whose cell is clamped odd.
+// it -- without a second pair of conversions but for a point past the mesh's edge, whose cells
+// are clamped.  (Every trajectory that leaves has such a point in its last step; called odd,
+// it made the whole warp take a step with IEEE operations, one warp step in ten of 100,000
+// short trajectories on a planar 81 x 31 mesh with boxes: 6.8 ms of windows for 4.9, or 5.2
+// with IEEE operations throughout.)
 template <class N>
 __device__ __forceinline__ void edge_field_cells(N &num, const bt_trace_args &a,
                                                  const PatchGeom &g, double sx, double sy,
@@ -126,15 +130,20 @@ __device__ __forceinline__ void edge_field_cells(N &num, const bt_trace_args &a,
         const int i = __double2int_rd(sx), j = __double2int_rd(sy);
         const double fi = (double)i, fj = (double)j;
         const bool up_i = hx >= fi + 1.0, up_j = hy >= fj + 1.0;
-        ix = clamp_index(i + (up_i ? 1 : 0), 0, pnx - 1);
+        ix = clamp_index(clamp_index(i, -1, pnx - 1) + (up_i ? 1 : 0), 0, pnx - 1);
         jx = clamp_index(j, 0, pny - 2);
         iy = clamp_index(i, 0, pnx - 2);
-        jy = clamp_index(j + (up_j ? 1 : 0), 0, pny - 1);
-        num.flag |= iy != i || jx != j;
+        jy = clamp_index(clamp_index(j, -1, pny - 1) + (up_j ? 1 : 0), 0, pny - 1);
         uy = sx - fi;
         wx = sy - fj;
         ux = hx - (up_i ? fi + 1.0 : fi);
         wy = hy - (up_j ? fj + 1.0 : fj);
+        if (iy != i || jx != j) {
+            ux = hx - (double)ix;
+            wx = sy - (double)jx;
+            uy = sx - (double)iy;
+            wy = hy - (double)jy;
+        }
     } else {
         ix = cell_weight(hx, pnx - 1, ux);
         jx = cell_weight(sy, pny - 2, wx);
