@@ -402,29 +402,34 @@ __device__ __forceinline__ void pull(double qm, const double *E, const double *B
     }
 }
 
-// One step from S to T, its deposit in D and its step time in dt_out; the rounding of every
-// operation is the reference's.  FAST: straight-line arithmetic (Num<true>), false where it
-// may not hold -- the caller steps again with FAST false.
+// One step from S to T and its deposit in D; the rounding of every operation is the
+// reference's.  The forms but kIeee: straight-line arithmetic (Num<true>), false where it may
+// not hold -- the caller steps again with kIeee.
 //
-// FAST also takes the step as limited by the speed, whose time the step before has left in
-// S.dt0, and only checks that the acceleration would not shorten it, with a margin of 1e-9
-// against rounding: |a| < 2 v^2 / h, all squared, no root or quotient.  So the time does not
+// kSpeculated also takes the step as limited by the speed, whose time the step before has left
+// in S.dt0, and only checks that the acceleration would not shorten it (`limited` where it
+// may), with a margin of 1e-9 against rounding: |a| < 2 v^2 / h, all squared, no root or quotient.  So the time does not
 // wait for the first field: the points of the second stage (x + dt/2 v) and of the first are
 // looked up together, as are those of the third (which needs the first stage's field) and
 // the fourth (the second's), the chain of a Runge-Kutta step two lookups long instead of
 // four with the step time's two roots and quotient between.  A step limited by the
-// acceleration (a beam starting nearly at rest) is taken twice.
+// acceleration (a beam starting nearly at rest, or turning back) is taken again as kTimed,
+// which waits for the field: 100,000 ions turned back at points of their own in a 41 x 21
+// mesh take 1.69 ms (planar 1.44), as kIeee 2.07 (1.56); all steps so, 1.72 (1.34).  (A loop
+// around the straight-line step in kTimed's place cost the other traces 7 %.)
 //
 // Bound by latency still: one warp a scheduler on 20,000 rings, 1,013 instructions of 500 in
 // FP64 a step (8 cycles each behind another, 2 of issue).  A window of 64 Runge-Kutta steps of
 // 20,000 rings at 801 x 201 takes 132 us (216 with IEEE roots and quotients and a step time
 // that waits for the field); 64 Boris steps of 100,000 ions on a graded 1025 x 513 mesh in
 // a solenoid 965 us before, 465 now (a pass's 68 windows on average).
-template <int CYL, int INTEG, bool GENERAL, bool MAG, bool FAST>
+enum StepForm { kIeee = 0, kSpeculated = 1, kTimed = 2 };
+
+template <int CYL, int INTEG, bool GENERAL, bool MAG, StepForm FORM>
 __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magnetic &mag,
                                         const Geo &G, const State &S, State &T, Share &D,
-                                        double &dt_out) {
-    Num<FAST> num;
+                                        bool &limited) {
+    Num<FORM != kIeee> num;
     const double qm = G.qm, inv_c2 = G.inv_c2;
     const double gv = GENERAL ? S.gv : 1.0;
     double E[3], B[3] = {0.0, 0.0, 0.0}, a1[3];
@@ -445,16 +450,16 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
     }
     const double acc2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
     double dt = S.dt0;
-    if (FAST) {
-        num.flag |= !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2));
-        num.flag |= !(dt > 0.0);
+    if (FORM == kSpeculated) {
+        limited = !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2)) || !(dt > 0.0);
     } else {
-        const double accel = num.root(acc2);
+        const double accel = sqrt(acc2);
         if (accel > 0.0) {
             const double d2 = sqrt(2.0 * S.hloc / accel);
             if (dt < 0.0 || d2 < dt) dt = d2;
         }
         if (dt < 0.0) dt = S.hloc;
+        limited = false;
     }
     dt = G.fraction * dt;
     const double hdt = 0.5 * dt;
@@ -595,7 +600,6 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
     D.c01 = (1.0 - u) * wr * ch;
     D.c10 = u * (1.0 - wr) * ch;
     D.c11 = u * wr * ch;
-    dt_out = dt;
     // (an intermediate value out of range leaves the end state, or its root, out of range)
     num.not_huge(y[0]);
     if (CYL != 1) num.not_huge(y[1]);
@@ -606,8 +610,19 @@ __device__ __forceinline__ bool advance(const bt_trace_args &a, const bt_magneti
 template <int CYL, int INTEG, bool GENERAL, bool MAG>
 __device__ __noinline__ void advance_plain(const bt_trace_args &a, const bt_magnetic &mag,
                                            const Geo &G, const State &S, State &T, Share &D) {
-    double dt;
-    advance<CYL, INTEG, GENERAL, MAG, false>(a, mag, G, S, T, D, dt);
+    bool limited;
+    advance<CYL, INTEG, GENERAL, MAG, kIeee>(a, mag, G, S, T, D, limited);
+    // (the root's reciprocal, for the straight-line quotients by the radius)
+    T.at.y = T.at.r > 0.0 ? 1.0 / T.at.r : 0.0;
+}
+
+// The straight-line step with the time that the acceleration sets, out of line: for the steps
+// that it limits.
+template <int CYL, int INTEG, bool GENERAL, bool MAG>
+__device__ __noinline__ bool advance_timed(const bt_trace_args &a, const bt_magnetic &mag,
+                                           const Geo &G, const State &S, State &T, Share &D) {
+    bool limited;
+    return advance<CYL, INTEG, GENERAL, MAG, kTimed>(a, mag, G, S, T, D, limited);
 }
 
 // The place and pace of a state whose position and velocity are set.
@@ -715,19 +730,21 @@ __device__ __forceinline__ bool trace_thread(const Trace &tr, const i64 *__restr
         if (ns >= a.max_steps) break;
         State next;
         Share D;
-        double dt;
-        const bool ok = advance<CYL, INTEG, GENERAL, MAG, true>(a, tr.mag, G, now, next, D, dt);
+        bool limited;
+        const bool ok =
+            advance<CYL, INTEG, GENERAL, MAG, kSpeculated>(a, tr.mag, G, now, next, D, limited) &&
+            G.fast;
         // the end's cell in the electrode table: asked for here, where the lookup runs beside
         // the rest of the step's arithmetic
         i64 cell = cell_at(next.at);
-        if (!(ok && G.fast)) {
+        if (!ok || limited) {
             // copies, so that only this branch keeps anything in memory
             const State from = now;
             const Geo g = G;
             State to;
             Share d;
-            advance_plain<CYL, INTEG, GENERAL, MAG>(a, tr.mag, g, from, to, d);
-            to.at.y = to.at.r > 0.0 ? 1.0 / to.at.r : 0.0;
+            if (!ok || !advance_timed<CYL, INTEG, GENERAL, MAG>(a, tr.mag, g, from, to, d))
+                advance_plain<CYL, INTEG, GENERAL, MAG>(a, tr.mag, g, from, to, d);
             next = to;
             D = d;
             cell = cell_at(next.at);
