@@ -307,15 +307,20 @@ __device__ __forceinline__ void pull3(N &, double qm, const Fields3 &F, const do
 }
 
 // One step from S to T and its deposit: the 2D trace's `advance` in three dimensions (the
-// same straight-line roots and quotients, the same step time known in advance, false where
-// either may not hold).  With IEEE operations a step was 2,429 instructions, its quotients by
-// the spacing and its roots behind one another: 509 us a window of 32 Runge-Kutta steps of
-// 100,000 trajectories; 1,620 instructions and 346 us now, the L1 data path busy 64 % of them
-// with the 96 corner loads a step.  Three blocks a multiprocessor (168 registers) hide more
-// of the loads than two with 255 (384 us).
-template <int INTEG, bool HASB, bool FAST>
+// same straight-line roots and quotients, false where they may not hold, the same step time
+// known in advance, `limited` where the acceleration may set it).  With IEEE operations a
+// step was 2,429 instructions, its quotients by the spacing and its roots behind one another:
+// 509 us a window of 32 Runge-Kutta steps of 100,000 trajectories; 1,620 instructions and 346
+// us now, the L1 data path busy 64 % of them with the 96 corner loads a step.  Three blocks a
+// multiprocessor (168 registers) hide more of the loads than two with 255 (384 us).  (300,000
+// ions turned back at points of their own in 41^3 nodes, whose steps the acceleration limits
+// there: 8.7 ms a trace by kTimed, 10.6 by kIeee, 8.8 with IEEE operations throughout.)
+enum StepForm3 { kIeee = 0, kSpeculated = 1, kTimed = 2 };
+
+template <int INTEG, bool HASB, StepForm3 FORM>
 __device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G, const State3 &S,
-                                         State3 &T, Deposit3 &D) {
+                                         State3 &T, Deposit3 &D, bool &limited) {
+    constexpr bool FAST = FORM != kIeee;
     Num<FAST> num;
     const double qm = G.qm, inv_c2 = a.inv_c2, gv = FAST ? 1.0 : S.gv;
     Fields3 F;
@@ -327,9 +332,8 @@ __device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G
     pull3<HASB>(num, qm, F, S.v, gv, a1);
     const double acc2 = a1[0] * a1[0] + a1[1] * a1[1] + a1[2] * a1[2];
     double dt = S.dt0;
-    if (FAST) {
-        num.flag |= !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2));
-        num.flag |= !(dt > 0.0);
+    if (FORM == kSpeculated) {
+        limited = !((acc2 * S.hloc) * S.hloc < (4.0 - 4e-9) * (S.speed2 * S.speed2)) || !(dt > 0.0);
     } else {
         const double accel = sqrt(acc2);
         if (accel > 0.0) {
@@ -337,6 +341,7 @@ __device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G
             if (dt < 0.0 || d2 < dt) dt = d2;
         }
         if (dt < 0.0) dt = S.hloc;
+        limited = false;
     }
     dt = a.step_fraction * dt;
     const double hdt = 0.5 * dt;
@@ -428,7 +433,14 @@ __device__ __forceinline__ bool advance3(const bt_trace3d_args &a, const Geo3 &G
 template <int INTEG, bool HASB>
 __device__ __noinline__ void advance3_plain(const bt_trace3d_args &a, const Geo3 &G,
                                             const State3 &S, State3 &T, Deposit3 &D) {
-    advance3<INTEG, HASB, false>(a, G, S, T, D);
+    bool limited;
+    advance3<INTEG, HASB, kIeee>(a, G, S, T, D, limited);
+}
+template <int INTEG, bool HASB>
+__device__ __noinline__ bool advance3_timed(const bt_trace3d_args &a, const Geo3 &G,
+                                            const State3 &S, State3 &T, Deposit3 &D) {
+    bool limited;
+    return advance3<INTEG, HASB, kTimed>(a, G, S, T, D, limited);
 }
 
 // One window of trajectory m (of the active list): at most S steps from its state.  The
@@ -493,16 +505,17 @@ __global__ void __launch_bounds__(128, 3) trace3d_window(const __grid_constant__
         for (; s < S && ns < a.max_steps; ++s) {
             State3 next;
             Deposit3 D;
-            bool ok = false;
-            if (TRY) ok = advance3<INTEG, HASB, true>(a, G, now, next, D);
-            if (!TRY) advance3<INTEG, HASB, false>(a, G, now, next, D);
-            if (TRY && !ok) {
+            bool ok = false, limited = false;
+            if (TRY) ok = advance3<INTEG, HASB, kSpeculated>(a, G, now, next, D, limited);
+            if (!TRY) advance3<INTEG, HASB, kIeee>(a, G, now, next, D, limited);
+            if (TRY && (!ok || limited)) {
                 // copies, so that only this branch keeps anything in memory
                 const State3 from = now;
                 const Geo3 g = G;
                 State3 to;
                 Deposit3 d;
-                advance3_plain<INTEG, HASB>(a, g, from, to, d);
+                if (!ok || !advance3_timed<INTEG, HASB>(a, g, from, to, d))
+                    advance3_plain<INTEG, HASB>(a, g, from, to, d);
                 next = to;
                 D = d;
             }
