@@ -250,7 +250,9 @@ struct Num {
     // the operands' smallest magnitude (below) and largest high word
     unsigned low = 0xffffffffu, high = 0u;
 
-    __device__ __forceinline__ bool odd() const { return flag || low < 2u * kLow - 1u || high > kHigh; }
+    __device__ __forceinline__ bool odd() const {
+        return flag || low < 2u * kLow - 1u || high > kHigh;
+    }
     // twice the high word of |v|, less one where the low word is zero: a zero alone wraps past
     // every exponent (some subnormals have bits in the low word only).  The low word's borrow,
     // so that it takes the two additions that the high word's mask and decrement took.

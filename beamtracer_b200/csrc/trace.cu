@@ -6,11 +6,11 @@
 // crossings, kept paths, exit and electrode sub-cell tests: the reference's step, term by
 // term, in FP64 with no contracted multiply-add, so a trajectory ends bit for bit where the
 // reference's CPU kernel ends it; the only fused multiply-adds are those of `div_known` and
-// `Num`, whose quotients and roots are the IEEE operations').  Instead of adding its charge to the mesh with
-// atomics, every step writes one deposit record (cell, u, w, dq dt) to a slot fixed by
-// (window, step, trajectory); between windows the live trajectories are compacted in order,
-// and the records are sorted by cell and reduced per cell in record order (deposit.cu), so
-// the node charges are deterministic.  The deposits run on a side stream under the next
+// `Num`, whose quotients and roots are the IEEE operations').  Instead of adding its charge
+// to the mesh with atomics, every step writes one deposit record (cell, u, w, dq dt) to a
+// slot fixed by (window, step, trajectory); between windows the live trajectories are
+// compacted in order, and the records are sorted by cell and reduced per cell in record order
+// (deposit.cu), so the node charges are deterministic.  The deposits run on a side stream under the next
 // windows, in the order the record buffers were filled.  Short windows bound the tail of a
 // warp (its threads wait only for the longest trajectory of the window, not of the whole
 // trace).
@@ -408,11 +408,11 @@ __device__ __forceinline__ void pull(double qm, const double *E, const double *B
 //
 // kSpeculated also takes the step as limited by the speed, whose time the step before has left
 // in S.dt0, and only checks that the acceleration would not shorten it (`limited` where it
-// may), with a margin of 1e-9 against rounding: |a| < 2 v^2 / h, all squared, no root or quotient.  So the time does not
-// wait for the first field: the points of the second stage (x + dt/2 v) and of the first are
-// looked up together, as are those of the third (which needs the first stage's field) and
-// the fourth (the second's), the chain of a Runge-Kutta step two lookups long instead of
-// four with the step time's two roots and quotient between.  A step limited by the
+// may), with a margin of 1e-9 against rounding: |a| < 2 v^2 / h, all squared, no root or
+// quotient.  So the time does not wait for the first field: the points of the second stage
+// (x + dt/2 v) and of the first are looked up together, as are those of the third (which
+// needs the first stage's field) and the fourth (the second's), the chain of a Runge-Kutta
+// step two lookups long instead of four with the step time's two roots and quotient between.  A step limited by the
 // acceleration (a beam starting nearly at rest, or turning back) is taken again as kTimed,
 // which waits for the field: 100,000 ions turned back at points of their own in a 41 x 21
 // mesh take 1.69 ms (planar 1.44), as kIeee 2.07 (1.56); all steps so, 1.72 (1.34).  (A loop
